@@ -53,7 +53,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_act_mul": [_vp, _vp, _i, _i, _i, _i, _i, _f, _vp],
         "xr_residual_add": [_vp, _vp, _i, _i, _i, _vp],
         "xr_gemm_simt": [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _ll, _ll, _f, _vp],
-        "xr_attention_simt": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _f, _i, _vp, _i, _vp],
+        "xr_attention_simt": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _f, _i, _vp, _i, _i, _vp],
         "xr_gemm_tc": [_vp, _vp, _vp, _vp, _i, _i, _i, _f, _f, _i, _i, _i, _ll, _ll, _vp, _ll, _vp, _i, _i, ctypes.POINTER(ctypes.c_int), _i, _vp],
         "xr_finish_add_rmsnorm": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
         "xr_finish_plain": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _ll, _vp],
@@ -314,8 +314,9 @@ def _bias_len(bias: Optional[torch.Tensor]) -> int:
 def attention_simt(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cache_k_ptr: int, positions, tok_seg,
                    block_tables, page_stride: int, v_offset: int, H: int, K: int, hd: int, max_pages: int,
                    page_size: int, window: int, scale: float, sink: Optional[torch.Tensor] = None, softcap: float = 0.0,
-                   keep_first: int = 0, bias: Optional[torch.Tensor] = None) -> None:
-    """Causal attention of every token of the step over its request's pages, float32 arithmetic.  `sink`: float32 [H];
+                   keep_first: int = 0, bias: Optional[torch.Tensor] = None, portions: int = 0) -> None:
+    """Causal attention of every token of the step over its request's pages, float32 arithmetic (`portions`: how many requests they
+    belong to, 0: not said; many tokens a request then share the reads of its keys).  `sink`: float32 [H];
     exp(sink[h]) joins the denominator of head h's softmax once (it has no key and no value).  `softcap` c > 0: every scaled
     score s becomes c tanh(s / c).  `keep_first`: with a window, a request's first keys stay visible behind it.  `bias`
     (float32 [H, L]): the query of head h at distance d from a key adds scale * bias[h, min(d, L - 1)] to the score."""
@@ -327,7 +328,7 @@ def attention_simt(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cache_
     _check(lib().xr_attention_simt(q.data_ptr(), out.data_ptr(), dtype_code(out.dtype), cache_k_ptr,
                                    positions.data_ptr(), tok_seg.data_ptr(), block_tables.data_ptr(), page_stride,
                                    v_offset, q_row_stride, n, H, K, hd, max_pages, page_size, window, float(scale),
-                                   _ptr(sink), float(softcap), int(keep_first), _ptr(bias), _bias_len(bias), _stream()), "attention_simt")
+                                   _ptr(sink), float(softcap), int(keep_first), _ptr(bias), _bias_len(bias), int(portions), _stream()), "attention_simt")
     _count()
 
 

@@ -303,9 +303,11 @@ class GQAAttention(Mixer):
                                       bias=self.dist_bias)
                 counters["mma"] += 1
         else:
+            # (a window that no token of the step reaches past masks nothing)
+            window = self.window if self.window and ctx.max_kv_len > self.window else 0
             kernels.attention_simt(qkv, qkv_dim, o, k_ptr, ctx.positions, ctx.tok_seg, bt, page_stride, v_offset,
-                                   self.H, self.K, self.hd, ctx.max_pages, ctx.page_size, self.window or 0, self.scale, sink=self.sink, softcap=self.softcap,
-                                   keep_first=self.keep_first, bias=self.dist_bias)
+                                   self.H, self.K, self.hd, ctx.max_pages, ctx.page_size, window, self.scale, sink=self.sink, softcap=self.softcap,
+                                   keep_first=self.keep_first, bias=self.dist_bias, portions=ctx.n_seg)
             counters["simt"] += 1
         if self.gate is not None:
             kernels.sigmoid_gate(o, proj[:, gate_at:gate_at + self.gate_cols], self.H, self.hd, self.Vd, self.gate == "each")
