@@ -1,4 +1,5 @@
 """The kernels and dispatch branches that take steps of many tokens, at the edges of their tiles."""
+import numpy as np
 import pytest
 import torch
 
@@ -39,3 +40,78 @@ def test_float32_attention_of_packed_rows_gives_the_same_bits(H, K, hd, page, ex
                                0, hd ** -0.5, portions=portions, **opt)
         outs.append(out)
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+
+
+# ---- attention over expanded keys ------------------------------------------------------------------------------------
+@pytest.mark.parametrize("H,D,R,V,page,window,gate", [(3, 128, 64, 128, 64, 0, "each"), (2, 64, 32, 64, 16, 100, "head"), (2, 64, 8, 128, 64, 0, ""),
+                                                      (1, 128, 40, 64, 8, 300, "head")])
+def test_attention_over_expanded_keys(H, D, R, V, page, window, gate):
+    """Portions that start a request, continue one, are too short (another kernel's), and see keys behind a window, with one key that
+    stands out; the rows' gather, then the attention, against float64 over the same operands."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(D + R)
+    C = 24
+    specs = [(0, 130), (700, 5), (515, 33), (128, 128)]
+    mp = -(-max(p + n for p, n in specs) // page)
+    pages = mp * len(specs)
+    cache = torch.zeros(pages, page, C + R).bfloat16()
+    bt = torch.randperm(pages, generator=g).view(len(specs), mp).int()
+    rows = [torch.randn(p + n, C + R, generator=g).bfloat16() for p, n in specs]
+    for s, r in enumerate(rows):
+        for j in range(len(r)):
+            cache[bt[s, j // page], j % page] = r[j]
+        if window:                                                   # pages behind the window of the portion's first token are gone
+            for i in range(max(0, specs[s][0] - window + 1) // page):
+                bt[s, i] = -1
+    n = sum(m for _, m in specs)
+    starts = [sum(m for _, m in specs[:s]) for s in range(len(specs))]
+    wk, wv = torch.randn(H * D, C, generator=g) * C ** -0.5, torch.randn(H * V, C, generator=g) * C ** -0.5
+    q = torch.randn(n, H * (D + R) + 8, generator=g).bfloat16()
+    gates = torch.randn(n, H * V if gate == "each" else H, generator=g).bfloat16()
+    first = [int(kernels.flat_first_key(np.int64(p), window)) for p, _ in specs]
+    keys = sum(p + m - f for (p, m), f in zip(specs, first) if m >= 32)
+    flat = torch.full((keys, C + R), 9.0, dtype=torch.bfloat16, device=DEV)
+    seg_len, pos0 = _i32([m for _, m in specs]), _i32([p for p, _ in specs])
+    cache_d, bt_d = cache.to(DEV), bt.to(DEV)
+    kernels.flat_rows(cache_d.data_ptr(), page * (C + R), flat, seg_len, pos0, bt_d, len(specs), mp, page, window, 32)
+    want_rows = []
+    for s, (p, m) in enumerate(specs):
+        if m >= 32:
+            r = rows[s].clone()
+            if window:
+                r[:max(0, p - window + 1) // page * page] = 0
+            want_rows.append(r[first[s]:])
+    want_rows = torch.cat(want_rows)
+    assert torch.equal(flat.cpu(), want_rows)
+    kv = torch.cat([want_rows[:, :C].float() @ wk.T, want_rows[:, :C].float() @ wv.T], dim=1).bfloat16()
+    scale = (D + R) ** -0.5
+    # head 0 of the third portion's last token looks for that request's key 500 or what the window leaves of it
+    far = 540
+    at = sum(len(rows[s]) - first[s] for s in (0,)) + far - first[2]
+    q[starts[2] + 32, :D] = (kv[at, :D].float() * 6).bfloat16()
+    out = torch.full((n, H * V), 5.0, dtype=torch.bfloat16, device=DEV)
+    tiles = sum(-(-m // 128) for _, m in specs if m >= 32)
+    kernels.attention_tc_flat(q.to(DEV), kv.to(DEV), flat[:, C:], out, _i32(starts), seg_len, pos0, len(specs), H, D, R, V, window, scale, 32, tiles,
+                              gate=gates.to(DEV) if gate else None, gate_each=gate == "each")
+    kernels.tc_check_status(torch.device(DEV))
+    got = out.cpu().double()
+    assert (got[starts[1]:starts[1] + 5] == 5.0).all()
+    at = 0
+    for s, (p, m) in enumerate(specs):
+        if m < 32:
+            continue
+        k = kv[at:at + p + m - first[s]].double()
+        tail = want_rows[at:at + p + m - first[s], C:].double()
+        at += len(k)
+        pos, key = torch.arange(p, p + m)[:, None], torch.arange(first[s], p + m)[None, :]
+        see = (key <= pos) & ((pos - key < window) if window else torch.ones_like(key <= pos))
+        for h in range(H):
+            qh = q[starts[s]:starts[s] + m, h * (D + R):(h + 1) * (D + R)].double()
+            sc = (qh[:, :D] @ k[:, h * D:(h + 1) * D].T + qh[:, D:] @ tail.T) * scale
+            o = torch.softmax(sc.masked_fill(~see, float("-inf")), dim=-1) @ k[:, H * D + h * V:H * D + (h + 1) * V]
+            if gate:
+                z = gates[starts[s]:starts[s] + m].double()
+                o = o * torch.sigmoid(z[:, h * V:(h + 1) * V] if gate == "each" else z[:, h:h + 1])
+            # probabilities are rounded to bfloat16 (2^-9 of each, weights that sum to one) and the result once more
+            top = k[:, H * D + h * V:H * D + (h + 1) * V].abs().max()
+            assert ((got[starts[s]:starts[s] + m, h * V:(h + 1) * V] - o).abs() <= 2.0 ** -8 * o.abs() + 2.0 ** -8 * top).all(), (s, h)

@@ -58,6 +58,12 @@ struct AttnTcArgs {
     int keep_first;              // with a window: the first keys that stay visible behind it
     XrBias bias;
     int bias_stride;             // floats between the heads' rows in shared memory; 0: the rows do not fit and are read where they are
+    // FLAT only (xr_attention_tc_flat)
+    int flat_min;                // portions of fewer tokens are not this launch's
+    int k_col, v_col;            // where head 0's keys and values begin in a row of the flat array
+    const __nv_bfloat16* gate;   // output gate's pre-activations or null: one a head, or with gate_each one an element
+    long long ld_gate;
+    int gate_each;
 };
 
 __device__ __forceinline__ uint32_t ta_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -164,12 +170,19 @@ __host__ __device__ constexpr uint32_t ta_idesc(bool b_mn, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
-// HD: head size, 64 or 128.  Shared memory keeps the layout of head size 128 (a stage of K or V is two halves
-// apart); at head size 64 only the first half of each is filled and read.
-template <int HD, bool BIAS>
+// The keys of a portion in the flat array: from this one on (the first its first token sees, at a tile's border) to its last.
+__host__ __device__ __forceinline__ int ta_flat_first(int pos0, int window) { return window > 0 && pos0 >= window ? (pos0 - window + 1) / TA_KEYS * TA_KEYS : 0; }
+
+// NK, NV: 64-column halves of a query or key and of a value.  Shared memory keeps the layout of two halves where there is one.
+// FLAT: keys and values do not come from the pages but from an array of their own, one row a key, the portions' keys one portion
+// after another (ta_flat_first): a head's keys at k_col + h 64 (NK - 1) and its values at v_col + h 64 NV, and the last half of every
+// key from a second array (tail_map), whose rows all heads share and which may be narrower than 64 columns (the query's row ends
+// there too: what is copied behind either is zeros).
+template <int NK, int NV, bool BIAS, bool FLAT>
 __global__ void __launch_bounds__(TA_THREADS, 1)
-k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, AttnTcArgs a) {
-    // 10 half tiles of 16 KB; the array is declared 1 KB aligned (what the
+k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap kv_map, const __grid_constant__ CUtensorMap tail_map,
+               AttnTcArgs a) {
+    // half tiles of 16 KB, 10 of them for heads of 128; the array is declared 1 KB aligned (what the
     // swizzled TMA boxes and the matrix descriptors need) and the kernel refuses to run if it is not
     extern __shared__ __align__(1024) uint8_t ta_smem_raw[];
     uint8_t* smem = ta_smem_raw;
@@ -178,11 +191,12 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
         return;
     }
     constexpr int HALF = TA_ROWS * 128;                   // bytes of one [128 rows][64 columns] half tile
-    constexpr int NH = HD / 64;                           // 64-column halves of a head
-    static_assert(HD == 64 || HD == 128, "head size 64 or 128");
-    uint8_t* q_s = smem;                                  // [2 halves][128 rows][128 B]
-    uint8_t* k_s = q_s + 2 * HALF;                        // [2 stages][2 halves (hd)][128 keys][128 B]
-    uint8_t* v_s = k_s + 4 * HALF;                        // [2 stages][2 halves (hd)][128 keys][128 B]
+    constexpr int HV = 64 * NV;                           // value elements of a head
+    constexpr int LK = NK < 2 ? 2 : NK;                   // halves a key stage has room for
+    static_assert(NK >= 1 && NK <= 3 && NV >= 1 && NV <= 2, "what fits shared memory");
+    uint8_t* q_s = smem;                                  // [LK halves][128 rows][128 B]
+    uint8_t* k_s = q_s + LK * HALF;                       // [2 stages][LK halves][128 keys][128 B]
+    uint8_t* v_s = k_s + 2 * LK * HALF;                        // [2 stages][2 halves (hd)][128 keys][128 B]
     uint64_t* bars = (uint64_t*)(v_s + 4 * HALF);
     uint64_t* q_full = bars;            // 1
     uint64_t* k_full = bars + 1;        // 2
@@ -202,14 +216,17 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
     // keys, start first.
     const int kvh = blockIdx.y;
     int seg = -1, tile = 0;
+    int flat_row0 = 0;                                              // FLAT: the row of the portion's key 0 (it may lie before the array)
     {
         const int want = (int)gridDim.x - 1 - (int)blockIdx.x;
         int before = 0;
         for (int s = 0; s < a.n_seg; s++) {
             const int rows = a.seg_len[s] * a.G;
-            const int t = rows > 16 ? (rows + TA_ROWS - 1) / TA_ROWS : 0;
+            const int t = rows > (FLAT ? a.flat_min - 1 : 16) ? (rows + TA_ROWS - 1) / TA_ROWS : 0;
+            if (FLAT && t > 0) flat_row0 -= ta_flat_first(a.seg_pos0[s], a.window);
             if (want < before + t) { seg = s; tile = want - before; break; }
             before += t;
+            if (FLAT && t > 0) flat_row0 += a.seg_pos0[s] + rows;            // (one row a token)
         }
     }
     if (seg < 0) return;                                            // (the caller gave an upper bound of the tiles)
@@ -252,9 +269,9 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
         if (lane == 0) {
             const bool keys = warp == 8;
             if (keys) {
-                ta_expect(q_full, NH * HALF);
+                ta_expect(q_full, NK * HALF);
                 int tok0 = tok_base + row0 / a.G;
-                for (int c = 0; c < NH; c++) ta_tma_3d(q_s + c * HALF, &q_map, c * 64, kvh * a.G, tok0, q_full);
+                for (int c = 0; c < NK; c++) ta_tma_3d(q_s + c * HALF, &q_map, c * 64, kvh * a.G, tok0, q_full);
             }
             const int box_rows = a.page_size < 64 ? a.page_size : 64;
             uint64_t* full = keys ? k_full : v_full;
@@ -263,29 +280,40 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             for (int j = 0; j < n_tiles; j++) {
                 int s = j & 1;
                 if (j >= 2) ta_wait(&empty[s], ((j >> 1) - 1) & 1, gave_up);
-                ta_expect(&full[s], NH * HALF);
+                ta_expect(&full[s], (keys ? NK : NV) * HALF);
                 int key0 = xr_walk_tile(j, kept_tiles, t_lo) * TA_KEYS;
+                if (FLAT) {
+                    const int row = flat_row0 + key0;
+                    if (keys) {
+                        for (int c = 0; c < NK - 1; c++) ta_tma_2d(base + (s * LK + c) * HALF, &kv_map, a.k_col + (kvh * (NK - 1) + c) * 64, row, &full[s]);
+                        ta_tma_2d(base + (s * LK + NK - 1) * HALF, &tail_map, 0, row, &full[s]);
+                    } else {
+                        for (int c = 0; c < NV; c++) ta_tma_2d(base + (s * 2 + c) * HALF, &kv_map, a.v_col + (kvh * NV + c) * 64, row, &full[s]);
+                    }
+                    continue;
+                }
                 for (int r0 = 0; r0 < TA_KEYS; r0 += box_rows) {
                     int kp = key0 + r0;
                     int pi = kp >> a.page_shift;
                     int page = pi < a.max_pages ? a.block_tables[(size_t)seg * a.max_pages + pi] : -1;
                     long long row = ((((long long)page * a.n_layers + a.layer) * 2 + (keys ? 0 : 1)) * a.K + kvh) * a.page_size + (kp & (a.page_size - 1));
                     if (page < 0) row = -1024;                          // outside the tensor: the copy fills zeros
-                    for (int c = 0; c < NH; c++) ta_tma_2d(base + (s * 2 + c) * HALF + r0 * 128, &kv_map, c * 64, (int)row, &full[s]);
+                    for (int c = 0; c < (keys ? NK : NV); c++)
+                        ta_tma_2d(base + (s * (keys ? LK : 2) + c) * HALF + r0 * 128, &kv_map, c * 64, (int)row, &full[s]);
                 }
             }
         }
     } else if (warp == 9) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            constexpr uint32_t id_qk = ta_idesc(false, TA_KEYS), id_pv = ta_idesc(true, HD);
+            constexpr uint32_t id_qk = ta_idesc(false, TA_KEYS), id_pv = ta_idesc(true, HV);
             auto issue_qk = [&](int j) {
                 int s = j & 1;
                 ta_wait(&k_full[s], (j >> 1) & 1, gave_up);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                uint32_t qa = ta_smem(q_s), kb = ta_smem(k_s + s * 2 * HALF);
+                uint32_t qa = ta_smem(q_s), kb = ta_smem(k_s + s * LK * HALF);
 #pragma unroll
-                for (int kk = 0; kk < HD / 16; kk++) {
+                for (int kk = 0; kk < NK * 4; kk++) {
                     uint32_t off = (kk >> 2) * HALF + (kk & 3) * 32;
                     ta_mma((j & 1) ? tm_s1 : tm_s0, ta_desc_k(qa + off), ta_desc_k(kb + off), id_qk, kk > 0 ? 1u : 0u);
                 }
@@ -393,11 +421,11 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 l *= corr;
 #pragma unroll 1
-                for (int c = 0; c < NH; c++) {
-                    ta_ld32(tm_o + lane_off + half * (HD / 2) + c * 32, v);
+                for (int c = 0; c < NV; c++) {
+                    ta_ld32(tm_o + lane_off + half * (HV / 2) + c * 32, v);
 #pragma unroll
                     for (int i = 0; i < 32; i++) v[i] *= corr;
-                    ta_st32(tm_o + lane_off + half * (HD / 2) + c * 32, v);
+                    ta_st32(tm_o + lane_off + half * (HV / 2) + c * 32, v);
                 }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             }
@@ -443,7 +471,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                 int s = j & 1;
                 ta_wait(&v_full[s], (j >> 1) & 1, gave_up);
                 int first_bad = hi + 1 - tile0;
-                constexpr int CH = HD / 8;                               // 16-byte chunks of a value row
+                constexpr int CH = HV / 8;                               // 16-byte chunks of a value row
                 for (int e = half * 128 + r; e < (TA_KEYS - first_bad) * CH; e += 256) {
                     int row = first_bad + e / CH, ch = e % CH;
                     *reinterpret_cast<uint4*>(v_s + (s * 2 + (ch >> 3)) * HALF + row * 128 + (((ch & 7) ^ (row & 7)) << 4)) = make_uint4(0, 0, 0, 0);
@@ -467,12 +495,21 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             // a sink has no key and no value: it only enters the sum, at the offset the sum carries
             if (live && a.sink != nullptr) l += ta_exp2(fmaf(a.sink[kvh * a.G + pr % a.G], 1.4426950408889634f, -m));
             float inv = live ? 1.0f / l : 0.f;
-            __nv_bfloat16* dst = a.out + ((long long)(tok_base + (live ? pr : 0) / a.G) * a.H + (kvh * a.G + (live ? pr : 0) % a.G)) * HD + half * (HD / 2);
+            const __nv_bfloat16* gate = nullptr;                     // FLAT: this thread's gates
+            if (FLAT && a.gate != nullptr && live) {
+                gate = a.gate + (long long)(tok_base + pr) * a.ld_gate + (a.gate_each ? kvh * HV + half * (HV / 2) : kvh);
+                if (!a.gate_each) inv = __fdividef(inv, 1.0f + __expf(-__bfloat162float(*gate)));
+            }
+            __nv_bfloat16* dst = a.out + ((long long)(tok_base + (live ? pr : 0) / a.G) * a.H + (kvh * a.G + (live ? pr : 0) % a.G)) * HV + half * (HV / 2);
             float v[32];
 #pragma unroll 1
-            for (int c = 0; c < NH; c++) {
-                ta_ld32(tm_o + lane_off + half * (HD / 2) + c * 32, v);      // warp-wide: rows past the portion load too
+            for (int c = 0; c < NV; c++) {
+                ta_ld32(tm_o + lane_off + half * (HV / 2) + c * 32, v);      // warp-wide: rows past the portion load too
                 if (!live) continue;
+                if (FLAT && gate != nullptr && a.gate_each) {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) v[i] = __fdividef(v[i], 1.0f + __expf(-__bfloat162float(gate[c * 32 + i])));
+                }
 #pragma unroll
                 for (int i = 0; i < 32; i += 8) {
                     uint32_t w[4];
@@ -577,10 +614,10 @@ XR_EXPORT int xr_attention_tc(const void* q, void* out, const void* cache_base, 
     }
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(k_attention_tc<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
+        if (cudaFuncSetAttribute(k_attention_tc<2, 2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_attention_tc<1, 1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(k_attention_tc<2, 2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess ||
+            cudaFuncSetAttribute(k_attention_tc<1, 1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
             return XR_ERR_LAUNCH;
         configured = true;
     }
@@ -589,9 +626,115 @@ XR_EXPORT int xr_attention_tc(const void* q, void* out, const void* cache_base, 
     long long tiles = row_tiles > 0 ? row_tiles : (((long long)max_seg_len * G + TA_ROWS - 1) / TA_ROWS) * n_seg;
     if (tiles > 0x7fffffffLL) return XR_ERR_ARG;
     const dim3 grid((unsigned)tiles, K, 1);
-    if (bias != nullptr && hd == 128) xr_launch((k_attention_tc<128, true>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, a);
-    else if (bias != nullptr) xr_launch((k_attention_tc<64, true>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, a);
-    else if (hd == 128) xr_launch((k_attention_tc<128, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, a);
-    else xr_launch((k_attention_tc<64, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, a);
+    if (bias != nullptr && hd == 128) xr_launch((k_attention_tc<2, 2, true, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, kvm, a);
+    else if (bias != nullptr) xr_launch((k_attention_tc<1, 1, true, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, kvm, a);
+    else if (hd == 128) xr_launch((k_attention_tc<2, 2, false, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, kvm, a);
+    else xr_launch((k_attention_tc<1, 1, false, false>), grid, dim3(TA_THREADS), smem, stream, qm, kvm, kvm, a);
+    return xr_launch_status();
+}
+
+// ---------------------------------------------------------------------------------------------
+// Portions of many tokens whose keys and values were expanded into a flat array (latent attention): every query head has keys of
+// its own, 64 (NK - 1) columns of the array and a tail of `tail` columns that all heads share.
+// ---------------------------------------------------------------------------------------------
+XR_EXPORT int xr_attention_tc_flat_supported(int D, int R, int V) {
+    return (D == 64 || D == 128) && (V == 64 || V == 128) && R >= 8 && R <= 64 && R % 8 == 0;
+}
+
+template <int NK, int NV>
+static int launch_flat(const CUtensorMap& qm, const CUtensorMap& kvm, const CUtensorMap& tm, const AttnTcArgs& a, long long tiles, cudaStream_t stream) {
+    constexpr int SMEM = (3 * (NK < 2 ? 2 : NK) + 4) * TA_ROWS * 128 + 128 + 2 * 2 * 128 * 4;
+    static const bool ready = cudaFuncSetAttribute(k_attention_tc<NK, NV, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess;
+    if (!ready) return XR_ERR_LAUNCH;
+    xr_launch((k_attention_tc<NK, NV, false, true>), dim3((unsigned)tiles, a.H), dim3(TA_THREADS), SMEM, stream, qm, kvm, tm, a);
+    return xr_launch_status();
+}
+
+// [rows][cols] bfloat16, `ld` elements apart; a box is 64 columns x 128 rows
+static bool ta_flat_map(CUtensorMap* m, const void* base, long long rows, long long cols, long long ld) {
+    TaEncodeFn enc = ta_encode();
+    if (!enc) return false;
+    const XrMapKey key{base, {(unsigned long long)cols, (unsigned long long)rows, 0}, {(unsigned long long)ld * 2, 0}, {64, TA_KEYS, 0}, 2, 2};
+    return xr_cached_map(m, key, [&](CUtensorMap* out) {
+        cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+        cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+        cuuint32_t box[2] = {64, TA_KEYS};
+        cuuint32_t estr[2] = {1, 1};
+        return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    });
+}
+
+// q: row t, head h at q + t * ld_q + h * (D + R), [D plain | R rotated].  kv [keys][ld_kv]: head h's plain keys at column h D, its
+// values at H D + h V; tail [keys][ld_tail]: the rotated part, R columns.  The keys are those of the portions of at least `min_len`
+// tokens, one portion after another, each from the first that its first token sees, down to a multiple of 128, to its last.
+// out [n][H V]; gate (optional): pre-activations, head h of token t at gate + t * ld_gate + h, or with gate_each + h V + i.
+// row_tiles: the 128-token tiles of those portions, summed.
+XR_EXPORT int xr_attention_tc_flat(const void* q, long long ld_q, const void* kv, long long ld_kv, const void* tail, long long ld_tail, void* out,
+                                   const int* seg_start, const int* seg_len, const int* seg_pos0, int* status, int n, int n_seg, int H, int D, int R,
+                                   int V, long long keys, int window, float scale, int min_len, long long row_tiles, const void* gate, long long ld_gate,
+                                   int gate_each, cudaStream_t stream) {
+    if (!xr_attention_tc_flat_supported(D, R, V) || n < 1 || n_seg < 1 || H < 1 || H > 65535 || keys < 1 || keys > 0x3fffffffLL || window < 0 || min_len < 1 ||
+        row_tiles < 1 || row_tiles > 0x7fffffffLL || status == nullptr)
+        return XR_ERR_ARG;
+    if (((uintptr_t)q | (uintptr_t)kv | (uintptr_t)tail | (uintptr_t)out) & 15 || (ld_q | ld_kv | ld_tail) % 8 || ld_q < (long long)H * (D + R) ||
+        ld_kv < (long long)H * (D + V) || ld_tail < R)
+        return XR_ERR_ARG;
+    TaEncodeFn enc = ta_encode();
+    if (!enc) return -3;
+    CUtensorMap qm, kvm, tm;
+    const XrMapKey key{q, {(unsigned long long)(D + R), (unsigned long long)H, (unsigned long long)n}, {(unsigned long long)(D + R) * 2, (unsigned long long)ld_q * 2},
+                       {64, 1, TA_ROWS}, 3, 1};
+    if (!xr_cached_map(&qm, key, [&](CUtensorMap* m) {
+            cuuint64_t dims[3] = {(cuuint64_t)(D + R), (cuuint64_t)H, (cuuint64_t)n};
+            cuuint64_t strides[2] = {(cuuint64_t)(D + R) * 2, (cuuint64_t)ld_q * 2};
+            cuuint32_t box[3] = {64, 1, TA_ROWS};
+            cuuint32_t estr[3] = {1, 1, 1};
+            return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+        }))
+        return -3;
+    if (!ta_flat_map(&kvm, kv, keys, (long long)H * (D + V), ld_kv) || !ta_flat_map(&tm, tail, keys, R, ld_tail)) return -3;
+    AttnTcArgs a{(__nv_bfloat16*)out, seg_start, seg_len, seg_pos0, nullptr, status, H, H, 1, 0, 1, 0, window, 1, 0, scale * 1.4426950408889634f, n_seg,
+                 nullptr, 0.f, 0.f, 0, {nullptr, 0}, 0, min_len, 0, H * D, (const __nv_bfloat16*)gate, ld_gate, gate_each};
+    if (D == 64 && V == 64) return launch_flat<2, 1>(qm, kvm, tm, a, row_tiles, stream);
+    if (D == 64) return launch_flat<2, 2>(qm, kvm, tm, a, row_tiles, stream);
+    if (V == 64) return launch_flat<3, 1>(qm, kvm, tm, a, row_tiles, stream);
+    return launch_flat<3, 2>(qm, kvm, tm, a, row_tiles, stream);
+}
+
+// The cached rows of those portions' keys, `width` elements each, one after another: a warp a row, 16 bytes a lane.
+__global__ void __launch_bounds__(256)
+k_flat_rows(const uint4* __restrict__ cache, long long page_stride, uint4* __restrict__ out, const int* __restrict__ seg_len,
+            const int* __restrict__ seg_pos0, const int* __restrict__ block_tables, int n_seg, int keys, int width, int max_pages, int page_size,
+            int window, int min_len) {
+    xr_pdl_launch();
+    const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= keys) return;
+    int seg = -1, key = 0, before = 0;
+    for (int s = 0; s < n_seg; s++) {
+        const int len = seg_len[s];
+        if (len < min_len) continue;
+        const int first = ta_flat_first(seg_pos0[s], window), count = seg_pos0[s] + len - first;
+        if (row < before + count) { seg = s; key = first + row - before; break; }
+        before += count;
+    }
+    if (seg < 0) return;
+    const int page = block_tables[(size_t)seg * max_pages + key / page_size];
+    xr_pdl_wait();                                       // (the portion's own rows are stored by a kernel of this step)
+    if (page < 0) {                                      // (a page behind the window was given back: nobody sees its keys)
+        for (int i = lane; i < width; i += 32) out[(size_t)row * width + i] = make_uint4(0, 0, 0, 0);
+        return;
+    }
+    const uint4* src = cache + (size_t)page * page_stride + (size_t)(key % page_size) * width;
+    for (int i = lane; i < width; i += 32) out[(size_t)row * width + i] = src[i];
+}
+
+XR_EXPORT int xr_flat_rows(const void* cache, long long page_stride, void* out, const int* seg_len, const int* seg_pos0, const int* block_tables,
+                           int n_seg, int keys, int width, int max_pages, int page_size, int window, int min_len, cudaStream_t stream) {
+    if (n_seg < 1 || keys < 1 || width < 8 || width % 8 || page_stride % 8 || page_size < 1 || window < 0 || min_len < 1) return XR_ERR_ARG;
+    if (((uintptr_t)cache | (uintptr_t)out) & 15) return XR_ERR_ARG;
+    xr_launch(k_flat_rows, dim3((unsigned)((keys + 7) / 8)), dim3(256), 0, stream, (const uint4*)cache, page_stride / 8, (uint4*)out, seg_len, seg_pos0,
+              block_tables, n_seg, keys, width / 8, max_pages, page_size, window, min_len);
     return xr_launch_status();
 }

@@ -65,6 +65,9 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_attention_wait_probe": [_vp, _vp, ctypes.c_uint, _vp],
         "xr_attention_tc_supported": [_i, _i, _i, _i],
         "xr_attention_tc": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _ll, _ll, _i, _i, _vp, _f, _i, _vp, _i, _vp],
+        "xr_attention_tc_flat_supported": [_i, _i, _i],
+        "xr_attention_tc_flat": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _ll, _i, _f, _i, _ll, _vp, _ll, _i, _vp],
+        "xr_flat_rows": [_vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
         "xr_sample": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp],
         "xr_sample_one_block": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
         "xr_logprob": [_vp, _ll, _i, _i, _vp, _vp, _vp],
@@ -709,6 +712,50 @@ def attention_tc(qkv: torch.Tensor, out: torch.Tensor, seg_start, seg_len, seg_p
                                  seg_pos0.data_ptr(), block_tables.data_ptr(), status.data_ptr(), qkv.stride(0), n, n_seg,
                                  H, K, hd, max_pages, page_size, window, float(scale), max_seg_len, row_tiles, group[1], group[2],
                                  group[3], _ptr(sink), float(softcap), int(keep_first), _ptr(bias), _bias_len(bias), _stream()), "attention_tc")
+    _count()
+
+
+FLAT_TILE = 128       # the flat array's first key of a portion is a multiple of this
+
+
+def attention_tc_flat_supported(act_dtype: torch.dtype, D: int, R: int, V: int) -> bool:
+    return act_dtype == torch.bfloat16 and lib().xr_attention_tc_flat_supported(D, R, V) == 1
+
+
+def flat_first_key(pos0, window: int):
+    """The first key of a portion that the flat array holds (numpy arrays or numbers)."""
+    first = (pos0 - window + 1) // FLAT_TILE * FLAT_TILE
+    return first * ((window > 0) & (pos0 >= window))
+
+
+def flat_rows(cache_ptr: int, page_stride: int, out: torch.Tensor, seg_len, seg_pos0, block_tables, n_seg: int, max_pages: int,
+              page_size: int, window: int, min_len: int) -> None:
+    """out [keys, width] bfloat16 = the cached rows of the keys of the portions of at least `min_len` tokens, one portion after
+    another, each from ``flat_first_key`` to its last."""
+    _dev(out, seg_len, seg_pos0, block_tables)
+    assert out.dtype == torch.bfloat16
+    _check(lib().xr_flat_rows(cache_ptr, page_stride, out.data_ptr(), seg_len.data_ptr(), seg_pos0.data_ptr(), block_tables.data_ptr(), n_seg,
+                              out.shape[0], out.shape[1], max_pages, page_size, window, min_len, _stream()), "flat_rows")
+    _count()
+
+
+def attention_tc_flat(q: torch.Tensor, kv: torch.Tensor, tail: torch.Tensor, out: torch.Tensor, seg_start, seg_len, seg_pos0, n_seg: int,
+                      H: int, D: int, R: int, V: int, window: int, scale: float, min_len: int, row_tiles: int,
+                      gate: Optional[torch.Tensor] = None, gate_each: bool = False) -> None:
+    """Causal attention on tcgen05 of the portions of at least `min_len` tokens over expanded keys and values.  q [n, >= H (D + R)]:
+    heads [D plain | R rotated]; kv [keys, H (D + V)]: all heads' plain keys, then all heads' values; tail [keys, R]: the rotated key
+    part that all heads share; the keys in the order of ``flat_rows``.  out [n, H V] (rows of other portions are left alone), times
+    sigmoid(gate): one value a head, or with `gate_each` one an element.  q, kv, tail and gate may be strided by rows.
+    `row_tiles`: the 128-token tiles of those portions."""
+    _dev(out, seg_start, seg_len, seg_pos0)
+    n, keys = q.shape[0], kv.shape[0]
+    assert all(t.dtype == torch.bfloat16 and t.is_cuda and t.stride(1) == 1 for t in (q, kv, tail, out))
+    assert q.shape[1] >= H * (D + R) and kv.shape[1] == H * (D + V) and tail.shape == (keys, R) and out.shape == (n, H * V)
+    assert gate is None or (gate.dtype == torch.bfloat16 and gate.is_cuda and gate.stride(1) == 1 and gate.shape == (n, H * V if gate_each else H))
+    _check(lib().xr_attention_tc_flat(q.data_ptr(), q.stride(0), kv.data_ptr(), kv.stride(0), tail.data_ptr(), tail.stride(0), out.data_ptr(),
+                                      seg_start.data_ptr(), seg_len.data_ptr(), seg_pos0.data_ptr(), workspace(out.device).status_ptr, n, n_seg,
+                                      H, D, R, V, keys, window, float(scale), min_len, row_tiles, _ptr(gate), 0 if gate is None else gate.stride(0),
+                                      int(gate_each), _stream()), "attention_tc_flat")
     _count()
 
 

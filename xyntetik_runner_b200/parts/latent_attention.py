@@ -6,9 +6,12 @@ With h the mixer's input, H heads, per head D plain and R rotated query/key elem
     k_h = [W_uk,h c | r],  v_h = W_uv,h c
     s_ij = (q_plain . W_uk,h c_j + rotate(q_rot) . r_j) * scale,  j <= i;  a = softmax(s);  o_h = sum_j a_ij v_hj
     y = W_o concat_h(sigmoid(W_g h)_h * o_h)
-Only [c | r] is cached: one row of C + R values per token (one plane, one "kv head"), whatever H is.  The kernels
-never expand a key: the query is taken into the latent space, attention runs over the cached rows, and the result is
-expanded by W_uv afterwards (csrc/latent_attention.cu).  The rotation uses the first `rotary_dim` of the R elements
+Only [c | r] is cached: one row of C + R values per token (one plane, one "kv head"), whatever H is.  Two orders of the
+same sums.  Few tokens over many keys (a decode step): no key is expanded, the query is taken into the latent space,
+attention runs over the cached rows with C + R columns a score and C a value, and the result is expanded by W_uv
+afterwards (csrc/latent_attention.cu).  Portions of many tokens: the keys and values of all heads are expanded once, by one
+dense product over the portion's cached rows, and attention runs with D + R and V columns on tcgen05 (csrc/attention_tc.cu,
+``_flat_plan`` says when).  The rotation uses the first `rotary_dim` of the R elements
 in the pairing the position encoding names (half-split or adjacent).
 
 Options, all off by default:
@@ -34,7 +37,12 @@ from .linear import Linear
 
 # the tensor-core kernel for the sizes it takes (a module attribute, so that a test can compare the two kernels)
 USE_MMA = True
-counters = {"mma": 0, "simt": 0}
+USE_FLAT = True
+counters = {"mma": 0, "simt": 0, "flat": 0}
+
+# Portions of at least so many tokens may have their keys expanded, over at most so many keys a step (16 KB a key and layer at
+# 32 heads of 128: what the expanded rows may take of the memory).
+FLAT_MIN, FLAT_KEYS = 32, 65536
 
 
 class LatentAttention(Mixer):
@@ -100,6 +108,10 @@ class LatentAttention(Mixer):
             self.w_uk_packed = kernels.pack_weight_groups(self.w_uk.view(self.H, self.D, self.C).transpose(1, 2).contiguous())
             self.w_uv_packed = kernels.pack_weight_groups(self.w_uv.view(self.H, self.V, self.C))
         self._heads_of_tiles = {}
+        self.expand = None
+        if (self.w_uk_packed is not None and (self.C + self.R) % 8 == 0
+                and kernels.attention_tc_flat_supported(rt.act_dtype, self.D, self.R, self.V)):
+            self.expand = Linear(torch.cat([self.w_uk, self.w_uv], dim=0)).prepare(rt)
         self.norm_w = tensors[n["norm"]].to(torch.float32).contiguous() if self.own_rows else None
         self.position.prepare(rt)
         rot = self.position.rotary()
@@ -124,6 +136,73 @@ class LatentAttention(Mixer):
     def weight_bytes(self):
         return (self.proj.nbytes() + self.out.nbytes() + self.w_uk.numel() * self.w_uk.element_size()
                 + self.w_uv.numel() * self.w_uv.element_size() + (self.up_q.nbytes() if self.up_q is not None else 0))
+
+    def _flat_plan(self, ctx, n: int):
+        """(keys to expand, 128-token tiles, token ranges left to the other order) where expanding keys pays, else None.  The times
+        (microseconds) behind it are rates measured on one B200: the kernel over the latent rows does 70 TFLOP/s on 2 C + R columns
+        a head and key, its per-head products 300; expanding costs a product at 900 TFLOP/s and attention at 300 on D + R + V columns,
+        and 25 us of launches.  2,048 tokens of one request, 16 heads of 128 + 64 over a latent of 512: 1,200 us a layer
+        over the latent rows, 85 so (51 of them attention); 512 of one request beside 16 single tokens, two layers: 540 us and 300."""
+        H, D, R, V, C, window = self.H, self.D, self.R, self.V, self.C, self.window or 0
+        length, pos0, start = (ctx.host[k].astype(np.int64) for k in ("seg_len", "seg_pos0", "seg_start"))
+        many = length >= FLAT_MIN
+        if not many.any():
+            return None
+        mean = pos0[many] + (length[many] + 1) / 2.0
+        pairs = float((np.minimum(mean, window) if window else mean).dot(length[many]))
+        keys = int((pos0 + length - kernels.flat_first_key(pos0, window))[many].sum())
+        tokens = int(length[many].sum())
+        if keys > FLAT_KEYS:
+            return None
+        absorbed = pairs * H * 2 * (2 * C + R) / 70e6 + tokens * 2.0 * H * C * (D + V) / 300e6
+        flat = 25.0 + keys * 2.0 * C * H * (D + V) / 900e6 + pairs * H * 2 * (D + R + V) / 300e6
+        if flat >= absorbed:
+            return None
+        # the tokens of the other portions, neighbours together
+        rest = []
+        for s in np.argsort(start[~many], kind="stable"):
+            at, end = int(start[~many][s]), int(start[~many][s] + length[~many][s])
+            if rest and rest[-1][1] == at:
+                rest[-1][1] = end
+            else:
+                rest.append([at, end])
+        if len(rest) > 4:
+            return None                     # (scattered one by one between long portions: not worth a launch each)
+        return keys, int((-(-length[many] // 128)).sum()), rest
+
+    def _absorbed(self, ctx, qt, positions, tok_seg, bt, cache_ptr, page_stride, o, gate, gate_col, window):
+        """Attention over the latent rows of the tokens whose queries are qt's rows, into o's."""
+        n, H, D, R, V, C = qt.shape[0], self.H, self.D, self.R, self.V, self.C
+        reach = min(ctx.max_kv_len, window) if window else ctx.max_kv_len
+        chunk, splits = ctx.once(("latent_splits", n, H, window), lambda: kernels.latent_attention_splits(n, H, reach))
+        po = pm = None
+        if splits > 1:
+            mt = -(-H // 16)
+            po = ctx.buf("latent_part_o", (n * mt * splits * 16 * C,), torch.float32)
+            pm = ctx.buf("latent_part_ml", (n * mt * splits * 32,), torch.float32)
+        args = (cache_ptr, page_stride, positions, tok_seg, bt, H, C, R, ctx.max_pages, ctx.page_size, self.scale, chunk, splits)
+        if self.w_uk_packed is not None:
+            # the two per-head products on tcgen05: rows of one head together (n_pad a head), one grouped product each
+            bn = 16 if n <= 16 else (32 if n <= 32 else (64 if n <= 64 else 128))
+            n_pad = -(-n // bn) * bn
+            groups = self._tile_heads(n_pad // bn, o.device)
+            qh = ctx.buf("latent_qh", (H * n_pad, D), torch.bfloat16)
+            kernels.heads_gather(qt, 0, D + R, qh, n, n_pad, H, D)
+            ql = ctx.buf("latent_q", (H * n_pad, C), torch.bfloat16)
+            kernels.gemm_tc_grouped(qh, self.w_uk_packed, ql, groups, bn, C)
+            ol = ctx.buf("latent_o", (H * n_pad, C), torch.bfloat16)
+            kernels.latent_attention_mma(ql, qt, D, D + R, ol, po, pm, *args, n_pad=n_pad, window=window)
+            oh = ctx.buf("latent_oh", (H * n_pad, V), torch.float32)
+            kernels.gemm_tc_grouped(ol, self.w_uv_packed, oh, groups, bn, V)
+            kernels.heads_scatter_gate(oh, o, gate, gate_col, n, n_pad, H, V, gate_each=self.gate_each)
+        else:
+            # the plain query parts, taken through W_uk^T into the latent space (bfloat16: an operand of the tensor cores)
+            ql = ctx.buf("latent_q", (n, H * C), torch.bfloat16)
+            kernels.head_matmul(qt, 0, D + R, self.w_uk, False, ql, n, H, D, C)
+            ol = ctx.buf("latent_o", (n, H * C), torch.float32)
+            kernels.latent_attention_mma(ql, qt, D, D + R, ol, po, pm, *args, window=window)
+            kernels.head_matmul(ol, 0, C, self.w_uv, True, o, n, H, C, V, gate=gate, gate_col=gate_col, gate_each=self.gate_each)
+        counters["mma"] += 1
 
     def forward(self, ctx, h, x, lay):
         n, H, D, R, V, C = h.shape[0], self.H, self.D, self.R, self.V, self.C
@@ -154,36 +233,23 @@ class LatentAttention(Mixer):
         gate = proj if self.gated else None
         window = self.window or 0
         if USE_MMA and D > 0 and kernels.latent_attention_mma_supported(ctx.act_dtype, D, R, C):
-            reach = min(ctx.max_kv_len, window) if window else ctx.max_kv_len
-            chunk, splits = ctx.once(("latent_splits", H, window), lambda: kernels.latent_attention_splits(n, H, reach))
-            po = pm = None
-            if splits > 1:
-                mt = -(-H // 16)
-                po = ctx.buf("latent_part_o", (n * mt * splits * 16 * C,), torch.float32)
-                pm = ctx.buf("latent_part_ml", (n * mt * splits * 32,), torch.float32)
-            args = (cache_ptr, page_stride, ctx.positions, ctx.tok_seg, bt, H, C, R, ctx.max_pages, ctx.page_size, self.scale, chunk, splits)
-            if self.w_uk_packed is not None:
-                # the two per-head products on tcgen05: rows of one head together (n_pad a head), one grouped product each
-                bn = 16 if n <= 16 else (32 if n <= 32 else (64 if n <= 64 else 128))
-                n_pad = -(-n // bn) * bn
-                groups = self._tile_heads(n_pad // bn, h.device)
-                qh = ctx.buf("latent_qh", (H * n_pad, D), torch.bfloat16)
-                kernels.heads_gather(qt, 0, D + R, qh, n, n_pad, H, D)
-                ql = ctx.buf("latent_q", (H * n_pad, C), torch.bfloat16)
-                kernels.gemm_tc_grouped(qh, self.w_uk_packed, ql, groups, bn, C)
-                ol = ctx.buf("latent_o", (H * n_pad, C), torch.bfloat16)
-                kernels.latent_attention_mma(ql, qt, D, D + R, ol, po, pm, *args, n_pad=n_pad, window=window)
-                oh = ctx.buf("latent_oh", (H * n_pad, V), torch.float32)
-                kernels.gemm_tc_grouped(ol, self.w_uv_packed, oh, groups, bn, V)
-                kernels.heads_scatter_gate(oh, o, gate, gate_col, n, n_pad, H, V, gate_each=self.gate_each)
+            flat = ctx.once(("latent_flat", H, D, R, V, C, window), lambda: self._flat_plan(ctx, n)) if USE_FLAT and self.expand is not None else None
+            if flat:
+                keys, tiles, rest = flat
+                # (rows for a power of two of keys: a buffer that grows invalidates the step graphs)
+                room = 1 << (keys - 1).bit_length()
+                rows = ctx.buf("latent_rows", (room, C + R), torch.bfloat16)[:keys]
+                kernels.flat_rows(cache_ptr, page_stride, rows, ctx.seg_len, ctx.seg_pos0, bt, ctx.n_seg, ctx.max_pages, ctx.page_size, window, FLAT_MIN)
+                kv = ctx.buf("latent_kv", (room, H * (D + V)), torch.bfloat16)[:keys]
+                self.expand.forward(rows[:, :C], kv)
+                kernels.attention_tc_flat(qt, kv, rows[:, C:], o, ctx.seg_start, ctx.seg_len, ctx.seg_pos0, ctx.n_seg, H, D, R, V, window, self.scale,
+                                          FLAT_MIN, tiles, gate=None if gate is None else gate[:, gate_col:], gate_each=self.gate_each)
+                counters["flat"] += 1
+                for at, end in rest:
+                    self._absorbed(ctx, qt[at:end], ctx.positions[at:end], ctx.tok_seg[at:end], bt, cache_ptr, page_stride, o[at:end],
+                                   None if gate is None else gate[at:end], gate_col, window)
             else:
-                # the plain query parts, taken through W_uk^T into the latent space (bfloat16: an operand of the tensor cores)
-                ql = ctx.buf("latent_q", (n, H * C), torch.bfloat16)
-                kernels.head_matmul(qt, 0, D + R, self.w_uk, False, ql, n, H, D, C)
-                ol = ctx.buf("latent_o", (n, H * C), torch.float32)
-                kernels.latent_attention_mma(ql, qt, D, D + R, ol, po, pm, *args, window=window)
-                kernels.head_matmul(ol, 0, C, self.w_uv, True, o, n, H, C, V, gate=gate, gate_col=gate_col, gate_each=self.gate_each)
-            counters["mma"] += 1
+                self._absorbed(ctx, qt, ctx.positions, ctx.tok_seg, bt, cache_ptr, page_stride, o, gate, gate_col, window)
         else:
             ql = ctx.buf("latent_q", (n, H * C), torch.float32)
             if D > 0:
