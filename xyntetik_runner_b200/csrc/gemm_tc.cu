@@ -174,10 +174,13 @@ struct TcParams {
     const int* tile_group;
     int group_row_tiles;        // row tiles of one matrix in the packed array
     float alpha = 1.f;          // factor on the accumulator, ahead of bias and activation (not for gated products)
+    // Grouped products on CTA pairs (xr_gemm_tc_grouped_pairs): [0] the number of token tiles, then per tile its matrix, its first
+    // row and its rows (at most TC2_BN), written by a kernel of this step; group_row_tiles as above
+    const int* tiles = nullptr;
 };
 
 // ---------------------------------------------------------------------------------------------
-// Epilogue of one tile, run by warps 2..9 once the accumulator is complete.  A warp may only read the 32
+// Epilogue of one tile (`bn` tokens from tok0 on, those from n_end on do not exist), run by warps 2..9 once the accumulator is complete.  A warp may only read the 32
 // tensor-memory lanes of its index mod 4, so two warps share each quarter and take alternate 16-column
 // chunks (with sixteen epilogue warps, four share a quarter).
 //
@@ -186,7 +189,7 @@ struct TcParams {
 // up lanes columns 8..15; each gets the other half of what it needs from its partner lane (lane xor 16) by shuffle.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_base, int row0, int tok0, int warp, int lane,
-                                            int warps_per_quarter = 2, int split = (int)blockIdx.z) {
+                                            int warps_per_quarter, int split, int bn, int n_end) {
     const int quad = warp & 3, chunk_first = (warp - 2) >> 2;
     const int r = row0 + quad * 32 + lane;            // row of the product that this thread's lane holds
     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
@@ -197,8 +200,8 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
     const float b = (p.bias != nullptr && row_ok && (p.epilogue == TC_EPI_STORE || p.epilogue == TC_EPI_ADD) && split == 0)
                         ? p.bias[r] : 0.f;
 #pragma unroll 1
-    for (int c0 = chunk_first * 16; c0 < p.bn; c0 += 16 * warps_per_quarter) {
-        if (tok0 + c0 >= p.n) break;               // warp-uniform
+    for (int c0 = chunk_first * 16; c0 < bn; c0 += 16 * warps_per_quarter) {
+        if (tok0 + c0 >= n_end) break;             // warp-uniform
         float g[16];
         tc_ld16(taddr + c0, g);
         if (gated_out) {
@@ -215,12 +218,12 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
                 __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)col0 * p.ldo + f;
 #pragma unroll
                 for (int c = 0; c < 8; c++)
-                    if (col0 + c < p.n) dst[(size_t)c * p.ldo] = __float2bfloat16_rn(v[c]);
+                    if (col0 + c < n_end) dst[(size_t)c * p.ldo] = __float2bfloat16_rn(v[c]);
             } else {
                 float* dst = (float*)p.out + (size_t)col0 * p.ldo + f;
 #pragma unroll
                 for (int c = 0; c < 8; c++)
-                    if (col0 + c < p.n) dst[(size_t)c * p.ldo] = v[c];
+                    if (col0 + c < n_end) dst[(size_t)c * p.ldo] = v[c];
             }
             continue;
         }
@@ -230,16 +233,16 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
             float* dst = (float*)p.out + (size_t)(tok0 + c0) * p.ldo + r;
             float old[16];
 #pragma unroll
-            for (int c = 0; c < 16; c++) old[c] = xr_ld_now(dst + (size_t)(tok0 + c0 + c < p.n ? c : 0) * p.ldo);
+            for (int c = 0; c < 16; c++) old[c] = xr_ld_now(dst + (size_t)(tok0 + c0 + c < n_end ? c : 0) * p.ldo);
 #pragma unroll
             for (int c = 0; c < 16; c++) xr_ld_fence(old[c]);
 #pragma unroll
             for (int c = 0; c < 16; c++)
-                if (tok0 + c0 + c < p.n) dst[(size_t)c * p.ldo] = old[c] + fmaf(p.alpha, g[c], b);
+                if (tok0 + c0 + c < n_end) dst[(size_t)c * p.ldo] = old[c] + fmaf(p.alpha, g[c], b);
             continue;
         }
         // a chunk that runs past the last token stores only what exists
-        const int live = p.n - (tok0 + c0) < 16 ? p.n - (tok0 + c0) : 16;
+        const int live = n_end - (tok0 + c0) < 16 ? n_end - (tok0 + c0) : 16;
         if (p.epilogue == TC_EPI_PARTIAL) {
             const size_t width = p.gated ? (size_t)((p.n_out + 63) / 64) * 128 : (size_t)p.n_out;
             float* dst = p.partial + ((size_t)split * p.n + tok0 + c0) * width + r;
@@ -377,7 +380,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         // ---------------- epilogue: warps 2..9 ----------------
         bool ok = mbar_wait(acc_ready, 0, abort_flag);
         tc_fence_after();
-        if (ok) tc_epilogue(p, tmem_base, row0, tok0, warp, lane);
+        if (ok) tc_epilogue(p, tmem_base, row0, tok0, warp, lane, 2, (int)blockIdx.z, p.bn, p.n);
     }
     tc_fence_before();
     __syncthreads();
@@ -434,6 +437,7 @@ __host__ __device__ constexpr uint32_t instr_desc_pair(int bn) {
 }
 
 #define TC2_BN 256         // token capacity of a pair's tile; each CTA stages half
+#define TC2_XBOX 32         // grouped products: tokens per TMA box
 #define TC2_THREADS 576    // producer warp, MMA warp, sixteen epilogue warps (the tile is wide: four per quarter)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
@@ -446,7 +450,28 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_cluster_addr) {
 // of stages runs on across tiles (the producer fetches the next tile's operands while the epilogue of this one
 // runs), and two accumulators are kept in tensor memory, so that the MMAs of the next tile overlap the epilogue
 // too (a gated product as well: its gate and up rows are interleaved in one tile, so it has one accumulator a tile).
-template <int STAGES>
+//
+// GROUPED: the rows of X are sorted by the matrix they meet and a table of this step (p.tiles) says which rows make a tile: at most
+// TC2_BN of them, of one matrix, as many as the matrix has or an equal share of them.  The instruction's N is the tile's own row
+// count rounded up to 32, so a matrix that meets 190 rows costs 192 columns and its weights are fetched once.
+// The tiles of one stretch of rows follow one another (all of its matrix's row tiles, then the next stretch): the clusters that work at
+// the same time share that stretch of X in L2, and every matrix streams through once.  The other order, all stretches for one pair of
+// row tiles, fetches X from memory again for every pair once it no longer fits beside the matrices (the gated product of 64 experts of
+// 1,408 at width 2,048, 192 rows each: 184 us so, 204 so ordered, 433 on single CTAs with padded tiles of 128).
+struct TcTile { int tok0, n_end, bn, row_tile0, pair; };
+template <bool GROUPED>
+__device__ __forceinline__ TcTile tc_pair_tile(const TcParams& p, int tile, int tok_tiles) {
+    if constexpr (GROUPED) {
+        const int pairs = (p.group_row_tiles + 1) / 2;
+        const int* e = p.tiles + 1 + 3 * (tile / pairs);
+        const int group = e[0], first = e[1], rows = e[2];
+        return {first, first + rows, (rows + 31) / 32 * 32, group * p.group_row_tiles, tile % pairs};
+    } else {
+        return {tile % tok_tiles * p.bn, p.n, p.bn, 0, tile / tok_tiles};
+    }
+}
+
+template <int STAGES, bool GROUPED>
 __global__ void __launch_bounds__(TC2_THREADS, 1)
 k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, TcParams p) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -466,9 +491,7 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = tc_cluster_rank();                 // 0: issues the MMAs
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
-    const int half = p.bn >> 1;                              // tokens this CTA stages
     const int nkb = (p.K + TC_BK - 1) / TC_BK;
-    const uint32_t stage_bytes = W_BYTES + half * TC_BK * 2;
     constexpr int ACC_BUFS = 2;                              // two accumulators of TC2_BN columns each
 
     if (threadIdx.x == 0) {
@@ -486,27 +509,35 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     xr_pdl_wait();
+    const int tok_tiles = GROUPED ? p.tiles[0] : p.tok_tiles;
+    const int pair_tiles = GROUPED ? tok_tiles * ((p.group_row_tiles + 1) / 2) : p.pair_tiles;
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
         if (lane == 0) {
             int it = 0;                                      // K blocks fetched so far, over all tiles
             bool ok = true;
-            for (int item = cluster_id; item < p.pair_tiles * p.splits && ok; item += n_clusters) {
-                const int tile = item % p.pair_tiles, split = item / p.pair_tiles;
-                const int row_tile = 2 * (tile / p.tok_tiles) + (int)rank;
-                const int tok0 = (tile % p.tok_tiles) * p.bn;
+            for (int item = cluster_id; item < pair_tiles * p.splits && ok; item += n_clusters) {
+                const int tile = item % pair_tiles, split = item / pair_tiles;
+                const TcTile at = tc_pair_tile<GROUPED>(p, tile, tok_tiles);
+                const int row_tile = at.row_tile0 + 2 * at.pair + (int)rank;
+                const int half = at.bn >> 1;                     // tokens this CTA stages
+                // grouped: boxes of TC2_XBOX tokens, as many as hold the half (a box may reach into rows of other tiles: columns
+                // of the accumulator that nobody reads)
+                const int boxes = GROUPED ? (half + TC2_XBOX - 1) / TC2_XBOX : 1;
+                const uint32_t stage_bytes = W_BYTES + (GROUPED ? boxes * TC2_XBOX : half) * TC_BK * 2;
                 const int kb0 = (int)(((long long)split * nkb) / p.splits), kb1 = (int)(((long long)(split + 1) * nkb) / p.splits);
                 for (int i = kb0; i < kb1; i++, it++) {
                     int s = it % STAGES;
                     if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag)) { ok = false; break; }
                     uint8_t* st = smem + s * STAGE_BYTES;
                     const uint32_t bar = tc_map_to_rank(smem_u32(&full[s]), 0);
+                    const int kx = i * TC_BK;
                     if (rank == 0) mbar_expect_tx(&full[s], 2 * stage_bytes);
-                    int kx = i * TC_BK;
                     if (p.packed) tma_load_2d_pair(st, &map_w, 0, (row_tile * p.w_kblocks + i) * TC_BM, bar);
                     else tma_load_2d_pair(st, &map_w, kx, row_tile * TC_BM, bar);
-                    tma_load_2d_pair(st + W_BYTES, &map_x, kx, tok0 + (int)rank * half, bar);
+                    for (int x = 0; x < boxes; x++)
+                        tma_load_2d_pair(st + W_BYTES + x * TC2_XBOX * TC_BK * 2, &map_x, kx, at.tok0 + (int)rank * half + x * TC2_XBOX, bar);
                 }
             }
             if (*abort_flag) {
@@ -519,11 +550,11 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA only) ----------------
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = instr_desc_pair(p.bn);
             bool ok = true;
             int it = 0, j = 0;                               // K blocks and tiles done so far
-            for (int item = cluster_id; item < p.pair_tiles * p.splits && ok; item += n_clusters, j++) {
-                const int split = item / p.pair_tiles;
+            for (int item = cluster_id; item < pair_tiles * p.splits && ok; item += n_clusters, j++) {
+                const int split = item / pair_tiles;
+                const uint32_t idesc = instr_desc_pair(tc_pair_tile<GROUPED>(p, item % pair_tiles, tok_tiles).bn);
                 const int kb0 = (int)(((long long)split * nkb) / p.splits), kb1 = (int)(((long long)(split + 1) * nkb) / p.splits);
                 const int b = j % ACC_BUFS;
                 if (j >= ACC_BUFS) {                         // the epilogues of both CTAs have emptied this accumulator
@@ -551,13 +582,14 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         // ---------------- epilogue: warps 2..17 of both CTAs, each CTA its own 128 rows ----------------
         const uint32_t acc_empty_bar0 = tc_map_to_rank(smem_u32(&acc_empty[0]), 0);
         int j = 0;
-        for (int item = cluster_id; item < p.pair_tiles * p.splits; item += n_clusters, j++) {
-            const int tile = item % p.pair_tiles, split = item / p.pair_tiles;
+        for (int item = cluster_id; item < pair_tiles * p.splits; item += n_clusters, j++) {
+            const int tile = item % pair_tiles, split = item / pair_tiles;
             const int b = j % ACC_BUFS;
             if (!mbar_wait(&acc_full[b], (j / ACC_BUFS) & 1, abort_flag)) break;
             tc_fence_after();
-            const int row0 = (2 * (tile / p.tok_tiles) + (int)rank) * TC_BM, tok0 = (tile % p.tok_tiles) * p.bn;
-            tc_epilogue(p, tmem_base + (uint32_t)b * TC2_BN, row0, tok0, warp, lane, 4, split);
+            const TcTile at = tc_pair_tile<GROUPED>(p, tile, tok_tiles);
+            const int row0 = (2 * at.pair + (int)rank) * TC_BM;
+            tc_epilogue(p, tmem_base + (uint32_t)b * TC2_BN, row0, at.tok0, warp, lane, 4, split, at.bn, at.n_end);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(acc_empty_bar0 + (uint32_t)b * 8);
@@ -696,21 +728,24 @@ struct PairLaunch {
             config(cfg, attr, xr_sm_count() / 2, nullptr);
             cfg.numAttrs = 1;
             int nc = 0;
-            if (cudaFuncSetAttribute(k_gemm_tc_pair<TC2_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
-                cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc_pair<TC2_STAGES>, &cfg) == cudaSuccess && nc > 0)
+            if (cudaFuncSetAttribute(k_gemm_tc_pair<TC2_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
+                cudaFuncSetAttribute(k_gemm_tc_pair<TC2_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
+                cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc_pair<TC2_STAGES, false>, &cfg) == cudaSuccess && nc > 0)
                 n = nc;
             else
                 cudaGetLastError();        // the single-CTA kernel takes over; leave no error behind
         }
         return n;
     }
+    // (grouped: p.pair_tiles is an upper bound, the kernel reads the true number of tiles)
     static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, cudaStream_t stream) {
         const int most = clusters();
         if (most < 1) return XR_ERR_LAUNCH;
         cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[2];
         const int items = p.pair_tiles * p.splits;
         config(cfg, attr, items < most ? items : most, stream);
-        cudaLaunchKernelEx(&cfg, k_gemm_tc_pair<TC2_STAGES>, mw, mx, p);
+        if (p.tiles != nullptr) cudaLaunchKernelEx(&cfg, k_gemm_tc_pair<TC2_STAGES, true>, mw, mx, p);
+        else cudaLaunchKernelEx(&cfg, k_gemm_tc_pair<TC2_STAGES, false>, mw, mx, p);
         return xr_launch_status();
     }
 };
@@ -893,6 +928,33 @@ XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int ou
         case 64: return launch_tc<64, 4, 2>(mw, mx, p, grid, stream);
         default: return launch_tc<128, 5, 1>(mw, mx, p, grid, stream);
     }
+}
+
+// The same on CTA pairs, for groups that meet many rows: `tiles` (int [1 + 3 max_tiles], on the device) holds the number of token
+// tiles and then per tile its group, its first row and its rows (1 .. 256), see xr_moe_plan_tiles; every group's rows lie in tiles of
+// their own.  n: rows of X and out.
+XR_EXPORT int xr_gemm_tc_pairs_available() { return PairLaunch::clusters() > 0 ? 1 : 0; }
+
+XR_EXPORT int xr_gemm_tc_grouped_pairs(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit,
+                                       int n, int n_out, int K, long long ldx, long long ldo, const int* tiles, int max_tiles, int groups,
+                                       int* status, cudaStream_t stream) {
+    if (n < 1 || n_out < 1 || K < 8 || (K % 8) != 0 || (ldx % 8) != 0 || ldx < K || ldo < n_out || groups < 1 || max_tiles < 1) return XR_ERR_ARG;
+    if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || tiles == nullptr) return XR_ERR_ARG;
+    if (epilogue != TC_EPI_STORE && epilogue != TC_EPI_GATED) return XR_ERR_ARG;
+    if (out_dtype != XR_F32 && out_dtype != XR_BF16) return XR_ERR_ARG;
+    const bool gated = epilogue == TC_EPI_GATED;
+    if (act != TC_ACT_NONE && act != TC_ACT_SILU && act != TC_ACT_GELU_TANH && act != TC_ACT_RELU2 && !(act == TC_ACT_SWISH_CLAMP && gated)) return XR_ERR_ARG;
+    const int row_tiles = gated ? (n_out + 63) / 64 : (n_out + TC_BM - 1) / TC_BM;
+    const int total_kb = (K + TC_BK - 1) / TC_BK;
+    const long long most = (long long)max_tiles * ((row_tiles + 1) / 2);
+    if (most > 0x7fffffffLL) return XR_ERR_ARG;
+    CUtensorMap mw, mx;
+    if (!make_map(&mw, W, (long long)groups * row_tiles * TC_BM * total_kb, TC_BK, TC_BK, TC_BM)) return -3;
+    if (!make_map(&mx, X, n, K, ldx, TC2_XBOX)) return -3;
+    TcParams p{out, nullptr, nullptr, status, ldo, n, n_out, K, 1, epilogue, out_dtype, act, act_limit, gated ? 1 : 0, TC2_BN, 1, total_kb,
+               max_tiles, (int)most, nullptr, row_tiles};
+    p.tiles = tiles;
+    return PairLaunch::launch(mw, mx, p, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -197,6 +197,67 @@ k_moe_plan(const int* __restrict__ ids, int* __restrict__ row_src, int* __restri
     (void)used;
 }
 
+// The same for the product on CTA pairs (xr_gemm_tc_grouped_pairs): the pairs sorted by expert, every expert's rows starting at a
+// multiple of 16, and a table of tiles, [0] their number, then per tile (expert, first row, rows): ceil(count / cap) tiles an expert,
+// its rows shared out evenly in multiples of 32.  At most pairs / cap + E tiles, pairs + 15 E rows.
+__global__ void __launch_bounds__(1024)
+k_moe_plan_tiles(const int* __restrict__ ids, int* __restrict__ row_src, int* __restrict__ pair_row, int* __restrict__ tiles,
+                 int pairs, int E, int cap, int max_rows) {
+    xr_pdl_launch();
+    __shared__ int count[MOE_MAX_E], cursor[MOE_MAX_E], tile0[MOE_MAX_E];
+    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
+    xr_pdl_wait();
+    __syncthreads();
+    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+        const int e = ids[p];
+        if (e < E) atomicAdd(&count[e], 1);
+    }
+    for (int r = threadIdx.x; r < max_rows; r += blockDim.x) row_src[r] = -1;
+    __syncthreads();
+    // starts: a warp's running sums over 32 experts at a time
+    if (threadIdx.x < 32) {
+        int rows_before = 0, tiles_before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + threadIdx.x, c = e < E ? count[e] : 0;
+            int rows = (c + 15) / 16 * 16, nt = (c + cap - 1) / cap;
+            const int own_rows = rows, own_nt = nt;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int a = __shfl_up_sync(0xffffffffu, rows, o), b = __shfl_up_sync(0xffffffffu, nt, o);
+                if ((int)threadIdx.x >= o) { rows += a; nt += b; }
+            }
+            if (e < E) { cursor[e] = rows_before + rows - own_rows; tile0[e] = tiles_before + nt - own_nt; }
+            rows_before += __shfl_sync(0xffffffffu, rows, 31);
+            tiles_before += __shfl_sync(0xffffffffu, nt, 31);
+        }
+        if (threadIdx.x == 0) tiles[0] = tiles_before;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        const int c = count[e], nt = (c + cap - 1) / cap;
+        const int share = nt > 0 ? ((c + nt - 1) / nt + 31) / 32 * 32 : 0;
+        for (int t = 0; t < nt; t++) {
+            int* out = tiles + 1 + 3 * (tile0[e] + t);
+            out[0] = e; out[1] = cursor[e] + t * share; out[2] = min(share, c - t * share);
+        }
+    }
+    __syncthreads();
+    for (int p = threadIdx.x; p < pairs; p += blockDim.x) {
+        const int e = ids[p];
+        if (e >= E) { pair_row[p] = -1; continue; }
+        const int r = atomicAdd(&cursor[e], 1);
+        row_src[r] = p;
+        pair_row[p] = r;
+    }
+}
+
+XR_EXPORT int xr_moe_plan_tiles(const int* ids, int* row_src, int* pair_row, int* tiles, int pairs, int E, int cap, int max_tiles, int max_rows,
+                                cudaStream_t stream) {
+    if (pairs < 1 || E < 1 || E > MOE_MAX_E || cap < 32 || cap % 32 || max_tiles < pairs / cap + E || (long long)max_rows < pairs + 15LL * E) return XR_ERR_ARG;
+    xr_launch(k_moe_plan_tiles, dim3(1), dim3(1024), 0, stream, ids, row_src, pair_row, tiles, pairs, E, cap, max_rows);
+    return xr_launch_status();
+}
+
 XR_EXPORT int xr_moe_plan(const int* ids, int* row_src, int* pair_row, int* tile_group, int pairs, int E, int align, int max_tiles,
                           cudaStream_t stream) {
     if (pairs < 1 || E < 1 || E > MOE_MAX_E || align < 1 || max_tiles < pairs / align + E) return XR_ERR_ARG;
@@ -207,7 +268,8 @@ XR_EXPORT int xr_moe_plan(const int* ids, int* row_src, int* pair_row, int* tile
 // ---------------------------------------------------------------------------------------------
 // out[r] = h[row_src[r] / top] for the rows of tiles that hold any, zeros for rows of padding: the first product's
 // input in the order of the plan, for the tensor-core product (which reads its rows through a tensor map).  T: what a thread moves at a
-// time (an element, or 16 bytes of them; ldh and width are counted in it).
+// time (an element, or 16 bytes of them; ldh and width are counted in it).  tile_group null (a plan of xr_moe_plan_tiles): rows of
+// padding are left as they are, nobody reads what they come to.
 // ---------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(256)
@@ -216,10 +278,11 @@ k_moe_gather(const T* __restrict__ h, long long ldh, T* __restrict__ out, const 
     xr_pdl_launch();
     xr_pdl_wait();
     const int r = blockIdx.x;
-    if (tile_group[r / align] < 0) return;
+    if (tile_group != nullptr && tile_group[r / align] < 0) return;
     const int src = row_src[r];
     T* o = out + (size_t)r * width;
     if (src < 0) {
+        if (tile_group == nullptr) return;
         for (int i = threadIdx.x; i < width; i += blockDim.x) o[i] = T{};
         return;
     }

@@ -94,6 +94,9 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_moe_plan": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
         "xr_moe_gather": [_vp, _i, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
         "xr_gemm_tc_grouped": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _i, _vp, _i, _vp, _vp],
+        "xr_gemm_tc_pairs_available": [],
+        "xr_gemm_tc_grouped_pairs": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _vp, _i, _i, _vp, _vp],
+        "xr_moe_plan_tiles": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
         "xr_moe_tile_rows": [],
         "xr_moe_gemm": [_vp, _i, _ll, _vp, _i, _vp, _i, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp],
         "xr_route_groups": [_vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _f, _vp],
@@ -1055,12 +1058,54 @@ def moe_plan(ids: torch.Tensor, row_src, pair_row, tile_group, E: int, align: in
     _count()
 
 
-def moe_gather(h: torch.Tensor, out: torch.Tensor, row_src, tile_group, top: int, align: int) -> None:
-    """out[r] = h[row_src[r] // top] for the rows of the plan's tiles (zeros for rows of padding)."""
+PAIR_TILE = 256       # rows a tile of the grouped product on CTA pairs holds at most
+
+
+def pairs_available() -> bool:
+    """Whether the device runs the product on pairs of CTAs."""
+    return lib().xr_gemm_tc_pairs_available() == 1
+
+
+def moe_tiles_room(pairs: int, E: int):
+    """(tiles, rows) that a plan of ``moe_plan_tiles`` over `pairs` rows and E experts can need at most."""
+    return pairs // PAIR_TILE + E, pairs + 15 * E
+
+
+def moe_plan_tiles(ids: torch.Tensor, row_src, pair_row, tiles, E: int) -> None:
+    """Like ``moe_plan``, for ``gemm_tc_grouped_pairs``: row_src [rows] and tiles [1 + 3 tiles] of the sizes ``moe_tiles_room`` gives;
+    tiles = the number of tiles, then (expert, first row, rows) of each; see k_moe_plan_tiles in csrc/moe.cu."""
+    _dev(ids, row_src, pair_row, tiles)
+    pairs = ids.numel()
+    max_tiles, max_rows = moe_tiles_room(pairs, E)
+    assert row_src.numel() >= max_rows and pair_row.numel() >= pairs and tiles.numel() >= 1 + 3 * max_tiles
+    _check(lib().xr_moe_plan_tiles(ids.data_ptr(), row_src.data_ptr(), pair_row.data_ptr(), tiles.data_ptr(), pairs, E, PAIR_TILE,
+                                   max_tiles, max_rows, _stream()), "moe_plan_tiles")
+    _count()
+
+
+def gemm_tc_grouped_pairs(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, tiles: torch.Tensor, max_tiles: int, n_out: int,
+                          epilogue: int = EPI_STORE, act: int = ACT_NONE, act_limit: float = 0.0) -> None:
+    """``gemm_tc_grouped`` on pairs of CTAs, over the tiles of ``moe_plan_tiles`` (rows of x that belong to no tile are left out)."""
+    _dev(x, w_packed, out, tiles)
+    n, k = x.shape
+    assert x.dtype == torch.bfloat16 and w_packed.dtype == torch.bfloat16 and w_packed.dim() == 5
+    row_tiles = -(-n_out // GATED_FEATURES) if epilogue == EPI_GATED else -(-n_out // TILE_ROWS)
+    assert w_packed.shape[1] == row_tiles and w_packed.shape[2] == -(-k // TILE_K) and out.shape == (n, n_out)
+    assert tiles.dtype == torch.int32 and tiles.numel() >= 1 + 3 * max_tiles
+    ws = workspace(x.device)
+    _check(lib().xr_gemm_tc_grouped_pairs(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
+                                          float(act_limit), n, n_out, k, x.stride(0), out.stride(0), tiles.data_ptr(), max_tiles,
+                                          w_packed.shape[0], ws.status_ptr, _stream()), "gemm_tc_grouped_pairs")
+    _count()
+
+
+def moe_gather(h: torch.Tensor, out: torch.Tensor, row_src, tile_group: Optional[torch.Tensor], top: int, align: int = 1) -> None:
+    """out[r] = h[row_src[r] // top] for the rows of the plan's tiles (zeros for rows of padding; with `tile_group` None, a plan of
+    ``moe_plan_tiles``, those stay as they are)."""
     _dev(out, row_src, tile_group)
     assert h.stride(1) == 1 and out.shape[1] == h.shape[1] and out.dtype == h.dtype and out.shape[0] % align == 0
     _check(lib().xr_moe_gather(h.data_ptr(), dtype_code(h.dtype), h.stride(0), out.data_ptr(), row_src.data_ptr(),
-                               tile_group.data_ptr(), top, h.shape[1], align, out.shape[0], _stream()), "moe_gather")
+                               _ptr(tile_group), top, h.shape[1], align, out.shape[0], _stream()), "moe_gather")
     _count()
 
 

@@ -218,10 +218,11 @@ FAMILIES = {
     "finish_plain": "products (tcgen05)", "finish_add_rmsnorm": "norms", "rmsnorm": "norms", "finish_rope_store": "rotation + cache store",
     "rope_store": "rotation + cache store", "attention_tc": "attention", "attention_mma": "attention", "attention_simt": "attention",
     "latent_prep": "rotation + cache store", "head_matmul": "latent attention: per-head products", "latent_attention": "latent attention: scores and sums",
-    "latent_attention_mma": "latent attention: scores and sums", "gemm_tc_grouped": "grouped products (experts, per-head)",
+    "latent_attention_mma": "latent attention: scores and sums", "gemm_tc_grouped": "grouped products (experts, per-head)", "gemm_tc_grouped_pairs": "grouped products (experts, per-head)",
+    "flat_rows": "latent attention: per-head products", "attention_tc_flat": "latent attention: scores and sums",
     "moe_gather": "grouped products (experts, per-head)", "heads_gather": "grouped products (experts, per-head)",
     "heads_scatter_gate": "grouped products (experts, per-head)",
-    "mlstm": "mlstm recurrence", "route_topk": "routing", "moe_plan": "routing", "moe_gemm": "experts' products", "moe_combine": "experts' sum",
+    "mlstm": "mlstm recurrence", "route_topk": "routing", "moe_plan": "routing", "moe_plan_tiles": "routing", "moe_gemm": "experts' products", "moe_combine": "experts' sum",
     "delta": "delta recurrence", "head_norm_gate": "gated norm of the recurrence", "qk_norm_rope_store": "rotation + cache store",
     "rmsnorm_act": "norms", "ssd": "state-space recurrence", "silu_gate_norm": "gated norm of the recurrence", "route_groups": "routing",
     "sigmoid_gate": "output gates", "stream_step": "stream kernels",

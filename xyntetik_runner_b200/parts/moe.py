@@ -31,6 +31,13 @@ from . import linear_tc
 from .linear import Linear
 
 
+# A plan of more rows an expert than this (on average) goes to the product on CTA pairs, whose tiles hold what an expert has (up to
+# 256 rows).  Both products of an expert, microseconds, padded tiles of one CTA against pairs: 64 experts of 1,408 at width 2,048:
+# 19 rows 200 / 193, 38 rows 238 / 197, 73 rows 367 / 229, 192 rows 660 / 284; 16 of 1,408 at width 1,024: 25 rows 35 / 38,
+# 50 rows 41 / 39, 97 rows 66 / 48.
+PAIRS_FROM = 32
+
+
 class PendingExperts:
     """The weighted sum of a step's expert outputs (and of the shared expert's), still to be added into x: by ``finish``, or by the
     norm that follows, in one pass with it."""
@@ -150,29 +157,45 @@ class RoutedExperts(FeedForward):
     def forward(self, ctx, h, x):
         n, top, E = h.shape[0], self.top, self.E
         pairs = n * top
+        on_pairs = self.tensor_cores and pairs > PAIRS_FROM * E and kernels.pairs_available()
         zs = ctx.buf("moe_logits", (n, self.router.n_out), torch.float32)
+        wts = ctx.buf("moe_weights", (n, top), torch.float32)
         self.router.forward(h, zs)
         z = zs if self.router.n_out == self.outputs else zs[:, :self.outputs]        # (a shared expert's gate is one column more)
         ids = ctx.buf("moe_ids", (n, top), torch.int32)
-        wts = ctx.buf("moe_weights", (n, top), torch.float32)
         if self.softmax_all:
             kernels.route_groups(z, ids, wts, top, self.correction, *self.groups, self.scale)
         elif self.sigmoid:
             kernels.route_topk(z, ids, wts, top, sigmoid_scores=True, correction=self.correction)
         else:
             kernels.route_topk(z, ids, wts, top)
-        align = self._row_tile(pairs, E) if self.tensor_cores else kernels.moe_tile_rows()
-        max_tiles = kernels.moe_max_tiles(pairs, E, align)
-        rows = max_tiles * align
-        row_src = ctx.buf("moe_row_src", (rows,), torch.int32)
+        align = 1 if on_pairs else (self._row_tile(pairs, E) if self.tensor_cores else kernels.moe_tile_rows())
+        if on_pairs:
+            max_tiles, rows = kernels.moe_tiles_room(pairs, E)
+        else:
+            max_tiles = kernels.moe_max_tiles(pairs, E, align)
+            rows = max_tiles * align
         pair_row = ctx.buf("moe_pair_row", (pairs,), torch.int32)
-        tile_group = ctx.buf("moe_tile_group", (max_tiles,), torch.int32)
-        kernels.moe_plan(ids, row_src, pair_row, tile_group, E, align)
-        y = ctx.buf("moe_act", (rows, self.inner), ctx.act_dtype)
-        zz = ctx.buf("moe_out", (rows, self.width), torch.float32)
+        if not on_pairs:
+            tile_group = ctx.buf("moe_tile_group", (max_tiles,), torch.int32)
         if self.tensor_cores:
             xs = ctx.buf("moe_rows", (rows, self.width), ctx.act_dtype)
-            kernels.moe_gather(h, xs, row_src, tile_group, top, align)
+        row_src = ctx.buf("moe_row_src", (rows,), torch.int32)
+        if on_pairs:
+            tiles = ctx.buf("moe_tiles", (1 + 3 * max_tiles,), torch.int32)
+            kernels.moe_plan_tiles(ids, row_src, pair_row, tiles, E)
+            kernels.moe_gather(h, xs, row_src, None, top)
+        else:
+            kernels.moe_plan(ids, row_src, pair_row, tile_group, E, align)
+            if self.tensor_cores:
+                kernels.moe_gather(h, xs, row_src, tile_group, top, align)
+        y = ctx.buf("moe_act", (rows, self.inner), ctx.act_dtype)
+        zz = ctx.buf("moe_out", (rows, self.width), torch.float32)
+        if on_pairs:
+            kernels.gemm_tc_grouped_pairs(xs, self.w_gate_up, y, tiles, max_tiles, self.inner, kernels.EPI_GATED if self.gated else kernels.EPI_STORE,
+                                          self.act, self.limit)
+            kernels.gemm_tc_grouped_pairs(y, self.w_down, zz, tiles, max_tiles, self.width)
+        elif self.tensor_cores:
             kernels.gemm_tc_grouped(xs, self.w_gate_up, y, tile_group, align, self.inner, kernels.EPI_GATED if self.gated else kernels.EPI_STORE,
                                     self.act, self.limit)
             kernels.gemm_tc_grouped(y, self.w_down, zz, tile_group, align, self.width)
