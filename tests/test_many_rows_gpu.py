@@ -11,6 +11,25 @@ def _i32(v):
     return torch.tensor(v, dtype=torch.int32, device=DEV)
 
 
+# ---- float32 products ------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n,n_out,k,wdt", [(1, 33, 7, torch.float32), (8, 100, 260, torch.bfloat16), (9, 65, 64, torch.bfloat16), (40, 3001, 36, torch.float32),
+                                           (300, 2001, 40, torch.bfloat16), (301, 8001, 33, torch.float32), (700, 13001, 36, torch.float32)])
+def test_float32_product_in_every_tile(n, n_out, k, wdt):
+    """Few tokens, few tiles, many of every size; K off and on the copies' border.  A float32 sum of k products
+    is off by at most k 2^-24 times the sum of their sizes; and a row is the same whatever stands beside it."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn(n, k, generator=g), torch.randn(n_out, k, generator=g).to(wdt)
+    out = torch.empty(n, n_out, device=DEV)
+    kernels.gemm_simt(x.to(DEV), w.to(DEV), out)
+    bound = (x.double().abs() @ w.double().abs().T) * (k + 2) * 2.0 ** -24
+    assert ((out.cpu().double() - x.double() @ w.double().T).abs() <= bound).all()
+    for t in {0, n // 2, n - 1}:
+        one = torch.empty(1, n_out, device=DEV)
+        kernels.gemm_simt(x[t:t + 1].to(DEV), w.to(DEV), one)
+        assert torch.equal(one[0], out[t])
+
+
 # ---- float32 attention -----------------------------------------------------------------------------------------------
 @pytest.mark.parametrize("H,K,hd,page,extra", [(8, 2, 128, 16, ""), (4, 4, 64, 8, "sink"), (16, 1, 64, 64, "cap"), (6, 3, 256, 32, "bias"), (4, 1, 128, 64, "short")])
 def test_float32_attention_of_packed_rows_gives_the_same_bits(H, K, hd, page, extra):
@@ -40,6 +59,58 @@ def test_float32_attention_of_packed_rows_gives_the_same_bits(H, K, hd, page, ex
                                0, hd ** -0.5, portions=portions, **opt)
         outs.append(out)
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+
+
+# ---- grouped products on CTA pairs -----------------------------------------------------------------------------------
+@pytest.mark.parametrize("counts,width,inner,gated", [([1, 0, 32, 33, 256, 257, 15], 72, 200, True), ([300, 513], 128, 136, False), ([0, 0, 5], 64, 64, True),
+                                                      ([700], 136, 264, False)])
+def test_grouped_products_on_pairs(counts, width, inner, gated):
+    """Experts that nobody chose, that got one row, a whole tile, a row more; row tiles in odd number; the plan's table, and both
+    products against float64 over the rounded operands: a bfloat16 result of a float32 sum is off by 2^-8 of itself and K 2^-24 of
+    the sum of the products' sizes."""
+    from xyntetik_runner_b200 import kernels
+    if not kernels.pairs_available():
+        pytest.skip("no pairs of CTAs on this device")
+    g = torch.Generator().manual_seed(sum(counts))
+    E, pairs = len(counts), sum(counts)
+    ids = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])[torch.randperm(pairs, generator=g)].int().view(pairs, 1).to(DEV)
+    h = torch.randn(pairs, width, generator=g).bfloat16()
+    first = (torch.randn(E, (2 if gated else 1) * inner, width, generator=g) * width ** -0.5).bfloat16()
+    second = (torch.randn(E, width, inner, generator=g) * inner ** -0.5).bfloat16()
+    max_tiles, rows = kernels.moe_tiles_room(pairs, E)
+    row_src, pair_row = torch.empty(rows, dtype=torch.int32, device=DEV), torch.empty(pairs, dtype=torch.int32, device=DEV)
+    tiles = torch.full((1 + 3 * max_tiles,), -7, dtype=torch.int32, device=DEV)
+    kernels.moe_plan_tiles(ids, row_src, pair_row, tiles, E)
+    table = tiles[1:1 + 3 * int(tiles[0])].view(-1, 3).cpu().tolist()
+    seen = {}
+    for e, at, n in table:
+        assert 1 <= n <= kernels.PAIR_TILE and at >= 0 and at + n <= rows
+        for r in range(at, at + n):
+            assert r not in seen
+            seen[r] = e
+    assert sorted(seen) == sorted(pair_row.tolist()) and len(table) == sum(-(-c // kernels.PAIR_TILE) for c in counts)
+    assert all(seen[r] == int(e) for r, e in zip(pair_row.tolist(), ids[:, 0].tolist()))
+    assert row_src[pair_row.long()].tolist() == list(range(pairs)) and int((row_src >= 0).sum()) == pairs
+    xs = torch.full((rows, width), float("nan"), dtype=torch.bfloat16, device=DEV)
+    kernels.moe_gather(h.to(DEV), xs, row_src, None, 1)
+    y = torch.full((rows, inner), float("nan"), dtype=torch.bfloat16, device=DEV)
+    act = kernels.ACT_SILU if gated else kernels.ACT_RELU2
+    kernels.gemm_tc_grouped_pairs(xs, kernels.pack_weight_groups(first.to(DEV), 2 if gated else 1), y, tiles, max_tiles, inner,
+                                  kernels.EPI_GATED if gated else kernels.EPI_STORE, act)
+    zz = torch.full((rows, width), float("nan"), device=DEV)
+    kernels.gemm_tc_grouped_pairs(y, kernels.pack_weight_groups(second.to(DEV)), zz, tiles, max_tiles, width)
+    kernels.tc_check_status(torch.device(DEV))
+    got_y, got = y[pair_row.long()].cpu().double(), zz[pair_row.long()].cpu().double()
+    for e in range(E):
+        mine = (ids[:, 0] == e).cpu()
+        w = first[e].double()
+        a = h[mine].double()
+        z = a @ w.T
+        want = torch.nn.functional.silu(z[:, :inner]) * z[:, inner:] if gated else torch.relu(z) ** 2
+        # (the sums' own error, width 2^-24 of sums of a few units, is far below the rounding; the hardware's exponential is good to 2^-21)
+        assert ((got_y[mine] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+        b, v = got_y[mine], second[e].double()
+        assert ((got[mine] - b @ v.T).abs() <= (inner + 2) * 2.0 ** -24 * (b.abs() @ v.abs().T) + 1e-12).all()
 
 
 # ---- attention over expanded keys ------------------------------------------------------------------------------------
@@ -115,55 +186,3 @@ def test_attention_over_expanded_keys(H, D, R, V, page, window, gate):
             # probabilities are rounded to bfloat16 (2^-9 of each, weights that sum to one) and the result once more
             top = k[:, H * D + h * V:H * D + (h + 1) * V].abs().max()
             assert ((got[starts[s]:starts[s] + m, h * V:(h + 1) * V] - o).abs() <= 2.0 ** -8 * o.abs() + 2.0 ** -8 * top).all(), (s, h)
-
-
-# ---- grouped products on CTA pairs -----------------------------------------------------------------------------------
-@pytest.mark.parametrize("counts,width,inner,gated", [([1, 0, 32, 33, 256, 257, 15], 72, 200, True), ([300, 513], 128, 136, False), ([0, 0, 5], 64, 64, True),
-                                                      ([700], 136, 264, False)])
-def test_grouped_products_on_pairs(counts, width, inner, gated):
-    """Experts that nobody chose, that got one row, a whole tile, a row more; row tiles in odd number; the plan's table, and both
-    products against float64 over the rounded operands: a bfloat16 result of a float32 sum is off by 2^-8 of itself and K 2^-24 of
-    the sum of the products' sizes."""
-    from xyntetik_runner_b200 import kernels
-    if not kernels.pairs_available():
-        pytest.skip("no pairs of CTAs on this device")
-    g = torch.Generator().manual_seed(sum(counts))
-    E, pairs = len(counts), sum(counts)
-    ids = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)])[torch.randperm(pairs, generator=g)].int().view(pairs, 1).to(DEV)
-    h = torch.randn(pairs, width, generator=g).bfloat16()
-    first = (torch.randn(E, (2 if gated else 1) * inner, width, generator=g) * width ** -0.5).bfloat16()
-    second = (torch.randn(E, width, inner, generator=g) * inner ** -0.5).bfloat16()
-    max_tiles, rows = kernels.moe_tiles_room(pairs, E)
-    row_src, pair_row = torch.empty(rows, dtype=torch.int32, device=DEV), torch.empty(pairs, dtype=torch.int32, device=DEV)
-    tiles = torch.full((1 + 3 * max_tiles,), -7, dtype=torch.int32, device=DEV)
-    kernels.moe_plan_tiles(ids, row_src, pair_row, tiles, E)
-    table = tiles[1:1 + 3 * int(tiles[0])].view(-1, 3).cpu().tolist()
-    seen = {}
-    for e, at, n in table:
-        assert 1 <= n <= kernels.PAIR_TILE and at >= 0 and at + n <= rows
-        for r in range(at, at + n):
-            assert r not in seen
-            seen[r] = e
-    assert sorted(seen) == sorted(pair_row.tolist()) and len(table) == sum(-(-c // kernels.PAIR_TILE) for c in counts)
-    assert all(seen[r] == int(e) for r, e in zip(pair_row.tolist(), ids[:, 0].tolist()))
-    assert row_src[pair_row.long()].tolist() == list(range(pairs)) and int((row_src >= 0).sum()) == pairs
-    xs = torch.full((rows, width), float("nan"), dtype=torch.bfloat16, device=DEV)
-    kernels.moe_gather(h.to(DEV), xs, row_src, None, 1)
-    y = torch.full((rows, inner), float("nan"), dtype=torch.bfloat16, device=DEV)
-    act = kernels.ACT_SILU if gated else kernels.ACT_RELU2
-    kernels.gemm_tc_grouped_pairs(xs, kernels.pack_weight_groups(first.to(DEV), 2 if gated else 1), y, tiles, max_tiles, inner,
-                                  kernels.EPI_GATED if gated else kernels.EPI_STORE, act)
-    zz = torch.full((rows, width), float("nan"), device=DEV)
-    kernels.gemm_tc_grouped_pairs(y, kernels.pack_weight_groups(second.to(DEV)), zz, tiles, max_tiles, width)
-    kernels.tc_check_status(torch.device(DEV))
-    got_y, got = y[pair_row.long()].cpu().double(), zz[pair_row.long()].cpu().double()
-    for e in range(E):
-        mine = (ids[:, 0] == e).cpu()
-        w = first[e].double()
-        a = h[mine].double()
-        z = a @ w.T
-        want = torch.nn.functional.silu(z[:, :inner]) * z[:, inner:] if gated else torch.relu(z) ** 2
-        # (the sums' own error, width 2^-24 of sums of a few units, is far below the rounding; the hardware's exponential is good to 2^-21)
-        assert ((got_y[mine] - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
-        b, v = got_y[mine], second[e].double()
-        assert ((got[mine] - b @ v.T).abs() <= (inner + 2) * 2.0 ** -24 * (b.abs() @ v.abs().T) + 1e-12).all()

@@ -298,7 +298,8 @@ XR_EXPORT int xr_attention_simt(const void* q, void* out, int dtype, const void*
     AttnArgs a{q, out, cache_k, positions, tok_seg, block_tables, page_stride, v_offset, q_row_stride,
                n, H, K, hd, max_pages, page_size, window, scale, sink, softcap, window > 0 ? keep_first : 0, {bias, bias_len}};
     // Many tokens a request: the rows of 16 / G tokens share their keys.  A step of single tokens has nothing to share, and a window
-    // starts every row's chunks elsewhere.  (The copies and stores are 16 bytes wide.)
+    // starts every row's chunks elsewhere.  (The copies and stores are 16 bytes wide.)  8 tokens of one request, 8 heads on 2, 128
+    // columns, a warp a row against this: 11 / 9 us, behind 1,000 keys 590 / 111, behind 4,000 2,340 / 418.
     const int G = H / K;
     const bool even = !(((uintptr_t)out | (uintptr_t)cache_k) & 15) && !((page_stride | v_offset) & 3);
     if (dtype == XR_F32 && portions > 0 && n >= 8 * portions && window == 0 && G <= AT_ROWS && AT_ROWS % G == 0 && even && K <= 65535) {

@@ -7,84 +7,92 @@
 // (the property the reference demands of its batched kernels,
 // src/kernels.cu:2415-2454).  The reference's counterparts are the warp-per-row
 // kernels `k_mv_*` / `k_mv_*_b` (src/kernels.cu:116-144, 534-549).
-#include "common.cuh"
+#include "simt_tile.cuh"
 
-#define GS_BM 64
-#define GS_BN 64
-#define GS_BK 16
-
-template <typename TX, typename TW, typename TO, bool ACCUM>
-__global__ void __launch_bounds__(256)
+// What bounds it: the FMA pipes (70 TFLOP/s measured) where there are enough tiles, else the chain of copies and of K dependent
+// multiply-adds, which is why a product with few tiles takes small ones: see launch_simt.  Earlier form (one 64 x 64 tile, blocks of
+// 16, no ring) against this, bfloat16 W, us: 256 tokens x 1,024 rows of 1,024: 70 / 29; 256 x 5,632 x 1,024: 156 / 91; 256 x 1,024 x 2,816:
+// 185 / 71; 2,048 x 5,632 x 1,024: 970 / 577 (41 TFLOP/s); 1 x 1,024 x 2,816: 160 / 35.
+template <typename TX, typename TW, typename TO, bool ACCUM, int WM, int WN, int TM, int TN>
+__global__ void __launch_bounds__(32 * WM * WN)
 k_gemm_simt(const TX* __restrict__ X, const TW* __restrict__ W, const float* __restrict__ bias,
-            TO* __restrict__ out, int n, int n_out, int K, long long ldx, long long ldo, float alpha) {
-    __shared__ float Xs[GS_BK][GS_BM + 4];
-    __shared__ float Ws[GS_BK][GS_BN + 4];
-    int tid = threadIdx.x;
-    int t0 = blockIdx.y * GS_BM, r0 = blockIdx.x * GS_BN;
-    int ty = tid / 16, tx = tid % 16;
-    float acc[4][4];
+            TO* __restrict__ out, int n, int n_out, int K, long long ldx, long long ldo, float alpha, int vec) {
+    constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN;
+    extern __shared__ __align__(16) unsigned char gs_sm[];
+    const int t0 = blockIdx.y * BM, r0 = blockIdx.x * BN;
+    float acc[TM][TN];
+    gs_tile<TX, TW, WM, WN, TM, TN>(
+        gs_sm, K, vec, [&](int i) { return t0 + i < n ? X + (size_t)(t0 + i) * ldx : (const TX*)nullptr; },
+        [&](int i) { return r0 + i < n_out ? W + (size_t)(r0 + i) * K : (const TW*)nullptr; }, acc);
+    const int tm = gs_token<WN, TM>(), rn = gs_row<WN, TN>();
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-
-    int lrow = tid / 4, lk = (tid % 4) * 4;
-    for (int k0 = 0; k0 < K; k0 += GS_BK) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            int k = k0 + lk + q;
-            int t = t0 + lrow, r = r0 + lrow;
-            Xs[lk + q][lrow] = (t < n && k < K) ? xr_to_f32<TX>(X[(size_t)t * ldx + k]) : 0.f;
-            Ws[lk + q][lrow] = (r < n_out && k < K) ? xr_to_f32<TW>(W[(size_t)r * K + k]) : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GS_BK; kk++) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) a[i] = Xs[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; j++) b[j] = Ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int t = t0 + ty * 4 + i;
+    for (int i = 0; i < TM; i++) {
+        const int t = t0 + tm + 4 * i;
         if (t >= n) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int r = r0 + tx * 4 + j;
+        for (int j = 0; j < TN; j++) {
+            const int r = r0 + rn + 8 * j;
             if (r >= n_out) continue;
             float v = alpha * acc[i][j];
             if (bias) v += bias[r];
-            size_t o = (size_t)t * ldo + r;
+            const size_t o = (size_t)t * ldo + r;
             if (ACCUM) out[o] = xr_from_f32<TO>(xr_to_f32<TO>(out[o]) + v);
             else out[o] = xr_from_f32<TO>(v);
         }
     }
 }
 
+template <typename TX, typename TW, typename TO, bool ACCUM, int WM, int WN, int TM, int TN>
+static int launch_simt_tile(const void* X, const void* W, const float* bias, void* out, int n, int n_out, int K, long long ldx, long long ldo,
+                            float alpha, cudaStream_t stream) {
+    constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN;
+    constexpr size_t SMEM = gs_smem<TX, TW, BM, BN>();
+    const dim3 grid((n_out + BN - 1) / BN, (n + BM - 1) / BM);
+    if (grid.y > 65535) return XR_ERR_ARG;
+    static const bool ready = SMEM <= 48 * 1024 || cudaFuncSetAttribute(k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN>,
+                                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess;
+    if (!ready) return XR_ERR_LAUNCH;
+    constexpr int PX = 16 / (int)sizeof(TX), PW = 16 / (int)sizeof(TW);
+    const int vec = !(((uintptr_t)X | (uintptr_t)W) & 15) && ldx % PX == 0 && K % PX == 0 && K % PW == 0;
+    k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN><<<grid, 32 * WM * WN, SMEM, stream>>>((const TX*)X, (const TW*)W, bias, (TO*)out, n, n_out, K, ldx, ldo, alpha, vec);
+    return xr_launch_status();
+}
+
+// Which tile: every element's arithmetic is the same in all of them.  The widest of which there are enough to keep the machine busy:
+// wide ones read fewer words a multiply-add from shared memory, narrow ones spread a small product over more SMs.  Measured, us, tiles
+// 8x32 / 32x32 / 32x64 / 64x64 / 128x128: 44 x 1,024 x 1,024: 17 21 29 43 114; 256 x 1,024 x 1,024: 35 29 29 45 115; 256 x 5,632 x 1,024:
+// 163 103 91 98 117; 256 x 32,000 x 1,024: 881 535 464 433 451; 2,048 x 5,632 x 1,024: 1,235 745 642 613 577.
+template <typename TX, typename TW, typename TO, bool ACCUM>
+static int launch_simt_out(const void* X, const void* W, const float* bias, void* out, int n, int n_out, int K, long long ldx, long long ldo,
+                           float alpha, cudaStream_t stream) {
+#define GS(WM, WN, TM, TN) return launch_simt_tile<TX, TW, TO, ACCUM, WM, WN, TM, TN>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, stream)
+    const long long sms = xr_sm_count();
+    auto tiles = [&](int bm, int bn) { return (long long)((n + bm - 1) / bm) * ((n_out + bn - 1) / bn); };
+    int pick;
+    if (n <= 8 || tiles(32, 32) < sms) pick = 0;
+    else if (tiles(128, 128) >= 4 * sms) pick = 4;
+    else if (tiles(64, 64) >= 4 * sms) pick = 3;
+    else pick = tiles(32, 64) >= 2 * sms ? 2 : 1;
+    switch (pick) {
+        case 0: GS(1, 4, 2, 1);            // 8 tokens x 32 rows
+        case 1: GS(2, 2, 4, 2);            // 32 x 32
+        case 2: GS(2, 2, 4, 4);            // 32 x 64
+        case 3: GS(2, 2, 8, 4);            // 64 x 64
+        default: GS(4, 2, 8, 8);           // 128 x 128
+    }
+#undef GS
+}
+
 template <typename TX, typename TW>
 static int launch_simt(const void* X, const void* W, const float* bias, void* out, int out_dtype, int accumulate,
                        int n, int n_out, int K, long long ldx, long long ldo, float alpha, cudaStream_t stream) {
-    dim3 grid((n_out + GS_BN - 1) / GS_BN, (n + GS_BM - 1) / GS_BM);
-    if (grid.y > 65535) return XR_ERR_ARG;
     if (accumulate) {
         if (out_dtype != XR_F32) return XR_ERR_ARG;
-        k_gemm_simt<TX, TW, float, true><<<grid, 256, 0, stream>>>((const TX*)X, (const TW*)W, bias, (float*)out, n, n_out, K, ldx, ldo, alpha);
-    } else if (out_dtype == XR_F32) {
-        k_gemm_simt<TX, TW, float, false><<<grid, 256, 0, stream>>>((const TX*)X, (const TW*)W, bias, (float*)out, n, n_out, K, ldx, ldo, alpha);
-    } else if (out_dtype == XR_BF16) {
-        k_gemm_simt<TX, TW, __nv_bfloat16, false><<<grid, 256, 0, stream>>>((const TX*)X, (const TW*)W, bias, (__nv_bfloat16*)out, n, n_out, K, ldx, ldo, alpha);
-    } else {
-        return XR_ERR_ARG;
+        return launch_simt_out<TX, TW, float, true>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, stream);
     }
-    return xr_launch_status();
+    if (out_dtype == XR_F32) return launch_simt_out<TX, TW, float, false>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, stream);
+    if (out_dtype == XR_BF16) return launch_simt_out<TX, TW, __nv_bfloat16, false>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, stream);
+    return XR_ERR_ARG;
 }
 
 // X: [n, K] with row stride ldx; W: [n_out, K] dense; out: [n, n_out] with row stride ldo.
