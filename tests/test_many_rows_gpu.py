@@ -186,3 +186,62 @@ def test_attention_over_expanded_keys(H, D, R, V, page, window, gate):
             # probabilities are rounded to bfloat16 (2^-9 of each, weights that sum to one) and the result once more
             top = k[:, H * D + h * V:H * D + (h + 1) * V].abs().max()
             assert ((got[starts[s]:starts[s] + m, h * V:(h + 1) * V] - o).abs() <= 2.0 ** -8 * o.abs() + 2.0 ** -8 * top).all(), (s, h)
+
+
+# ---- the gated linear recurrence of long portions --------------------------------------------------------------------
+@pytest.mark.parametrize("R,B,taps,lens,dtype", [(48, 2, 4, [70, 1, 33], torch.bfloat16), (33, 3, 1, [65], torch.bfloat16),
+                                                 (256, 1, 3, [31, 320], torch.float32), (1280, 5, 4, [300, 257], torch.bfloat16)])
+def test_gated_recurrence_of_long_portions(R, B, taps, lens, dtype):
+    """Portions of fewer tokens than segments, of a token more, of many; the products in each of their tiles; two launches, the second
+    from the state the first left.  Decays near one over 300 steps: the float32 walk's error grows with the steps it sums over."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(R)
+    Bs = R // B
+    f = lambda *s: torch.randn(*s, generator=g)
+    conv, cb, wa, wi, ba, bi, lam = f(R, taps), f(R), f(B, Bs, Bs) / Bs ** 0.5, f(B, Bs, Bs) / Bs ** 0.5, f(R), f(R), -4.0 + f(R)
+    rows = [f(n, 2 * R) for n in lens]
+
+    def plain(x):
+        x = x.double()
+        u = cb.double().expand(len(x), R).clone()
+        for j in range(taps):
+            u[j:] += conv[:, taps - 1 - j].double() * x[:len(x) - j, R:]
+        ub = u.view(len(x), B, Bs)
+        r = torch.sigmoid(torch.einsum("boi,tbi->tbo", wa.double(), ub).reshape(len(x), R) + ba)
+        i = torch.sigmoid(torch.einsum("boi,tbi->tbo", wi.double(), ub).reshape(len(x), R) + bi)
+        log_a = -8.0 * r * torch.nn.functional.softplus(lam.double())
+        inp = torch.sqrt(-torch.expm1(2 * log_a)) * i * u
+        S, out = torch.zeros(R, dtype=torch.float64), []
+        for t in range(len(x)):
+            S = torch.exp(log_a[t]) * S + inp[t]
+            out.append(S)
+        return torch.stack(out) * torch.nn.functional.gelu(x[:, :R], approximate="tanh"), S
+
+    state = torch.zeros(len(lens) + 1, kernels.rglru_state_floats(R, taps), device=DEV)
+    slots = list(range(len(lens), 0, -1))
+    cut = [max(1, n // 3) for n in lens]
+    got = [[] for _ in lens]
+    for part in range(2):
+        xs = [r[:c] if part == 0 else r[c:] for r, c in zip(rows, cut)]
+        use = [s for s, x in enumerate(xs) if len(x)]
+        x = torch.cat([xs[s] for s in use]).to(DEV)
+        ln = [len(xs[s]) for s in use]
+        st = [sum(ln[:i]) for i in range(len(ln))]
+        n = len(x)
+        a, b, u = (torch.empty(n, R, device=DEV) for _ in range(3))
+        out = torch.empty(n, R, dtype=dtype, device=DEV)
+        kernels.rglru(x, conv.to(DEV), cb.to(DEV), None, None, wa.to(DEV), wi.to(DEV), ba.to(DEV), bi.to(DEV), lam.to(DEV), state,
+                      _i32([i for i, m in enumerate(ln) for _ in range(m)]), _i32(st), _i32(ln), _i32([slots[s] for s in use]), a, b, u, out, len(ln), R, B,
+                      taps, 8.0)
+        for i, s in enumerate(use):
+            got[s].append(out[st[i]:st[i] + ln[i]].cpu().double())
+    assert state[0].abs().sum() == 0
+    for s, r in enumerate(rows):
+        want, end = plain(r)
+        assert torch.allclose(torch.cat(got[s]), want, rtol=5e-5 + (2.0 ** -8 if dtype == torch.bfloat16 else 0.0), atol=1e-5)
+        assert torch.allclose(state[slots[s], :R].cpu().double(), end, rtol=5e-5, atol=1e-5)
+        tail = torch.zeros(taps - 1, R)
+        keep = min(taps - 1, len(r))
+        if keep:
+            tail[taps - 1 - keep:] = r[len(r) - keep:, R:]
+        assert torch.equal(state[slots[s], R:].cpu().view(taps - 1, R), tail)

@@ -7,9 +7,9 @@
 //       a   = exp(-c r softplus(lam)),  S <- a S + sqrt(1 - a^2) (i u)  c a constant of the design (an argument)
 //       out = S * gelu_tanh(y')
 //     State per slot: S [R], then the last taps - 1 rows x' [taps-1][R].
-//     k_rglru_gates, a block per (tile of tokens, channel block): convolution into shared memory, then both gate products
-//     with one output channel a thread (the matrices are given transposed, [b][in][out], so that a warp reads a row), then
-//     a, the recurrence's input and the gated branch's activation.  k_rglru_scan, a thread a channel: the walk over a
+//     k_rglru_conv, a thread an element: the convolution u.  k_rglru_gates, a block per tile of tokens and outputs of a channel block
+//     (k_rglru_gates_few: a warp an output, for few tokens): both gate products, then a, the recurrence's input and the gated branch's
+//     activation.  k_rglru_scan, a thread a channel (k_rglru_scan_segments: a warp a segment of the portion): the walk over a
 //     portion's tokens, the read-out times the gated branch, and the slot's new tail.
 //
 // (2) Linear attention with a constant decay per head ("lightning attention"): S [D][V] per head,
@@ -26,8 +26,9 @@
 //     S [H][V][N], then the last taps - 1 inputs of the convolution [taps-1][H V + 2 G N].
 //
 // Everything here is float32 in both precisions, and the walks go token by token: the state after a token does not depend
-// on how the tokens were cut into steps, bit for bit.
-#include "common.cuh"
+// on how the tokens were cut into steps, bit for bit.  (Not so where a portion of many tokens of a bfloat16 model is cut into segments
+// or chunks: k_rglru_scan_segments, chunked.cuh; there the last bits depend on the cuts.)
+#include "simt_tile.cuh"
 #include "conv_tail.cuh"
 #include <math.h>
 
@@ -44,28 +45,6 @@ __device__ __forceinline__ float rc_softplus(float z) { return z > 30.0f ? z : l
 __device__ __forceinline__ float rc_silu(float z) { return z < -80.0f ? 0.0f : z / (1.0f + expf(-z)); }
 __device__ __forceinline__ float rc_gelu_tanh(float z) { return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z))); }
 
-#define RG_COLS 128              // output channels a block of the gates kernel takes (a thread each)
-
-// The convolution of tokens t0 .. t0 + nt - 1 over the channels of block b into shared memory; u[e * stride_e + tt * stride_t].
-__device__ __forceinline__ void rg_conv_tile(float* u, int stride_e, int stride_t, const float* __restrict__ proj, long long ldp, int x_col,
-                                             const float* __restrict__ conv_w, const float* __restrict__ conv_b, const float* __restrict__ state,
-                                             long long state_stride, const int* __restrict__ tok_seg, const int* __restrict__ seg_start,
-                                             const int* __restrict__ seg_slot, int t0, int nt, int c0, int R, int Bs, int taps) {
-    for (int idx = threadIdx.x; idx < nt * Bs; idx += blockDim.x) {
-        const int tt = idx / Bs, e = idx % Bs, t = t0 + tt, ch = c0 + e;
-        const int seg = tok_seg[t], i = t - seg_start[seg];
-        const float* tail = state + (size_t)seg_slot[seg] * state_stride + R;
-        const float* w = conv_w + (size_t)ch * taps;
-        float acc = conv_b[ch];
-        for (int j = taps - 1; j >= 0; j--) {                            // oldest input first
-            const int ip = i - j;
-            const float x = ip >= 0 ? proj[(size_t)(t - j) * ldp + x_col + ch] : tail[(size_t)(taps - 1 + ip) * R + ch];
-            acc = fmaf(w[taps - 1 - j], x, acc);
-        }
-        u[e * stride_e + tt * stride_t] = acc;
-    }
-}
-
 // a and the recurrence's input from the gates' sums; the gated branch's activation in place (nothing else reads those columns)
 __device__ __forceinline__ void rg_finish(float ra, float ri, float u, float rate, float* a_out, float* b_out, float* y) {
     *y = rc_gelu_tanh(*y);
@@ -74,66 +53,71 @@ __device__ __forceinline__ void rg_finish(float ra, float ri, float u, float rat
     *b_out = sqrtf(-expm1f(2.0f * log_a)) * (rc_sigmoid(ri) * u);          // sqrt(1 - a^2) without the cancellation near a = 1
 }
 
-// Many tokens: a block per (TT tokens, channel block, 64 output channels), a thread an output channel with TT sums of each gate.
-// The tile of u lies in shared memory input-major, [in][TT], so that a thread reads four tokens' values at once.
-template <int TT>
-__global__ void __launch_bounds__(RG_COLS)
-k_rglru_gates(float* __restrict__ proj, long long ldp, int y_col, int x_col, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
-              const float* __restrict__ wa_t, const float* __restrict__ wi_t, const float* __restrict__ ba, const float* __restrict__ bi,
-              const float* __restrict__ lam, const float* __restrict__ state, long long state_stride, const int* __restrict__ tok_seg,
-              const int* __restrict__ seg_start, const int* __restrict__ seg_slot, float* __restrict__ a_out, float* __restrict__ b_out,
-              int n, int R, int Bs, int taps, float c) {
+// Many tokens: both gate products as one tile product (simt_tile.cuh) over a channel block's inputs u: a tile's rows are, eight and
+// eight, rows of Wa and of Wi for the same outputs, so that a thread holds both sums of its outputs and finishes them in registers.
+// What bounds it: the float32 FMA pipes; the matrices come from L2.  1,901 tokens, 2,560 channels in ten blocks: 180 us,
+// where a thread an output with eight tokens' sums, which reads its weights from L2 for every eight tokens, took 360.
+template <int WM, int WN, int TM, int TN>
+__global__ void __launch_bounds__(32 * WM * WN)
+k_rglru_gates(float* __restrict__ proj, long long ldp, int y_col, const float* __restrict__ u, const float* __restrict__ wa, const float* __restrict__ wi,
+              const float* __restrict__ ba, const float* __restrict__ bi, const float* __restrict__ lam, float* __restrict__ a_out,
+              float* __restrict__ b_out, int n, int R, int Bs, float c, int vec) {
+    static_assert(TN % 2 == 0, "rows of both matrices a thread");
+    constexpr int BM = 4 * TM * WM, OUT = 8 * TN * WN / 2;          // outputs a tile
+    extern __shared__ __align__(16) unsigned char gs_sm[];
     xr_pdl_launch();
-    extern __shared__ __align__(16) float rg_u[];                // [Bs][TT]
-    const int t0 = blockIdx.x * TT, b = blockIdx.y, c0 = b * Bs;
-    const int nt = min(TT, n - t0);
+    const int t0 = blockIdx.y * BM, o0 = blockIdx.x * OUT, b = blockIdx.z, c0 = b * Bs;
+    const float* wab = wa + (size_t)b * Bs * Bs;
+    const float* wib = wi + (size_t)b * Bs * Bs;
     xr_pdl_wait();
-    if (nt < TT)
-        for (int idx = threadIdx.x; idx < TT * Bs; idx += blockDim.x) rg_u[idx] = 0.f;
-    __syncthreads();
-    rg_conv_tile(rg_u, TT, 1, (const float*)proj, ldp, x_col, conv_w, conv_b, state, state_stride, tok_seg, seg_start, seg_slot, t0, nt, c0, R, Bs, taps);
-    __syncthreads();
-    const float* wa = wa_t + (size_t)b * Bs * Bs;
-    const float* wi = wi_t + (size_t)b * Bs * Bs;
-    for (int o = blockIdx.z * RG_COLS + threadIdx.x; o < Bs; o += gridDim.z * RG_COLS) {
-        float ra[TT], ri[TT];
+    float acc[TM][TN];
+    gs_tile<float, float, WM, WN, TM, TN>(
+        gs_sm, Bs, vec, [&](int i) { return t0 + i < n ? u + (size_t)(t0 + i) * R + c0 : (const float*)nullptr; },
+        [&](int i) {
+            const int o = o0 + i / 16 * 8 + i % 8;                  // rows 16 q .. + 7: Wa's, + 8 .. + 15: Wi's of the same outputs
+            return o < Bs ? (i & 8 ? wib : wab) + (size_t)o * Bs : (const float*)nullptr;
+        },
+        acc);
+    const int tm = gs_token<WN, TM>(), rn = gs_row<WN, TN>();
 #pragma unroll
-        for (int tt = 0; tt < TT; tt++) { ra[tt] = ba[c0 + o]; ri[tt] = bi[c0 + o]; }
-        // eight inputs' weights are fetched in one run of loads ahead of their multiply-adds (they come from the L2 cache, and
-        // the few warps an SM holds of this kernel do not hide that latency otherwise)
-        for (int k0 = 0; k0 < Bs; k0 += 8) {
-            float va[8], vi[8];
+    for (int j = 0; j < TN; j += 2) {
+        const int row = rn + 8 * j, o = o0 + row / 16 * 8 + row % 8;
+        if (o >= Bs) continue;
+        const float rate = -c * rc_softplus(lam[c0 + o]), bias_a = ba[c0 + o], bias_i = bi[c0 + o];
+        float us[TM], ys[TM];                            // (all on their way at once)
 #pragma unroll
-            for (int kk = 0; kk < 8; kk++) {
-                const int k = min(k0 + kk, Bs - 1);
-                va[kk] = rc_ld_weight(wa + (size_t)k * Bs + o); vi[kk] = rc_ld_weight(wi + (size_t)k * Bs + o);
-            }
-#pragma unroll
-            for (int kk = 0; kk < 8; kk++) { xr_ld_fence(va[kk]); xr_ld_fence(vi[kk]); }
-#pragma unroll
-            for (int kk = 0; kk < 8; kk++) {
-                if (k0 + kk < Bs) {
-                    const float4* uk = reinterpret_cast<const float4*>(rg_u + (size_t)(k0 + kk) * TT);
-#pragma unroll
-                    for (int q4 = 0; q4 < TT / 4; q4++) {
-                        const float4 u = uk[q4];
-                        ra[4 * q4] = fmaf(va[kk], u.x, ra[4 * q4]); ri[4 * q4] = fmaf(vi[kk], u.x, ri[4 * q4]);
-                        ra[4 * q4 + 1] = fmaf(va[kk], u.y, ra[4 * q4 + 1]); ri[4 * q4 + 1] = fmaf(vi[kk], u.y, ri[4 * q4 + 1]);
-                        ra[4 * q4 + 2] = fmaf(va[kk], u.z, ra[4 * q4 + 2]); ri[4 * q4 + 2] = fmaf(vi[kk], u.z, ri[4 * q4 + 2]);
-                        ra[4 * q4 + 3] = fmaf(va[kk], u.w, ra[4 * q4 + 3]); ri[4 * q4 + 3] = fmaf(vi[kk], u.w, ri[4 * q4 + 3]);
-                    }
-                }
-            }
+        for (int i = 0; i < TM; i++) {
+            const int t = min(t0 + tm + 4 * i, n - 1);
+            us[i] = xr_ld_now(u + (size_t)t * R + c0 + o);
+            ys[i] = xr_ld_now(proj + (size_t)t * ldp + y_col + c0 + o);
         }
-        const float rate = -c * rc_softplus(lam[c0 + o]);
 #pragma unroll
-        for (int tt = 0; tt < TT; tt++) {
-            if (tt < nt) {
-                const size_t at = (size_t)(t0 + tt) * R + c0 + o;
-                rg_finish(ra[tt], ri[tt], rg_u[(size_t)o * TT + tt], rate, a_out + at, b_out + at, proj + (size_t)(t0 + tt) * ldp + y_col + c0 + o);
-            }
+        for (int i = 0; i < TM; i++) {
+            const int t = t0 + tm + 4 * i;
+            if (t >= n) continue;
+            const size_t at = (size_t)t * R + c0 + o;
+            xr_ld_fence(us[i]);
+            xr_ld_fence(ys[i]);
+            rg_finish(acc[i][j] + bias_a, acc[i][j + 1] + bias_i, us[i], rate, a_out + at, b_out + at, ys + i);
+            proj[(size_t)t * ldp + y_col + c0 + o] = ys[i];
         }
     }
+}
+
+template <int WM, int WN, int TM, int TN>
+static int launch_rglru_gates(float* proj, long long ldp, int y_col, const float* u, const float* wa, const float* wi, const float* ba, const float* bi,
+                              const float* lam, float* a_s, float* b_s, int n, int R, int B, float c, cudaStream_t stream) {
+    constexpr int BM = 4 * TM * WM, OUT = 8 * TN * WN / 2;
+    constexpr size_t SMEM = gs_smem<float, float, BM, 2 * OUT>();
+    const int Bs = R / B;
+    static const bool ready = SMEM <= 48 * 1024 || cudaFuncSetAttribute(k_rglru_gates<WM, WN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                                        (int)SMEM) == cudaSuccess;
+    if (!ready) return XR_ERR_LAUNCH;
+    const int vec = Bs % 4 == 0 && !(((uintptr_t)u | (uintptr_t)wa | (uintptr_t)wi) & 15);
+    const dim3 grid((Bs + OUT - 1) / OUT, (n + BM - 1) / BM, B);
+    if (grid.y > 65535) return XR_ERR_ARG;
+    xr_launch((k_rglru_gates<WM, WN, TM, TN>), grid, dim3(32 * WM * WN), SMEM, stream, proj, ldp, y_col, u, wa, wi, ba, bi, lam, a_s, b_s, n, R, Bs, c, vec);
+    return XR_OK;
 }
 
 // The convolution alone, a thread an element: u [n][R].  Ahead of k_rglru_gates_few, whose many small blocks would each compute
@@ -159,14 +143,50 @@ __global__ void k_rglru_conv(const float* __restrict__ proj, long long ldp, int 
     u[idx] = acc;
 }
 
+// The same sums for many tokens, four taps: a thread four channels of RC_RUN tokens, whose rows it reads once, 16 bytes at a time and
+// all on their way at once.  What bounds it: memory.  1,901 tokens of 2,560 channels: 8 us, a thread an element 39.
+#define RC_RUN 8
+__global__ void __launch_bounds__(128)
+k_rglru_conv_rows(const float* __restrict__ proj, long long ldp, int x_col, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
+                  const float* __restrict__ state, long long state_stride, const int* __restrict__ tok_seg, const int* __restrict__ seg_start,
+                  const int* __restrict__ seg_slot, float* __restrict__ u, int n, int R) {
+    xr_pdl_launch();
+    const int ch = (blockIdx.x * 128 + threadIdx.x) * 4, t0 = blockIdx.y * RC_RUN;
+    if (ch >= R) return;
+    float4 w[4];                                                     // [channel]: its four taps
+#pragma unroll
+    for (int k = 0; k < 4; k++) w[k] = *reinterpret_cast<const float4*>(conv_w + (size_t)(ch + k) * 4);
+    const float4 bias = make_float4(conv_b[ch], conv_b[ch + 1], conv_b[ch + 2], conv_b[ch + 3]);
+    xr_pdl_wait();
+    float4 x[RC_RUN + 3];                                            // rows t0 - 3 ..
+#pragma unroll
+    for (int r = 0; r < RC_RUN + 3; r++) x[r] = *reinterpret_cast<const float4*>(proj + (size_t)max(0, min(t0 + r - 3, n - 1)) * ldp + x_col + ch);
+#pragma unroll
+    for (int r = 0; r < RC_RUN; r++) {
+        const int t = t0 + r;
+        if (t >= n) break;
+        const int seg = tok_seg[t], i = t - seg_start[seg];
+        const float* tail = state + (size_t)seg_slot[seg] * state_stride + R + ch;
+        float4 acc = bias;
+#pragma unroll
+        for (int j = 3; j >= 0; j--) {                               // oldest input first
+            const float4 v = i - j >= 0 ? x[r + 3 - j] : *reinterpret_cast<const float4*>(tail + (size_t)(3 + i - j) * R);
+            const float* wk = reinterpret_cast<const float*>(w);
+            acc.x = fmaf(wk[3 - j], v.x, acc.x);
+            acc.y = fmaf(wk[4 + 3 - j], v.y, acc.y);
+            acc.z = fmaf(wk[8 + 3 - j], v.z, acc.z);
+            acc.w = fmaf(wk[12 + 3 - j], v.w, acc.w);
+        }
+        *reinterpret_cast<float4*>(u + (size_t)t * R + ch) = acc;
+    }
+}
+
 // Few tokens (a step of single tokens): a warp an output channel, its lanes share the inputs, so that the matrices' rows (as
 // stored, [b][out][in]) are read by whole warps and every load of a thread is in flight at once.  A block: 8 tokens, 8 channels.
 __global__ void __launch_bounds__(256)
-k_rglru_gates_few(float* __restrict__ proj, long long ldp, int y_col, int x_col, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
-                  const float* __restrict__ wa, const float* __restrict__ wi, const float* __restrict__ ba, const float* __restrict__ bi,
-                  const float* __restrict__ lam, const float* __restrict__ state, long long state_stride, const int* __restrict__ tok_seg,
-                  const int* __restrict__ seg_start, const int* __restrict__ seg_slot, float* __restrict__ a_out, float* __restrict__ b_out,
-                  int n, int R, int Bs, int taps, float c, int groups, const float* __restrict__ u_in) {
+k_rglru_gates_few(float* __restrict__ proj, long long ldp, int y_col, const float* __restrict__ wa, const float* __restrict__ wi,
+                  const float* __restrict__ ba, const float* __restrict__ bi, const float* __restrict__ lam, float* __restrict__ a_out,
+                  float* __restrict__ b_out, int n, int R, int Bs, float c, int groups, const float* __restrict__ u_in) {
     xr_pdl_launch();
     extern __shared__ __align__(16) float rg_u[];                // [8][Bs]
     const int t0 = blockIdx.x * 8, b = blockIdx.y / groups, c0 = b * Bs;
@@ -253,46 +273,114 @@ k_rglru_scan(const float* __restrict__ proj, long long ldp, int y_col, int x_col
     for (int r = 0; r < taps - 1; r++) tail[(size_t)r * R + ch] = keep[r];
 }
 
+// Long portions: a warp a segment of the portion's tokens, a lane a channel, RS_WARPS segments a block.  Every warp first walks its
+// segment from zero (the end state and the product of the decays), the segments' start states follow from one another, and the
+// second walk starts from the right state and writes.  The chain of dependent steps is a thirty-second of the portion, twice; the
+// gates' results are read twice, the second time from L2.  1,901 tokens, 2,560 channels: 34 us, a thread a channel for all of them 90.
+#define RS_WARPS 32
+template <typename T>
+__global__ void __launch_bounds__(32 * RS_WARPS)
+k_rglru_scan_segments(const float* __restrict__ proj, long long ldp, int y_col, int x_col, const float* __restrict__ a_in, const float* __restrict__ b_in,
+                      float* __restrict__ state, long long state_stride, const int* __restrict__ seg_start, const int* __restrict__ seg_len,
+                      const int* __restrict__ seg_slot, T* __restrict__ out, int R, int taps) {
+    __shared__ float ends[RS_WARPS][32], decays[RS_WARPS][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ch = blockIdx.x * 32 + lane, seg = blockIdx.y, cc = min(ch, R - 1);
+    const int start = seg_start[seg], len = seg_len[seg];
+    const int per = (len + RS_WARPS - 1) / RS_WARPS, i0 = min(len, warp * per), i1 = min(len, i0 + per);
+    float* st = state + (size_t)seg_slot[seg] * state_stride;
+    const float* ap = a_in + (size_t)start * R + cc;
+    const float* bp = b_in + (size_t)start * R + cc;
+    float S = 0.f, A = 1.f;
+    for (int i = i0; i < i1; i += 8) {
+        float a[8], b[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) { const size_t at = (size_t)min(i + k, i1 - 1) * R; a[k] = xr_ld_now(ap + at); b[k] = xr_ld_now(bp + at); }
+#pragma unroll
+        for (int k = 0; k < 8; k++) { xr_ld_fence(a[k]); xr_ld_fence(b[k]); }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (i + k < i1) { S = fmaf(a[k], S, b[k]); A *= a[k]; }
+    }
+    ends[warp][lane] = S; decays[warp][lane] = A;
+    __syncthreads();
+    S = st[cc];
+    for (int w = 0; w < warp; w++) S = fmaf(decays[w][lane], S, ends[w][lane]);
+    const float* yp = proj + (size_t)start * ldp + y_col + cc;
+    for (int i = i0; i < i1; i += 8) {
+        float a[8], b[8], y[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const size_t t = (size_t)min(i + k, i1 - 1);
+            a[k] = xr_ld_now(ap + t * R); b[k] = xr_ld_now(bp + t * R); y[k] = xr_ld_now(yp + t * ldp);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) { xr_ld_fence(a[k]); xr_ld_fence(b[k]); xr_ld_fence(y[k]); }
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (i + k < i1) {
+                S = fmaf(a[k], S, b[k]);
+                if (ch < R) out[(size_t)(start + i + k) * R + ch] = xr_from_f32<T>(S * y[k]);
+            }
+    }
+    __syncthreads();                                     // every warp has read the state as it was
+    if (len > 0 && i0 < len && i1 == len && ch < R) {    // the warp with the last token
+        st[ch] = S;
+        float keep[RG_MAX_TAPS];
+        float* tail = st + R;
+        for (int r = 0; r < taps - 1; r++) {
+            const int i = len - (taps - 1) + r;
+            keep[r] = i >= 0 ? proj[(size_t)(start + i) * ldp + x_col + ch] : tail[(size_t)(r + len) * R + ch];
+        }
+        for (int r = 0; r < taps - 1; r++) tail[(size_t)r * R + ch] = keep[r];
+    }
+}
+
 // proj [n][ldp] float32: the gated branch's pre-activations at y_col, the convolution's inputs at x_col, R columns each.
-// conv_w [R][taps], conv_b [R]; wa_t, wi_t [B][R/B (in)][R/B (out)] and wa, wi the same matrices as stored, [B][out][in]; ba, bi,
+// conv_w [R][taps], conv_b [R]; wa, wi [B][R/B (out)][R/B (in)] as stored; ba, bi,
 // lam [R]; all float32.
 // state [slots][state_stride] float32: S [R], tail [taps-1][R].  a_s, b_s, u_s [n][R] float32 scratch.  out [n][R] dtype `dtype`.
-XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa_t,
-                       const float* wi_t, const float* wa, const float* wi, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
+XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
                        const int* tok_seg, const int* seg_start, const int* seg_len, const int* seg_slot, float* a_s, float* b_s, float* u_s, void* out,
                        int dtype, int n, int n_seg, int R, int B, int taps, float c, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || R < 1 || B < 1 || R % B || taps < 1 || taps > RG_MAX_TAPS || n_seg > 65535 || B > 65535 ||
         state_stride < (long long)R * taps)
         return XR_ERR_ARG;
     const int Bs = R / B;
-    // (a tile of eight tokens of one channel block in shared memory: wide blocks ask for more than the default 48 KB)
-    const size_t smem8 = (size_t)8 * Bs * sizeof(float);
-    if (smem8 > 200 * 1024) return XR_ERR_ARG;
-    if (smem8 > 48 * 1024 &&
-        (cudaFuncSetAttribute(k_rglru_gates_few, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem8) != cudaSuccess ||
-         cudaFuncSetAttribute(k_rglru_gates<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem8) != cudaSuccess))
-        return XR_ERR_LAUNCH;
-#define RG_ARGS(A, I) proj, ldp, y_col, x_col, conv_w, conv_b, A, I, ba, bi, lam, (const float*)state, state_stride, tok_seg, seg_start, seg_slot, a_s, b_s, n, R, Bs, taps, c
-    if (n <= 16) {
-        const int groups = (Bs + 7) / 8;
+    if ((long long)n * R > 0x7fffffffLL - 255) return XR_ERR_ARG;
+    const bool rows = taps == 4 && n >= 64 && !((R | ldp | x_col | state_stride) & 3) &&
+                      !(((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)state | (uintptr_t)u_s) & 15) && (n + RC_RUN - 1) / RC_RUN <= 65535;
+    if (rows)
+        xr_launch(k_rglru_conv_rows, dim3((R / 4 + 127) / 128, (n + RC_RUN - 1) / RC_RUN), dim3(128), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b,
+                  (const float*)state, state_stride, tok_seg, seg_start, seg_slot, u_s, n, R);
+    else
         xr_launch(k_rglru_conv, dim3((n * R + 255) / 256), dim3(256), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b, (const float*)state,
                   state_stride, tok_seg, seg_start, seg_slot, u_s, n, R, taps);
-        xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, RG_ARGS(wa, wi), groups, (const float*)u_s);
-    } else if (n >= 64 && (size_t)32 * Bs * sizeof(float) <= 48 * 1024) {
-        xr_launch((k_rglru_gates<32>), dim3((n + 31) / 32, B, (Bs + RG_COLS - 1) / RG_COLS), dim3(RG_COLS), (size_t)32 * Bs * sizeof(float), stream, RG_ARGS(wa_t, wi_t));
+    const size_t smem8 = (size_t)8 * Bs * sizeof(float);
+    if (n <= 16 && smem8 <= 48 * 1024) {
+        // (one token to a few: a warp an output, its lanes share the inputs)
+        const int groups = (Bs + 7) / 8;
+        xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, proj, ldp, y_col, wa, wi, ba, bi, lam, a_s, b_s,
+                  n, R, Bs, c, groups, (const float*)u_s);
     } else {
-        xr_launch((k_rglru_gates<8>), dim3((n + 7) / 8, B, (Bs + RG_COLS - 1) / RG_COLS), dim3(RG_COLS), smem8, stream, RG_ARGS(wa_t, wi_t));
+        int rc;
+        // enough tiles of 64 tokens x 32 outputs to fill the machine twice, else of 16 x 16.  The whole part (convolution, gates, scan) at 2,560
+        // channels, us, 64 x 32 / 16 x 16: 32 tokens 34 / 18, 200 tokens 45 / 41, 512 tokens 71 / 82, 1,901 tokens 236 / 267
+        const long long mid = (long long)((n + 63) / 64) * ((Bs + 31) / 32) * B;
+        if (mid >= 2 * xr_sm_count()) rc = launch_rglru_gates<2, 2, 8, 4>(proj, ldp, y_col, u_s, wa, wi, ba, bi, lam, a_s, b_s, n, R, B, c, stream);
+        else rc = launch_rglru_gates<1, 2, 4, 2>(proj, ldp, y_col, u_s, wa, wi, ba, bi, lam, a_s, b_s, n, R, B, c, stream);
+        if (rc != XR_OK) return rc;
     }
-#undef RG_ARGS
     dim3 gs((R + 127) / 128, n_seg);
     // (a step with long portions is a few long-lived blocks: they start behind the gates kernel, not into its last wave)
-    const bool walk = n > 4 * n_seg;
-    if (walk && dtype == XR_F32)
+    const bool behind = n > 4 * n_seg;
+    // (the true 32-bit path promises the same bits however portions are cut: a thread a channel there)
+    if (behind && dtype == XR_BF16)
+        xr_launch_behind((k_rglru_scan_segments<__nv_bfloat16>), dim3((R + 31) / 32, n_seg), dim3(32 * RS_WARPS), 0, stream, (const float*)proj, ldp, y_col,
+                         x_col, (const float*)a_s, (const float*)b_s, state, state_stride, seg_start, seg_len, seg_slot, (__nv_bfloat16*)out, R, taps);
+    else if (behind && dtype == XR_F32)
         xr_launch_behind((k_rglru_scan<float>), gs, dim3(128), 0, stream, (const float*)proj, ldp, y_col, x_col, (const float*)a_s, (const float*)b_s, state,
                          state_stride, seg_start, seg_len, seg_slot, (float*)out, R, taps);
-    else if (walk && dtype == XR_BF16)
-        xr_launch_behind((k_rglru_scan<__nv_bfloat16>), gs, dim3(128), 0, stream, (const float*)proj, ldp, y_col, x_col, (const float*)a_s, (const float*)b_s, state,
-                         state_stride, seg_start, seg_len, seg_slot, (__nv_bfloat16*)out, R, taps);
     else if (dtype == XR_F32)
         xr_launch((k_rglru_scan<float>), gs, dim3(128), 0, stream, (const float*)proj, ldp, y_col, x_col, (const float*)a_s, (const float*)b_s, state,
                   state_stride, seg_start, seg_len, seg_slot, (float*)out, R, taps);

@@ -107,7 +107,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_cast_rows": [_vp, _vp, _i, _ll, _vp],
         "xr_depth_average": [_vp, _vp, _vp, _vp, _vp, _i, _i, _ll, _vp],
         "xr_rotate_heads": [_vp, _i, _ll, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _f, _i, _vp],
-        "xr_rglru": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
+        "xr_rglru": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
                      _f, _vp],
         "xr_row_norm_gate": [_vp, _vp, _ll, _vp, _vp, _i, _i, _i, _f, _f, _vp],
         "xr_ssd": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
@@ -1264,20 +1264,20 @@ def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, s
     """The real-gated linear recurrent unit over the step's tokens, request by request, from and into `state`.  proj [n, >= 2R]
     float32 (rows may be strided): the gated branch's pre-activations in columns [0, R), the convolution's inputs in [R, 2R).
     out [n, R] = S * gelu_tanh(gated branch).  wa, wi: the gates' matrices [B, out, in]; wa_t, wi_t: the same transposed to
-    [B, in, out] (steps of many tokens read those).  See csrc/recurrent.cu for the other arguments."""
-    _dev(conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, state, tok_seg, seg_start, seg_len, seg_slot, a_s, b_s, u_s, out)
+    [B, in, out], or None (no kernel reads them).  See csrc/recurrent.cu for the other arguments."""
+    _dev(conv_w, conv_b, wa, wi, ba, bi, lam, state, tok_seg, seg_start, seg_len, seg_slot, a_s, b_s, u_s, out)
     n = proj.shape[0]
     Bs = R // B
     assert u_s.dtype == torch.float32 and u_s.numel() >= n * R
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[1] >= 2 * R and out.shape == (n, R)
-    assert all(t.dtype == torch.float32 for t in (conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, state, a_s, b_s))
-    assert conv_w.shape == (R, taps) and all(t.shape == (B, Bs, Bs) for t in (wa_t, wi_t, wa, wi)) and a_s.numel() >= n * R and b_s.numel() >= n * R
+    assert all(t.dtype == torch.float32 for t in (conv_w, conv_b, wa, wi, ba, bi, lam, state, a_s, b_s))
+    assert conv_w.shape == (R, taps) and all(t.shape == (B, Bs, Bs) for t in (wa, wi)) and a_s.numel() >= n * R and b_s.numel() >= n * R
     assert state.dim() == 2 and state.shape[1] >= rglru_state_floats(R, taps)
-    _check(lib().xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(), wa_t.data_ptr(), wi_t.data_ptr(),
+    _check(lib().xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(),
                           wa.data_ptr(), wi.data_ptr(), ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
                           seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), u_s.data_ptr(), out.data_ptr(),
                           dtype_code(out.dtype), n, n_seg, R, B, taps, float(c), _stream()), "rglru")
-    _count(3 if n <= 16 else 2)
+    _count(3)
 
 
 def decay_attention(proj: torch.Tensor, cols, decay: torch.Tensor, state: torch.Tensor, seg_start, seg_len, seg_slot, o: torch.Tensor,
