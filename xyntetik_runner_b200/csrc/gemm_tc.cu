@@ -81,6 +81,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     *abort_flag = 1;
     return false;
 }
+// One lane of a whole warp, the same one every time.  The copies', MMAs' and commits' operands live in registers that a warp shares:
+// behind this the compiler knows that one lane runs, behind `lane == 0` it does not and moves every operand over one by one.  Cycles a K
+// block of the pair kernel, `lane == 0` / elected: tiles of 64 and 128 tokens 620 / 323, of 256 tokens 620 / 512, which are the tensor
+// pipe's own; 2,048 x 4,096 x 4,096: 56 / 50 us.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
@@ -253,7 +262,11 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
         }
         float v[16];
 #pragma unroll
-        for (int c = 0; c < 16; c++) v[c] = tc_act(p.act, fmaf(p.alpha, g[c], b));
+        for (int c = 0; c < 16; c++) v[c] = fmaf(p.alpha, g[c], b);
+        if (p.act != TC_ACT_NONE) {             // (one branch a chunk: asked for value by value, every function's steps are taken for every value)
+#pragma unroll
+            for (int c = 0; c < 16; c++) v[c] = tc_act(p.act, v[c]);
+        }
         if (p.out_dtype == XR_BF16) {
             __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)(tok0 + c0) * p.ldo + r;
 #pragma unroll
@@ -334,13 +347,13 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         }
     };
     const int early = nkb < STAGES ? nkb : STAGES;
-    if (warp == 0 && lane == 0)
+    if (warp == 0 && tc_elect())
         for (int i = 0; i < early; i++) load_w(i);
     xr_pdl_wait();
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        if (tc_elect()) {
             int issued = early;
             for (int i = 0; i < nkb; i++) {
                 int s = i % STAGES;
@@ -359,20 +372,20 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (tc_elect()) {
             const uint32_t idesc = instr_desc(p.bn);
+            const uint64_t first = smem_desc_sw128(smem_u32(smem));
             bool ok = true;
+            uint32_t s = 0, phase = 0;
             for (int i = 0; i < nkb && ok; i++) {
-                int s = i % STAGES;
-                ok = mbar_wait(&full[s], (i / STAGES) & 1, abort_flag);
+                ok = mbar_wait(&full[s], phase, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-                uint32_t b_addr = a_addr + W_BYTES;
+                const uint64_t a_desc = first + s * (STAGE_BYTES >> 4), b_desc = a_desc + (W_BYTES >> 4);
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; k++)
-                    tc_mma(tmem_base, smem_desc_sw128(a_addr + k * 32), smem_desc_sw128(b_addr + k * 32), idesc, (i > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < TC_BK / 16; k++) tc_mma(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
                 tc_commit(&empty[s]);          // the stage is free once these MMAs have read it
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
             if (ok) tc_commit(acc_ready);      // accumulators complete
         }
@@ -514,8 +527,9 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        if (lane == 0) {
+        if (tc_elect()) {
             int it = 0;                                      // K blocks fetched so far, over all tiles
+            uint32_t s = 0, phase = 1;                       // the ring's place
             bool ok = true;
             for (int item = cluster_id; item < pair_tiles * p.splits && ok; item += n_clusters) {
                 const int tile = item % pair_tiles, split = item / pair_tiles;
@@ -528,8 +542,7 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 const uint32_t stage_bytes = W_BYTES + (GROUPED ? boxes * TC2_XBOX : half) * TC_BK * 2;
                 const int kb0 = (int)(((long long)split * nkb) / p.splits), kb1 = (int)(((long long)(split + 1) * nkb) / p.splits);
                 for (int i = kb0; i < kb1; i++, it++) {
-                    int s = it % STAGES;
-                    if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort_flag)) { ok = false; break; }
+                    if (it >= STAGES && !mbar_wait(&empty[s], phase, abort_flag)) { ok = false; break; }
                     uint8_t* st = smem + s * STAGE_BYTES;
                     const uint32_t bar = tc_map_to_rank(smem_u32(&full[s]), 0);
                     const int kx = i * TC_BK;
@@ -538,6 +551,7 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     else tma_load_2d_pair(st, &map_w, kx, row_tile * TC_BM, bar);
                     for (int x = 0; x < boxes; x++)
                         tma_load_2d_pair(st + W_BYTES + x * TC2_XBOX * TC_BK * 2, &map_x, kx, at.tok0 + (int)rank * half + x * TC2_XBOX, bar);
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
             }
             if (*abort_flag) {
@@ -549,9 +563,11 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA only) ----------------
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && tc_elect()) {
             bool ok = true;
-            int it = 0, j = 0;                               // K blocks and tiles done so far
+            const uint64_t first = smem_desc_sw128(smem_u32(smem));
+            uint32_t s = 0, phase = 0;                       // the ring's place
+            int j = 0;                                       // tiles done so far
             for (int item = cluster_id; item < pair_tiles * p.splits && ok; item += n_clusters, j++) {
                 const int split = item / pair_tiles;
                 const uint32_t idesc = instr_desc_pair(tc_pair_tile<GROUPED>(p, item % pair_tiles, tok_tiles).bn);
@@ -563,17 +579,15 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                     tc_fence_after();
                 }
                 const uint32_t acc_addr = tmem_base + (uint32_t)b * TC2_BN;
-                for (int i = kb0; i < kb1; i++, it++) {
-                    int s = it % STAGES;
-                    ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag);
+                for (int i = kb0; i < kb1; i++) {
+                    ok = mbar_wait(&full[s], phase, abort_flag);
                     if (!ok) break;
                     tc_fence_after();
-                    uint32_t a_addr = smem_u32(smem + s * STAGE_BYTES);
-                    uint32_t b_addr = a_addr + W_BYTES;
+                    const uint64_t a_desc = first + s * (STAGE_BYTES >> 4), b_desc = a_desc + (W_BYTES >> 4);
 #pragma unroll
-                    for (int k = 0; k < TC_BK / 16; k++)
-                        tc_mma_pair(acc_addr, smem_desc_sw128(a_addr + k * 32), smem_desc_sw128(b_addr + k * 32), idesc, (i > kb0 || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < TC_BK / 16; k++) tc_mma_pair(acc_addr, a_desc + 2 * k, b_desc + 2 * k, idesc, (i > kb0 || k > 0) ? 1u : 0u);
                     tc_commit_pair(&empty[s]);
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
                 if (ok) tc_commit_pair(&acc_full[b]);
             }
