@@ -245,3 +245,131 @@ def test_gated_recurrence_of_long_portions(R, B, taps, lens, dtype):
         if keep:
             tail[taps - 1 - keep:] = r[len(r) - keep:, R:]
         assert torch.equal(state[slots[s], R:].cpu().view(taps - 1, R), tail)
+
+
+# ---- recurrences in chunks -------------------------------------------------------------------------------------------
+def _walk(q, k, v, decay, S):
+    """S <- decay S + k v^T, o = S^T q in float64; q, k [T, H, D], v [T, H, V], decay [T, H, D]."""
+    out = []
+    for t in range(len(q)):
+        S = decay[t][:, :, None] * S + k[t][:, :, None] * v[t][:, None, :]
+        out.append(torch.einsum("hdv,hd->hv", S, q[t]))
+    return torch.stack(out), S
+
+
+def _close(got, want, walk):
+    """No further from float64 than a few units of float32 of the largest value, and no further than three times the walk is."""
+    far, near = (got.double() - want).abs().max(), (walk.double() - want).abs().max()
+    assert far <= max(3.0 * near, 4e-6 * want.abs().max()), (far, near, want.abs().max())
+
+
+CHUNKED = [("head", 2, 64, 64), ("head", 1, 128, 128), ("key", 2, 64, 128), ("key", 1, 128, 64), ("key deep", 1, 64, 64)]
+
+
+@pytest.mark.parametrize("kind,H,D,V", CHUNKED)
+def test_recurrences_in_chunks(kind, H, D, V):
+    """Portions of a token, of a chunk, of a chunk and a token, of several, from states that hold something, against float64 and
+    beside the walk on the same inputs: read-outs, new states, other slots.  "deep": decays that clear the memory within a chunk next
+    to decays near one, where exponentials of sums would overflow or lose their digits."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(H * D + V + len(kind))
+    f = lambda *s: torch.randn(*s, generator=g)
+    lens, slots = [130, 1, 64, 65], [3, 0, 4, 1]
+    n, S = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(S)]
+    state0 = f(6, H * V * D)
+    q, k, v = f(n, H, D), f(n, H, D) * D ** -0.5, f(n, H, V)
+    if kind == "head":
+        dec = torch.tensor([1.0 - 2.0 ** -(2 + 6 * h) for h in range(H)])
+        proj = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1)], 1).to(DEV)
+        decay = dec.double()[None, :, None].expand(n, H, D)
+
+        def run(state, scratch):
+            o = torch.empty(n, H * V, device=DEV)
+            kernels.decay_attention(proj, (0, H * D, 2 * H * D), dec.to(DEV), state, _i32(starts), _i32(lens), _i32(slots), o, S, H, D, V, silu=False,
+                                    read_scale=0.5, scratch=scratch)
+            return o
+        floats = kernels.chunked_floats(n, S, H, D, V, "head")
+    else:
+        R, tau = 8, 12.0
+        inner, w_t, bias = f(n, R), f(R, H * D), 2.0 + f(H * D)
+        if kind.endswith("deep"):
+            inner[::13] *= 200.0
+        proj = torch.cat([q.reshape(n, -1), k.reshape(n, -1), v.reshape(n, -1), inner], 1).to(DEV)
+        z = inner.double() @ w_t.double() + bias
+        decay = torch.exp(torch.nn.functional.logsigmoid(z) / tau).view(n, H, D)
+
+        def run(state, scratch):
+            o = torch.empty(n, H * V, device=DEV)
+            kernels.key_decay_attention(proj, (0, H * D, 2 * H * D, 2 * H * D + H * V), R, w_t.to(DEV), bias.to(DEV), tau, torch.empty(n, H * D, device=DEV),
+                                        state, _i32(starts), _i32(lens), _i32(slots), o, S, H, D, V, read_scale=0.5, scratch=scratch)
+            return o
+        floats = kernels.chunked_floats(n, S, H, D, V, "key")
+    q = q * 0.5
+    assert floats > 0
+    walk_state, state = state0.to(DEV).clone(), state0.to(DEV).clone()
+    by_walk = run(walk_state, None).cpu()
+    got = run(state, torch.full((floats,), float("nan"), device=DEV)).cpu()
+    assert torch.equal(state[2].cpu(), state0[2]) and torch.equal(state[5].cpu(), state0[5])
+    for i, (m, slot) in enumerate(zip(lens, slots)):
+        at = slice(starts[i], starts[i] + m)
+        before = state0[slot].double().view(H, V, D).transpose(1, 2)
+        want, end = _walk(q[at].double(), k[at].double(), v[at].double(), decay[at].double(), before)
+        _close(got[at], want.reshape(m, -1), by_walk[at])
+        _close(state[slot].cpu(), end.transpose(1, 2).reshape(-1), walk_state[slot].cpu())
+
+
+@pytest.mark.parametrize("H,D,V,dtype", [(2, 64, 128, torch.float32), (1, 128, 64, torch.bfloat16), (3, 128, 256, torch.bfloat16)])
+def test_matrix_memory_with_gates_in_chunks(H, D, V, dtype):
+    """The same for the cell with exponential input gates: gates far apart, a maximum that moves, a forget gate near zero."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(H * D + V)
+    f = lambda *s: torch.randn(*s, generator=g)
+    lens, slots, cap = [300, 1, 64], [2, 0, 3], 15.0
+    n, S = sum(lens), len(lens)
+    starts = [sum(lens[:i]) for i in range(S)]
+    proj = f(n, 2 * H * D + 2 * H * V).to(dtype)
+    gates = torch.cat([4.0 * f(n, H), 3.0 + 2.0 * f(n, H)], dim=1)
+    gates[::41, H:] = -40.0
+    size = D * V + D + 1
+    state0 = f(4, H, size)
+    state0[..., -1] = state0[..., -1].abs()
+    norm_w = torch.ones(H * V)
+
+    def run(state, scratch):
+        o, y = torch.empty(n, H * V, device=DEV), torch.empty(n, H * V, dtype=dtype, device=DEV)
+        kernels.mlstm(proj.to(DEV), (0, H * D, 2 * H * D, 2 * H * D + H * V), gates.to(DEV), state, torch.empty(n, 3 * H, device=DEV), o, norm_w.to(DEV), y,
+                      _i32(starts), _i32(lens), _i32(slots), S, H, D, V, cap, 1e-6, scratch=scratch)
+        return o.cpu()
+    walk_state, state = state0.reshape(4, -1).to(DEV).clone(), state0.reshape(4, -1).to(DEV).clone()
+    by_walk = run(walk_state, None)
+    got = run(state, torch.full((kernels.chunked_floats(n, S, H, D, V, "mlstm"),), float("nan"), device=DEV))
+    assert torch.equal(state[1].cpu(), state0[1].reshape(-1))
+    p = proj.double()
+    q, k, v = p[:, :H * D].view(n, H, D) * D ** -0.5, p[:, H * D:2 * H * D].view(n, H, D), p[:, 2 * H * D:2 * H * D + H * V].view(n, H, V)
+    li = cap * torch.tanh(gates[:, :H].double() / cap)
+    lf = torch.nn.functional.logsigmoid(cap * torch.tanh(gates[:, H:].double() / cap))
+    for i, (m, slot) in enumerate(zip(lens, slots)):
+        st = state0[slot].double()
+        Sm, nm, mx = st[:, :D * V].reshape(H, D, V), st[:, D * V:D * V + D], st[:, -1]
+        Sa, na = Sm.abs(), nm.abs()                      # the same sums over sizes: what a rounding of a term can be a share of
+        out, bound = [], []
+        for t in range(starts[i], starts[i] + m):
+            new = torch.maximum(lf[t] + mx, li[t])
+            a, s = torch.exp(lf[t] + mx - new), torch.exp(li[t] - new)
+            Sm = a[:, None, None] * Sm + s[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+            nm = a[:, None] * nm + s[:, None] * k[t]
+            mx = new
+            Sa = a[:, None, None] * Sa + s[:, None, None] * k[t].abs()[:, :, None] * v[t].abs()[:, None, :]
+            na = a[:, None] * na + s[:, None] * k[t].abs()
+            den = torch.maximum((nm * q[t]).sum(-1).abs(), torch.exp(-mx)) + 1e-6
+            o = torch.einsum("hdv,hd->hv", Sm, q[t]) / den[:, None]
+            size = torch.einsum("hdv,hd->hv", Sa, q[t].abs()) + o.abs() * (na * q[t].abs()).sum(-1)[:, None]
+            out.append(o.reshape(-1))
+            bound.append((size / den[:, None]).reshape(-1))
+        at = slice(starts[i], starts[i] + m)
+        # numerator and denominator: a term passes at most 64 additions of its chunk's memory, 6 of the scan, 16 + 8 of a score, 32 + 6
+        # of the last product, and a dozen products and exponentials; the denominator may cancel, so the terms' sizes count
+        assert ((got[at].double() - torch.stack(out)).abs() <= 144 * 2.0 ** -24 * torch.stack(bound)).all()
+        end = torch.cat([Sm.reshape(H, -1), nm, mx[:, None]], dim=1).reshape(-1)
+        _close(state[slot].cpu(), end, walk_state[slot].cpu())

@@ -15,7 +15,7 @@
 // each head's o by its root mean square, multiplies by the norm weight and the sigmoid of the output gate.
 // The walk is token by token in both, so the state after a token does not depend on how the tokens were cut into
 // steps, bit for bit.
-#include "common.cuh"
+#include "chunked.cuh"
 #include <math.h>
 
 #define ML_VS 32          // value columns per block of the scan
@@ -25,7 +25,7 @@
 __device__ __forceinline__ float ml_logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
 // state layout per slot: [H][D * V + D + 1]
-__device__ __forceinline__ size_t ml_state_head(int D, int V) { return (size_t)D * V + D + 1; }
+__host__ __device__ __forceinline__ size_t ml_state_head(int D, int V) { return (size_t)D * V + D + 1; }
 
 // Tokens are taken `stage` at a time, in four steps a chunk, so that nothing but a few scalar operations per token is
 // serial: (1) the logarithms of the gates of the chunk's tokens, a thread a token; (2) one thread walks the chunk's
@@ -290,13 +290,112 @@ k_mlstm_out(const float* __restrict__ o, const TG* __restrict__ proj, long long 
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// Portions of many tokens go through the recurrence in chunks (chunked.cuh), with  a_t = f  and  s_t = i  in logarithms:
+//   log f_t = lf_t + m_(t-1) - m_t <= 0,   s_t = exp(li_t - m_t),   floor_t = exp(-m_t).
+// m is a running maximum of sums, m_t = max(m_(t-1) + lf_t, li_t): a block per (head, portion), a thread a run of tokens; a run is
+// the map m -> max(m + A, B), the runs' maps are joined over the block, then every thread walks its run from its own start.
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, float* __restrict__ log_f, float* __restrict__ in_scale,
+                float* __restrict__ floor_n, const int* __restrict__ seg_start, const int* __restrict__ seg_len, const int* __restrict__ seg_slot,
+                int H, int D, int V, float cap) {
+    xr_pdl_launch();
+    __shared__ float sa[256], sb[256];
+    const int h = blockIdx.x, seg = blockIdx.y, tid = threadIdx.x;
+    const int start = seg_start[seg], len = seg_len[seg];
+    const int per = (len + 255) / 256, i0 = min(len, tid * per), i1 = min(len, i0 + per);
+    float* m_at = state + ((size_t)seg_slot[seg] * H + h) * ml_state_head(D, V) + (size_t)D * V + D;
+    xr_pdl_wait();
+    const float m0 = *m_at;
+    auto logs = [&](int i, float& li, float& lf) {
+        const float* row = gates + (size_t)(start + i) * 2 * H + h;
+        li = cap * tanhf(row[0] / cap);
+        lf = ml_logsigmoid(cap * tanhf(row[H] / cap));
+    };
+    float A = 0.f, B = -INFINITY;
+    for (int i = i0; i < i1; i++) {
+        float li, lf;
+        logs(i, li, lf);
+        B = fmaxf(B + lf, li); A += lf;
+    }
+    sa[tid] = A; sb[tid] = B;
+    __syncthreads();
+    for (int o = 1; o < 256; o <<= 1) {                  // the maps of all runs up to this one, joined
+        float pa = 0.f, pb = -INFINITY;
+        if (tid >= o) { pa = sa[tid - o]; pb = sb[tid - o]; }
+        __syncthreads();
+        if (tid >= o) { sb[tid] = fmaxf(pb + sa[tid], sb[tid]); sa[tid] += pa; }
+        __syncthreads();
+    }
+    float m = tid == 0 ? m0 : fmaxf(m0 + sa[tid - 1], sb[tid - 1]), first_m = 0.f, first_lf = 0.f;
+    for (int i = i0; i < i1; i++) {
+        float li, lf;
+        logs(i, li, lf);
+        const float m_new = fmaxf(lf + m, li);
+        const size_t at = (size_t)(start + i) * H + h;
+        if (i == i0) { first_m = m_new; first_lf = lf; }
+        else log_f[at] = fminf(lf + m - m_new, 0.f);
+        in_scale[at] = expf(li - m_new); floor_n[at] = expf(-m_new);
+        m = m_new;
+    }
+    // a run's first decay leads over from the very m that the run before ended with (joined in another order, the sums differ in
+    // their last bits, and S is kept relative to m)
+    __syncthreads();
+    sa[tid] = m;
+    __syncthreads();
+    if (i0 < i1) log_f[(size_t)(start + i0) * H + h] = fminf(first_lf + (tid == 0 ? m0 : sa[tid - 1]) - first_m, 0.f);
+    if (len > 0 && i0 < len && i1 == len) *m_at = m;     // (every thread has read it, barriers ago)
+}
+
+// q / sqrt(D), k and v as float32 rows [n][2 H D + H V]
+template <typename T>
+__global__ void __launch_bounds__(256)
+k_mlstm_rows(const T* __restrict__ proj, long long ldp, int q_col, int k_col, int v_col, float* __restrict__ out, int n, int HD, int HV, float qs) {
+    xr_pdl_launch();
+    xr_pdl_wait();
+    const int cols = 2 * HD + HV;
+    for (size_t e = (size_t)blockIdx.x * 256 + threadIdx.x; e < (size_t)n * cols; e += (size_t)gridDim.x * 256) {
+        const size_t t = e / cols;
+        const int c = (int)(e % cols);
+        const T* row = proj + t * ldp;
+        out[e] = c < HD ? xr_to_f32<T>(row[q_col + c]) * qs : (c < 2 * HD ? xr_to_f32<T>(row[k_col + c - HD]) : xr_to_f32<T>(row[v_col + c - 2 * HD]));
+    }
+}
+
+template <typename T>
+static int mlstm_chunked(const T* proj, long long ldp, int q_col, int k_col, int v_col, const float* gates, float* state, float* o, const int* seg_start,
+                         const int* seg_len, const int* seg_slot, int n, int n_seg, int H, int D, int V, float cap, float* scratch,
+                         long long scratch_floats, cudaStream_t stream) {
+    const int HD = H * D, HV = H * V;
+    const long long cols = 2LL * HD + HV;
+    if (scratch_floats < ck_floats(n, n_seg, H, D, V, H, true) + n * (cols + 3LL * H) + 16) return XR_ERR_ARG;
+    float* rows = reinterpret_cast<float*>(((uintptr_t)scratch + 15) & ~(uintptr_t)15);
+    float* log_f = rows + n * cols;
+    float* in_scale = log_f + (size_t)n * H;
+    float* floor_n = in_scale + (size_t)n * H;
+    float* rest = reinterpret_cast<float*>(((uintptr_t)(floor_n + (size_t)n * H) + 15) & ~(uintptr_t)15);
+    const long long head = (long long)ml_state_head(D, V);
+    ChunkArgs a{rows, rows + HD, rows + 2 * HD, cols, cols, cols, H, V, nullptr, nullptr, in_scale, nullptr, nullptr, nullptr, state, (long long)H * head,
+                head, 1, seg_start, seg_len, seg_slot, n_seg, o, 1.0f, floor_n};
+    double* cum = ck_lay_out(a, rest, n, D, true);
+    a.cum = cum;
+    const size_t total = (size_t)n * cols;
+    const int most = xr_sm_count() * 8, blocks = (int)((total + 255) / 256 < (size_t)most ? (total + 255) / 256 : most);
+    xr_launch((k_mlstm_rows<T>), dim3(blocks), dim3(256), 0, stream, proj, ldp, q_col, k_col, v_col, rows, n, HD, HV, 1.0f / sqrtf((float)D));
+    xr_launch(k_mlstm_scalars, dim3(H, n_seg), dim3(256), 0, stream, gates, state, log_f, in_scale, floor_n, seg_start, seg_len, seg_slot, H, D, V, cap);
+    xr_launch(ck_cumulate, dim3((H + 127) / 128, (unsigned)ck_chunks(n, n_seg)), dim3(128), 0, stream, (const float*)log_f, (long long)H, cum, H, a);
+    return ck_run<CK_TOKEN, true>(a, n, D, stream);
+}
+
 // proj [n][ldp] (activation dtype): q at q_col [H][D], k at k_col [H][D], v at v_col [H][V], output gate at g_col [H][V];
 // gates [n][2H] float32 (input-gate pre-activations, then forget-gate ones, biases included);
 // state [slots][H][D*V + D + 1] float32;  coef [n][H][3], o [n][H][V]: float32 scratch;  y [n][H*V] activation dtype.
+// scratch (null: the walk): the recurrence in chunks, where it takes the sizes; xr_chunked_floats says how much it needs.
 XR_EXPORT int xr_mlstm(const void* proj, int dtype, long long ldp, int q_col, int k_col, int v_col, int g_col, const float* gates,
                        float* state, float* coef, float* o, const float* norm_w, void* y, const int* seg_start,
                        const int* seg_len, const int* seg_slot, int n, int n_seg, int H, int D, int V, float cap, float eps,
-                       cudaStream_t stream) {
+                       float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || H < 1 || D < 1 || V < 1 || !(cap > 0.f) || n_seg > 65535 || H > 65535) return XR_ERR_ARG;
     // tokens a chunk of the gates kernel: what fits 44 KB of shared memory, at most 32; its threads own up to 4 elements of n each
     if (D > 1024) return XR_ERR_ARG;
@@ -323,9 +422,15 @@ XR_EXPORT int xr_mlstm(const void* proj, int dtype, long long ldp, int q_col, in
         if (D > 256 && smem_s > 48 * 1024 &&                                                                                                     \
             cudaFuncSetAttribute(k_mlstm_scan_wide<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_s) != cudaSuccess)      \
             return XR_ERR_LAUNCH;                                                                                                     \
+        if (scratch != nullptr && ck_takes(D, V) && ck_chunks(n, n_seg) <= 65535) {                                                   \
+            const int rc = mlstm_chunked<T>((const T*)proj, ldp, q_col, k_col, v_col, gates, state, o, seg_start, seg_len, seg_slot, n, n_seg, H, D, V, \
+                                            cap, scratch, scratch_floats, stream);                                                    \
+            if (rc != XR_OK) return rc;                                                                                               \
+        } else {                                                                                                                      \
         xr_launch((k_mlstm_gates<T>), gg, dim3(D <= 128 ? 128 : 256), smem_g, stream, (const T*)proj, ldp, q_col, k_col, gates, state, coef, seg_start, \
                   seg_len, seg_slot, H, D, V, cap, stage);                                                                            \
         SCAN(T);                                                                                                                      \
+        }                                                                                                                             \
         xr_launch((k_mlstm_out<T>), dim3(gb), dim3(128), 0, stream, (const float*)o, (const T*)proj, ldp, g_col, norm_w, (T*)y, n, H, \
                   V, eps, V, 0);                                                                                                         \
     } while (0)

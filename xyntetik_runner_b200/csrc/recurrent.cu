@@ -30,6 +30,7 @@
 // or chunks: k_rglru_scan_segments, chunked.cuh; there the last bits depend on the cuts.)
 #include "simt_tile.cuh"
 #include "conv_tail.cuh"
+#include "chunked.cuh"
 #include <math.h>
 
 #define RG_MAX_TAPS 16
@@ -749,9 +750,10 @@ static int launch_decay_scan(const float* proj, long long ldp, int q_col, int k_
 // proj [n][ldp] float32: q at q_col [H][D], k at k_col [H][D], v at v_col [H][V]; with `silu` their pre-activations (columns from the
 // first of q to the last of v, which a step of many tokens activates in place), else as they are; decay [H] float32; state
 // [slots][state_stride] float32, S [H][V][D];  o [n][H V] float32 receives the read-outs, times read_scale.
+// scratch (null: the walk): the recurrence in chunks (chunked.cuh), all decays then in (0, 1]; xr_chunked_floats says how much it takes.
 XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_col, int v_col, const float* decay, float* state,
                                  long long state_stride, const int* seg_start, const int* seg_len, const int* seg_slot, float* o, int n, int n_seg,
-                                 int H, int D, int V, int silu, float read_scale, cudaStream_t stream) {
+                                 int H, int D, int V, int silu, float read_scale, float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || H < 1 || D < 1 || V < 1 || D > 256 || n_seg > 65535 || H > 65535 || state_stride < (long long)H * D * V)
         return XR_ERR_ARG;
     // q, k, v lie side by side from q_col on (the caller's layout): one pass activates them all
@@ -761,12 +763,19 @@ XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_co
         const int blocks = (int)((total + 255) / 256 < (size_t)xr_sm_count() * 16 ? (total + 255) / 256 : xr_sm_count() * 16);
         xr_launch(k_silu_cols, dim3(blocks), dim3(256), 0, stream, proj + q_col, ldp, 2 * H * D + H * V, total);
     }
+    if (scratch != nullptr && ck_takes(D, V) && (many || !silu)) {
+        if (scratch_floats < ck_floats(n, n_seg, H, D, V, 0, false)) return XR_ERR_ARG;
+        ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, decay, nullptr, nullptr, nullptr, nullptr, nullptr, state,
+                    state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
+        ck_lay_out(a, scratch, n, D, false);
+        if (ck_aligned(a)) return ck_run<CK_HEAD, false>(a, n, D, stream);
+    }
     return launch_decay_scan<DS_HEAD>(proj, ldp, q_col, k_col, v_col, decay, state, state_stride, seg_start, seg_len, seg_slot, o, n, n_seg, H, D, V,
                                       many || !silu, KeyDecayArgs{nullptr, read_scale}, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
-// Decays per key channel: out[t][c] = sigmoid(z)^(1/tau) = exp(log sigmoid(z) / tau), z = bias[c] + sum_r w_t[r][c] in[t][r]; `in` R
+// Decays per key channel: out[t][c] = sigmoid(z)^(1/tau) = exp(log sigmoid(z) / tau) (with `logs` its logarithm), z = bias[c] + sum_r w_t[r][c] in[t][r]; `in` R
 // columns of a wider float32 row, w_t the matrix transposed ([R][C], so that a warp reads a row).  A thread a channel with KD_T
 // tokens' sums; the tokens' rows lie in shared memory, R of them at a time.
 // ---------------------------------------------------------------------------------------------
@@ -774,7 +783,7 @@ XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_co
 template <int KD_T>
 __global__ void __launch_bounds__(128)
 k_key_decay(const float* __restrict__ in, long long ld_in, const float* __restrict__ w_t, const float* __restrict__ bias, float* __restrict__ out,
-            int n, int R, int C, float inv_tau, int early) {
+            int n, int R, int C, float inv_tau, int early, int logs) {
     if (early) xr_pdl_launch();                  // (a walk of long portions stays behind this kernel: see xr_launch_behind)
     __shared__ float rows[KD_R][KD_T];
     const int c = blockIdx.x * 128 + threadIdx.x, t0 = blockIdx.y * KD_T, cc = min(c, C - 1);
@@ -801,20 +810,35 @@ k_key_decay(const float* __restrict__ in, long long ld_in, const float* __restri
     if (c >= C) return;
 #pragma unroll
     for (int i = 0; i < KD_T; i++)
-        if (t0 + i < n) out[(size_t)(t0 + i) * C + c] = expf((fminf(z[i], 0.f) - log1pf(expf(-fabsf(z[i])))) * inv_tau);
+        if (t0 + i < n) {
+            const float log_a = (fminf(z[i], 0.f) - log1pf(expf(-fabsf(z[i])))) * inv_tau;
+            out[(size_t)(t0 + i) * C + c] = logs ? log_a : expf(log_a);
+        }
 }
 
 // Linear attention with a decay per key channel: q, k, v as in xr_decay_attention without an activation; the decays' inner values at
-// a_col (R columns of proj), w_t [R][H D], bias [H D] float32; decays [n][H D] float32 scratch.
+// a_col (R columns of proj), w_t [R][H D], bias [H D] float32; decays [n][H D] float32 scratch.  scratch: as in xr_decay_attention.
 XR_EXPORT int xr_key_decay_attention(const float* proj, long long ldp, int q_col, int k_col, int v_col, int a_col, const float* w_t, const float* bias,
                                      int R, float tau, float* decays, float* state, long long state_stride, const int* seg_start, const int* seg_len,
-                                     const int* seg_slot, float* o, int n, int n_seg, int H, int D, int V, float read_scale, cudaStream_t stream) {
+                                     const int* seg_slot, float* o, int n, int n_seg, int H, int D, int V, float read_scale,
+                                     float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || H < 1 || D < 1 || V < 1 || D > 256 || R < 1 || !(tau > 0.f) || n_seg > 65535 || H > 65535 || n > 65535 * 4 ||
         state_stride < (long long)H * D * V)
         return XR_ERR_ARG;
-    const int C = H * D, early = n > 4 * n_seg ? 0 : 1;
-    if (n > 64) xr_launch((k_key_decay<16>), dim3((C + 127) / 128, (n + 15) / 16), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early);
-    else xr_launch((k_key_decay<4>), dim3((C + 127) / 128, (n + 3) / 4), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early);
+    const int C = H * D;
+    ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
+                state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
+    const int chunked = scratch != nullptr && ck_takes(D, V) && ck_aligned(a) && ck_chunks(n, n_seg) <= 65535;
+    if (chunked && scratch_floats < ck_floats(n, n_seg, H, D, V, C, false)) return XR_ERR_ARG;
+    const int early = chunked || n <= 4 * n_seg;
+    if (n > 64) xr_launch((k_key_decay<16>), dim3((C + 127) / 128, (n + 15) / 16), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early, chunked);
+    else xr_launch((k_key_decay<4>), dim3((C + 127) / 128, (n + 3) / 4), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early, chunked);
+    if (chunked) {
+        double* cum = ck_lay_out(a, scratch, n, D, false);
+        a.cum = cum;
+        xr_launch(ck_cumulate, dim3((C + 127) / 128, (unsigned)ck_chunks(n, n_seg)), dim3(128), 0, stream, (const float*)decays, (long long)C, cum, C, a);
+        return ck_run<CK_KEY, false>(a, n, D, stream);
+    }
     return launch_decay_scan<DS_KEY>(proj, ldp, q_col, k_col, v_col, nullptr, state, state_stride, seg_start, seg_len, seg_slot, o, n, n_seg, H, D, V,
                                      true, KeyDecayArgs{decays, read_scale}, stream);
 }
@@ -921,4 +945,14 @@ XR_EXPORT int xr_ssd(const float* proj, long long ldp, int x_col, int dt_col, co
 #undef SS1
 #undef SS_ARGS
     return xr_launch_status();
+}
+
+// float32 values of scratch that a recurrence in chunks takes for a step of n tokens in n_seg portions: H heads with key size D and
+// value size V; decays: CK_HEAD constant per head, CK_TOKEN per token and head (mLSTM, with the sum of keys and its gates' numbers),
+// CK_KEY per key channel.  0: these sizes are the walk's.
+XR_EXPORT long long xr_chunked_floats(int n, int n_seg, int H, int D, int V, int decays) {
+    if (n < 1 || n_seg < 1 || H < 1 || !ck_takes(D, V) || ck_chunks(n, n_seg) > 65535) return 0;
+    const bool norm = decays == CK_TOKEN;
+    const int cols = decays == CK_HEAD ? 0 : (norm ? H : H * D);
+    return ck_floats(n, n_seg, H, D, V, cols, norm) + (norm ? (long long)n * (2LL * H * D + (long long)H * V + 3LL * H) + 16 : 0);
 }

@@ -89,7 +89,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_rmsnorm_act": [_vp, _i, _ll, _vp, _vp, _ll, _i, _i, _f, _vp],
         "xr_delta": [_vp, _i, _ll, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
         "xr_head_norm_gate": [_vp, _vp, _i, _ll, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _vp],
-        "xr_mlstm": [_vp, _i, _ll, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp],
+        "xr_mlstm": [_vp, _i, _ll, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp, _ll, _vp],
         "xr_route_topk": [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _i, _vp],
         "xr_moe_plan": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
         "xr_moe_gather": [_vp, _i, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
@@ -112,13 +112,15 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_row_norm_gate": [_vp, _vp, _ll, _vp, _vp, _i, _i, _i, _f, _f, _vp],
         "xr_ssd": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
         "xr_silu_gate_norm": [_vp, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _f, _vp],
-        "xr_decay_attention": [_vp, _ll, _i, _i, _i, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp],
-        "xr_key_decay_attention": [_vp, _ll, _i, _i, _i, _i, _vp, _vp, _i, _f, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp],
+        "xr_decay_attention": [_vp, _ll, _i, _i, _i, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _ll, _vp],
+        "xr_chunked_floats": [_i, _i, _i, _i, _i, _i],
+        "xr_key_decay_attention": [_vp, _ll, _i, _i, _i, _i, _vp, _vp, _i, _f, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp, _ll, _vp],
     }
     for name, args in sig.items():
         fn = getattr(L, name)
         fn.argtypes = args
         fn.restype = ctypes.c_int
+    L.xr_chunked_floats.restype = _ll
 
 
 def _check(code: int, what: str) -> None:
@@ -938,13 +940,24 @@ def mlstm_state_floats(H: int, D: int, V: int) -> int:
     return H * (D * V + D + 1)
 
 
+def chunked_floats(n: int, n_seg: int, H: int, D: int, V: int, kind: str) -> int:
+    """float32 values of `scratch` with which ``decay_attention`` (kind "head"), ``mlstm`` ("mlstm") and ``key_decay_attention`` ("key")
+    run their recurrence in chunks (csrc/chunked.cuh) instead of token by token, for n tokens in n_seg portions; 0: not for these sizes."""
+    return int(lib().xr_chunked_floats(n, n_seg, H, D, V, ("head", "mlstm", "key").index(kind)))
+
+
+def _floats(scratch: Optional[torch.Tensor]) -> int:
+    assert scratch is None or scratch.dtype == torch.float32
+    return 0 if scratch is None else scratch.numel()
+
+
 def mlstm(proj: torch.Tensor, cols, gates: torch.Tensor, state: torch.Tensor, coef: torch.Tensor, o: torch.Tensor,
           norm_w: torch.Tensor, y: torch.Tensor, seg_start, seg_len, seg_slot, n_seg: int, H: int, D: int, V: int,
-          cap: float, eps: float) -> None:
+          cap: float, eps: float, scratch: Optional[torch.Tensor] = None) -> None:
     """The recurrence over the step's tokens, request by request, from and into `state` [slots, H * (D V + D + 1)].
     proj [n, *]: q, k, v and the output gate at the columns `cols` = (q, k, v, g); gates [n, 2H] float32; coef
-    [n, 3H] and o [n, H V] float32 scratch; y [n, H V] = o / rms(o per head) * norm_w * sigmoid(g)."""
-    _dev(gates, state, coef, o, norm_w, y, seg_start, seg_len, seg_slot)
+    [n, 3H] and o [n, H V] float32 scratch; y [n, H V] = o / rms(o per head) * norm_w * sigmoid(g).  `scratch`: see ``chunked_floats``."""
+    _dev(gates, state, coef, o, norm_w, y, seg_start, seg_len, seg_slot, scratch)
     n = proj.shape[0]
     assert proj.stride(1) == 1 and gates.dtype == torch.float32 and gates.shape == (n, 2 * H) and state.dtype == torch.float32
     assert state.shape[1] == mlstm_state_floats(H, D, V) and coef.numel() >= 3 * n * H and o.shape == (n, H * V)
@@ -952,8 +965,8 @@ def mlstm(proj: torch.Tensor, cols, gates: torch.Tensor, state: torch.Tensor, co
     _check(lib().xr_mlstm(proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), cols[0], cols[1], cols[2], cols[3],
                           gates.data_ptr(), state.data_ptr(), coef.data_ptr(), o.data_ptr(), norm_w.data_ptr(), y.data_ptr(),
                           seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), n, n_seg, H, D, V, float(cap), float(eps),
-                          _stream()), "mlstm")
-    _count(3)
+                          _ptr(scratch), _floats(scratch), _stream()), "mlstm")
+    _count(3 if scratch is None else 8)
 
 
 def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, gate_col: int, w: Optional[torch.Tensor], y: torch.Tensor, H: int, V: int, eps: float,
@@ -1281,28 +1294,28 @@ def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, s
 
 
 def decay_attention(proj: torch.Tensor, cols, decay: torch.Tensor, state: torch.Tensor, seg_start, seg_len, seg_slot, o: torch.Tensor,
-                    n_seg: int, H: int, D: int, V: int, silu: bool = True, read_scale: float = 1.0) -> None:
+                    n_seg: int, H: int, D: int, V: int, silu: bool = True, read_scale: float = 1.0, scratch: Optional[torch.Tensor] = None) -> None:
     """Linear attention with a constant decay per head: S <- decay_h S + k v^T, o = read_scale * S^T q, with q, k, v = proj's columns at
     cols = (q, k, v), behind SiLU or (`silu` False) as they are; proj float32 [n, *] (a step of many tokens activates those columns in
-    place), state float32 [slots, >= H D V], o float32 [n, H V]."""
-    _dev(decay, state, seg_start, seg_len, seg_slot, o)
+    place), state float32 [slots, >= H D V], o float32 [n, H V].  `scratch`: see ``chunked_floats`` (decays in (0, 1] then)."""
+    _dev(scratch, decay, state, seg_start, seg_len, seg_slot, o)
     n = proj.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and o.shape == (n, H * V) and o.dtype == torch.float32
     assert decay.dtype == torch.float32 and decay.numel() == H and state.dtype == torch.float32 and state.shape[1] >= H * D * V
     _check(lib().xr_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], decay.data_ptr(), state.data_ptr(),
                                     state.stride(0), seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), o.data_ptr(), n, n_seg, H, D, V,
-                                    int(silu), float(read_scale), _stream()), "decay_attention")
-    _count(2 if silu and n > 16 else 1)
+                                    int(silu), float(read_scale), _ptr(scratch), _floats(scratch), _stream()), "decay_attention")
+    _count((2 if silu and n > 16 else 1) + (0 if scratch is None else 3))
 
 
 def key_decay_attention(proj: torch.Tensor, cols, inner: int, w_t: torch.Tensor, bias: torch.Tensor, tau: float, decays: torch.Tensor,
                         state: torch.Tensor, seg_start, seg_len, seg_slot, o: torch.Tensor, n_seg: int, H: int, D: int, V: int,
-                        read_scale: float = 1.0) -> None:
+                        read_scale: float = 1.0, scratch: Optional[torch.Tensor] = None) -> None:
     """Linear attention with a decay per key channel and token: S <- diag(a) S + k v^T, o = read_scale * S^T q, a = sigmoid(z)^(1/tau),
     z = w_t^T proj[:, cols[3] : cols[3] + inner] + bias.  proj float32 [n, *]: q, k, v and the decays' inner values at
     cols = (q, k, v, inner); w_t float32 [inner, H D], bias float32 [H D]; decays float32 [n, H D] scratch; state float32
-    [slots, >= H D V], o float32 [n, H V]."""
-    _dev(w_t, bias, decays, state, seg_start, seg_len, seg_slot, o)
+    [slots, >= H D V], o float32 [n, H V].  `scratch`: see ``chunked_floats``."""
+    _dev(scratch, w_t, bias, decays, state, seg_start, seg_len, seg_slot, o)
     n = proj.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and o.shape == (n, H * V) and o.dtype == torch.float32
     assert w_t.dtype == torch.float32 and w_t.shape == (inner, H * D) and bias.dtype == torch.float32 and bias.numel() == H * D
@@ -1310,8 +1323,8 @@ def key_decay_attention(proj: torch.Tensor, cols, inner: int, w_t: torch.Tensor,
     assert state.dtype == torch.float32 and state.shape[1] >= H * D * V
     _check(lib().xr_key_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], cols[3], w_t.data_ptr(), bias.data_ptr(), int(inner),
                                         float(tau), decays.data_ptr(), state.data_ptr(), state.stride(0), seg_start.data_ptr(), seg_len.data_ptr(),
-                                        seg_slot.data_ptr(), o.data_ptr(), n, n_seg, H, D, V, float(read_scale), _stream()), "key_decay_attention")
-    _count(2)
+                                        seg_slot.data_ptr(), o.data_ptr(), n, n_seg, H, D, V, float(read_scale), _ptr(scratch), _floats(scratch), _stream()), "key_decay_attention")
+    _count(2 if scratch is None else 6)
 
 
 def ssd_state_floats(H: int, G: int, N: int, V: int, taps: int) -> int:

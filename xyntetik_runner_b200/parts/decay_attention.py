@@ -24,6 +24,7 @@ import torch
 from .. import kernels
 from ..weights.loader import TensorSpec
 from .base import Mixer, StateNeed, register_mixer
+from .chunks import chunk_scratch
 from .linear import Linear
 
 
@@ -106,8 +107,10 @@ class DecayLinearAttention(_LinearAttention):
         self.decay = torch.tensor(self.decay_values, dtype=torch.float32, device=rt.device)
 
     def walk(self, ctx, proj, cols, lay, o):
+        # (in chunks a decay is an exponential of its logarithm)
+        scratch = chunk_scratch(ctx, "head", self.H, self.D, self.V) if all(0.0 < d <= 1.0 for d in self.decay_values) else None
         kernels.decay_attention(proj, cols, self.decay, lay.state, ctx.seg_start, ctx.seg_len, ctx.seg_slot, o, ctx.n_seg, self.H, self.D,
-                                self.V, silu=self.silu, read_scale=self.read_scale)
+                                self.V, silu=self.silu, read_scale=self.read_scale, scratch=scratch)
 
 
 class KeyDecayLinearAttention(_LinearAttention):
@@ -149,7 +152,8 @@ class KeyDecayLinearAttention(_LinearAttention):
         H, D, V = self.H, self.D, self.V
         decays = ctx.buf("decay_keys", (proj.shape[0], H * D), torch.float32)
         kernels.key_decay_attention(proj, cols + (2 * H * D + 2 * H * V,), self.inner, self.a2_t, self.a2_b, self.tau, decays, lay.state,
-                                    ctx.seg_start, ctx.seg_len, ctx.seg_slot, o, ctx.n_seg, H, D, V, read_scale=self.read_scale)
+                                    ctx.seg_start, ctx.seg_len, ctx.seg_slot, o, ctx.n_seg, H, D, V, read_scale=self.read_scale,
+                                    scratch=chunk_scratch(ctx, "key", H, D, V))
 
 
 register_mixer("decay_linear_attention", DecayLinearAttention)

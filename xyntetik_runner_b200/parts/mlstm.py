@@ -16,6 +16,7 @@ import torch
 from .. import kernels
 from ..weights.loader import TensorSpec
 from .base import Mixer, StateNeed, register_mixer
+from .chunks import chunk_scratch
 from .linear import Linear
 
 
@@ -73,7 +74,8 @@ class MLSTM(Mixer):
         o = ctx.buf("mlstm_o", (n, H * V), torch.float32)
         y = ctx.buf("attn_out", (n, H * V), ctx.act_dtype)
         kernels.mlstm(proj, (0, H * D, 2 * H * D, 2 * H * D + H * V), gates, lay.state, coef, o, self.norm_w, y,
-                      ctx.seg_start, ctx.seg_len, ctx.seg_slot, ctx.n_seg, H, D, V, self.cap, self.eps)
+                      ctx.seg_start, ctx.seg_len, ctx.seg_slot, ctx.n_seg, H, D, V, self.cap, self.eps,
+                      scratch=chunk_scratch(ctx, "mlstm", H, D, V))
         ctx.set_pending(x, self.out.forward(y, x, accumulate=True, defer=True))
 
 
