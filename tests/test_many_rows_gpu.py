@@ -373,3 +373,38 @@ def test_matrix_memory_with_gates_in_chunks(H, D, V, dtype):
         assert ((got[at].double() - torch.stack(out)).abs() <= 144 * 2.0 ** -24 * torch.stack(bound)).all()
         end = torch.cat([Sm.reshape(H, -1), nm, mx[:, None]], dim=1).reshape(-1)
         _close(state[slot].cpu(), end, walk_state[slot].cpu())
+
+
+# ---- recurrences a token a step ---------------------------------------------------------------------------------------
+@pytest.mark.parametrize("kind,H,D,V", [("head", 3, 64, 40), ("head", 2, 128, 128), ("head", 1, 100, 4), ("key", 2, 36, 24), ("key", 1, 128, 72), ("ssd", 2, 64, 64),
+                                        ("ssd", 4, 100, 20)])
+def test_single_tokens_follow_the_walk_bit_for_bit(kind, H, D, V):
+    """Two requests' tokens in steps of one token each against the same tokens in one step: read-outs, states and tails."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(H * D + V)
+    f = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    S, T, taps, slots = 2, 7, 4, [2, 0]
+    G, R = H // 2 if kind == "ssd" else H, 8
+    CH = H * V + 2 * G * D
+    width = CH + H if kind == "ssd" else 2 * H * D + H * V + (R if kind == "key" else 0)
+    rows = f(S, T, width)
+    dec, w_t, bias = torch.rand(H, generator=g).to(DEV), f(R, H * D), f(H * D)
+    conv, cb, dtb, neg_a, skip = f(CH, taps), f(CH), f(H), -torch.rand(H, generator=g).to(DEV), f(H)
+    state0 = f(4, kernels.ssd_state_floats(H, G, D, V, taps) if kind == "ssd" else H * D * V)
+
+    def step(x, counts, state):
+        n = x.shape[0]
+        starts, o = [0, counts[0]], torch.empty(n, H * V, device=DEV)
+        where = (state, _i32(starts), _i32(counts), _i32(slots))
+        if kind == "head":
+            kernels.decay_attention(x.clone(), (0, H * D, 2 * H * D), dec, *where, o, S, H, D, V, read_scale=0.5)
+        elif kind == "key":
+            kernels.key_decay_attention(x, (0, H * D, 2 * H * D, 2 * H * D + H * V), R, w_t, bias, 3.0, torch.empty(n, H * D, device=DEV), *where, o, S, H, D, V)
+        else:
+            kernels.ssd(x, 0, CH, conv, cb, dtb, neg_a, skip, state, _i32([0] * counts[0] + [1] * counts[1]), *where[1:], torch.empty(n, CH, device=DEV),
+                        torch.empty(n, 2 * H, device=DEV), o, S, H, G, D, V, taps)
+        return o.view(S, -1, H * V)
+    whole, single = state0.clone(), state0.clone()
+    want = step(rows.reshape(S * T, width), [T, T], whole)
+    got = torch.cat([step(rows[:, t].contiguous(), [1, 1], single) for t in range(T)], dim=1)
+    assert torch.equal(got, want) and torch.equal(single, whole) and torch.equal(whole[1], state0[1]) and not torch.equal(whole[0], state0[0])

@@ -56,7 +56,7 @@ __device__ __forceinline__ void rg_finish(float ra, float ri, float u, float rat
 
 // Many tokens: both gate products as one tile product (simt_tile.cuh) over a channel block's inputs u: a tile's rows are, eight and
 // eight, rows of Wa and of Wi for the same outputs, so that a thread holds both sums of its outputs and finishes them in registers.
-// What bounds it: the float32 FMA pipes; the matrices come from L2.  1,901 tokens, 2,560 channels in ten blocks: 180 us,
+// What bounds it: the float32 FMA pipes; the matrices come from L2.  1,901 tokens, 2,560 channels in ten blocks: 193 us,
 // where a thread an output with eight tokens' sums, which reads its weights from L2 for every eight tokens, took 360.
 template <int WM, int WN, int TM, int TN>
 __global__ void __launch_bounds__(32 * WM * WN)
@@ -701,6 +701,114 @@ k_decay_scan(const float* __restrict__ proj, long long ldp, int q_col, int k_col
                                   blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
 }
 
+// A step of single tokens (JD 2: D <= 64, JD 4: D <= 128; everything on 16-byte borders): a warp eight value columns, whose state it has
+// on its way at once, four warps a block, many blocks an SM.  What bounds it: the state's way to and from memory; the walk above, whose
+// blocks hold two chunks of rows that one token does not fill, has too little of it in flight.  The arithmetic is the walk's, sum for
+// sum, so a state does not depend on which of the two a token took.  32 requests, 8 heads of 128 x 128: 7.3 us, the walk 20.6; 1
+// request, 4 heads of 128 x 128: 2.8 / 4.9.
+#define DT_COLS 8
+template <int JD, int KIND>
+__global__ void __launch_bounds__(128)
+k_decay_step(const float* __restrict__ proj, long long ldp, int q_col, int k_col, int v_col, const float* __restrict__ decay, float* __restrict__ state,
+             long long state_stride, const int* __restrict__ seg_start, const int* __restrict__ seg_len, const int* __restrict__ seg_slot,
+             float* __restrict__ o, int H, int D, int V, int activated, SsdArgs ssd, KeyDecayArgs key) {
+    xr_pdl_launch();
+    constexpr bool SSD = KIND == DS_SSD, KEY = KIND == DS_KEY;
+    constexpr int NP = JD / 2;
+    const int lane = threadIdx.x & 31, v0 = (blockIdx.x * 4 + (threadIdx.x >> 5)) * DT_COLS, h = blockIdx.y, seg = blockIdx.z;
+    const int start = seg_start[seg], len = seg_len[seg], g = SSD ? h / ssd.rep : h;
+    const float dec = KIND == DS_HEAD ? decay[h] : 0.f, skip = SSD ? ssd.skip[h] : 0.f;
+    float* slot = state + (size_t)seg_slot[seg] * state_stride;
+    float* st = slot + (size_t)h * D * V + lane * JD;
+    const bool live = lane * JD < D;
+    auto pairs = [&](const float* p, F2* out) {
+        if constexpr (JD == 4) {
+            const ulonglong2 x = live ? *reinterpret_cast<const ulonglong2*>(p) : make_ulonglong2(0, 0);
+            out[0] = x.x; out[1] = x.y;
+        } else {
+            out[0] = live ? *reinterpret_cast<const F2*>(p) : 0;
+        }
+    };
+    auto silu = [&](F2 x) { const float2 y = f2_unpack(x); return f2_pack(rc_silu(y.x), rc_silu(y.y)); };
+    xr_pdl_wait();
+    F2 s[DT_COLS][NP];
+#pragma unroll
+    for (int c = 0; c < DT_COLS; c++) pairs(st + (size_t)min(v0 + c, V - 1) * D, s[c]);
+    for (int t = start; t < start + len; t++) {
+        const float* row = proj + (size_t)t * ldp;
+        F2 q[NP], k[NP], ak[KEY ? NP : 1];
+        pairs(row + q_col + g * D + lane * JD, q);
+        pairs(row + k_col + g * D + lane * JD, k);
+        if constexpr (KEY) pairs(key.rows + ((size_t)t * H + h) * D + lane * JD, ak);
+        float v = lane < DT_COLS && v0 + lane < V ? row[v_col + h * V + v0 + lane] : 0.f;
+        float2 ad = make_float2(dec, 1.f);
+        if constexpr (SSD) ad = *reinterpret_cast<const float2*>(ssd.coef + ((size_t)t * H + h) * 2);
+        if (!activated) {
+#pragma unroll
+            for (int j = 0; j < NP; j++) { q[j] = silu(q[j]); k[j] = silu(k[j]); }
+            v = rc_silu(v);
+        }
+        const F2 a = f2_pack(ad.x, ad.x);
+        float acc[DT_COLS];
+#pragma unroll
+        for (int c = 0; c < DT_COLS; c++) {
+            float vc = __shfl_sync(0xffffffffu, v, c);
+            if constexpr (SSD) vc *= ad.y;
+            const F2 vv = f2_pack(vc, vc);
+            F2 y;
+#pragma unroll
+            for (int j = 0; j < NP; j++) {
+                s[c][j] = f2_fma(KEY ? ak[KEY ? j : 0] : a, s[c][j], f2_mul(k[j], vv));
+                y = j == 0 ? f2_mul(s[c][j], q[j]) : f2_fma(s[c][j], q[j], y);
+            }
+            const float2 sum = f2_unpack(y);
+            acc[c] = sum.x + sum.y;
+        }
+        // eight sums a lane -> one, over lanes 16, 8, 4, 2, 1 apart like the walk
+#pragma unroll
+        for (int w = 4, bit = 16; w > 0; w >>= 1, bit >>= 1) {
+            const bool upper = lane & bit;
+#pragma unroll
+            for (int c = 0; c < w; c++) {
+                const float send = upper ? acc[c] : acc[c + w], keep = upper ? acc[c + w] : acc[c];
+                acc[c] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+            }
+        }
+        float y = acc[0];
+        y += __shfl_xor_sync(0xffffffffu, y, 2);
+        y += __shfl_xor_sync(0xffffffffu, y, 1);
+        const int c = lane >> 2;
+        const float raw = __shfl_sync(0xffffffffu, v, c);
+        if (SSD) y = fmaf(skip, raw, y);
+        else y *= key.read_scale;
+        if ((lane & 3) == 0 && v0 + c < V) o[(size_t)t * H * V + (size_t)h * V + v0 + c] = y;
+    }
+    if (live)
+#pragma unroll
+        for (int c = 0; c < DT_COLS; c++)
+            if (v0 + c < V) {
+                if constexpr (JD == 4) *reinterpret_cast<ulonglong2*>(st + (size_t)(v0 + c) * D) = make_ulonglong2(s[c][0], s[c][1]);
+                else *reinterpret_cast<F2*>(st + (size_t)(v0 + c) * D) = s[c][0];
+            }
+    if constexpr (SSD)
+        if (ssd.taps > 1)
+            xr_tail_update<float>(ssd.raw, ssd.ld_raw, slot + (size_t)H * V * D, start, len, ssd.CH, ssd.taps, blockIdx.y * gridDim.x + blockIdx.x,
+                                  gridDim.x * gridDim.y);
+}
+
+// Launches the kernel above where it applies: a step of single tokens, sizes and addresses on 16-byte borders.
+template <int KIND>
+static bool launch_decay_step(const float* proj, long long ldp, int q_col, int k_col, int v_col, const float* decay, float* state, long long state_stride,
+                              const int* seg_start, const int* seg_len, const int* seg_slot, float* o, int n, int n_seg, int H, int D, int V, int activated,
+                              const SsdArgs& ssd, const KeyDecayArgs& key, cudaStream_t stream) {
+    const bool even = !((D | ldp | q_col | k_col | state_stride) & 3) && !(((uintptr_t)proj | (uintptr_t)state | (uintptr_t)key.rows) & 15);
+    if (n != n_seg || D <= 32 || D > 128 || !even) return false;
+    const dim3 grid((V + 4 * DT_COLS - 1) / (4 * DT_COLS), H, n_seg);
+    if (D <= 64) xr_launch((k_decay_step<2, KIND>), grid, dim3(128), 0, stream, proj, ldp, q_col, k_col, v_col, decay, state, state_stride, seg_start, seg_len, seg_slot, o, H, D, V, activated, ssd, key);
+    else xr_launch((k_decay_step<4, KIND>), grid, dim3(128), 0, stream, proj, ldp, q_col, k_col, v_col, decay, state, state_stride, seg_start, seg_len, seg_slot, o, H, D, V, activated, ssd, key);
+    return true;
+}
+
 // Value columns a warp: two where the walk's length is what counts (few blocks, each with its SM to itself), four where there are more
 // blocks than the machine holds at once (half the reads of shared memory per state element).  A column's arithmetic is the same.
 static inline bool decay_scan_wide(int V, int H, int n_seg) { return (long long)((V + 15) / 16) * H * n_seg > 2LL * xr_sm_count(); }
@@ -714,6 +822,9 @@ template <int KIND>
 static int launch_decay_scan(const float* proj, long long ldp, int q_col, int k_col, int v_col, const float* decay, float* state, long long state_stride,
                              const int* seg_start, const int* seg_len, const int* seg_slot, float* o, int n, int n_seg, int H, int D, int V, bool ready,
                              KeyDecayArgs key, cudaStream_t stream) {
+    if (launch_decay_step<KIND>(proj, ldp, q_col, k_col, v_col, decay, state, state_stride, seg_start, seg_len, seg_slot, o, n, n_seg, H, D, V, ready ? 1 : 0,
+                                SsdArgs{}, key, stream))
+        return xr_launch_status();
     // (a step with long portions is a few long-lived blocks: they start behind the kernel ahead, not into its last wave)
     const bool walk = n > 4 * n_seg;
     // 16 bytes a load where every row, column offset and size falls on a 16-byte border
@@ -922,6 +1033,9 @@ XR_EXPORT int xr_ssd(const float* proj, long long ldp, int x_col, int dt_col, co
     const bool walk = n > 4 * n_seg;
     const bool vec = !((N | V) & 3) && !((uintptr_t)xbc & 15);
     const SsdArgs ssd{coef, skip, proj + x_col, ldp, CH, taps, H / G};
+    if (launch_decay_step<DS_SSD>((const float*)xbc, (long long)CH, H * V + G * N, H * V, 0, nullptr, state, state_stride, seg_start, seg_len, seg_slot, y, n, n_seg, H, N, V,
+                                  1, ssd, KeyDecayArgs{nullptr, 1.0f}, stream))
+        return xr_launch_status();
 #define SS_ARGS(JD, VC, CK) dim3((V + VC * DA_WARPS - 1) / (VC * DA_WARPS), H, n_seg), dim3(32 * DA_WARPS), decay_scan_smem(JD, VC, CK, DS_SSD), stream, (const float*)xbc, (long long)CH,            \
                     H * V + G * N, H * V, 0, (const float*)nullptr, state, state_stride, seg_start, seg_len, seg_slot, y, H, N, V, 1, ssd, KeyDecayArgs{nullptr, 1.0f}
 #define SS1(JD, VC, CK, VEC)                                                                                                                 \
