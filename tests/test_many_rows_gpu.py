@@ -408,3 +408,35 @@ def test_single_tokens_follow_the_walk_bit_for_bit(kind, H, D, V):
     want = step(rows.reshape(S * T, width), [T, T], whole)
     got = torch.cat([step(rows[:, t].contiguous(), [1, 1], single) for t in range(T)], dim=1)
     assert torch.equal(got, want) and torch.equal(single, whole) and torch.equal(whole[1], state0[1]) and not torch.equal(whole[0], state0[0])
+
+
+# ---- streams of many rows ----------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n,width,dtype", [(33, 2048, torch.bfloat16), (40, 4096, torch.float32), (35, 2052, torch.bfloat16), (34, 70, torch.bfloat16),
+                                           (33, 36, torch.float32)])
+def test_streams_of_many_rows(n, width, dtype):
+    """Rows that take 16 bytes an access and rows that do not, the widest that stay in registers: the norm that is added, the average over
+    depth, the scaled sum; what is cleared is zero.  A norm's sum of `width` squares and three more roundings; an average's k + 1 terms."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + width)
+    f = lambda *s: torch.randn(*s, generator=g)
+    eps32 = 2.0 ** -24
+    half = 2.0 ** -8 if dtype == torch.bfloat16 else eps32
+    d0, x0, gain = f(n, width), f(n, width), torch.tensor([0.7])
+    d, x, cast = d0.to(DEV), x0.to(DEV), torch.empty(n, width, dtype=dtype, device=DEV)
+    kernels.norm_add(d, x, gain.to(DEV), 1e-5, cast=cast, clear=True)
+    add = d0.double() / torch.sqrt(d0.double().pow(2).mean(1, keepdim=True) + 1e-5) * 0.7
+    want = x0.double() + add
+    tol = eps32 * (want.abs() + (width + 4) * add.abs())
+    assert ((x.cpu().double() - want).abs() <= tol).all() and ((cast.cpu().double() - want).abs() <= tol + half * want.abs()).all() and not d.any()
+    k = 10
+    first, hist, w = f(n, width), f(k, n, width), f(k + 1)
+    x, past = x0.to(DEV), hist.to(DEV)
+    kernels.depth_average(x, first.to(DEV), past, w.to(DEV), k, cast=cast)
+    terms = torch.cat([first[None], hist[:k - 1], x0[None]]).double() * w.double()[:, None, None]
+    want, tol = terms.sum(0), (k + 1) * eps32 * terms.abs().sum(0)
+    assert ((x.cpu().double() - want).abs() <= tol).all() and ((cast.cpu().double() - want).abs() <= tol + half * want.abs()).all()
+    assert torch.equal(past.cpu(), torch.cat([hist[:k - 1], x0[None]]))
+    for clear in (False, True):
+        d, x = d0.to(DEV), x0.to(DEV)
+        kernels.scaled_add(x, d, 0.3, clear=clear)
+        assert torch.allclose(x.cpu(), x0 + 0.3 * d0, rtol=1e-6, atol=1e-6) and torch.equal(d.cpu(), torch.zeros_like(d0) if clear else d0)

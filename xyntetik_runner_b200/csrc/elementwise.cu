@@ -813,20 +813,35 @@ XR_EXPORT int xr_residual_add(float* x, const void* dlt, int dtype, int n, int d
 
 // ---------------------------------------------------------------------------
 // x[t][i] += m * d[t][i] on float32 streams: a block that runs its sublayers side by side collects their sum in d
-// and adds it to the residual stream once, times the model's residual multiplier.
+// and adds it to the residual stream once, times the model's residual multiplier; with `clear`, d is zeroed behind the read, ready
+// for the next block's sublayers to add into.  What bounds it: memory; UNIT floats an access.
 // ---------------------------------------------------------------------------
-__global__ void k_scaled_add(float* __restrict__ x, const float* __restrict__ d, float m, size_t total) {
+template <int UNIT>
+__global__ void k_scaled_add(float* __restrict__ x, float* __restrict__ d, float m, int clear, size_t total) {
     xr_pdl_launch();
     xr_pdl_wait();
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x)
-        x[i] = fmaf(m, d[i], x[i]);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total / UNIT; i += (size_t)gridDim.x * blockDim.x) {
+        if constexpr (UNIT == 4) {
+            float4 v = reinterpret_cast<const float4*>(x)[i];
+            const float4 a = reinterpret_cast<const float4*>(d)[i];
+            v = make_float4(fmaf(m, a.x, v.x), fmaf(m, a.y, v.y), fmaf(m, a.z, v.z), fmaf(m, a.w, v.w));
+            reinterpret_cast<float4*>(x)[i] = v;
+            if (clear) reinterpret_cast<float4*>(d)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        } else {
+            x[i] = fmaf(m, d[i], x[i]);
+            if (clear) d[i] = 0.f;
+        }
+    }
 }
 
-XR_EXPORT int xr_scaled_add(float* x, const float* d, float m, int n, int width, cudaStream_t stream) {
+XR_EXPORT int xr_scaled_add(float* x, float* d, float m, int clear, int n, int width, cudaStream_t stream) {
     if (n < 1 || width < 1) return XR_ERR_ARG;
-    size_t total = (size_t)n * width;
-    int blocks = (int)((total + 255) / 256 < (size_t)xr_sm_count() * 16 ? (total + 255) / 256 : xr_sm_count() * 16);
-    xr_launch(k_scaled_add, dim3(blocks), dim3(256), 0, stream, x, d, m, total);
+    const size_t total = (size_t)n * width;
+    const bool four = !(total & 3) && !(((uintptr_t)x | (uintptr_t)d) & 15);
+    const size_t units = four ? total / 4 : total;
+    const int blocks = (int)((units + 255) / 256 < (size_t)xr_sm_count() * 16 ? (units + 255) / 256 : xr_sm_count() * 16);
+    if (four) xr_launch(k_scaled_add<4>, dim3(blocks), dim3(256), 0, stream, x, d, m, clear, total);
+    else xr_launch(k_scaled_add<1>, dim3(blocks), dim3(256), 0, stream, x, d, m, clear, total);
     return xr_launch_status();
 }
 

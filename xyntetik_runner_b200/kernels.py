@@ -72,7 +72,7 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_sample_one_block": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
         "xr_logprob": [_vp, _ll, _i, _i, _vp, _vp, _vp],
         "xr_random_normal": [_vp, _i, _ll, ctypes.c_ulonglong, ctypes.c_ulonglong, _f, _f, _vp],
-        "xr_scaled_add": [_vp, _vp, _f, _i, _i, _vp],
+        "xr_scaled_add": [_vp, _vp, _f, _i, _i, _i, _vp],
         "xr_stream_step": [_vp, _vp, _vp, _i, _i, _vp],
         "xr_sigmoid_gate": [_vp, _ll, _vp, _ll, _i, _i, _i, _i, _i, _i, _vp],
         "xr_concat_cast": [_vp, _vp, _vp, _i, _i, _i, _vp],
@@ -766,11 +766,11 @@ def attention_tc_flat(q: torch.Tensor, kv: torch.Tensor, tail: torch.Tensor, out
 
 # ---------------------------------------------------------------------------
 # Kernels of blocks that run their sublayers side by side, of joined streams and of capped logits
-def scaled_add(x: torch.Tensor, d: torch.Tensor, m: float) -> None:
-    """x += m * d on float32 streams."""
+def scaled_add(x: torch.Tensor, d: torch.Tensor, m: float, clear: bool = False) -> None:
+    """x += m * d on float32 streams; with `clear`, d is zero afterwards."""
     _dev(x, d)
     assert x.dtype == torch.float32 and d.dtype == torch.float32 and x.shape == d.shape
-    _check(lib().xr_scaled_add(x.data_ptr(), d.data_ptr(), float(m), x.shape[0], x.shape[1], _stream()), "scaled_add")
+    _check(lib().xr_scaled_add(x.data_ptr(), d.data_ptr(), float(m), int(clear), x.shape[0], x.shape[1], _stream()), "scaled_add")
     _count()
 
 

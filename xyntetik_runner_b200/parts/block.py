@@ -113,12 +113,13 @@ class ParallelBlock(Block):
                 self.feed_forward.forward(ctx, h2, x)
             return
         d = ctx.buf("block_sum", (n, width), torch.float32)
-        d.zero_()
+        # the sum starts at zero once a step; every block clears it behind its read
+        ctx.once(("block_sum", d.data_ptr()), lambda: (d.zero_(), True)[1])
         self.mixer.forward(ctx, h, d, lay)
         if self.feed_forward is not None:
             self.feed_forward.forward(ctx, h2, d)
         ctx.materialize(d)
-        kernels.scaled_add(x, d, self.mult)
+        kernels.scaled_add(x, d, self.mult, clear=True)
 
 
 register_block("parallel", ParallelBlock)
