@@ -440,3 +440,45 @@ def test_streams_of_many_rows(n, width, dtype):
         d, x = d0.to(DEV), x0.to(DEV)
         kernels.scaled_add(x, d, 0.3, clear=clear)
         assert torch.allclose(x.cpu(), x0 + 0.3 * d0, rtol=1e-6, atol=1e-6) and torch.equal(d.cpu(), torch.zeros_like(d0) if clear else d0)
+
+
+# ---- choice, plan and gather of few tokens in one launch -------------------------------------------------------------
+@pytest.mark.parametrize("n,E,identity,top,mode,splits,align", [(1, 16, 0, 2, 0, 1, 16), (8, 64, 0, 6, 0, 8, 16), (32, 16, 0, 2, 1, 3, 16), (40, 12, 4, 2, 2, 2, 16),
+                                                                (64, 3, 0, 3, 0, 9, 32), (85, 40, 0, 3, 1, 1, 16)])
+def test_route_few_against_its_parts(n, E, identity, top, mode, splits, align):
+    """The same choice and weights as the kernels it stands for; a plan that gives every pair a row in a tile of its expert and no two
+    the same; the rows themselves; tiles without rows marked; columns behind the router's outputs carried along."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + E)
+    outputs, W, extra = E + identity, 64, 0 if mode == 2 else 1
+    ldz = outputs + extra
+    parts = torch.randn(splits, n, ldz, generator=g).to(DEV)
+    h = torch.randn(n, W, generator=g).bfloat16().to(DEV)
+    corr = None if mode == 0 else (0.3 * torch.randn(outputs, generator=g)).to(DEV)
+    total = parts[0].clone()
+    for s in range(1, splits):
+        total += parts[s]
+    zs = total.clone() if splits == 1 else torch.full((n, ldz), float("nan"), device=DEV)
+    pairs = n * top
+    mt = kernels.moe_max_tiles(pairs, E, align)
+    wts, pair_row = torch.empty(n, top, device=DEV), torch.empty(pairs, dtype=torch.int32, device=DEV)
+    tile_group = torch.full((mt,), 77, dtype=torch.int32, device=DEV)
+    xs = torch.full((mt * align, W), 3.0, dtype=torch.bfloat16, device=DEV)
+    groups = (4, 2) if mode == 2 else (1, 1)
+    kernels.route_few(zs if splits == 1 else parts, splits, zs, outputs, E, top, wts, pair_row, tile_group, align, h, xs, mode, corr, *groups, 1.7)
+    assert torch.equal(zs, total)
+    ids, want = torch.empty(n, top, dtype=torch.int32, device=DEV), torch.empty(n, top, device=DEV)
+    if mode == 2:
+        kernels.route_groups(zs, ids, want, top, corr, *groups, 1.7)
+    else:
+        kernels.route_topk(zs[:, :outputs], ids, want, top, sigmoid_scores=mode == 1, correction=corr)
+    assert torch.equal(wts, want)
+    ids, rows, tiles = ids.reshape(-1).tolist(), pair_row.tolist(), tile_group.tolist()
+    real = [r for r in rows if r >= 0]
+    assert len(set(real)) == len(real)
+    for p, (e, r) in enumerate(zip(ids, rows)):
+        assert (r < 0) == (e >= E)
+        if r >= 0:
+            assert tiles[r // align] == e and torch.equal(xs[r], h[p // top])
+    used = sum(-(-ids.count(e) // align) for e in range(E))
+    assert all(0 <= t < E for t in tiles[:used]) and all(t == -1 for t in tiles[used:])

@@ -94,6 +94,8 @@ def _declare(L: ctypes.CDLL) -> None:
         "xr_moe_plan": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
         "xr_moe_gather": [_vp, _i, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
         "xr_gemm_tc_grouped": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _i, _vp, _i, _vp, _vp],
+        "xr_route_few_supported": [_i, _i, _i, _i, _i, _i],
+        "xr_route_few": [_vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _f, _vp, _vp, _vp, _i, _i, _vp, _ll, _vp, _i, _vp],
         "xr_gemm_tc_pairs_available": [],
         "xr_gemm_tc_grouped_pairs": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _vp, _i, _i, _vp, _vp],
         "xr_moe_plan_tiles": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
@@ -1109,6 +1111,29 @@ def gemm_tc_grouped_pairs(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Te
     _check(lib().xr_gemm_tc_grouped_pairs(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
                                           float(act_limit), n, n_out, k, x.stride(0), out.stride(0), tiles.data_ptr(), max_tiles,
                                           w_packed.shape[0], ws.status_ptr, _stream()), "gemm_tc_grouped_pairs")
+    _count()
+
+
+def route_few_supported(n: int, ldz: int, outputs: int, E: int, top: int, width: int) -> bool:
+    return lib().xr_route_few_supported(n, ldz, outputs, E, top, width) == 1
+
+
+def route_few(z: torch.Tensor, splits: int, zs: torch.Tensor, outputs: int, E: int, top: int, wts: torch.Tensor, pair_row: torch.Tensor,
+              tile_group: torch.Tensor, align: int, h: torch.Tensor, xs: torch.Tensor, mode: int = 0, correction: Optional[torch.Tensor] = None,
+              groups: int = 1, keep: int = 1, scale: float = 1.0) -> None:
+    """Choice, plan and gather of a step of few tokens in one launch: ``route_topk`` (mode 0, or 1 with sigmoid scores) or ``route_groups``
+    (mode 2) over the logits zs [n, *], whose first `outputs` columns count, then ``moe_plan`` and ``moe_gather`` (rows of padding are
+    left as they are).  With splits > 1, z holds the partial sums [splits][n][zs' columns] and zs receives them added; else z is zs."""
+    _dev(z, zs, wts, pair_row, tile_group, xs, correction)
+    n, ldz = zs.shape
+    max_tiles = moe_max_tiles(n * top, E, align)
+    assert zs.dtype == torch.float32 and z.dtype == torch.float32 and z.numel() >= splits * n * ldz and wts.dtype == torch.float32
+    assert correction is None or (correction.dtype == torch.float32 and correction.numel() == outputs)
+    assert h.dtype == torch.bfloat16 and xs.dtype == torch.bfloat16 and h.stride(1) == 1 and h.shape == (n, xs.shape[1])
+    assert wts.numel() >= n * top and pair_row.numel() >= n * top and tile_group.numel() >= max_tiles and xs.shape[0] >= max_tiles * align
+    _check(lib().xr_route_few(z.data_ptr(), splits, zs.data_ptr(), ldz, n, outputs, E, top, _ptr(correction), mode, groups, keep, float(scale),
+                              wts.data_ptr(), pair_row.data_ptr(), tile_group.data_ptr(), align, max_tiles, h.data_ptr(), h.stride(0), xs.data_ptr(),
+                              h.shape[1], _stream()), "route_few")
     _count()
 
 

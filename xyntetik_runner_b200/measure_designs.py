@@ -222,7 +222,7 @@ FAMILIES = {
     "flat_rows": "latent attention: per-head products", "attention_tc_flat": "latent attention: scores and sums",
     "moe_gather": "grouped products (experts, per-head)", "heads_gather": "grouped products (experts, per-head)",
     "heads_scatter_gate": "grouped products (experts, per-head)",
-    "mlstm": "mlstm recurrence", "route_topk": "routing", "moe_plan": "routing", "moe_plan_tiles": "routing", "moe_gemm": "experts' products", "moe_combine": "experts' sum",
+    "mlstm": "mlstm recurrence", "route_topk": "routing", "moe_plan": "routing", "moe_plan_tiles": "routing", "route_few": "routing", "moe_gemm": "experts' products", "moe_combine": "experts' sum",
     "delta": "delta recurrence", "head_norm_gate": "gated norm of the recurrence", "qk_norm_rope_store": "rotation + cache store",
     "rmsnorm_act": "norms", "ssd": "state-space recurrence", "silu_gate_norm": "gated norm of the recurrence", "route_groups": "routing",
     "sigmoid_gate": "output gates", "stream_step": "stream kernels",

@@ -37,6 +37,9 @@ from .linear import Linear
 # 50 rows 41 / 39, 97 rows 66 / 48.
 PAIRS_FROM = 32
 
+# The choice, the plan and the gather of a step of so few single tokens are one kernel: csrc/moe.cu, k_route_few.
+FEW_TOKENS = 8
+
 
 class PendingExperts:
     """The weighted sum of a step's expert outputs (and of the shared expert's), still to be added into x: by ``finish``, or by the
@@ -158,17 +161,12 @@ class RoutedExperts(FeedForward):
         n, top, E = h.shape[0], self.top, self.E
         pairs = n * top
         on_pairs = self.tensor_cores and pairs > PAIRS_FROM * E and kernels.pairs_available()
+        # (steps of single tokens, which are chains of launches; in a portion's step the choice stays a kernel of its own)
+        few = (self.tensor_cores and ctx.decode_only and n <= FEW_TOKENS and not on_pairs and h.stride(0) % 8 == 0
+               and kernels.route_few_supported(n, self.router.n_out, self.outputs, E, top, self.width))
         zs = ctx.buf("moe_logits", (n, self.router.n_out), torch.float32)
         wts = ctx.buf("moe_weights", (n, top), torch.float32)
-        self.router.forward(h, zs)
-        z = zs if self.router.n_out == self.outputs else zs[:, :self.outputs]        # (a shared expert's gate is one column more)
-        ids = ctx.buf("moe_ids", (n, top), torch.int32)
-        if self.softmax_all:
-            kernels.route_groups(z, ids, wts, top, self.correction, *self.groups, self.scale)
-        elif self.sigmoid:
-            kernels.route_topk(z, ids, wts, top, sigmoid_scores=True, correction=self.correction)
-        else:
-            kernels.route_topk(z, ids, wts, top)
+        pend = self.router.forward(h, zs, defer=few)
         align = 1 if on_pairs else (self._row_tile(pairs, E) if self.tensor_cores else kernels.moe_tile_rows())
         if on_pairs:
             max_tiles, rows = kernels.moe_tiles_room(pairs, E)
@@ -180,15 +178,29 @@ class RoutedExperts(FeedForward):
             tile_group = ctx.buf("moe_tile_group", (max_tiles,), torch.int32)
         if self.tensor_cores:
             xs = ctx.buf("moe_rows", (rows, self.width), ctx.act_dtype)
-        row_src = ctx.buf("moe_row_src", (rows,), torch.int32)
-        if on_pairs:
-            tiles = ctx.buf("moe_tiles", (1 + 3 * max_tiles,), torch.int32)
-            kernels.moe_plan_tiles(ids, row_src, pair_row, tiles, E)
-            kernels.moe_gather(h, xs, row_src, None, top)
+        if few:
+            kernels.route_few(zs if pend is None else pend.partial, 1 if pend is None else pend.splits, zs, self.outputs, E, top, wts, pair_row, tile_group,
+                              align, h, xs, 2 if self.softmax_all else int(self.sigmoid), self.correction, *self.groups, self.scale)
+            if pend is not None:
+                pend.release()
         else:
-            kernels.moe_plan(ids, row_src, pair_row, tile_group, E, align)
-            if self.tensor_cores:
-                kernels.moe_gather(h, xs, row_src, tile_group, top, align)
+            z = zs if self.router.n_out == self.outputs else zs[:, :self.outputs]        # (a shared expert's gate is one column more)
+            ids = ctx.buf("moe_ids", (n, top), torch.int32)
+            if self.softmax_all:
+                kernels.route_groups(z, ids, wts, top, self.correction, *self.groups, self.scale)
+            elif self.sigmoid:
+                kernels.route_topk(z, ids, wts, top, sigmoid_scores=True, correction=self.correction)
+            else:
+                kernels.route_topk(z, ids, wts, top)
+            row_src = ctx.buf("moe_row_src", (rows,), torch.int32)
+            if on_pairs:
+                tiles = ctx.buf("moe_tiles", (1 + 3 * max_tiles,), torch.int32)
+                kernels.moe_plan_tiles(ids, row_src, pair_row, tiles, E)
+                kernels.moe_gather(h, xs, row_src, None, top)
+            else:
+                kernels.moe_plan(ids, row_src, pair_row, tile_group, E, align)
+                if self.tensor_cores:
+                    kernels.moe_gather(h, xs, row_src, tile_group, top, align)
         y = ctx.buf("moe_act", (rows, self.inner), ctx.act_dtype)
         zz = ctx.buf("moe_out", (rows, self.width), torch.float32)
         if on_pairs:
