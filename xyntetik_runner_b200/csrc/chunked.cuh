@@ -19,7 +19,7 @@
 // than the walk's, so a state depends in its last bits on where portions were cut; callers that promise the same bits take the walk.
 // 2,048 tokens of one request, 8 heads, us, walk / chunks: constant decay, 128 x 128 values: 166 / 79; decay per channel, 128 x 256:
 // 222 / 164; mLSTM, 128 x 256: 906 / 197.  Root mean square error of the read-outs against float64, 2,040 tokens, walk / chunks: 2.3e-7 /
-// 2.1e-7; 2.1e-6 / 2.1e-7; 6.9e-7 / 7.3e-7 (it divides by a sum that may cancel; 300 and 1,024 tokens 5.3e-7 / 5.4e-7).
+// 1.7e-7; 2.1e-6 / 1.8e-7; 6.9e-7 / 6.5e-7.
 #pragma once
 #include "common.cuh"
 #include <math.h>
@@ -397,20 +397,19 @@ ck_out(ChunkArgs a) {
 #pragma unroll
     for (int b = 0; b < CK_ST - 1; b++) { fill(b); asm volatile("cp.async.commit_group;" ::: "memory"); }
     if (NORM) {
-        // the denominators: the same rows times [sum of keys; ones], two threads a token
+        // the denominators: the same rows times [sum of keys; ones], two threads a token; in float64, because they may cancel
         const float* nm = a.mem_n + at * D;
         const float* r = rows + (tid >> 1) * LR;
-        float total = 0.f;
-        for (int b = 0; b < BLOCKS; b++) {
-            float part = 0.f;
-            for (int k = b * CK_KB + (tid & 1) * 4; k < (b + 1) * CK_KB; k += 8) {
-                const float4 x = *reinterpret_cast<const float4*>(r + k);
-                const float4 y = k < D ? *reinterpret_cast<const float4*>(nm + k) : make_float4(1.f, 1.f, 1.f, 1.f);
-                part = fmaf(x.x, y.x, part); part = fmaf(x.y, y.y, part); part = fmaf(x.z, y.z, part); part = fmaf(x.w, y.w, part);
-            }
-            total += part;
+        double part[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int k = (tid & 1) * 4; k < LR; k += 8) {
+            const float4 x = *reinterpret_cast<const float4*>(r + k);
+            const float4 y = k < D ? *reinterpret_cast<const float4*>(nm + k) : make_float4(1.f, 1.f, 1.f, 1.f);
+            part[0] = fma((double)x.x, (double)y.x, part[0]); part[1] = fma((double)x.y, (double)y.y, part[1]);
+            part[2] = fma((double)x.z, (double)y.z, part[2]); part[3] = fma((double)x.w, (double)y.w, part[3]);
         }
-        total += __shfl_xor_sync(0xffffffffu, total, 1);
+        double sum64 = (part[0] + part[1]) + (part[2] + part[3]);
+        sum64 += __shfl_xor_sync(0xffffffffu, sum64, 1);
+        const float total = (float)sum64;
         if (!(tid & 1)) den[tid >> 1] = (tid >> 1) < p.count ? fmaxf(fabsf(total), a.floor_n[(size_t)(p.t0 + (tid >> 1)) * a.H + h]) + 1e-6f : 1.f;
     }
     for (int b = 0; b < BLOCKS; b++) {
