@@ -61,6 +61,26 @@ def test_float32_attention_of_packed_rows_gives_the_same_bits(H, K, hd, page, ex
     assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
 
 
+# ---- dense products on CTA pairs ----------------------------------------------------------------------------------------
+@pytest.mark.parametrize("n,n_out,k", [(300, 1024, 1024), (401, 3071, 2048), (300, 5632, 1024), (400, 5632, 1024), (512, 5632, 1024), (640, 5632, 1024),
+                                       (1025, 4098, 520), (129, 70, 72)])
+def test_dense_products_in_every_width(n, n_out, k):
+    """Products whose sizes choose tiles of 64, 96, .. 256 tokens, cut and uncut, rows that pair up for a store and rows that do not: a
+    sum of k products in float32, and a bfloat16 store's rounding."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + n_out)
+    x, w = torch.randn(n, k, generator=g).bfloat16(), (torch.randn(n_out, k, generator=g) * k ** -0.5).bfloat16()
+    bias, old = torch.randn(n_out, generator=g), torch.randn(n, n_out, generator=g)
+    want = x.double() @ w.double().T + bias.double()
+    bound = ((x.double().abs() @ w.double().abs().T) + bias.double().abs()) * (k + 4) * 2.0 ** -24
+    xd, wd = x.to(DEV), kernels.pack_weight(w.to(DEV))
+    out, wide = torch.full((n + 1, n_out), 7.0, dtype=torch.bfloat16, device=DEV), old.to(DEV)
+    kernels.gemm_tc(xd, wd, out[:n], bias.to(DEV), kernels.EPI_STORE, packed_rows=n_out)
+    kernels.gemm_tc(xd, wd, wide, bias.to(DEV), kernels.EPI_ADD, packed_rows=n_out)
+    assert ((out[:n].cpu().double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all() and (out[n] == 7.0).all()
+    assert ((wide.cpu().double() - want - old.double()).abs() <= bound + 2.0 ** -23 * (want.abs() + old.abs())).all()
+
+
 # ---- grouped products on CTA pairs -----------------------------------------------------------------------------------
 @pytest.mark.parametrize("counts,width,inner,gated", [([1, 0, 32, 33, 256, 257, 15], 72, 200, True), ([300, 513], 128, 136, False), ([0, 0, 5], 64, 64, True),
                                                       ([700], 136, 264, False)])

@@ -135,6 +135,12 @@ __device__ __forceinline__ float tc_act(int act, float g) {
     if (act == TC_ACT_RELU2) { const float r = fmaxf(g, 0.f); return r * r; }
     return act == TC_ACT_SILU ? tc_silu(g) : (act == TC_ACT_GELU_TANH ? tc_gelu_tanh(g) : g);
 }
+// a chunk's values (one branch a chunk: asked for value by value, every function's steps are taken for every value)
+__device__ __forceinline__ void tc_act16(int act, float (&v)[16]) {
+    if (act == TC_ACT_NONE) return;
+#pragma unroll
+    for (int c = 0; c < 16; c++) v[c] = tc_act(act, v[c]);
+}
 // What a gated product stores for a feature with gate sum g and up sum u: act(g) * u, or for TC_ACT_SWISH_CLAMP
 // g' sigmoid(1.702 g') (u' + 1) with g' = min(g, limit) and u' = u clamped to [-limit, limit].
 __device__ __forceinline__ float tc_gate(int act, float limit, float g, float u) {
@@ -197,6 +203,7 @@ struct TcParams {
 // lanes 0..15 and their up rows in lanes 16..31.  Of a 16-column chunk the gate lanes finish columns 0..7 and the
 // up lanes columns 8..15; each gets the other half of what it needs from its partner lane (lane xor 16) by shuffle.
 // ---------------------------------------------------------------------------------------------
+template <bool PAIRS>
 __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_base, int row0, int tok0, int warp, int lane,
                                             int warps_per_quarter, int split, int bn, int n_end) {
     const int quad = warp & 3, chunk_first = (warp - 2) >> 2;
@@ -208,6 +215,10 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
     const bool row_ok = gated_out ? f < p.n_out : r < (p.gated ? ((p.n_out + 63) / 64) * 128 : p.n_out);
     const float b = (p.bias != nullptr && row_ok && (p.epilogue == TC_EPI_STORE || p.epilogue == TC_EPI_ADD) && split == 0)
                         ? p.bias[r] : 0.f;
+    // bfloat16 rows r and r + 1 of a token in one store where they lie on a border of four bytes: the even lane of a pair has tokens 0..7 of
+    // both rows, the odd lane tokens 8..15.  Half as many stores: 512 x 2,048 x 2,048 17.9 -> 16.7 us.  (PAIRS: not for a few tokens, whose
+    // epilogue is a chain and no traffic: Llama-3.2-1B decode 739 us without, 750 with.)
+    const bool odd = lane & 1, paired = PAIRS && p.epilogue == TC_EPI_STORE && p.out_dtype == XR_BF16 && !((p.n_out | (int)p.ldo) & 1) && !((uintptr_t)p.out & 3);
 #pragma unroll 1
     for (int c0 = chunk_first * 16; c0 < bn; c0 += 16 * warps_per_quarter) {
         if (tok0 + c0 >= n_end) break;             // warp-uniform
@@ -236,6 +247,24 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
             }
             continue;
         }
+        // a chunk that runs past the last token stores only what exists
+        const int live = n_end - (tok0 + c0) < 16 ? n_end - (tok0 + c0) : 16;
+        if (paired) {
+            float v[16];
+#pragma unroll
+            for (int c = 0; c < 16; c++) v[c] = fmaf(p.alpha, g[c], b);
+            tc_act16(p.act, v);
+            float other[8];
+#pragma unroll
+            for (int c = 0; c < 8; c++) other[c] = __shfl_xor_sync(0xffffffffu, odd ? v[c] : v[8 + c], 1);
+            if (!row_ok) continue;
+            __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)(tok0 + c0 + (odd ? 8 : 0)) * p.ldo + (r & ~1);
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                if (c + (odd ? 8 : 0) < live)
+                    *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)c * p.ldo) = odd ? __floats2bfloat162_rn(other[c], v[8 + c]) : __floats2bfloat162_rn(v[c], other[c]);
+            continue;
+        }
         if (!row_ok) continue;
         if (p.epilogue == TC_EPI_ADD) {
             // read-modify-write of the float32 residual: all loads first, so that they overlap
@@ -250,8 +279,6 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
                 if (tok0 + c0 + c < n_end) dst[(size_t)c * p.ldo] = old[c] + fmaf(p.alpha, g[c], b);
             continue;
         }
-        // a chunk that runs past the last token stores only what exists
-        const int live = n_end - (tok0 + c0) < 16 ? n_end - (tok0 + c0) : 16;
         if (p.epilogue == TC_EPI_PARTIAL) {
             const size_t width = p.gated ? (size_t)((p.n_out + 63) / 64) * 128 : (size_t)p.n_out;
             float* dst = p.partial + ((size_t)split * p.n + tok0 + c0) * width + r;
@@ -263,10 +290,7 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
         float v[16];
 #pragma unroll
         for (int c = 0; c < 16; c++) v[c] = fmaf(p.alpha, g[c], b);
-        if (p.act != TC_ACT_NONE) {             // (one branch a chunk: asked for value by value, every function's steps are taken for every value)
-#pragma unroll
-            for (int c = 0; c < 16; c++) v[c] = tc_act(p.act, v[c]);
-        }
+        tc_act16(p.act, v);
         if (p.out_dtype == XR_BF16) {
             __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (size_t)(tok0 + c0) * p.ldo + r;
 #pragma unroll
@@ -393,7 +417,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         // ---------------- epilogue: warps 2..9 ----------------
         bool ok = mbar_wait(acc_ready, 0, abort_flag);
         tc_fence_after();
-        if (ok) tc_epilogue(p, tmem_base, row0, tok0, warp, lane, 2, (int)blockIdx.z, p.bn, p.n);
+        if (ok) tc_epilogue<(BN > 64)>(p, tmem_base, row0, tok0, warp, lane, 2, (int)blockIdx.z, p.bn, p.n);
     }
     tc_fence_before();
     __syncthreads();
@@ -603,7 +627,7 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             tc_fence_after();
             const TcTile at = tc_pair_tile<GROUPED>(p, tile, tok_tiles);
             const int row0 = (2 * at.pair + (int)rank) * TC_BM;
-            tc_epilogue(p, tmem_base + (uint32_t)b * TC2_BN, row0, at.tok0, warp, lane, 4, split, at.bn, at.n_end);
+            tc_epilogue<true>(p, tmem_base + (uint32_t)b * TC2_BN, row0, at.tok0, warp, lane, 4, split, at.bn, at.n_end);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(acc_empty_bar0 + (uint32_t)b * 8);
@@ -768,11 +792,9 @@ struct PairLaunch {
 // two per SM (three for the 16-token tile, of which the grids fill two), one otherwise.
 static int resident_ctas(int bn, int sms) { return bn <= 64 ? 2 * sms : sms; }
 
-// Tokens per tile for a kernel whose buffers hold `cap` of them: up to `cap` tokens, the tokens rounded up to the
-// instruction's step of 16 (no work on padding); more, `cap` -- narrower tiles that would fill the last wave
-// better were measured (144..240 at 2,048 tokens) and are no faster, the product being bound by the operand
-// traffic of its tiles rather than by the number of waves.  The width changes nothing in the sums: every
-// output element is one accumulator over all of K.
+// Tokens per tile for the single-CTA kernel whose buffers hold `cap` of them: up to `cap` tokens, the tokens rounded up to the
+// instruction's step of 16 (no work on padding); more, `cap`.  The width changes nothing in the sums: every output element is one
+// accumulator over all of K.
 static int choose_token_tile(int n, int cap) {
     if (n <= cap) return (n + 15) / 16 * 16;
     return cap;
@@ -782,14 +804,20 @@ static int choose_token_tile(int n, int cap) {
 // for every entry point, so that two entry points given the same sizes and the same room for partial sums do the
 // same arithmetic.
 //
-// Costs are in units of the time one CTA needs for one K block (about 0.27 us).  A product runs in waves of
-// `slots` CTAs (CTA pairs in the pair kernel); a CTA costs a fixed part (launch, barrier and tensor-memory set-up,
-// filling the pipeline, the epilogue: about six units) plus its K blocks.  A product that is cut along K also pays
-// for its partial sums' way to memory and back (8 bytes per element and slice at about 5 TB/s, 170,000 elements a
-// unit in the pair kernel, whose partial sums are tens of megabytes; a quarter of that in the single-CTA kernel, whose
-// few megabytes stay in L2) and for the kernel that sums them (fifteen units; none when the caller's next kernel does
-// it in passing).
-// The cheapest number of slices is taken; only products with a single tile of tokens are cut (single-CTA kernel).
+// Costs are in hundredths of the time a CTA needs for one K block of 256 tokens (about 0.27 us).
+//
+// The pair kernel: `slots` pairs work through the tiles (or the tiles' slices along K) in rounds.  A K block costs its tokens' share of
+// 256, but no less than 72 (the thread that issues it, and the operands' way from L2); a tile's epilogue 100 + 800 x its share, hidden
+// behind the next tile's K blocks but for the last; a launch 600.  A product that is cut along K also pays for its partial sums' way to
+// memory and back (170,000 elements and slice a K block) and for the kernel that sums them (fifteen K blocks; none when the caller's next
+// kernel does it in passing).  The cheapest width (multiples of 32) and number of slices is taken.  Over 90 products of 257 to 2,048 tokens
+// by 1,024 to 11,264 rows of 1,024 to 5,632 this is 0.3 % from the fastest of the widths and cuts of one, two and four slices, where
+// always 256 tokens with the best cut is 30 %: 512 x 2,048 x 2,048 18.0 / 11.8 us (64 tokens a tile), 777 x 2,048 x 5,632 37.7 / 24.9 (96),
+// 1,024 x 1,024 x 1,024 13.0 / 7.9 (64), 1,901 x 3,072 x 2,048 28.6 / 22.8 (160), 2,048 x 2,048 x 2,048 19.1 both ways (256).
+//
+// The single-CTA kernel runs in waves of `slots` CTAs; a CTA costs a fixed part of six K blocks (launch, barrier and tensor-memory set-up,
+// filling the pipeline, the epilogue) plus its K blocks.  Its partial sums, a few megabytes, stay in L2: 700,000 elements and slice a K
+// block.  Only products with a single tile of tokens are cut.
 struct TcPlan {
     int bn;            // token capacity of the kernel's tile: 16, 32, 64, 128 or 256
     int bn_eff;        // tokens per tile as launched
@@ -813,33 +841,44 @@ static TcPlan plan_product(int n, int n_out, int K, bool gated, int force_splits
     const long long finish = deferred ? 0 : 15;
     const int pair_clusters = pl.bn == 256 ? PairLaunch::clusters() : 0;
     pl.pair = pair_clusters > 0;
-    int splits = 1, max_s;
-    long long tiles, slots;
-    if (pl.pair) {
-        pl.bn_eff = (pl.bn_eff + 31) / 32 * 32;
-        pl.tok_tiles = (n + pl.bn_eff - 1) / pl.bn_eff;
-        tiles = (long long)pl.tok_tiles * ((pl.row_tiles + 1) / 2);
-        slots = pair_clusters;
-        max_s = tiles < slots ? (pl.total_kb / 8 < 8 ? pl.total_kb / 8 : 8) : 1;
-    } else {
-        tiles = (long long)pl.row_tiles * pl.tok_tiles;
-        slots = resident_ctas(pl.bn, xr_sm_count());
-        max_s = (pl.tok_tiles > 1 || tiles >= 2 * slots) ? 1 : (pl.total_kb / 4 < 16 ? pl.total_kb / 4 : 16);
-    }
-    if (max_s < 1) max_s = 1;
-    if (force_splits > 0) splits = force_splits;
-    else {
-        long long best_cost = -1;
-        for (int sp = 1; sp <= max_s; sp++) {
-            long long rounds = (tiles * sp + slots - 1) / slots;
-            long long cost = rounds * (6 + (pl.total_kb + sp - 1) / sp);
-            if (sp > 1) cost += pl.pair ? finish + sp * per_slice / 170000 : finish + sp * per_slice / 700000;
-            if (best_cost < 0 || cost < best_cost) { best_cost = cost; splits = sp; }
-        }
-    }
-    if (splits > pl.total_kb) splits = pl.total_kb;
     // no room for the partial sums: the product runs uncut (slower, the same result up to the order of the sums)
-    if (splits > 1 && scratch_floats < (long long)splits * per_slice) splits = 1;
+    const long long room = per_slice > 0 ? scratch_floats / per_slice : 0;
+    int splits = 1;
+    long long best_cost = -1;
+    if (pl.pair) {
+        for (int bn = 256; bn >= 64; bn -= 32) {
+            if (bn - 32 >= n) continue;                                  // (more than one step of padding)
+            const int tok_tiles = (n + bn - 1) / bn;
+            const long long tiles = (long long)tok_tiles * ((pl.row_tiles + 1) / 2), block = bn <= 184 ? 72 : 100 * bn / 256, out = 100 + 800 * bn / 256;
+            int first = 1, last = tiles < pair_clusters ? (pl.total_kb / 8 < 8 ? pl.total_kb / 8 : 8) : 1;
+            if (force_splits > 0) first = last = force_splits;
+            if (last > pl.total_kb) last = pl.total_kb;
+            if (last > room) last = (int)room;
+            if (last < 1) last = 1;
+            if (first > last) first = last;
+            for (int sp = first; sp <= last; sp++) {
+                const long long rounds = (tiles * sp + pair_clusters - 1) / pair_clusters, main = (pl.total_kb + sp - 1) / sp * block;
+                long long cost = 600 + (rounds - 1) * (main > out ? main : out) + main + out;
+                if (sp > 1) cost += 100 * finish + 100 * sp * per_slice / 170000;
+                if (best_cost < 0 || cost < best_cost) { best_cost = cost; splits = sp; pl.bn_eff = bn; pl.tok_tiles = tok_tiles; }
+            }
+        }
+    } else {
+        const long long tiles = (long long)pl.row_tiles * pl.tok_tiles;
+        const int slots = resident_ctas(pl.bn, xr_sm_count());
+        int max_s = (pl.tok_tiles > 1 || tiles >= 2LL * slots) ? 1 : (pl.total_kb / 4 < 16 ? pl.total_kb / 4 : 16);
+        if (max_s < 1) max_s = 1;
+        if (force_splits > 0) splits = force_splits;
+        else
+            for (int sp = 1; sp <= max_s; sp++) {
+                const long long rounds = (tiles * sp + slots - 1) / slots;
+                long long cost = 100 * rounds * (6 + (pl.total_kb + sp - 1) / sp);
+                if (sp > 1) cost += 100 * finish + 100 * (sp * per_slice / 700000);
+                if (best_cost < 0 || cost < best_cost) { best_cost = cost; splits = sp; }
+            }
+        if (splits > pl.total_kb) splits = pl.total_kb;
+        if (splits > 1 && splits > room) splits = 1;
+    }
     pl.splits = splits;
     return pl;
 }
