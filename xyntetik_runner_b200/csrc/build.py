@@ -13,10 +13,13 @@ compile error the caller gets an exception.
 from __future__ import annotations
 
 import hashlib
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -41,6 +44,10 @@ if TRACE:
 
 
 class BuildError(RuntimeError):
+    pass
+
+
+class NoHeaders(BuildError):
     pass
 
 
@@ -217,6 +224,61 @@ def host_library_path(build: bool = True) -> str:
     raise BuildError("no writable folder for the build: " + ", ".join(_build_dirs()))
 
 
+# ---------------------------------------------------------------------------------------------
+# The extension that calls the CUDA library's launchers (calls.py), built with the C++ compiler for this Python, by the same rules.
+# ---------------------------------------------------------------------------------------------
+CALLS_LIB = "xrb200_calls.so"
+CALLS_FLAGS = ["-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden"]
+
+
+def calls_path(build: bool = True) -> str:
+    """Path of an up-to-date extension; compiles it if needed (and allowed)."""
+    from . import calls as made
+    text, include = made.source(), sysconfig.get_paths()["include"]
+    digest = hashlib.sha256("\n".join([sys.version] + CALLS_FLAGS + [text]).encode()).hexdigest()
+    for d in _build_dirs():
+        lib, stamp = os.path.join(d, CALLS_LIB), os.path.join(d, "digest_calls.txt")
+        if os.path.isfile(lib) and os.path.isfile(stamp):
+            with open(stamp) as f:
+                if f.read().strip() == digest:
+                    return lib
+    if not build:
+        raise BuildError("the extension of direct calls is not built")
+    if not os.path.isfile(os.path.join(include, "Python.h")):
+        raise NoHeaders(f"no Python.h in {include}: the extension of direct calls cannot be built")
+    for d in _build_dirs():
+        if not _writable(d):
+            continue
+        src, tmp_lib = os.path.join(d, f".calls.{os.getpid()}.cpp"), os.path.join(d, f".{CALLS_LIB}.{os.getpid()}")
+        env = dict(os.environ)
+        env.setdefault("TMPDIR", d)
+        try:
+            with open(src, "w") as f:
+                f.write(text)
+            r = subprocess.run([find_cxx()] + CALLS_FLAGS + ["-I", include, "-o", tmp_lib, src, "-ldl"], capture_output=True, text=True, env=env)
+            if r.returncode != 0:
+                raise BuildError(f"the C++ compiler failed on the extension of direct calls:\n{r.stdout}\n{r.stderr}")
+        finally:
+            if os.path.exists(src):
+                os.remove(src)
+        lib = os.path.join(d, CALLS_LIB)
+        os.replace(tmp_lib, lib)
+        with open(os.path.join(d, "digest_calls.txt"), "w") as f:
+            f.write(digest + "\n")
+        return lib
+    raise BuildError("no writable folder for the build: " + ", ".join(_build_dirs()))
+
+
+def calls(library: str):
+    """The extension, its functions bound to `library`."""
+    loader = importlib.machinery.ExtensionFileLoader("xrb200_calls", calls_path())
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("xrb200_calls", loader))
+    loader.exec_module(module)
+    module.bind(library)
+    return module
+
+
 if __name__ == "__main__":
     print(library_path())
     print(host_library_path())
+    print(calls_path())

@@ -54,6 +54,9 @@ class StepEntry:
     want: Sequence[int] = ()           # indices into `tokens` whose logits are wanted
 
 
+MOST_VIEWS = 4096       # views of step buffers that are kept at most (a shape of a step has some tens)
+
+
 class StepContext:
     """What the parts see of one step.  Tensors are on the device; `host` holds the same as numpy."""
 
@@ -71,7 +74,7 @@ class StepContext:
         self.host: Dict[str, np.ndarray] = {}
         self.max_kv_len = 0            # longest key range any token of the step reads
         self._pending = {}
-        self._views: Dict[tuple, torch.Tensor] = {}
+        self._views = eng._views
         self._memo: Dict[object, object] = {}
         self.decode_only = False       # every segment is a single token
         self.uneven = False            # the requests' lengths differ much (a hint for kernels that split work by request)
@@ -79,11 +82,14 @@ class StepContext:
         self.stream_cast = None        # address of the stream whose rounding to the activation dtype lies in "block_normed"
 
     def buf(self, name: str, shape, dtype: torch.dtype) -> torch.Tensor:
-        # (every layer asks for the same few views: made once a step)
-        key = (name, tuple(shape), dtype)
+        # (every layer of every step asks for the same few views: made once a shape, until a buffer is replaced)
+        key = (name, shape if type(shape) is tuple else tuple(shape), dtype)
         t = self._views.get(key)
         if t is None:
-            t = self._views[key] = self._eng._buf(name, shape, dtype)
+            t = self._eng._buf(name, shape, dtype)
+            if len(self._views) >= MOST_VIEWS:
+                self._views.clear()
+            self._views[key] = t
         return t
 
     def once(self, key, make):
@@ -182,6 +188,7 @@ class Engine:
         self._pinned: List[Optional[torch.Tensor]] = [None] * 3
         self._pinned_done: List[Optional[torch.cuda.Event]] = [None] * 3
         self._pinned_next = 0
+        self._slot_states: Dict[int, List[List[torch.Tensor]]] = {}      # views of a slot's states, made when it is first used
         self._slot_generation = np.zeros(p.max_requests, dtype=np.int64)
         self.steps_run = 0
         self.h2d_bytes = 0               # bytes of step descriptions copied to the device so far
@@ -196,6 +203,7 @@ class Engine:
         self._fill_ok = self._graph_ok and not self.model.state_needs and self.embedding_state is None
         self._graph_seen: Dict[tuple, int] = {}
         self._buf_generation = 0
+        self._views: Dict[tuple, torch.Tensor] = {}      # see StepContext.buf
         self.graph_replays = 0
         self._graph_launches: Dict[tuple, int] = {}
         # the step description's device buffer is made once for the largest step the parameters name
@@ -218,6 +226,7 @@ class Engine:
             t = torch.empty(max(cap, 1), dtype=dtype, device=self.device)
             self._bufs[key] = t
             self._buf_generation += 1
+            self._views.clear()
             self._graphs.clear()
             self._uneven_of_shape.clear()
         return t[:n].view(*shape)
@@ -243,11 +252,17 @@ class Engine:
 
     def _open(self, request) -> int:
         slot = self.cache.open(request)
-        for lay in self.model.layers:
-            if lay.state is not None:
-                lay.state[slot].zero_()
-        if self.embedding_state is not None:
-            self.embedding_state[slot].zero_()
+        rows = self._slot_states.get(slot)
+        if rows is None:
+            states = [lay.state for lay in self.model.layers if lay.state is not None]
+            if self.embedding_state is not None:
+                states.append(self.embedding_state)
+            rows = {}                              # by dtype: all of one in one launch
+            for s in states:
+                rows.setdefault(s.dtype, []).append(s[slot])
+            self._slot_states[slot] = rows = list(rows.values())
+        for same in rows:
+            torch._foreach_zero_(same)
         return slot
 
     # ---- the step ----------------------------------------------------------------

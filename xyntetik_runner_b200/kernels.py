@@ -13,6 +13,7 @@ from typing import Optional
 import torch
 
 from .csrc import build as _build
+from .csrc.signatures import LONG, SIGNATURES
 
 F32, BF16 = 0, 1
 _ERR = {-1: "the kernel refuses these sizes or dtypes", -2: "CUDA refused the launch", -3: "tensor map encoding failed",
@@ -37,92 +38,50 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+class _Calls:
+    """Stands for the direct calls (csrc/calls.py: an extension with one function per launcher, a third of ctypes' cost a call) until the
+    first is used; then the extension takes its place."""
+
+    def __getattr__(self, name):
+        global _c
+        L = lib()
+        try:
+            _c = _build.calls(_build.library_path(build=False))
+        except _build.NoHeaders:             # (a Python without its headers: the same calls through ctypes)
+            _c = _CtypesCalls(L)
+        return getattr(_c, name)
+
+
+class _CtypesCalls:
+    def __init__(self, L: ctypes.CDLL):
+        for name, letters in SIGNATURES.items():
+            setattr(self, name, self._setting(getattr(L, name), letters.index("o")) if "o" in letters else getattr(L, name))
+
+    @staticmethod
+    def _setting(fn, at: int):
+        def call(*args):
+            out = ctypes.c_int(0)
+            return fn(*args[:at], ctypes.byref(out), *args[at:]) or out.value
+        return call
+
+
+_c = _Calls()
+
+
 def library_file() -> str:
     lib()
     return _build.library_path(build=False)
 
 
-_vp, _i, _ll, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+_CTYPES = {"p": ctypes.c_void_p, "i": ctypes.c_int, "l": ctypes.c_longlong, "f": ctypes.c_float, "u": ctypes.c_uint, "U": ctypes.c_ulonglong,
+           "o": ctypes.POINTER(ctypes.c_int)}
 
 
 def _declare(L: ctypes.CDLL) -> None:
-    sig = {
-        "xr_embed": [_vp, _i, _vp, _vp, _i, _vp, _i, _i, _i, _f, _vp],
-        "xr_rmsnorm": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
-        "xr_rope_store": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp],
-        "xr_act_mul": [_vp, _vp, _i, _i, _i, _i, _i, _f, _vp],
-        "xr_residual_add": [_vp, _vp, _i, _i, _i, _vp],
-        "xr_gemm_simt": [_vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _ll, _ll, _f, _vp],
-        "xr_attention_simt": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _f, _i, _vp, _i, _i, _vp],
-        "xr_gemm_tc": [_vp, _vp, _vp, _vp, _i, _i, _i, _f, _f, _i, _i, _i, _ll, _ll, _vp, _ll, _vp, _i, _i, ctypes.POINTER(ctypes.c_int), _i, _vp],
-        "xr_finish_add_rmsnorm": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _vp],
-        "xr_finish_plain": [_vp, _i, _vp, _vp, _i, _i, _i, _i, _ll, _vp],
-        "xr_finish_rope_store": [_vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp],
-        "xr_attention_mma": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _f,
-                             _i, _i, _i, _i, _i, _vp, _ll, _i, _i, _vp, _vp, _i, _i, _ll, _vp, _f, _i, _vp, _i, _vp],
-        "xr_attention_mma_splits": [_i, _i, _ll],
-        "xr_attention_even_launches": [],
-        "xr_attention_wait_probe": [_vp, _vp, ctypes.c_uint, _vp],
-        "xr_attention_tc_supported": [_i, _i, _i, _i],
-        "xr_attention_tc": [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _ll, _ll, _i, _i, _vp, _f, _i, _vp, _i, _vp],
-        "xr_attention_tc_flat_supported": [_i, _i, _i],
-        "xr_attention_tc_flat": [_vp, _ll, _vp, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _ll, _i, _f, _i, _ll, _vp, _ll, _i, _vp],
-        "xr_flat_rows": [_vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-        "xr_sample": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp, _vp, _vp, _vp],
-        "xr_sample_one_block": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
-        "xr_logprob": [_vp, _ll, _i, _i, _vp, _vp, _vp],
-        "xr_random_normal": [_vp, _i, _ll, ctypes.c_ulonglong, ctypes.c_ulonglong, _f, _f, _vp],
-        "xr_scaled_add": [_vp, _vp, _f, _i, _i, _i, _vp],
-        "xr_stream_step": [_vp, _vp, _vp, _i, _i, _vp],
-        "xr_sigmoid_gate": [_vp, _ll, _vp, _ll, _i, _i, _i, _i, _i, _i, _vp],
-        "xr_concat_cast": [_vp, _vp, _vp, _i, _i, _i, _vp],
-        "xr_softcap": [_vp, _f, _ll, _vp],
-        "xr_latent_prep": [_vp, _i, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _vp],
-        "xr_head_matmul": [_vp, _i, _ll, _i, _vp, _i, _ll, _ll, _ll, _vp, _i, _ll, _vp, _i, _ll, _i, _i, _i, _i, _i, _vp],
-        "xr_latent_attention": [_vp, _vp, _i, _ll, _i, _vp, _vp, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _vp],
-        "xr_latent_attention_mma_supported": [_i, _i],
-        "xr_latent_attention_mma": [_vp, _ll, _ll, _vp, _ll, _i, _vp, _vp, _ll, _ll, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _i, _i, _i, _vp],
-        "xr_heads_gather": [_vp, _ll, _i, _vp, _i, _i, _i, _i, _vp],
-        "xr_heads_scatter_gate": [_vp, _vp, _vp, _ll, _i, _i, _i, _i, _i, _vp],
-        "xr_qk_norm_rope_store": [_vp, _i, _ll, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _ll, _i, _i, _i, _i, _i, _i, _i, _i, _i, _i, _f, _i, _f, _i,
-                                  _vp, _i, _vp, _i, _f, _i, _vp, _i, _f, _vp],
-        "xr_rmsnorm_act": [_vp, _i, _ll, _vp, _vp, _ll, _i, _i, _f, _vp],
-        "xr_delta": [_vp, _i, _ll, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-        "xr_head_norm_gate": [_vp, _vp, _i, _ll, _vp, _i, _i, _vp, _i, _i, _i, _i, _f, _vp],
-        "xr_mlstm": [_vp, _i, _ll, _i, _i, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _f, _vp, _ll, _vp],
-        "xr_route_topk": [_vp, _ll, _vp, _vp, _i, _i, _i, _vp, _i, _vp],
-        "xr_moe_plan": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
-        "xr_moe_gather": [_vp, _i, _ll, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
-        "xr_gemm_tc_grouped": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _i, _vp, _i, _vp, _vp],
-        "xr_route_few_supported": [_i, _i, _i, _i, _i, _i],
-        "xr_route_few": [_vp, _i, _vp, _i, _i, _i, _i, _i, _vp, _i, _i, _i, _f, _vp, _vp, _vp, _i, _i, _vp, _ll, _vp, _i, _vp],
-        "xr_gemm_tc_pairs_available": [],
-        "xr_gemm_tc_grouped_pairs": [_vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _i, _ll, _ll, _vp, _i, _i, _vp, _vp],
-        "xr_moe_plan_tiles": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
-        "xr_moe_tile_rows": [],
-        "xr_moe_gemm": [_vp, _i, _ll, _vp, _i, _vp, _i, _ll, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp],
-        "xr_route_groups": [_vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _f, _vp],
-        "xr_moe_combine": [_vp, _vp, _vp, _vp, _vp, _i, _ll, _vp, _i, _vp, _ll, _f, _vp, _vp, _i, _f, _i, _i, _i, _vp],
-        "xr_embed_pair": [_vp, _vp, _i, _vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _ll, _ll, _ll, _vp],
-        "xr_last_token": [_vp, _vp, _i, _vp, _vp, _vp, _vp, _i, _i, _vp],
-        "xr_norm_add": [_vp, _vp, _vp, _vp, _i, _i, _i, _f, _i, _vp, _vp, _i, _vp],
-        "xr_cast_rows": [_vp, _vp, _i, _ll, _vp],
-        "xr_depth_average": [_vp, _vp, _vp, _vp, _vp, _i, _i, _ll, _vp],
-        "xr_rotate_heads": [_vp, _i, _ll, _i, _i, _i, _i, _i, _i, _vp, _vp, _f, _f, _i, _vp],
-        "xr_rglru": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i,
-                     _f, _vp],
-        "xr_row_norm_gate": [_vp, _vp, _ll, _vp, _vp, _i, _i, _i, _f, _f, _vp],
-        "xr_ssd": [_vp, _ll, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _vp],
-        "xr_silu_gate_norm": [_vp, _vp, _ll, _vp, _vp, _i, _i, _i, _i, _f, _vp],
-        "xr_decay_attention": [_vp, _ll, _i, _i, _i, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _ll, _vp],
-        "xr_chunked_floats": [_i, _i, _i, _i, _i, _i],
-        "xr_key_decay_attention": [_vp, _ll, _i, _i, _i, _i, _vp, _vp, _i, _f, _vp, _vp, _ll, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _f, _vp, _ll, _vp],
-    }
-    for name, args in sig.items():
+    for name, letters in SIGNATURES.items():
         fn = getattr(L, name)
-        fn.argtypes = args
-        fn.restype = ctypes.c_int
-    L.xr_chunked_floats.restype = _ll
+        fn.argtypes = [_CTYPES[c] for c in letters]
+        fn.restype = ctypes.c_longlong if name in LONG else ctypes.c_int
 
 
 def _check(code: int, what: str) -> None:
@@ -178,7 +137,7 @@ def embed(table: torch.Tensor, ids: torch.Tensor, x: torch.Tensor, feed: Optiona
     n, d = x.shape
     assert ids.dtype == torch.int32 and ids.numel() >= n and x.dtype == torch.float32 and table.shape[1] == d
     assert feed is None or feed.dtype == torch.int32
-    _check(lib().xr_embed(table.data_ptr(), dtype_code(table.dtype), ids.data_ptr(), _ptr(feed),
+    _check(_c.xr_embed(table.data_ptr(), dtype_code(table.dtype), ids.data_ptr(), _ptr(feed),
                           0 if feed is None else feed.numel(), x.data_ptr(), n, d, table.shape[0], float(scale), _stream()), "embed")
     _count()
 
@@ -198,7 +157,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, eps: float, row
     assert x.dtype == torch.float32 and w.dtype == torch.float32 and x.shape[1] == d and w.numel() == d
     assert rows is None or (rows.dtype == torch.int32 and rows.numel() >= n)
     _second_norm(w2, out2, out, d)
-    _check(lib().xr_rmsnorm(x.data_ptr(), _ptr(rows), w.data_ptr(), out.data_ptr(), _ptr(w2), _ptr(out2), dtype_code(out.dtype), n, d,
+    _check(_c.xr_rmsnorm(x.data_ptr(), _ptr(rows), w.data_ptr(), out.data_ptr(), _ptr(w2), _ptr(out2), dtype_code(out.dtype), n, d,
                             float(eps), _stream()), "rmsnorm")
     _count()
 
@@ -213,7 +172,7 @@ def rope_store(qkv: torch.Tensor, positions, tok_seg, block_tables, inv_freq: Op
     n = qkv.shape[0]
     assert qkv.shape[1] == (H + 2 * K) * hd
     assert rotary_dim == 0 or (inv_freq is not None and inv_freq.dtype == torch.float32 and inv_freq.numel() >= rotary_dim // 2)
-    _check(lib().xr_rope_store(qkv.data_ptr(), dtype_code(qkv.dtype), positions.data_ptr(), tok_seg.data_ptr(),
+    _check(_c.xr_rope_store(qkv.data_ptr(), dtype_code(qkv.dtype), positions.data_ptr(), tok_seg.data_ptr(),
                                block_tables.data_ptr(), _ptr(inv_freq), cache_k_ptr, page_stride, v_offset,
                                n, H, K, hd, rotary_dim, max_pages, page_size, int(adjacent), float(mscale), _stream()),
            "rope_store")
@@ -232,7 +191,7 @@ def rmsnorm_act(inp: torch.Tensor, w: torch.Tensor, out: torch.Tensor, eps: floa
     n, d = inp.shape
     assert out.shape == (n, d) and inp.dtype == out.dtype and inp.stride(1) == 1 and out.stride(1) == 1 and inp.is_cuda and out.is_cuda
     assert w.dtype == torch.float32 and w.numel() == d
-    _check(lib().xr_rmsnorm_act(inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), n, d,
+    _check(_c.xr_rmsnorm_act(inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), w.data_ptr(), out.data_ptr(), out.stride(0), n, d,
                                 float(eps), _stream()), "rmsnorm_act")
     _count()
 
@@ -262,7 +221,7 @@ def qk_norm_rope_store(inp: torch.Tensor, q_out: torch.Tensor, positions, tok_se
     assert inp.stride(1) == 1 and q_out.stride(1) == 1 and inp.dtype == q_out.dtype and q_out.shape[0] == n and q_out.shape[1] >= H * hd
     assert inp.shape[1] >= (H + K) * D + K * Vd and (freq is None or (freq.dtype == torch.float64 and freq.numel() >= rotary_dim // 2))
     assert q_w is None or (q_w.dtype == torch.float32 and k_w.dtype == torch.float32 and q_w.numel() == D and k_w.numel() == D)
-    _check(lib().xr_qk_norm_rope_store(inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), q_out.data_ptr(), q_out.stride(0),
+    _check(_c.xr_qk_norm_rope_store(inp.data_ptr(), dtype_code(inp.dtype), inp.stride(0), q_out.data_ptr(), q_out.stride(0),
                                        positions.data_ptr(), tok_seg.data_ptr(), block_tables.data_ptr(), _ptr(freq), _ptr(q_w), _ptr(k_w),
                                        cache_k_ptr, page_stride, v_offset, n, H, K, D, Vd, hd, rotary_dim, max_pages, page_size,
                                        int(adjacent), float(eps), int(unit_norm), float(q_coef), int(q_every), _ptr(partial), int(splits),
@@ -279,7 +238,7 @@ def act_mul(gu: torch.Tensor, h: torch.Tensor, act: int = ACT_SILU, gated: bool 
     _dev(gu, h)
     n, F = h.shape
     assert gu.shape == (n, 2 * F if gated else F) and gu.dtype == h.dtype
-    _check(lib().xr_act_mul(gu.data_ptr(), h.data_ptr(), dtype_code(h.dtype), n, F, int(act), int(gated), float(limit), _stream()), "act_mul")
+    _check(_c.xr_act_mul(gu.data_ptr(), h.data_ptr(), dtype_code(h.dtype), n, F, int(act), int(gated), float(limit), _stream()), "act_mul")
     _count()
 
 
@@ -291,7 +250,7 @@ def residual_add(x: torch.Tensor, delta: torch.Tensor) -> None:
     _dev(x, delta)
     n, d = x.shape
     assert x.dtype == torch.float32 and delta.shape == x.shape
-    _check(lib().xr_residual_add(x.data_ptr(), delta.data_ptr(), dtype_code(delta.dtype), n, d, _stream()), "residual_add")
+    _check(_c.xr_residual_add(x.data_ptr(), delta.data_ptr(), dtype_code(delta.dtype), n, d, _stream()), "residual_add")
     _count()
 
 
@@ -306,7 +265,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optiona
     assert w.shape[1] == k and out.shape == (n, n_out) and w.is_contiguous()
     assert x.stride(1) == 1 and out.stride(1) == 1
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == n_out)
-    _check(lib().xr_gemm_simt(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), _ptr(bias),
+    _check(_c.xr_gemm_simt(x.data_ptr(), dtype_code(x.dtype), w.data_ptr(), dtype_code(w.dtype), _ptr(bias),
                               out.data_ptr(), dtype_code(out.dtype), int(accumulate), n, n_out, k,
                               x.stride(0), out.stride(0), float(alpha), _stream()), "gemm_simt")
     _count()
@@ -335,7 +294,7 @@ def attention_simt(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cache_
     n = out.shape[0]
     _check_bias(bias, H)
     assert out.shape[1] == H * hd and q.dtype == out.dtype
-    _check(lib().xr_attention_simt(q.data_ptr(), out.data_ptr(), dtype_code(out.dtype), cache_k_ptr,
+    _check(_c.xr_attention_simt(q.data_ptr(), out.data_ptr(), dtype_code(out.dtype), cache_k_ptr,
                                    positions.data_ptr(), tok_seg.data_ptr(), block_tables.data_ptr(), page_stride,
                                    v_offset, q_row_stride, n, H, K, hd, max_pages, page_size, window, float(scale),
                                    _ptr(sink), float(softcap), int(keep_first), _ptr(bias), _bias_len(bias), int(portions), _stream()), "attention_simt")
@@ -373,9 +332,9 @@ def sample(logits: torch.Tensor, temp, top_k, top_p, min_p, penalty, draw, recen
         assert exempt.numel() >= EXEMPT_IDS * rows and feed.dtype == torch.int32 and recent is not None
         assert out.data_ptr() != feed.data_ptr() and any_sampled and not one_block
     if one_block or not any_sampled:
-        _check(lib().xr_sample_one_block(*args, _stream()), "sample")
+        _check(_c.xr_sample_one_block(*args, _stream()), "sample")
     else:
-        _check(lib().xr_sample(*args, int(shortcuts), _ptr(pending), _ptr(feed), _ptr(exempt), _stream()), "sample")
+        _check(_c.xr_sample(*args, int(shortcuts), _ptr(pending), _ptr(feed), _ptr(exempt), _stream()), "sample")
     _count()
 
 
@@ -385,7 +344,7 @@ def logprob(logits: torch.Tensor, target: torch.Tensor, out: torch.Tensor) -> No
     rows, V = logits.shape
     assert logits.dtype == torch.float32 and logits.stride(1) == 1 and logits.is_cuda
     assert target.dtype == torch.int32 and target.numel() >= rows and out.dtype == torch.float32 and out.numel() >= rows
-    _check(lib().xr_logprob(logits.data_ptr(), logits.stride(0), rows, V, target.data_ptr(), out.data_ptr(), _stream()), "logprob")
+    _check(_c.xr_logprob(logits.data_ptr(), logits.stride(0), rows, V, target.data_ptr(), out.data_ptr(), _stream()), "logprob")
     _count()
 
 
@@ -393,7 +352,7 @@ def random_normal(out: torch.Tensor, key: int, mean: float, std: float, first: i
     """out.flat[i] = mean + std * z(key, first + i): the counter-based generator of csrc/random_fill.cu, whose
     values equal ``weights.random_fill.normal_values`` bit for bit."""
     _dev(out)
-    _check(lib().xr_random_normal(out.data_ptr(), dtype_code(out.dtype), out.numel(), key & 0xFFFFFFFFFFFFFFFF, first,
+    _check(_c.xr_random_normal(out.data_ptr(), dtype_code(out.dtype), out.numel(), key & 0xFFFFFFFFFFFFFFFF, first,
                                   float(mean), float(std), _stream()), "random_normal")
     _count()
 
@@ -535,19 +494,20 @@ class PartialSums:
             self._ws = None
 
 
-_SPLITS_USED = ctypes.c_int(1)           # where xr_gemm_tc says how it cut the product (read at once after the call)
-_SPLITS_USED_REF = ctypes.byref(_SPLITS_USED)
 
 
 def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, act_limit=0.0, alpha=1.0):
+    # (called once or several times a layer: shapes and strides are asked for once)
     n, k = x.shape
+    ldx, one = x.stride()
     gated = epilogue == EPI_GATED
     if packed_rows is not None:
         # w comes from pack_weight(); packed_rows is the logical number of output features
         n_out = packed_rows
         tiles = -(-n_out // GATED_FEATURES) if gated else -(-n_out // TILE_ROWS)
-        assert w.dim() == 4 and w.shape[0] == tiles and w.shape[1] == -(-k // TILE_K) and out.shape == (n, n_out)
-        assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and k % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+        ws = w.shape
+        assert len(ws) == 4 and ws[0] == tiles and ws[1] == -(-k // TILE_K) and out.shape == (n, n_out)
+        assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and k % 8 == 0 and one == 1 and ldx % 8 == 0
     else:
         if gated:
             raise KernelError("the gated product takes weights from pack_weight(w, halves=2)")
@@ -557,11 +517,11 @@ def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, a
     assert not defer or not gated
     ws = workspace(x.device)
     at, room = ws.room()
-    _check(lib().xr_gemm_tc(x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), float(alpha),
-                            n, n_out, k, x.stride(0), out.stride(0), at, room,
-                            ws.status_ptr, force_splits, int(defer), _SPLITS_USED_REF,
-                            int(packed_rows is not None), _stream()), "gemm_tc")
-    splits = _SPLITS_USED.value
+    splits = _c.xr_gemm_tc(x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), float(alpha),
+                           n, n_out, k, ldx, out.stride(0), at, room,
+                           ws.status_ptr, force_splits, int(defer), int(packed_rows is not None), _stream())
+    if splits < 0:
+        _check(splits, "gemm_tc")
     _count(1 if (splits == 1 or defer) else 2)
     if defer and splits > 1:
         rows = tiles * TILE_ROWS if (gated and packed_rows is not None) else n_out
@@ -598,7 +558,7 @@ def finish_add_rmsnorm(partial: torch.Tensor, splits: int, bias: Optional[torch.
     n, d = x.shape
     assert x.dtype == torch.float32 and w.dtype == torch.float32 and out.shape == (n, d) and partial.numel() >= splits * n * d
     _second_norm(w2, out2, out, d)
-    _check(lib().xr_finish_add_rmsnorm(partial.data_ptr(), splits, _ptr(bias), x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(w2),
+    _check(_c.xr_finish_add_rmsnorm(partial.data_ptr(), splits, _ptr(bias), x.data_ptr(), w.data_ptr(), out.data_ptr(), _ptr(w2),
                                        _ptr(out2), dtype_code(out.dtype), n, d, float(eps), _stream()), "finish_add_rmsnorm")
     _count()
 
@@ -608,7 +568,7 @@ def finish_plain(partial: torch.Tensor, splits: int, bias: Optional[torch.Tensor
     """out (+)= sum of the split-K partials (+ bias)."""
     n, width = out.shape
     assert out.stride(1) == 1 and partial.numel() >= splits * n * width
-    _check(lib().xr_finish_plain(partial.data_ptr(), splits, _ptr(bias), out.data_ptr(), dtype_code(out.dtype),
+    _check(_c.xr_finish_plain(partial.data_ptr(), splits, _ptr(bias), out.data_ptr(), dtype_code(out.dtype),
                                  int(accumulate), n, width, out.stride(0), _stream()), "finish_plain")
     _count()
 
@@ -622,7 +582,7 @@ def finish_rope_store(partial: torch.Tensor, splits: int, bias: Optional[torch.T
     _dev(qkv, positions, tok_seg, block_tables, inv_freq, bias)
     n = qkv.shape[0]
     assert qkv.dtype == torch.bfloat16 and qkv.shape[1] == (H + 2 * K) * hd and partial.numel() >= splits * n * qkv.shape[1]
-    _check(lib().xr_finish_rope_store(partial.data_ptr(), splits, _ptr(bias), qkv.data_ptr(), positions.data_ptr(),
+    _check(_c.xr_finish_rope_store(partial.data_ptr(), splits, _ptr(bias), qkv.data_ptr(), positions.data_ptr(),
                                       tok_seg.data_ptr(), block_tables.data_ptr(), _ptr(inv_freq), cache_k_ptr, page_stride,
                                       v_offset, n, H, K, hd, rotary_dim, max_pages, page_size, int(adjacent), float(mscale),
                                       _stream()), "finish_rope_store")
@@ -637,7 +597,7 @@ def attention_mma_supported(dtype: torch.dtype, H: int, K: int, hd: int) -> bool
 def attention_mma_splits(max_kv_len: int, window: int, items: int) -> int:
     """Slots of scratch per (segment, kv head) pair that the key-split kernel needs for a step with `items` such
     pairs: its spans per request, or its CTAs over the pairs where it cuts the step's tiles into even shares."""
-    return int(lib().xr_attention_mma_splits(max_kv_len, window, items))
+    return int(_c.xr_attention_mma_splits(max_kv_len, window, items))
 
 
 def long_row_tiles(seg_len_host, heads_per_kv_head: int, rows_per_tile: int) -> int:
@@ -649,7 +609,7 @@ def long_row_tiles(seg_len_host, heads_per_kv_head: int, rows_per_tile: int) -> 
 
 def attention_even_launches() -> int:
     """How often the decode attention was launched in even shares (rather than in spans) so far."""
-    return int(lib().xr_attention_even_launches())
+    return int(_c.xr_attention_even_launches())
 
 
 def attention_wait_probe(device: torch.device, limit: int = 1 << 12) -> None:
@@ -657,7 +617,7 @@ def attention_wait_probe(device: torch.device, limit: int = 1 << 12) -> None:
     status word of `device` says so, as it would for a hand-over that never came (``tc_check_status`` then raises).
     Nothing faults and nothing hangs; this exists so that tests can drive the host's handling of that word."""
     ws = workspace(device)
-    _check(lib().xr_attention_wait_probe(ws.flags.data_ptr() + 4 * (ws.flags.numel() - 1), ws.status.data_ptr(), int(limit),
+    _check(_c.xr_attention_wait_probe(ws.flags.data_ptr() + 4 * (ws.flags.numel() - 1), ws.status.data_ptr(), int(limit),
                                          _stream()), "attention_wait_probe")
 
 
@@ -685,7 +645,7 @@ def attention_mma(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cache_k
         assert part_acc is not None and part_acc.numel() >= n_seg * K * splits * 16 * hd
         assert part_ml is not None and part_ml.numel() >= n_seg * K * splits * 32
     ws = workspace(out.device)
-    _check(lib().xr_attention_mma(q.data_ptr(), out.data_ptr(), cache_k_ptr, seg_start.data_ptr(), seg_len.data_ptr(),
+    _check(_c.xr_attention_mma(q.data_ptr(), out.data_ptr(), cache_k_ptr, seg_start.data_ptr(), seg_len.data_ptr(),
                                   seg_pos0.data_ptr(), block_tables.data_ptr(), _ptr(part_acc), _ptr(part_ml),
                                   q_row_stride, page_stride, v_offset, n_seg, H, K, hd, max_pages, page_size, window,
                                   float(scale), max_seg_len, max_kv_len, splits, int(any_short), int(any_long),
@@ -697,7 +657,7 @@ def attention_mma(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, cache_k
 
 
 def attention_tc_supported(dtype: torch.dtype, H: int, K: int, hd: int, page_size: int) -> bool:
-    return dtype == torch.bfloat16 and bool(lib().xr_attention_tc_supported(H, K, hd, page_size))
+    return dtype == torch.bfloat16 and bool(_c.xr_attention_tc_supported(H, K, hd, page_size))
 
 
 def attention_tc(qkv: torch.Tensor, out: torch.Tensor, seg_start, seg_len, seg_pos0, block_tables, group: tuple,
@@ -715,7 +675,7 @@ def attention_tc(qkv: torch.Tensor, out: torch.Tensor, seg_start, seg_len, seg_p
     n = qkv.shape[0]
     assert qkv.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.shape == (n, H * hd)
     status = tc_workspace(out.device)[1]
-    _check(lib().xr_attention_tc(qkv.data_ptr(), out.data_ptr(), group[0], seg_start.data_ptr(), seg_len.data_ptr(),
+    _check(_c.xr_attention_tc(qkv.data_ptr(), out.data_ptr(), group[0], seg_start.data_ptr(), seg_len.data_ptr(),
                                  seg_pos0.data_ptr(), block_tables.data_ptr(), status.data_ptr(), qkv.stride(0), n, n_seg,
                                  H, K, hd, max_pages, page_size, window, float(scale), max_seg_len, row_tiles, group[1], group[2],
                                  group[3], _ptr(sink), float(softcap), int(keep_first), _ptr(bias), _bias_len(bias), _stream()), "attention_tc")
@@ -726,7 +686,7 @@ FLAT_TILE = 128       # the flat array's first key of a portion is a multiple of
 
 
 def attention_tc_flat_supported(act_dtype: torch.dtype, D: int, R: int, V: int) -> bool:
-    return act_dtype == torch.bfloat16 and lib().xr_attention_tc_flat_supported(D, R, V) == 1
+    return act_dtype == torch.bfloat16 and _c.xr_attention_tc_flat_supported(D, R, V) == 1
 
 
 def flat_first_key(pos0, window: int):
@@ -741,7 +701,7 @@ def flat_rows(cache_ptr: int, page_stride: int, out: torch.Tensor, seg_len, seg_
     another, each from ``flat_first_key`` to its last."""
     _dev(out, seg_len, seg_pos0, block_tables)
     assert out.dtype == torch.bfloat16
-    _check(lib().xr_flat_rows(cache_ptr, page_stride, out.data_ptr(), seg_len.data_ptr(), seg_pos0.data_ptr(), block_tables.data_ptr(), n_seg,
+    _check(_c.xr_flat_rows(cache_ptr, page_stride, out.data_ptr(), seg_len.data_ptr(), seg_pos0.data_ptr(), block_tables.data_ptr(), n_seg,
                               out.shape[0], out.shape[1], max_pages, page_size, window, min_len, _stream()), "flat_rows")
     _count()
 
@@ -759,7 +719,7 @@ def attention_tc_flat(q: torch.Tensor, kv: torch.Tensor, tail: torch.Tensor, out
     assert all(t.dtype == torch.bfloat16 and t.is_cuda and t.stride(1) == 1 for t in (q, kv, tail, out))
     assert q.shape[1] >= H * (D + R) and kv.shape[1] == H * (D + V) and tail.shape == (keys, R) and out.shape == (n, H * V)
     assert gate is None or (gate.dtype == torch.bfloat16 and gate.is_cuda and gate.stride(1) == 1 and gate.shape == (n, H * V if gate_each else H))
-    _check(lib().xr_attention_tc_flat(q.data_ptr(), q.stride(0), kv.data_ptr(), kv.stride(0), tail.data_ptr(), tail.stride(0), out.data_ptr(),
+    _check(_c.xr_attention_tc_flat(q.data_ptr(), q.stride(0), kv.data_ptr(), kv.stride(0), tail.data_ptr(), tail.stride(0), out.data_ptr(),
                                       seg_start.data_ptr(), seg_len.data_ptr(), seg_pos0.data_ptr(), workspace(out.device).status_ptr, n, n_seg,
                                       H, D, R, V, keys, window, float(scale), min_len, row_tiles, _ptr(gate), 0 if gate is None else gate.stride(0),
                                       int(gate_each), _stream()), "attention_tc_flat")
@@ -772,7 +732,7 @@ def scaled_add(x: torch.Tensor, d: torch.Tensor, m: float, clear: bool = False) 
     """x += m * d on float32 streams; with `clear`, d is zero afterwards."""
     _dev(x, d)
     assert x.dtype == torch.float32 and d.dtype == torch.float32 and x.shape == d.shape
-    _check(lib().xr_scaled_add(x.data_ptr(), d.data_ptr(), float(m), int(clear), x.shape[0], x.shape[1], _stream()), "scaled_add")
+    _check(_c.xr_scaled_add(x.data_ptr(), d.data_ptr(), float(m), int(clear), x.shape[0], x.shape[1], _stream()), "scaled_add")
     _count()
 
 
@@ -781,7 +741,7 @@ def stream_step(x: torch.Tensor, x0: Optional[torch.Tensor], v: Optional[torch.T
     _dev(x, x0, v)
     assert x.dtype == torch.float32 and x.is_contiguous() and (x0 is None or (x0.dtype == torch.float32 and x0.shape == x.shape and x0.is_contiguous()))
     assert v is None or (v.dtype == torch.float32 and v.numel() == x.shape[1] and v.is_contiguous())
-    _check(lib().xr_stream_step(x.data_ptr(), _ptr(x0), _ptr(v), x.shape[0], x.shape[1], _stream()), "stream_step")
+    _check(_c.xr_stream_step(x.data_ptr(), _ptr(x0), _ptr(v), x.shape[0], x.shape[1], _stream()), "stream_step")
     _count()
 
 
@@ -791,7 +751,7 @@ def sigmoid_gate(o: torch.Tensor, g: torch.Tensor, H: int, hd: int, Vd: int, eac
     _dev(o)
     n = o.shape[0]
     assert g.is_cuda and o.dtype == g.dtype and o.stride(1) == 1 and g.stride(1) == 1 and o.shape[1] == H * hd and g.shape == (n, H * Vd if each else H)
-    _check(lib().xr_sigmoid_gate(o.data_ptr(), o.stride(0), g.data_ptr(), g.stride(0), dtype_code(o.dtype), n, H, hd, Vd, int(each),
+    _check(_c.xr_sigmoid_gate(o.data_ptr(), o.stride(0), g.data_ptr(), g.stride(0), dtype_code(o.dtype), n, H, hd, Vd, int(each),
                                  _stream()), "sigmoid_gate")
     _count()
 
@@ -801,7 +761,7 @@ def concat_cast(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor) -> None:
     _dev(a, b, out)
     n, width = a.shape
     assert a.dtype == torch.float32 and b.dtype == torch.float32 and b.shape == a.shape and out.shape == (n, 2 * width)
-    _check(lib().xr_concat_cast(a.data_ptr(), b.data_ptr(), out.data_ptr(), dtype_code(out.dtype), n, width, _stream()), "concat_cast")
+    _check(_c.xr_concat_cast(a.data_ptr(), b.data_ptr(), out.data_ptr(), dtype_code(out.dtype), n, width, _stream()), "concat_cast")
     _count()
 
 
@@ -809,7 +769,7 @@ def softcap(z: torch.Tensor, cap: float) -> None:
     """z <- cap * tanh(z / cap) in place on float32 logits."""
     _dev(z)
     assert z.dtype == torch.float32
-    _check(lib().xr_softcap(z.data_ptr(), float(cap), z.numel(), _stream()), "softcap")
+    _check(_c.xr_softcap(z.data_ptr(), float(cap), z.numel(), _stream()), "softcap")
     _count()
 
 
@@ -828,7 +788,7 @@ def latent_prep(q: torch.Tensor, down: Optional[torch.Tensor], positions, tok_se
     if cache_ptr is not None:
         assert down is not None and down.stride(1) == 1 and down.dtype == q.dtype and down.shape[1] >= C + R
         assert norm_w.dtype == torch.float32 and norm_w.numel() == C
-    _check(lib().xr_latent_prep(q.data_ptr(), dtype_code(q.dtype), q.stride(0), _ptr(down), 0 if down is None else down.stride(0),
+    _check(_c.xr_latent_prep(q.data_ptr(), dtype_code(q.dtype), q.stride(0), _ptr(down), 0 if down is None else down.stride(0),
                                 positions.data_ptr(), tok_seg.data_ptr(), block_tables.data_ptr(), _ptr(freq), _ptr(norm_w), cache_ptr,
                                 page_stride, q.shape[0], H, D, R, C, rot_dims, max_pages, page_size, float(eps), int(adjacent), _stream()),
            "latent_prep")
@@ -846,7 +806,7 @@ def head_matmul(inp: torch.Tensor, in_col: int, head_in: int, w: torch.Tensor, t
     es = inp.element_size()
     w_head, w_k, w_j = (J * Kd, 1, Kd) if transposed else (Kd * J, J, 1)
     gptr = None if gate is None else gate.data_ptr() + gate_col * gate.element_size()
-    _check(lib().xr_head_matmul(inp.data_ptr() + in_col * es, dtype_code(inp.dtype), inp.stride(0), head_in, w.data_ptr(),
+    _check(_c.xr_head_matmul(inp.data_ptr() + in_col * es, dtype_code(inp.dtype), inp.stride(0), head_in, w.data_ptr(),
                                 dtype_code(w.dtype), w_head, w_k, w_j, out.data_ptr(), dtype_code(out.dtype), out.stride(0),
                                 gptr, 0 if gate is None else dtype_code(gate.dtype), 0 if gate is None else gate.stride(0),
                                 n, H, Kd, J, int(gate_each), _stream()), "head_matmul")
@@ -863,7 +823,7 @@ def latent_attention(ql: torch.Tensor, proj: torch.Tensor, qr_col: int, head_qr:
     _dev(ql, out, positions, tok_seg, block_tables)
     n = ql.shape[0]
     assert ql.dtype == torch.float32 and out.dtype == torch.float32 and ql.shape == (n, H * C) and out.shape == (n, H * C)
-    _check(lib().xr_latent_attention(ql.data_ptr(), proj.data_ptr() + qr_col * proj.element_size(), dtype_code(proj.dtype),
+    _check(_c.xr_latent_attention(ql.data_ptr(), proj.data_ptr() + qr_col * proj.element_size(), dtype_code(proj.dtype),
                                      proj.stride(0), head_qr, out.data_ptr(), cache_ptr, page_stride, positions.data_ptr(),
                                      tok_seg.data_ptr(), block_tables.data_ptr(), n, H, C, R, max_pages, page_size, float(scale),
                                      int(window), _stream()), "latent_attention")
@@ -873,7 +833,7 @@ def latent_attention(ql: torch.Tensor, proj: torch.Tensor, qr_col: int, head_qr:
 def latent_attention_mma_supported(dtype: torch.dtype, D: int, R: int, C: int) -> bool:
     """Whether the tensor-core kernel takes these sizes: bfloat16, latent size a multiple of 64 up to 512, rotated part
     a multiple of 8, an even plain part (the query's pieces are read in pairs)."""
-    return dtype == torch.bfloat16 and D % 2 == 0 and bool(lib().xr_latent_attention_mma_supported(C, R))
+    return dtype == torch.bfloat16 and D % 2 == 0 and bool(_c.xr_latent_attention_mma_supported(C, R))
 
 
 def latent_attention_splits(n: int, H: int, max_kv_len: int, sms: int = 148) -> tuple:
@@ -909,7 +869,7 @@ def latent_attention_mma(ql: torch.Tensor, proj: torch.Tensor, qr_col: int, head
         q_tok, q_head, o32, o16, o_tok, o_head = C, n_pad * C, None, out.data_ptr(), C, n_pad * C
     if splits > 1:
         assert part_o.numel() >= n * mt * splits * 16 * C and part_ml.numel() >= n * mt * splits * 32
-    _check(lib().xr_latent_attention_mma(ql.data_ptr(), q_tok, q_head, proj.data_ptr() + qr_col * 2, proj.stride(0), head_qr, o32, o16,
+    _check(_c.xr_latent_attention_mma(ql.data_ptr(), q_tok, q_head, proj.data_ptr() + qr_col * 2, proj.stride(0), head_qr, o32, o16,
                                          o_tok, o_head, _ptr(part_o), _ptr(part_ml), cache_ptr, page_stride, positions.data_ptr(),
                                          tok_seg.data_ptr(), block_tables.data_ptr(), n, H, C, R, max_pages, page_size, float(scale),
                                          chunk, splits, int(window), _stream()), "latent_attention_mma")
@@ -920,7 +880,7 @@ def heads_gather(inp: torch.Tensor, in_col: int, head_in: int, out: torch.Tensor
     """out[h * n_pad + t] = inp[t, in_col + h * head_in : ... + Kd] (bfloat16; rows t >= n are zeros)."""
     _dev(out)
     assert inp.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and out.shape == (H * n_pad, Kd) and inp.stride(1) == 1
-    _check(lib().xr_heads_gather(inp.data_ptr() + 2 * in_col, inp.stride(0), head_in, out.data_ptr(), n, n_pad, H, Kd, _stream()), "heads_gather")
+    _check(_c.xr_heads_gather(inp.data_ptr() + 2 * in_col, inp.stride(0), head_in, out.data_ptr(), n, n_pad, H, Kd, _stream()), "heads_gather")
     _count()
 
 
@@ -931,26 +891,26 @@ def heads_scatter_gate(inp: torch.Tensor, y: torch.Tensor, gate: Optional[torch.
     _dev(inp, y)
     assert inp.dtype == torch.float32 and y.dtype == torch.bfloat16 and inp.shape == (H * n_pad, J) and y.shape == (n, H * J)
     gptr = None if gate is None else gate.data_ptr() + 2 * gate_col
-    _check(lib().xr_heads_scatter_gate(inp.data_ptr(), y.data_ptr(), gptr, 0 if gate is None else gate.stride(0), n, n_pad, H, J, int(gate_each), _stream()),
+    _check(_c.xr_heads_scatter_gate(inp.data_ptr(), y.data_ptr(), gptr, 0 if gate is None else gate.stride(0), n, n_pad, H, J, int(gate_each), _stream()),
            "heads_scatter_gate")
     _count()
 
 
 # ---------------------------------------------------------------------------
 # Matrix-memory recurrence (csrc/mlstm.cu)
-def mlstm_state_floats(H: int, D: int, V: int) -> int:
-    return H * (D * V + D + 1)
-
-
 def chunked_floats(n: int, n_seg: int, H: int, D: int, V: int, kind: str) -> int:
     """float32 values of `scratch` with which ``decay_attention`` (kind "head"), ``mlstm`` ("mlstm") and ``key_decay_attention`` ("key")
     run their recurrence in chunks (csrc/chunked.cuh) instead of token by token, for n tokens in n_seg portions; 0: not for these sizes."""
-    return int(lib().xr_chunked_floats(n, n_seg, H, D, V, ("head", "mlstm", "key").index(kind)))
+    return int(_c.xr_chunked_floats(n, n_seg, H, D, V, ("head", "mlstm", "key").index(kind)))
 
 
 def _floats(scratch: Optional[torch.Tensor]) -> int:
     assert scratch is None or scratch.dtype == torch.float32
     return 0 if scratch is None else scratch.numel()
+
+
+def mlstm_state_floats(H: int, D: int, V: int) -> int:
+    return H * (D * V + D + 1)
 
 
 def mlstm(proj: torch.Tensor, cols, gates: torch.Tensor, state: torch.Tensor, coef: torch.Tensor, o: torch.Tensor,
@@ -964,7 +924,7 @@ def mlstm(proj: torch.Tensor, cols, gates: torch.Tensor, state: torch.Tensor, co
     assert proj.stride(1) == 1 and gates.dtype == torch.float32 and gates.shape == (n, 2 * H) and state.dtype == torch.float32
     assert state.shape[1] == mlstm_state_floats(H, D, V) and coef.numel() >= 3 * n * H and o.shape == (n, H * V)
     assert y.shape == (n, H * V) and y.dtype == proj.dtype and norm_w.dtype == torch.float32 and norm_w.numel() == H * V
-    _check(lib().xr_mlstm(proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), cols[0], cols[1], cols[2], cols[3],
+    _check(_c.xr_mlstm(proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), cols[0], cols[1], cols[2], cols[3],
                           gates.data_ptr(), state.data_ptr(), coef.data_ptr(), o.data_ptr(), norm_w.data_ptr(), y.data_ptr(),
                           seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), n, n_seg, H, D, V, float(cap), float(eps),
                           _ptr(scratch), _floats(scratch), _stream()), "mlstm")
@@ -981,7 +941,7 @@ def head_norm_gate(o: torch.Tensor, gate: torch.Tensor, gate_col: int, w: Option
     assert gate.dtype in (y.dtype, torch.float32)
     assert w is None or (w.dtype == torch.float32 and w.numel() == (H * V if per_head_weight else V))
     assert gate.shape[1] >= gate_col + H * V
-    _check(lib().xr_head_norm_gate(o.data_ptr(), gate.data_ptr() + gate_col * gate.element_size(), dtype_code(gate.dtype), gate.stride(0),
+    _check(_c.xr_head_norm_gate(o.data_ptr(), gate.data_ptr() + gate_col * gate.element_size(), dtype_code(gate.dtype), gate.stride(0),
                                    _ptr(w), V if per_head_weight else 0, int(silu), y.data_ptr(), dtype_code(y.dtype), n, H, V,
                                    float(eps), _stream()), "head_norm_gate")
     _count()
@@ -1010,7 +970,7 @@ def delta(proj: torch.Tensor, conv_w: torch.Tensor, gates: torch.Tensor, neg_a: 
     assert neg_a.dtype == torch.float32 and dt_bias.dtype == torch.float32
     assert qkv.shape == (n, CH) and qkv.dtype == torch.float32 and coef.numel() >= 2 * n * H and coef.dtype == torch.float32
     assert o.shape == (n, H * V) and o.dtype == torch.float32
-    _check(lib().xr_delta(proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), conv_w.data_ptr(), gates.data_ptr(), neg_a.data_ptr(),
+    _check(_c.xr_delta(proj.data_ptr(), dtype_code(proj.dtype), proj.stride(0), conv_w.data_ptr(), gates.data_ptr(), neg_a.data_ptr(),
                           dt_bias.data_ptr(), state.data_ptr(), state.stride(0), qkv.data_ptr(), coef.data_ptr(), o.data_ptr(),
                           tok_seg.data_ptr(), seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), n, n_seg, H, G, D, V, taps,
                           _stream()), "delta")
@@ -1030,7 +990,7 @@ def route_topk(z: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, top: int, 
     n, E = z.shape
     assert z.dtype == torch.float32 and ids.dtype == torch.int32 and wts.dtype == torch.float32
     assert ids.shape == (n, top) and wts.shape == (n, top)
-    _check(lib().xr_route_topk(z.data_ptr(), z.stride(0), ids.data_ptr(), wts.data_ptr(), n, E, top, _ptr(correction), int(sigmoid_scores),
+    _check(_c.xr_route_topk(z.data_ptr(), z.stride(0), ids.data_ptr(), wts.data_ptr(), n, E, top, _ptr(correction), int(sigmoid_scores),
                                _stream()), "route_topk")
     _count()
 
@@ -1045,14 +1005,14 @@ def route_groups(z: torch.Tensor, ids: torch.Tensor, wts: torch.Tensor, top: int
     assert correction is None or (correction.dtype == torch.float32 and correction.numel() == E)
     assert z.dtype == torch.float32 and ids.dtype == torch.int32 and wts.dtype == torch.float32
     assert ids.shape == (n, top) and wts.shape == (n, top)
-    _check(lib().xr_route_groups(z.data_ptr(), ids.data_ptr(), wts.data_ptr(), n, E, top, _ptr(correction), int(groups), int(keep), float(scale),
+    _check(_c.xr_route_groups(z.data_ptr(), ids.data_ptr(), wts.data_ptr(), n, E, top, _ptr(correction), int(groups), int(keep), float(scale),
                                  _stream()), "route_groups")
     _count()
 
 
 def moe_tile_rows() -> int:
     """Rows per tile of the FMA kernel of the experts' products (the alignment its plan needs)."""
-    return int(lib().xr_moe_tile_rows())
+    return int(_c.xr_moe_tile_rows())
 
 
 def moe_max_tiles(pairs: int, E: int, align: int) -> int:
@@ -1068,7 +1028,7 @@ def moe_plan(ids: torch.Tensor, row_src, pair_row, tile_group, E: int, align: in
     pairs = ids.numel()
     max_tiles = moe_max_tiles(pairs, E, align)
     assert row_src.numel() >= max_tiles * align and pair_row.numel() >= pairs and tile_group.numel() >= max_tiles
-    _check(lib().xr_moe_plan(ids.data_ptr(), row_src.data_ptr(), pair_row.data_ptr(), tile_group.data_ptr(), pairs, E, align,
+    _check(_c.xr_moe_plan(ids.data_ptr(), row_src.data_ptr(), pair_row.data_ptr(), tile_group.data_ptr(), pairs, E, align,
                              max_tiles, _stream()), "moe_plan")
     _count()
 
@@ -1078,7 +1038,7 @@ PAIR_TILE = 256       # rows a tile of the grouped product on CTA pairs holds at
 
 def pairs_available() -> bool:
     """Whether the device runs the product on pairs of CTAs."""
-    return lib().xr_gemm_tc_pairs_available() == 1
+    return _c.xr_gemm_tc_pairs_available() == 1
 
 
 def moe_tiles_room(pairs: int, E: int):
@@ -1093,7 +1053,7 @@ def moe_plan_tiles(ids: torch.Tensor, row_src, pair_row, tiles, E: int) -> None:
     pairs = ids.numel()
     max_tiles, max_rows = moe_tiles_room(pairs, E)
     assert row_src.numel() >= max_rows and pair_row.numel() >= pairs and tiles.numel() >= 1 + 3 * max_tiles
-    _check(lib().xr_moe_plan_tiles(ids.data_ptr(), row_src.data_ptr(), pair_row.data_ptr(), tiles.data_ptr(), pairs, E, PAIR_TILE,
+    _check(_c.xr_moe_plan_tiles(ids.data_ptr(), row_src.data_ptr(), pair_row.data_ptr(), tiles.data_ptr(), pairs, E, PAIR_TILE,
                                    max_tiles, max_rows, _stream()), "moe_plan_tiles")
     _count()
 
@@ -1108,14 +1068,14 @@ def gemm_tc_grouped_pairs(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Te
     assert w_packed.shape[1] == row_tiles and w_packed.shape[2] == -(-k // TILE_K) and out.shape == (n, n_out)
     assert tiles.dtype == torch.int32 and tiles.numel() >= 1 + 3 * max_tiles
     ws = workspace(x.device)
-    _check(lib().xr_gemm_tc_grouped_pairs(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
+    _check(_c.xr_gemm_tc_grouped_pairs(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
                                           float(act_limit), n, n_out, k, x.stride(0), out.stride(0), tiles.data_ptr(), max_tiles,
                                           w_packed.shape[0], ws.status_ptr, _stream()), "gemm_tc_grouped_pairs")
     _count()
 
 
 def route_few_supported(n: int, ldz: int, outputs: int, E: int, top: int, width: int) -> bool:
-    return lib().xr_route_few_supported(n, ldz, outputs, E, top, width) == 1
+    return _c.xr_route_few_supported(n, ldz, outputs, E, top, width) == 1
 
 
 def route_few(z: torch.Tensor, splits: int, zs: torch.Tensor, outputs: int, E: int, top: int, wts: torch.Tensor, pair_row: torch.Tensor,
@@ -1131,7 +1091,7 @@ def route_few(z: torch.Tensor, splits: int, zs: torch.Tensor, outputs: int, E: i
     assert correction is None or (correction.dtype == torch.float32 and correction.numel() == outputs)
     assert h.dtype == torch.bfloat16 and xs.dtype == torch.bfloat16 and h.stride(1) == 1 and h.shape == (n, xs.shape[1])
     assert wts.numel() >= n * top and pair_row.numel() >= n * top and tile_group.numel() >= max_tiles and xs.shape[0] >= max_tiles * align
-    _check(lib().xr_route_few(z.data_ptr(), splits, zs.data_ptr(), ldz, n, outputs, E, top, _ptr(correction), mode, groups, keep, float(scale),
+    _check(_c.xr_route_few(z.data_ptr(), splits, zs.data_ptr(), ldz, n, outputs, E, top, _ptr(correction), mode, groups, keep, float(scale),
                               wts.data_ptr(), pair_row.data_ptr(), tile_group.data_ptr(), align, max_tiles, h.data_ptr(), h.stride(0), xs.data_ptr(),
                               h.shape[1], _stream()), "route_few")
     _count()
@@ -1142,7 +1102,7 @@ def moe_gather(h: torch.Tensor, out: torch.Tensor, row_src, tile_group: Optional
     ``moe_plan_tiles``, those stay as they are)."""
     _dev(out, row_src, tile_group)
     assert h.stride(1) == 1 and out.shape[1] == h.shape[1] and out.dtype == h.dtype and out.shape[0] % align == 0
-    _check(lib().xr_moe_gather(h.data_ptr(), dtype_code(h.dtype), h.stride(0), out.data_ptr(), row_src.data_ptr(),
+    _check(_c.xr_moe_gather(h.data_ptr(), dtype_code(h.dtype), h.stride(0), out.data_ptr(), row_src.data_ptr(),
                                _ptr(tile_group), top, h.shape[1], align, out.shape[0], _stream()), "moe_gather")
     _count()
 
@@ -1157,7 +1117,7 @@ def moe_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, row_src, tile_
     E, rows, K = w.shape
     N = rows // 2 if gated else rows
     assert a.shape[1] == K and out.shape[1] == N and out.shape[0] % moe_tile_rows() == 0
-    _check(lib().xr_moe_gemm(a.data_ptr(), dtype_code(a.dtype), a.stride(0), w.data_ptr(), dtype_code(w.dtype), out.data_ptr(),
+    _check(_c.xr_moe_gemm(a.data_ptr(), dtype_code(a.dtype), a.stride(0), w.data_ptr(), dtype_code(w.dtype), out.data_ptr(),
                              dtype_code(out.dtype), out.stride(0), row_src.data_ptr(), tile_group.data_ptr(),
                              out.shape[0] // moe_tile_rows(), top, N, K, int(gated), int(gather), int(act), float(limit), _stream()), "moe_gemm")
     _count()
@@ -1180,7 +1140,7 @@ def gemm_tc_grouped(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, 
     assert w_packed.shape[1] == tiles and w_packed.shape[2] == -(-k // TILE_K) and out.shape == (n, n_out)
     assert tile_group.dtype == torch.int32 and tile_group.numel() >= n // bn
     ws = workspace(x.device)
-    _check(lib().xr_gemm_tc_grouped(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
+    _check(_c.xr_gemm_tc_grouped(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
                                     float(act_limit), n, n_out, k, x.stride(0), out.stride(0), bn, tile_group.data_ptr(),
                                     w_packed.shape[0], ws.status_ptr, _stream()), "gemm_tc_grouped")
     _count()
@@ -1200,7 +1160,7 @@ def moe_combine(d: torch.Tensor, z: torch.Tensor, wts: torch.Tensor, pair_row: t
     assert shared is None or (shared.dtype == torch.float32 and splits >= 1 and shared.numel() >= splits * n * width)
     assert gate is None or (shared is not None and gate.is_cuda and gate.dtype == torch.float32 and gate.shape == (n,))
     assert (norm_w is None) == (out is None) and (out is None or (out.shape == d.shape and norm_w.dtype == torch.float32 and norm_w.numel() == width))
-    _check(lib().xr_moe_combine(d.data_ptr(), z.data_ptr(), wts.data_ptr(), pair_row.data_ptr(), _ptr(h), 0 if h is None else dtype_code(h.dtype),
+    _check(_c.xr_moe_combine(d.data_ptr(), z.data_ptr(), wts.data_ptr(), pair_row.data_ptr(), _ptr(h), 0 if h is None else dtype_code(h.dtype),
                                 0 if h is None else h.stride(0), _ptr(shared), int(splits), _ptr(gate), 0 if gate is None else gate.stride(0), float(scale),
                                 _ptr(norm_w), _ptr(out), 0 if out is None else dtype_code(out.dtype), float(eps), n, width, top, _stream()),
            "moe_combine")
@@ -1217,7 +1177,7 @@ def embed_pair(table: torch.Tensor, pairs: torch.Tensor, ids, positions, tok_seg
     n, d = x.shape
     assert table.dtype == pairs.dtype and table.shape[1] == d and pairs.shape[1] == d and pairs.shape[0] >= 2
     assert x.dtype == torch.float32 and last.dtype == torch.int32 and ids.dtype == torch.int32
-    _check(lib().xr_embed_pair(table.data_ptr(), pairs.data_ptr(), dtype_code(table.dtype), ids.data_ptr(), _ptr(feed),
+    _check(_c.xr_embed_pair(table.data_ptr(), pairs.data_ptr(), dtype_code(table.dtype), ids.data_ptr(), _ptr(feed),
                                0 if feed is None else feed.numel(), positions.data_ptr(), tok_seg.data_ptr(), seg_start.data_ptr(),
                                seg_slot.data_ptr(), last.data_ptr(), x.data_ptr(), n, d, table.shape[0], pairs.shape[0] - 1, int(mul_prev),
                                int(mul_cur), _stream()), "embed_pair")
@@ -1227,7 +1187,7 @@ def embed_pair(table: torch.Tensor, pairs: torch.Tensor, ids, positions, tok_seg
 def last_token(ids, seg_start, seg_len, seg_slot, last: torch.Tensor, n_seg: int, vocab: int, feed: Optional[torch.Tensor] = None) -> None:
     """last[slot of portion s] = the portion's last token."""
     _dev(ids, seg_start, seg_len, seg_slot, last, feed)
-    _check(lib().xr_last_token(ids.data_ptr(), _ptr(feed), 0 if feed is None else feed.numel(), seg_start.data_ptr(), seg_len.data_ptr(),
+    _check(_c.xr_last_token(ids.data_ptr(), _ptr(feed), 0 if feed is None else feed.numel(), seg_start.data_ptr(), seg_len.data_ptr(),
                                seg_slot.data_ptr(), last.data_ptr(), n_seg, vocab, _stream()), "last_token")
     _count()
 
@@ -1243,7 +1203,7 @@ def norm_add(d: torch.Tensor, x: torch.Tensor, gain: torch.Tensor, eps: float, c
     n, w = x.shape
     assert d.shape == (n, w) and d.dtype == torch.float32 and x.dtype == torch.float32 and gain.dtype == torch.float32 and gain.numel() == 1
     assert cast is None or cast.shape == (n, w)
-    _check(lib().xr_norm_add(d.data_ptr(), x.data_ptr(), gain.data_ptr(), _ptr(cast), 0 if cast is None else dtype_code(cast.dtype), n, w,
+    _check(_c.xr_norm_add(d.data_ptr(), x.data_ptr(), gain.data_ptr(), _ptr(cast), 0 if cast is None else dtype_code(cast.dtype), n, w,
                              float(eps), int(clear), _ptr(partial), _ptr(bias), int(splits), _stream()), "norm_add")
     _count()
 
@@ -1255,7 +1215,7 @@ def row_norm_gate(o: torch.Tensor, gate: torch.Tensor, gate_col: int, w: torch.T
     n, width = o.shape
     assert o.dtype == torch.float32 and gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape[1] >= gate_col + width
     assert w.dtype == torch.float32 and w.numel() == width and y.shape == (n, width)
-    _check(lib().xr_row_norm_gate(o.data_ptr(), gate.data_ptr() + 4 * gate_col, gate.stride(0), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype),
+    _check(_c.xr_row_norm_gate(o.data_ptr(), gate.data_ptr() + 4 * gate_col, gate.stride(0), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype),
                                   n, width, float(eps), float(scale), _stream()), "row_norm_gate")
     _count()
 
@@ -1264,7 +1224,7 @@ def cast_rows(x: torch.Tensor, out: torch.Tensor) -> None:
     """out = x in out's dtype (x float32)."""
     _dev(x, out)
     assert x.dtype == torch.float32 and out.numel() == x.numel()
-    _check(lib().xr_cast_rows(x.data_ptr(), out.data_ptr(), dtype_code(out.dtype), x.numel(), _stream()), "cast_rows")
+    _check(_c.xr_cast_rows(x.data_ptr(), out.data_ptr(), dtype_code(out.dtype), x.numel(), _stream()), "cast_rows")
     _count()
 
 
@@ -1273,7 +1233,7 @@ def depth_average(x: torch.Tensor, x0: torch.Tensor, hist: torch.Tensor, w: torc
     _dev(x, x0, hist, w, cast)
     assert x.dtype == torch.float32 and x0.shape == x.shape and hist.dtype == torch.float32 and hist.shape[0] >= k and hist[0].numel() == x.numel()
     assert w.dtype == torch.float32 and w.numel() == k + 1
-    _check(lib().xr_depth_average(x.data_ptr(), x0.data_ptr(), hist.data_ptr(), w.data_ptr(), _ptr(cast),
+    _check(_c.xr_depth_average(x.data_ptr(), x0.data_ptr(), hist.data_ptr(), w.data_ptr(), _ptr(cast),
                                   0 if cast is None else dtype_code(cast.dtype), k, x.numel(), _stream()), "depth_average")
     _count()
 
@@ -1285,7 +1245,7 @@ def rotate_heads(rows: torch.Tensor, col0: int, heads: int, head_stride: int, di
     _dev(freq, positions)
     assert rows.stride(1) == 1 and rows.is_cuda and rows.shape[1] >= col0 + (heads - 1) * head_stride + live
     assert freq.dtype == torch.float64 and freq.numel() >= dims // 2
-    _check(lib().xr_rotate_heads(rows.data_ptr(), dtype_code(rows.dtype), rows.stride(0), col0, heads, head_stride, dims, live, int(adjacent),
+    _check(_c.xr_rotate_heads(rows.data_ptr(), dtype_code(rows.dtype), rows.stride(0), col0, heads, head_stride, dims, live, int(adjacent),
                                  freq.data_ptr(), positions.data_ptr(), float(sign), float(scale), rows.shape[0], _stream()), "rotate_heads")
     _count()
 
@@ -1311,7 +1271,7 @@ def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, s
     assert all(t.dtype == torch.float32 for t in (conv_w, conv_b, wa, wi, ba, bi, lam, state, a_s, b_s))
     assert conv_w.shape == (R, taps) and all(t.shape == (B, Bs, Bs) for t in (wa, wi)) and a_s.numel() >= n * R and b_s.numel() >= n * R
     assert state.dim() == 2 and state.shape[1] >= rglru_state_floats(R, taps)
-    _check(lib().xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(),
+    _check(_c.xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(),
                           wa.data_ptr(), wi.data_ptr(), ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
                           seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), u_s.data_ptr(), out.data_ptr(),
                           dtype_code(out.dtype), n, n_seg, R, B, taps, float(c), _stream()), "rglru")
@@ -1327,7 +1287,7 @@ def decay_attention(proj: torch.Tensor, cols, decay: torch.Tensor, state: torch.
     n = proj.shape[0]
     assert proj.dtype == torch.float32 and proj.stride(1) == 1 and o.shape == (n, H * V) and o.dtype == torch.float32
     assert decay.dtype == torch.float32 and decay.numel() == H and state.dtype == torch.float32 and state.shape[1] >= H * D * V
-    _check(lib().xr_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], decay.data_ptr(), state.data_ptr(),
+    _check(_c.xr_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], decay.data_ptr(), state.data_ptr(),
                                     state.stride(0), seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), o.data_ptr(), n, n_seg, H, D, V,
                                     int(silu), float(read_scale), _ptr(scratch), _floats(scratch), _stream()), "decay_attention")
     _count((2 if silu and n > 16 else 1) + (0 if scratch is None else 3))
@@ -1346,7 +1306,7 @@ def key_decay_attention(proj: torch.Tensor, cols, inner: int, w_t: torch.Tensor,
     assert w_t.dtype == torch.float32 and w_t.shape == (inner, H * D) and bias.dtype == torch.float32 and bias.numel() == H * D
     assert decays.dtype == torch.float32 and decays.numel() >= n * H * D and proj.shape[1] >= cols[3] + inner
     assert state.dtype == torch.float32 and state.shape[1] >= H * D * V
-    _check(lib().xr_key_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], cols[3], w_t.data_ptr(), bias.data_ptr(), int(inner),
+    _check(_c.xr_key_decay_attention(proj.data_ptr(), proj.stride(0), cols[0], cols[1], cols[2], cols[3], w_t.data_ptr(), bias.data_ptr(), int(inner),
                                         float(tau), decays.data_ptr(), state.data_ptr(), state.stride(0), seg_start.data_ptr(), seg_len.data_ptr(),
                                         seg_slot.data_ptr(), o.data_ptr(), n, n_seg, H, D, V, float(read_scale), _ptr(scratch), _floats(scratch), _stream()), "key_decay_attention")
     _count(2 if scratch is None else 6)
@@ -1370,7 +1330,7 @@ def ssd(proj: torch.Tensor, x_col: int, dt_col: int, conv_w, conv_b, dt_bias, ne
     assert conv_w.shape == (CH, taps) and conv_b.numel() == CH and all(t.numel() == H for t in (dt_bias, neg_a, skip))
     assert state.dim() == 2 and state.shape[1] >= ssd_state_floats(H, G, N, V, taps)
     assert xbc.shape == (n, CH) and coef.numel() >= 2 * n * H and y.shape == (n, H * V)
-    _check(lib().xr_ssd(proj.data_ptr(), proj.stride(0), x_col, dt_col, conv_w.data_ptr(), conv_b.data_ptr(), dt_bias.data_ptr(), neg_a.data_ptr(),
+    _check(_c.xr_ssd(proj.data_ptr(), proj.stride(0), x_col, dt_col, conv_w.data_ptr(), conv_b.data_ptr(), dt_bias.data_ptr(), neg_a.data_ptr(),
                         skip.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(), seg_start.data_ptr(), seg_len.data_ptr(),
                         seg_slot.data_ptr(), xbc.data_ptr(), coef.data_ptr(), y.data_ptr(), n, n_seg, H, G, N, V, taps, _stream()), "ssd")
     _count(2)
@@ -1383,6 +1343,6 @@ def silu_gate_norm(o: torch.Tensor, gate: torch.Tensor, gate_col: int, w: torch.
     n, width = o.shape
     assert o.dtype == torch.float32 and gate.dtype == torch.float32 and gate.stride(1) == 1 and gate.shape[1] >= gate_col + width
     assert w.dtype == torch.float32 and w.numel() == width and y.shape == (n, width)
-    _check(lib().xr_silu_gate_norm(o.data_ptr(), gate.data_ptr() + 4 * gate_col, gate.stride(0), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype),
+    _check(_c.xr_silu_gate_norm(o.data_ptr(), gate.data_ptr() + 4 * gate_col, gate.stride(0), w.data_ptr(), y.data_ptr(), dtype_code(y.dtype),
                                    n, width, int(groups), float(eps), _stream()), "silu_gate_norm")
     _count()
