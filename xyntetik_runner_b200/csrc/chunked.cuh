@@ -6,9 +6,9 @@
 // first token to t, S the memory before the chunk:
 //   o_i = (q_i exp(c_i))^T S + sum_(j <= i) P_ij v_j,      P_ij = s_j sum_d q_i[d] k_j[d] exp(c_i[d] - c_j[d])
 //   S'  = diag(exp(c_last)) S + sum_j (k_j s_j exp(c_last - c_j)) v_j^T
-// Four kernels: ck_scores (per chunk and head: the row [q_i exp(c_i) | P_i] of every token), ck_states (the sum of S'), ck_scan (the
-// memories before every chunk, one after another, in the place of the sums, and the slot's new state) and ck_out (one product of
-// [64 x (D + 64)] with [S; v]).  c is summed and subtracted in float64, so that a difference of two sums keeps float32's relative
+// Four kernels: ck_scores (per chunk and head: the row [q_i exp(c_i) | P_i] of every token and its key k~_j = k_j s_j exp(c_last - c_j)),
+// ck_states (the sum of S'), ck_scan (the memories before every chunk, one after another, in the place of the sums, and the slot's new
+// state) and ck_out (one product of [64 x (D + 64)] with [S; v]).  c is summed and subtracted in float64, so that a difference of two sums keeps float32's relative
 // precision however far both have gone; every exponential's argument is at or below zero, except in the short cut of decays per
 // channel (ck_scores).
 //
@@ -17,8 +17,8 @@
 // chunks at once.  It costs about half as many operations again and the memories' way through L2, so it is for portions of many
 // tokens: the callers say from how many (a short portion beside a long one is a chunk of its own).  The sums come in another order
 // than the walk's, so a state depends in its last bits on where portions were cut; callers that promise the same bits take the walk.
-// 2,048 tokens of one request, 8 heads, us, walk / chunks: constant decay, 128 x 128 values: 166 / 79; decay per channel, 128 x 256:
-// 222 / 164; mLSTM, 128 x 256: 906 / 197.  Root mean square error of the read-outs against float64, 2,040 tokens, walk / chunks: 2.3e-7 /
+// 2,048 tokens of one request, 8 heads, us, walk / chunks: constant decay, 128 x 128 values: 166 / 75; decay per channel, 128 x 256:
+// 223 / 138; mLSTM, 128 x 256: 906 / 193.  Root mean square error of the read-outs against float64, 2,040 tokens, walk / chunks: 2.3e-7 /
 // 1.7e-7; 2.1e-6 / 1.8e-7; 6.9e-7 / 6.5e-7.
 #pragma once
 #include "common.cuh"
@@ -36,6 +36,7 @@ struct ChunkArgs {
     const double* cum;               // c: CK_TOKEN [n][H], CK_KEY [n][H D]
     const float* in_scale;           // s: [n][H], or null (one)
     float* rows;                     // [chunks][H][64][D + 64]
+    float* keys;                     // k~: [chunks][H][64][D]
     float* mem;                      // [chunks][H][D][V]
     float* mem_n;                    // NORM: [chunks][H][D]
     float* state; long long state_stride, head_stride;   // a slot's head h at + h * head_stride: [V][D], or with `rows_first` [D][V]
@@ -107,27 +108,39 @@ ck_scores(ChunkArgs a) {
     float* qs = ck_sm;                       // [64][LD]
     float* ks = qs + CK_L * LD;              // [64][LD]; CK_KEY: 48 rows more behind it
     __shared__ double cs[CK_L];
+    __shared__ float ends[CK_L];
     __shared__ int deep;
     const int h = blockIdx.x, tid = threadIdx.x;
     const ChunkPlace p = ck_place(a, blockIdx.y);
     xr_pdl_wait();
     if (p.seg < 0) return;
     if (tid == 0) deep = 0;
-    if (KIND != CK_KEY && tid < CK_L)
-        cs[tid] = KIND == CK_HEAD ? (tid + 1) * log((double)a.decay[h]) : a.cum[(size_t)(p.t0 + min(tid, p.count - 1)) * a.H + h];
+    const int last = p.t0 + p.count - 1;
+    if (KIND != CK_KEY && tid < CK_L) {
+        // c, and what a key's outer product is worth at the chunk's end
+        const int t = min(tid, p.count - 1);
+        const double lad = KIND == CK_HEAD ? log((double)a.decay[h]) : 0.0;
+        cs[tid] = KIND == CK_HEAD ? (tid + 1) * lad : a.cum[(size_t)(p.t0 + t) * a.H + h];
+        float f = KIND == CK_HEAD ? (t == p.count - 1 ? 1.f : ck_exp((p.count - 1 - t) * lad)) : ck_exp(a.cum[(size_t)last * a.H + h] - a.cum[(size_t)(p.t0 + t) * a.H + h]);
+        if (a.in_scale != nullptr) f *= a.in_scale[(size_t)(p.t0 + t) * a.H + h];
+        ends[tid] = f;
+    }
     __syncthreads();
     if (KIND == CK_KEY && tid < D && a.cum[((size_t)(p.t0 + p.count - 1) * a.H + h) * D + tid] < -CK_DEEP) deep = 1;
     if (KIND == CK_KEY) __syncthreads();
     float* out = a.rows + ((size_t)blockIdx.y * a.H + h) * CK_L * LR;
+    float* keys = a.keys + ((size_t)blockIdx.y * a.H + h) * CK_L * D;
     for (int e = tid * 4; e < CK_L * D; e += 1024) {
         const int t = e / D, d = e % D;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q, r = q;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q, r = q, kt = q;
         if (t < p.count) {
             q = *reinterpret_cast<const float4*>(a.q + (size_t)(p.t0 + t) * a.ld_q + h * D + d);
             k = *reinterpret_cast<const float4*>(a.k + (size_t)(p.t0 + t) * a.ld_k + h * D + d);
             if (KIND == CK_KEY) {
                 const double* c = a.cum + ((size_t)(p.t0 + t) * a.H + h) * D + d;
                 const double c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+                const double* cl = a.cum + ((size_t)last * a.H + h) * D + d;
+                kt = make_float4(k.x * ck_exp(cl[0] - c0), k.y * ck_exp(cl[1] - c1), k.z * ck_exp(cl[2] - c2), k.w * ck_exp(cl[3] - c3));
                 r = make_float4(q.x * ck_exp(c0), q.y * ck_exp(c1), q.z * ck_exp(c2), q.w * ck_exp(c3));
                 if (!deep) {
                     q = r;
@@ -139,11 +152,14 @@ ck_scores(ChunkArgs a) {
             } else {
                 const float f = ck_exp(cs[t]);
                 r = make_float4(q.x * f, q.y * f, q.z * f, q.w * f);
+                float g = ends[t];
+                kt = make_float4(k.x * g, k.y * g, k.z * g, k.w * g);
             }
         }
         *reinterpret_cast<float4*>(qs + t * LD + d) = q;
         *reinterpret_cast<float4*>(ks + t * LD + d) = k;
         *reinterpret_cast<float4*>(out + t * LR + d) = r;
+        *reinterpret_cast<float4*>(keys + t * D + d) = kt;
     }
     __syncthreads();
     // thread: tokens i = ti + 16 r, keys j = tj + 16 r (r = 0..3): rows 16 apart, so that a warp's sixteen tj read neighbouring rows
@@ -236,76 +252,60 @@ ck_scores(ChunkArgs a) {
 }
 
 // ---- sum_j k~_j v_j^T -----------------------------------------------------------------------------------------------
-// 256 threads over D x 64: (D / 16) x 4 each, four channels and four columns at a time.
-template <int D, int KIND, bool NORM>
+// 256 threads over D x 64: (D / 16) x 4 each, four channels and four columns at a time; all of the chunk's keys (as ck_scores left them)
+// and values on their way at once.  (With the keys' exponentials taken here, once for every 64 value columns, the recurrence with decays
+// per channel took 164 us at 2,048 tokens, 8 heads of 128 x 256; 138 so.)
+template <int D, bool NORM>
 __global__ void __launch_bounds__(256)
 ck_states(ChunkArgs a) {
     xr_pdl_launch();
     constexpr int RD = D / 16;               // channels a thread: 4 (tid / 16) + 64 m + (0..3)
-    __shared__ __align__(16) float ks[32][D], vs[32][CK_VT];
+    __shared__ __align__(16) float ks[CK_L][D], vs[CK_L][CK_VT];
     const int v0 = blockIdx.x * CK_VT, h = blockIdx.y, tid = threadIdx.x;
     const ChunkPlace p = ck_place(a, blockIdx.z);
     xr_pdl_wait();
     if (p.seg < 0) return;
+    const size_t at = (size_t)blockIdx.z * a.H + h;
+    for (int e = tid * 4; e < CK_L * D; e += 1024)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(&ks[0][0] + e)), "l"(a.keys + at * CK_L * D + e) : "memory");
+    for (int e = tid * 4; e < CK_L * CK_VT; e += 1024) {
+        const int j = e / CK_VT, c = e % CK_VT, live = j < p.count ? 16 : 0;          // (no token: zeros)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(&vs[0][0] + e)),
+                     "l"(a.v + (size_t)(p.t0 + (live ? j : 0)) * a.ld_v + (size_t)h * a.V + v0 + c), "r"(live) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
     const int td = tid >> 4, tv = tid & 15;
-    float acc[RD][4], sum_n = 0.f;
+    float acc[RD][4];
 #pragma unroll
     for (int r = 0; r < RD; r++)
 #pragma unroll
         for (int s = 0; s < 4; s++) acc[r][s] = 0.f;
-    const int last = p.t0 + p.count - 1;
-    const double lad = KIND == CK_HEAD ? log((double)a.decay[h]) : 0.0;
-    for (int half = 0; half < p.count; half += 32) {
-        __syncthreads();
-        for (int e = tid * 4; e < 32 * D; e += 1024) {
-            const int j = half + e / D, d = e % D, t = p.t0 + j;
-            float4 k = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j < p.count) {
-                k = *reinterpret_cast<const float4*>(a.k + (size_t)t * a.ld_k + h * D + d);
-                if (KIND == CK_KEY) {
-                    const double* c = a.cum + ((size_t)t * a.H + h) * D + d;
-                    const double* cl = a.cum + ((size_t)last * a.H + h) * D + d;
-                    k = make_float4(k.x * expf((float)(cl[0] - c[0])), k.y * expf((float)(cl[1] - c[1])), k.z * expf((float)(cl[2] - c[2])),
-                                    k.w * expf((float)(cl[3] - c[3])));
-                } else {
-                    float f = KIND == CK_HEAD ? expf((float)((p.count - 1 - j) * lad)) : expf((float)(a.cum[(size_t)last * a.H + h] - a.cum[(size_t)t * a.H + h]));
-                    if (KIND == CK_HEAD && j == p.count - 1) f = 1.f;
-                    if (a.in_scale != nullptr) f *= a.in_scale[(size_t)t * a.H + h];
-                    k = make_float4(k.x * f, k.y * f, k.z * f, k.w * f);
-                }
-            }
-            *reinterpret_cast<float4*>(&ks[e / D][d]) = k;
-        }
-        for (int e = tid * 4; e < 32 * CK_VT; e += 1024) {
-            const int j = half + e / CK_VT, c = e % CK_VT;
-            *reinterpret_cast<float4*>(&vs[e / CK_VT][c]) =
-                j < p.count ? *reinterpret_cast<const float4*>(a.v + (size_t)(p.t0 + j) * a.ld_v + (size_t)h * a.V + v0 + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        __syncthreads();
 #pragma unroll 4
-        for (int j = 0; j < 32; j++) {
-            const float4 v = *reinterpret_cast<const float4*>(&vs[j][4 * tv]);
+    for (int j = 0; j < CK_L; j++) {
+        const float4 v = *reinterpret_cast<const float4*>(&vs[j][4 * tv]);
 #pragma unroll
-            for (int m = 0; m < RD / 4; m++) {
-                const float4 k = *reinterpret_cast<const float4*>(&ks[j][64 * m + 4 * td]);
-                const float kk[4] = {k.x, k.y, k.z, k.w};
+        for (int m = 0; m < RD / 4; m++) {
+            const float4 k = *reinterpret_cast<const float4*>(&ks[j][64 * m + 4 * td]);
+            const float kk[4] = {k.x, k.y, k.z, k.w};
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    acc[4 * m + r][0] = fmaf(kk[r], v.x, acc[4 * m + r][0]); acc[4 * m + r][1] = fmaf(kk[r], v.y, acc[4 * m + r][1]);
-                    acc[4 * m + r][2] = fmaf(kk[r], v.z, acc[4 * m + r][2]); acc[4 * m + r][3] = fmaf(kk[r], v.w, acc[4 * m + r][3]);
-                }
+            for (int r = 0; r < 4; r++) {
+                acc[4 * m + r][0] = fmaf(kk[r], v.x, acc[4 * m + r][0]); acc[4 * m + r][1] = fmaf(kk[r], v.y, acc[4 * m + r][1]);
+                acc[4 * m + r][2] = fmaf(kk[r], v.z, acc[4 * m + r][2]); acc[4 * m + r][3] = fmaf(kk[r], v.w, acc[4 * m + r][3]);
             }
         }
-        if (NORM && blockIdx.x == 0 && tid < D)
-            for (int j = 0; j < 32; j++) sum_n += ks[j][tid];
     }
-    float* out = a.mem + ((size_t)blockIdx.z * a.H + h) * D * a.V + v0 + 4 * tv;
+    float* out = a.mem + at * D * a.V + v0 + 4 * tv;
 #pragma unroll
     for (int m = 0; m < RD / 4; m++)
 #pragma unroll
         for (int r = 0; r < 4; r++)
             *reinterpret_cast<float4*>(out + (size_t)(64 * m + 4 * td + r) * a.V) = make_float4(acc[4 * m + r][0], acc[4 * m + r][1], acc[4 * m + r][2], acc[4 * m + r][3]);
-    if (NORM && blockIdx.x == 0 && tid < D) a.mem_n[((size_t)blockIdx.z * a.H + h) * D + tid] = sum_n;
+    if (NORM && blockIdx.x == 0 && tid < D) {
+        float sum = 0.f;
+        for (int j = 0; j < CK_L; j++) sum += ks[j][tid];
+        a.mem_n[at * D + tid] = sum;
+    }
 }
 
 // ---- the memories before the chunks ------------------------------------------------------------------------------------
@@ -472,16 +472,17 @@ ck_out(ChunkArgs a) {
 static inline bool ck_takes(int D, int V) { return (D == 64 || D == 128) && V >= CK_VT && V % CK_VT == 0; }
 // chunks of a step of n tokens in n_seg portions, at most
 static inline long long ck_chunks(int n, int n_seg) { return n / CK_L + n_seg; }
-// float32 of scratch: rows, memories (and sums of keys), then float64 sums c of `cum_cols` columns a token
+// float32 of scratch: rows, keys, memories (and sums of keys), then float64 sums c of `cum_cols` columns a token
 static inline long long ck_floats(int n, int n_seg, int H, int D, int V, int cum_cols, bool norm) {
-    const long long per = (long long)CK_L * (D + CK_L) + (long long)D * V + (norm ? D : 0);
+    const long long per = (long long)CK_L * (2 * D + CK_L) + (long long)D * V + (norm ? D : 0);
     return ck_chunks(n, n_seg) * H * per + 2LL * n * cum_cols + 8;
 }
 // lays the scratch out; returns where the sums c begin
 static inline double* ck_lay_out(ChunkArgs& a, float* scratch, int n, int D, bool norm) {
     const long long heads = ck_chunks(n, a.n_seg) * a.H;
     a.rows = scratch;
-    a.mem = a.rows + heads * CK_L * (D + CK_L);
+    a.keys = a.rows + heads * CK_L * (D + CK_L);
+    a.mem = a.keys + heads * CK_L * D;
     a.mem_n = norm ? a.mem + heads * D * a.V : nullptr;
     float* end = a.mem + heads * D * a.V + (norm ? heads * D : 0);
     return reinterpret_cast<double*>(((uintptr_t)end + 15) & ~(uintptr_t)15);
@@ -497,7 +498,7 @@ static int ck_launch(const ChunkArgs& a, int n, cudaStream_t stream) {
                               cudaFuncSetAttribute(ck_out<D, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S4) == cudaSuccess;
     if (!ready) return XR_ERR_LAUNCH;
     xr_launch((ck_scores<D, KIND>), dim3(a.H, chunks), dim3(256), S1, stream, a);
-    xr_launch((ck_states<D, KIND, NORM>), dim3(vt, a.H, chunks), dim3(256), 0, stream, a);
+    xr_launch((ck_states<D, NORM>), dim3(vt, a.H, chunks), dim3(256), 0, stream, a);
     xr_launch((ck_scan<D, KIND, NORM>), dim3((D * a.V + (NORM ? D : 0) + 255) / 256, a.H, a.n_seg), dim3(256), 0, stream, a);
     xr_launch((ck_out<D, NORM>), dim3(vt, a.H, chunks), dim3(128), S4, stream, a);
     return xr_launch_status();

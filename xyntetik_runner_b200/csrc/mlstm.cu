@@ -376,7 +376,7 @@ static int mlstm_chunked(const T* proj, long long ldp, int q_col, int k_col, int
     float* floor_n = in_scale + (size_t)n * H;
     float* rest = reinterpret_cast<float*>(((uintptr_t)(floor_n + (size_t)n * H) + 15) & ~(uintptr_t)15);
     const long long head = (long long)ml_state_head(D, V);
-    ChunkArgs a{rows, rows + HD, rows + 2 * HD, cols, cols, cols, H, V, nullptr, nullptr, in_scale, nullptr, nullptr, nullptr, state, (long long)H * head,
+    ChunkArgs a{rows, rows + HD, rows + 2 * HD, cols, cols, cols, H, V, nullptr, nullptr, in_scale, nullptr, nullptr, nullptr, nullptr, state, (long long)H * head,
                 head, 1, seg_start, seg_len, seg_slot, n_seg, o, 1.0f, floor_n};
     double* cum = ck_lay_out(a, rest, n, D, true);
     a.cum = cum;

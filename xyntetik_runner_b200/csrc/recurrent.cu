@@ -876,7 +876,7 @@ XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_co
     }
     if (scratch != nullptr && ck_takes(D, V) && (many || !silu)) {
         if (scratch_floats < ck_floats(n, n_seg, H, D, V, 0, false)) return XR_ERR_ARG;
-        ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, decay, nullptr, nullptr, nullptr, nullptr, nullptr, state,
+        ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, decay, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
                     state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
         ck_lay_out(a, scratch, n, D, false);
         if (ck_aligned(a)) return ck_run<CK_HEAD, false>(a, n, D, stream);
@@ -937,7 +937,7 @@ XR_EXPORT int xr_key_decay_attention(const float* proj, long long ldp, int q_col
         state_stride < (long long)H * D * V)
         return XR_ERR_ARG;
     const int C = H * D;
-    ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
+    ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
                 state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
     const int chunked = scratch != nullptr && ck_takes(D, V) && ck_aligned(a) && ck_chunks(n, n_seg) <= 65535;
     if (chunked && scratch_floats < ck_floats(n, n_seg, H, D, V, C, false)) return XR_ERR_ARG;

@@ -6,10 +6,10 @@ import torch
 from .. import kernels
 
 # Portions of at least so many tokens.  The walk takes about 0.1 us a token whatever stands beside it (mLSTM's 0.4); the chunks take
-# five to eight launches of a few microseconds each.  8 heads, us, walk / chunks: constant decay 512 tokens 45 / 48, 777 66 / 59; decay
-# per key channel 777 tokens 95 / 95, 1,024 120 / 106; mLSTM 128 tokens 64 / 73, 192 92 / 73.  (The state-space recurrence of Mamba-2,
+# five to eight launches of a few microseconds each.  8 heads, us, walk / chunks: constant decay 512 tokens 45 / 44, 777 66 / 58; decay
+# per key channel 512 tokens 68 / 81, 777 96 / 88; mLSTM 128 tokens 64 / 73, 192 92 / 73.  (The state-space recurrence of Mamba-2,
 # whose heads have 64 values and fill the machine, is as fast walked at every size up to 2,048.)
-CHUNKED_FROM = {"head": 768, "key": 1024, "mlstm": 192}
+CHUNKED_FROM = {"head": 640, "key": 768, "mlstm": 192}
 
 
 def chunk_scratch(ctx, kind: str, H: int, D: int, V: int):
