@@ -47,10 +47,6 @@ class BuildError(RuntimeError):
     pass
 
 
-class NoHeaders(BuildError):
-    pass
-
-
 def sources() -> List[str]:
     return sorted(f for f in os.listdir(HERE) if f.endswith(".cu"))
 
@@ -245,7 +241,7 @@ def calls_path(build: bool = True) -> str:
     if not build:
         raise BuildError("the extension of direct calls is not built")
     if not os.path.isfile(os.path.join(include, "Python.h")):
-        raise NoHeaders(f"no Python.h in {include}: the extension of direct calls cannot be built")
+        raise BuildError(f"no Python.h in {include}: the extension of direct calls cannot be built")
     for d in _build_dirs():
         if not _writable(d):
             continue

@@ -39,7 +39,7 @@ def lib() -> ctypes.CDLL:
 
 
 class _Calls:
-    """Stands for the direct calls (csrc/calls.py: an extension with one function per launcher, a third of ctypes' cost a call) until the
+    """Stands for the direct calls (csrc/calls.py: an extension with one function per launcher, a sixth of ctypes' cost a call) until the
     first is used; then the extension takes its place."""
 
     def __getattr__(self, name):
@@ -47,7 +47,7 @@ class _Calls:
         L = lib()
         try:
             _c = _build.calls(_build.library_path(build=False))
-        except _build.NoHeaders:             # (a Python without its headers: the same calls through ctypes)
+        except _build.BuildError:            # (a Python without its headers, or no compiler: the same calls through ctypes)
             _c = _CtypesCalls(L)
         return getattr(_c, name)
 
