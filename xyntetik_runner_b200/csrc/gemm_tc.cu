@@ -807,17 +807,20 @@ static int choose_token_tile(int n, int cap) {
 // Costs are in hundredths of the time a CTA needs for one K block of 256 tokens (about 0.27 us).
 //
 // The pair kernel: `slots` pairs work through the tiles (or the tiles' slices along K) in rounds.  A K block costs its tokens' share of
-// 256, but no less than 72 (the thread that issues it, and the operands' way from L2); a tile's epilogue 100 + 800 x its share, hidden
+// 256, but no less than 72 (its four instructions take 80 cycles each however narrow they are, and the operands' way from L2); a tile's epilogue 100 + 800 x its share, hidden
 // behind the next tile's K blocks but for the last; a launch 600.  A product that is cut along K also pays for its partial sums' way to
 // memory and back (170,000 elements and slice a K block) and for the kernel that sums them (fifteen K blocks; none when the caller's next
 // kernel does it in passing).  The cheapest width (multiples of 32) and number of slices is taken.  Over 90 products of 257 to 2,048 tokens
 // by 1,024 to 11,264 rows of 1,024 to 5,632 this is 0.3 % from the fastest of the widths and cuts of one, two and four slices, where
 // always 256 tokens with the best cut is 30 %: 512 x 2,048 x 2,048 18.0 / 11.8 us (64 tokens a tile), 777 x 2,048 x 5,632 37.7 / 24.9 (96),
 // 1,024 x 1,024 x 1,024 13.0 / 7.9 (64), 1,901 x 3,072 x 2,048 28.6 / 22.8 (160), 2,048 x 2,048 x 2,048 19.1 both ways (256).
+// 129 to 256 tokens likewise: 256 x 2,048 x 2,048 in one tile 15.8 us, in four of 64 tokens 11.4; 256 x 2,048 x 5,632 in one tile cut in
+// five 24.0, in two of 128 tokens cut in four 18.3.
 //
 // The single-CTA kernel runs in waves of `slots` CTAs; a CTA costs a fixed part of six K blocks (launch, barrier and tensor-memory set-up,
 // filling the pipeline, the epilogue) plus its K blocks.  Its partial sums, a few megabytes, stay in L2: 700,000 elements and slice a K
 // block.  Only products with a single tile of tokens are cut.
+#define XR_NOALLOC_SCRATCH_FLOATS (4u << 20)          // 16 MiB of float32 (xr_gemm_tc_noalloc), held by every GPU that loads the library
 struct TcPlan {
     int bn;            // token capacity of the kernel's tile: 16, 32, 64, 128 or 256
     int bn_eff;        // tokens per tile as launched
@@ -846,17 +849,36 @@ static TcPlan plan_product(int n, int n_out, int K, bool gated, int force_splits
     int splits = 1;
     long long best_cost = -1;
     if (pl.pair) {
-        for (int bn = 256; bn >= 64; bn -= 32) {
+        int most = force_splits > 0 ? force_splits : (pl.total_kb / 8 < 8 ? pl.total_kb / 8 : 8), only = force_splits;
+        // One tile of tokens cut so that its partial sums exceed the scratch array of xr_gemm_tc_noalloc stays so cut, and at its one tile's
+        // width: which products that entry point refuses hangs on it.  What fits the array is chosen freely, among what fits it.
+        const long long fits = per_slice > 0 ? (long long)XR_NOALLOC_SCRATCH_FLOATS / per_slice : 0;
+        long long most_room = room;
+        if (n <= 256 && force_splits <= 0) {
+            const long long tiles = (pl.row_tiles + 1) / 2;
+            for (int sp = 1; sp <= (tiles < pair_clusters && most > 1 ? most : 1); sp++) {
+                const long long rounds = (tiles * sp + pair_clusters - 1) / pair_clusters;
+                long long cost = rounds * (6 + (pl.total_kb + sp - 1) / sp);
+                if (sp > 1) cost += finish + sp * per_slice / 170000;
+                if (best_cost < 0 || cost < best_cost) { best_cost = cost; only = sp; }
+            }
+            best_cost = -1;
+            if (only <= 1 || only <= fits) {
+                only = 0;
+                if (most_room > fits) most_room = fits;
+            }
+        }
+        if (only > pl.total_kb) only = pl.total_kb;
+        if (only > 1 && only > room) only = 1;
+        const int narrowest = n <= 256 && only > 1 && only > fits ? (n + 31) / 32 * 32 : 64;
+        for (int bn = 256; bn >= narrowest; bn -= 32) {
             if (bn - 32 >= n) continue;                                  // (more than one step of padding)
             const int tok_tiles = (n + bn - 1) / bn;
             const long long tiles = (long long)tok_tiles * ((pl.row_tiles + 1) / 2), block = bn <= 184 ? 72 : 100 * bn / 256, out = 100 + 800 * bn / 256;
-            int first = 1, last = tiles < pair_clusters ? (pl.total_kb / 8 < 8 ? pl.total_kb / 8 : 8) : 1;
-            if (force_splits > 0) first = last = force_splits;
-            if (last > pl.total_kb) last = pl.total_kb;
-            if (last > room) last = (int)room;
+            int last = only > 0 ? only : (tiles < pair_clusters ? most : 1);
+            if (only <= 0 && last > most_room) last = (int)most_room;
             if (last < 1) last = 1;
-            if (first > last) first = last;
-            for (int sp = first; sp <= last; sp++) {
+            for (int sp = only > 0 ? only : 1; sp <= last; sp++) {
                 const long long rounds = (tiles * sp + pair_clusters - 1) / pair_clusters, main = (pl.total_kb + sp - 1) / sp * block;
                 long long cost = 600 + (rounds - 1) * (main > out ? main : out) + main + out;
                 if (sp > 1) cost += 100 * finish + 100 * sp * per_slice / 170000;
@@ -1019,7 +1041,6 @@ XR_EXPORT int xr_gemm_tc_grouped_pairs(const void* X, const void* W, void* out, 
 // can use comes from cudaGetSymbolAddress, asked once per device (with that device current) on the
 // entry point's first call there.
 // ---------------------------------------------------------------------------------------------
-#define XR_NOALLOC_SCRATCH_FLOATS (4u << 20)          // 16 MiB of float32, held by every GPU that loads the library
 #define XR_NOALLOC_MAX_DEVICES 64
 static __device__ __align__(256) float g_noalloc_scratch[XR_NOALLOC_SCRATCH_FLOATS];
 static __device__ __align__(256) int g_noalloc_status[64];
