@@ -100,6 +100,12 @@ class StepContext:
             v = self._memo[key] = make()
         return v
 
+    def forget(self) -> None:
+        """Nothing of a run through the layers stands: what ``once`` made (part of it may be work on the device) and pending sums."""
+        self._memo.clear()
+        self._pending.clear()
+        self.stream_cast = None
+
     # A part whose last product was split along K may leave the sum unfinished ("pending") on the residual
     # stream; the next norm finishes it in its own pass.  Anything else that reads or writes that tensor
     # directly calls ``materialize`` first.
@@ -423,8 +429,10 @@ class Engine:
             logits = self._forward(ctx)
         self._graph_launches[key] = kernels.launch_count - launches0
         if self._buf_generation != gen:
-            # a buffer was made during capture: the graph may hold a stale address; run plainly this time
+            # a buffer was made during capture: the graph may hold a stale address; run plainly this time.  (What the capture
+            # recorded did not run: work that is done once a step is still to be done.)
             self._graph_seen[key] = 1
+            ctx.forget()
             return self._forward(ctx)
         self._graphs[key] = graph
         graph.replay()
