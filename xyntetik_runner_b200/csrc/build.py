@@ -227,6 +227,11 @@ CALLS_LIB = "xrb200_calls.so"
 CALLS_FLAGS = ["-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden"]
 
 
+class CannotBuild(BuildError):
+    """This machine has not what the extension is built with (Python's headers, a C++ compiler, a folder): ctypes makes the calls
+    then.  A compiler that rejects the generated source is a plain BuildError, and nobody's fallback."""
+
+
 def calls_path(build: bool = True) -> str:
     """Path of an up-to-date extension; compiles it if needed (and allowed)."""
     from . import calls as made
@@ -241,7 +246,11 @@ def calls_path(build: bool = True) -> str:
     if not build:
         raise BuildError("the extension of direct calls is not built")
     if not os.path.isfile(os.path.join(include, "Python.h")):
-        raise BuildError(f"no Python.h in {include}: the extension of direct calls cannot be built")
+        raise CannotBuild(f"no Python.h in {include}: the extension of direct calls cannot be built")
+    try:
+        cxx = find_cxx()
+    except BuildError as e:
+        raise CannotBuild(str(e)) from None
     for d in _build_dirs():
         if not _writable(d):
             continue
@@ -251,7 +260,7 @@ def calls_path(build: bool = True) -> str:
         try:
             with open(src, "w") as f:
                 f.write(text)
-            r = subprocess.run([find_cxx()] + CALLS_FLAGS + ["-I", include, "-o", tmp_lib, src, "-ldl"], capture_output=True, text=True, env=env)
+            r = subprocess.run([cxx] + CALLS_FLAGS + ["-I", include, "-o", tmp_lib, src, "-ldl"], capture_output=True, text=True, env=env)
             if r.returncode != 0:
                 raise BuildError(f"the C++ compiler failed on the extension of direct calls:\n{r.stdout}\n{r.stderr}")
         finally:
@@ -262,7 +271,7 @@ def calls_path(build: bool = True) -> str:
         with open(os.path.join(d, "digest_calls.txt"), "w") as f:
             f.write(digest + "\n")
         return lib
-    raise BuildError("no writable folder for the build: " + ", ".join(_build_dirs()))
+    raise CannotBuild("no writable folder for the build: " + ", ".join(_build_dirs()))
 
 
 def calls(library: str):

@@ -47,7 +47,7 @@ class _Calls:
         L = lib()
         try:
             _c = _build.calls(_build.library_path(build=False))
-        except _build.BuildError:            # (a Python without its headers, or no compiler: the same calls through ctypes)
+        except _build.CannotBuild:           # (a Python without its headers, or no compiler: the same calls through ctypes)
             _c = _CtypesCalls(L)
         return getattr(_c, name)
 
