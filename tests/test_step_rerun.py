@@ -1,5 +1,8 @@
-"""A step whose capture made a buffer runs again plainly: work that a step does once (a sum that starts at zero) was only recorded
-by the capture and must be done by the run that counts."""
+"""What a step works out once.
+
+A step whose capture made a buffer runs again plainly: work that a step does once (a sum that starts at zero) was only recorded
+by the capture and must be done by the run that counts.  And an answer
+of None is an answer: no layer works it out again."""
 import contextlib
 
 import torch
@@ -40,3 +43,12 @@ def test_a_discarded_capture_leaves_nothing_behind(monkeypatch):
     eng._forward = forward
     assert eng._forward_graphed(ctx).abs().sum() == 0
     assert runs == ["capture", "plain"] and not eng._graphs
+
+
+def test_an_answer_of_none_is_kept():
+    ctx = object.__new__(StepContext)
+    ctx._memo = {}
+    asked = []
+    for _ in range(3):
+        assert ctx.once("plan", lambda: asked.append(1)) is None
+    assert len(asked) == 1

@@ -95,8 +95,8 @@ class StepContext:
     def once(self, key, make):
         """make() the first time `key` is asked for in this step, the same value afterwards: for what a part works out
         from the step's description on the host and every layer would work out again."""
-        v = self._memo.get(key)
-        if v is None:
+        v = self._memo.get(key, self)              # (self: not asked for yet; None is an answer)
+        if v is self:
             v = self._memo[key] = make()
         return v
 
