@@ -1435,28 +1435,22 @@ static int launch_keys_tma(const AttnMmaArgs& a, const void* cache_base, long lo
     constexpr int STAGE = 2 * ATT_TILE * HD * 2, REST = 16 * LD * 2 + 64 + 1024;
     constexpr int RECV = (16 * (HD / 4) + ATT_CLUSTER_MAX) * 16 + ATT_CLUSTER_MAX * 16 * 8 + 16;
     constexpr int S2 = 2 * STAGE + REST, S3 = 3 * STAGE + REST, S4 = 4 * STAGE + REST;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_attention_keys_tma<HD, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S2) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys_tma<HD, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S3) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys_tma<HD, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, S4) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys_tma<HD, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S2 + RECV) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys_tma<HD, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S3 + RECV) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys_tma<HD, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, S4 + RECV) != cudaSuccess)
-            return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] {
+            return xr_allow_smem(k_attention_keys_tma<HD, 2, false>, S2) && xr_allow_smem(k_attention_keys_tma<HD, 3, false>, S3) &&
+                   xr_allow_smem(k_attention_keys_tma<HD, 4, false>, S4) && xr_allow_smem(k_attention_keys_tma<HD, 2, true>, S2 + RECV) &&
+                   xr_allow_smem(k_attention_keys_tma<HD, 3, true>, S3 + RECV) && xr_allow_smem(k_attention_keys_tma<HD, 4, true>, S4 + RECV);
+        }))
+        return XR_ERR_LAUNCH;
     if (att_even_wanted((long long)n_seg * a.K, uneven) && flags != nullptr && n_seg <= ATT_EVEN_MAX_SEGS && att_cluster_merge_enabled()) {
         // even shares: as many CTAs as are resident at once
-        static bool even_configured = false;
+        static bool even_ready[XR_DEVICES];
         constexpr int EVEN_MAX = 2 * 4 * ATT_TILE * HD * 2 + 16 * LD * 2 + 4 * 16 * HD * 4 + 512 + 64 + 4 * (ATT_EVEN_MAX_SEGS + 4);
-        if (!even_configured) {
-            if (cudaFuncSetAttribute(k_attention_keys_even<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, EVEN_MAX) != cudaSuccess ||
-                cudaFuncSetAttribute(k_attention_keys_even<HD, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, EVEN_MAX) != cudaSuccess ||
-                cudaFuncSetAttribute(k_attention_keys_even<HD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, EVEN_MAX) != cudaSuccess)
-                return XR_ERR_LAUNCH;
-            even_configured = true;
-        }
+        if (!xr_once_per_device(even_ready, [] {
+                return xr_allow_smem(k_attention_keys_even<HD, 2>, EVEN_MAX) && xr_allow_smem(k_attention_keys_even<HD, 3>, EVEN_MAX) &&
+                       xr_allow_smem(k_attention_keys_even<HD, 4>, EVEN_MAX);
+            }))
+            return XR_ERR_LAUNCH;
         const int region = 16 * LD * 2 > 4 * a.recv_rows * HD * 4 ? 16 * LD * 2 : 4 * a.recv_rows * HD * 4;
         const int tail = (region + 512 + 8 * 4 + 4 * (n_seg + 2) + 15) & ~15;
         // the deepest ring with which three CTAs share an SM (measured: three with two stages stream faster than two with
@@ -1545,14 +1539,12 @@ static int launch_attention(const AttnMmaArgs& a, int n_seg, int max_seg_len, in
     constexpr int KEYS_TILES2 = (16 + 2 * 2 * ATT_TILE) * LD * 2, KEYS_TILES4 = (16 + 2 * 4 * ATT_TILE) * LD * 2;
     constexpr int SMEM_KEYS2 = KEYS_TILES2 > KEYS_MERGE ? KEYS_TILES2 : KEYS_MERGE;
     constexpr int SMEM_KEYS4 = KEYS_TILES4 > KEYS_MERGE ? KEYS_TILES4 : KEYS_MERGE;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_attention_rows<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ROWS) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_KEYS2) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_keys<HD, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_KEYS4) != cudaSuccess)
-            return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] {
+            return xr_allow_smem(k_attention_rows<HD>, SMEM_ROWS) && xr_allow_smem(k_attention_keys<HD, 2>, SMEM_KEYS2) &&
+                   xr_allow_smem(k_attention_keys<HD, 4>, SMEM_KEYS4);
+        }))
+        return XR_ERR_LAUNCH;
     if (any_long) {
         // row_tiles: the 64-row tiles of the portions with more than 16 packed rows, summed; 0: not known, and an upper
         // bound is taken (blocks beyond the true number return at once)

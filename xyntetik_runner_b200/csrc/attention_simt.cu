@@ -279,8 +279,8 @@ k_attention_simt_rows(AttnArgs a) {
 template <int HD>
 static int launch_simt_rows(const AttnArgs& a, cudaStream_t stream) {
     constexpr size_t SMEM = (2 * 32 * (HD + 4) + 2 * 32 * HD + AT_ROWS * HD + AT_ROWS * 32) * sizeof(float);
-    static const bool ready = cudaFuncSetAttribute(k_attention_simt_rows<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess;
-    if (!ready) return XR_ERR_LAUNCH;
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_attention_simt_rows<HD>, SMEM); })) return XR_ERR_LAUNCH;
     const int tokens = AT_ROWS / (a.H / a.K);
     k_attention_simt_rows<HD><<<dim3((a.n + tokens - 1) / tokens, a.K), 32 * AT_WARPS, SMEM, stream>>>(a);
     return xr_launch_status();

@@ -612,15 +612,12 @@ XR_EXPORT int xr_attention_tc(const void* q, void* out, const void* cache_base, 
         const int stride = bias_len + ((want - bias_len % 32) + 32) % 32;
         if (SMEM + (long long)G * stride * 4 <= SMEM_MOST) { a.bias_stride = stride; smem = SMEM + G * stride * 4; }
     }
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_attention_tc<2, 2, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<1, 1, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<2, 2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess ||
-            cudaFuncSetAttribute(k_attention_tc<1, 1, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MOST) != cudaSuccess)
-            return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] {
+            return xr_allow_smem(k_attention_tc<2, 2, false, false>, SMEM) && xr_allow_smem(k_attention_tc<1, 1, false, false>, SMEM) &&
+                   xr_allow_smem(k_attention_tc<2, 2, true, false>, SMEM_MOST) && xr_allow_smem(k_attention_tc<1, 1, true, false>, SMEM_MOST);
+        }))
+        return XR_ERR_LAUNCH;
     // row_tiles: the 128-row tiles of the portions with more than 16 packed rows, summed; 0: not known, and an upper
     // bound is taken (blocks beyond the true number return at once)
     long long tiles = row_tiles > 0 ? row_tiles : (((long long)max_seg_len * G + TA_ROWS - 1) / TA_ROWS) * n_seg;
@@ -644,8 +641,8 @@ XR_EXPORT int xr_attention_tc_flat_supported(int D, int R, int V) {
 template <int NK, int NV>
 static int launch_flat(const CUtensorMap& qm, const CUtensorMap& kvm, const CUtensorMap& tm, const AttnTcArgs& a, long long tiles, cudaStream_t stream) {
     constexpr int SMEM = (3 * (NK < 2 ? 2 : NK) + 4) * TA_ROWS * 128 + 128 + 2 * 2 * 128 * 4;
-    static const bool ready = cudaFuncSetAttribute(k_attention_tc<NK, NV, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess;
-    if (!ready) return XR_ERR_LAUNCH;
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_attention_tc<NK, NV, false, true>, SMEM); })) return XR_ERR_LAUNCH;
     xr_launch((k_attention_tc<NK, NV, false, true>), dim3((unsigned)tiles, a.H), dim3(TA_THREADS), SMEM, stream, qm, kvm, tm, a);
     return xr_launch_status();
 }

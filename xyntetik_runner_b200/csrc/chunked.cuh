@@ -494,9 +494,8 @@ static int ck_launch(const ChunkArgs& a, int n, cudaStream_t stream) {
     if (chunks > 65535 || a.H > 65535 || a.n_seg > 65535) return XR_ERR_ARG;
     constexpr size_t S1 = (2 * CK_L + (KIND == CK_KEY ? 48 : 0)) * (size_t)(D + 4) * sizeof(float);
     constexpr size_t S4 = (size_t)CK_ST * (CK_L * (CK_KB + 4) + CK_KB * CK_VT) * sizeof(float);
-    static const bool ready = cudaFuncSetAttribute(ck_scores<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S1) == cudaSuccess &&
-                              cudaFuncSetAttribute(ck_out<D, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S4) == cudaSuccess;
-    if (!ready) return XR_ERR_LAUNCH;
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(ck_scores<D, KIND>, S1) && xr_allow_smem(ck_out<D, NORM>, S4); })) return XR_ERR_LAUNCH;
     xr_launch((ck_scores<D, KIND>), dim3(a.H, chunks), dim3(256), S1, stream, a);
     xr_launch((ck_states<D, NORM>), dim3(vt, a.H, chunks), dim3(256), 0, stream, a);
     xr_launch((ck_scan<D, KIND, NORM>), dim3((D * a.V + (NORM ? D : 0) + 255) / 256, a.H, a.n_seg), dim3(256), 0, stream, a);

@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include "per_device.h"
 
 #define XR_F32 0
 #define XR_BF16 1
@@ -67,12 +68,24 @@ static inline bool xr_pdl_enabled() {
     return on == 1;
 }
 
+template <typename Ask>
+static inline bool xr_once_per_device(bool (&done)[XR_DEVICES], Ask ask) {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    return xr_once_on_device(done, dev, ask);
+}
+// `kernel` may be launched with `bytes` of dynamic shared memory on the current device from here on.
+template <typename Kernel>
+static inline bool xr_allow_smem(Kernel kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
+
 // Streaming multiprocessors of the current device (asked once per device): grids and wave models are sized by
 // it, so a part exposed with fewer of them than the full chip is not over-subscribed.
 static inline int xr_sm_count() {
-    static int known[64];
+    static int known[XR_DEVICES];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= XR_DEVICES) dev = 0;
     if (known[dev] == 0) {
         int v = 0;
         if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v < 1) v = 148;

@@ -49,9 +49,9 @@ static int launch_simt_tile(const void* X, const void* W, const float* bias, voi
     constexpr size_t SMEM = gs_smem<TX, TW, BM, BN>();
     const dim3 grid((n_out + BN - 1) / BN, (n + BM - 1) / BM);
     if (grid.y > 65535) return XR_ERR_ARG;
-    static const bool ready = SMEM <= 48 * 1024 || cudaFuncSetAttribute(k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN>,
-                                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM) == cudaSuccess;
-    if (!ready) return XR_ERR_LAUNCH;
+    static bool ready[XR_DEVICES];
+    if (SMEM > 48 * 1024 && !xr_once_per_device(ready, [] { return xr_allow_smem(k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN>, SMEM); }))
+        return XR_ERR_LAUNCH;
     constexpr int PX = 16 / (int)sizeof(TX), PW = 16 / (int)sizeof(TW);
     const int vec = !(((uintptr_t)X | (uintptr_t)W) & 15) && ldx % PX == 0 && K % PX == 0 && K % PW == 0;
     k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN><<<grid, 32 * WM * WN, SMEM, stream>>>((const TX*)X, (const TW*)W, bias, (TO*)out, n, n_out, K, ldx, ldo, alpha, vec);

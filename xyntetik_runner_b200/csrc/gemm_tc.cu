@@ -733,12 +733,8 @@ template <int BN, int STAGES, int MINB>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, dim3 grid, cudaStream_t stream) {
     constexpr int STAGE_BYTES = TC_BM * TC_BK * 2 + BN * TC_BK * 2;
     constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + (2 * STAGES + 1) * 8 + 16;
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_gemm_tc<BN, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess)
-            return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_gemm_tc<BN, STAGES, MINB>, SMEM); })) return XR_ERR_LAUNCH;
     xr_launch((k_gemm_tc<BN, STAGES, MINB>), dim3(grid), dim3(tc_threads(BN)), SMEM, stream, mw, mx, p);
     return xr_launch_status();
 }
@@ -759,21 +755,23 @@ struct PairLaunch {
     }
     // pairs of CTAs the device holds at once (one CTA per SM); 0 if it cannot run the kernel as clusters of two
     static int clusters() {
-        static int n = -1;
-        if (n < 0) {
-            n = 0;
+        static int known[XR_DEVICES];      // per device: 1 + the answer
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= XR_DEVICES) dev = 0;
+        if (known[dev] == 0) {
+            int n = 0;
             cudaLaunchConfig_t cfg; cudaLaunchAttribute attr[2];
             config(cfg, attr, xr_sm_count() / 2, nullptr);
             cfg.numAttrs = 1;
             int nc = 0;
-            if (cudaFuncSetAttribute(k_gemm_tc_pair<TC2_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
-                cudaFuncSetAttribute(k_gemm_tc_pair<TC2_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) == cudaSuccess &&
+            if (xr_allow_smem(k_gemm_tc_pair<TC2_STAGES, false>, SMEM) && xr_allow_smem(k_gemm_tc_pair<TC2_STAGES, true>, SMEM) &&
                 cudaOccupancyMaxActiveClusters(&nc, k_gemm_tc_pair<TC2_STAGES, false>, &cfg) == cudaSuccess && nc > 0)
                 n = nc;
             else
                 cudaGetLastError();        // the single-CTA kernel takes over; leave no error behind
+            known[dev] = 1 + n;
         }
-        return n;
+        return known[dev] - 1;
     }
     // (grouped: p.pair_tiles is an upper bound, the kernel reads the true number of tiles)
     static int launch(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, cudaStream_t stream) {

@@ -607,11 +607,8 @@ XR_EXPORT int xr_latent_attention_mma(const void* ql, long long ql_tok, long lon
     if (splits > 65535 || (H + 15) / 16 > 65535) return XR_ERR_ARG;
     const int Wp = (C + R + 15) / 16 * 16;
     const size_t smem = (size_t)(16 + 2 * LT_KT) * lt_row_bytes(Wp) + 16 * 33 * sizeof(float);
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_latent_attention_mma, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess) return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_latent_attention_mma, 200 * 1024); })) return XR_ERR_LAUNCH;
     const int mt = (H + 15) / 16;
     xr_launch(k_latent_attention_mma, dim3(n, mt, splits), dim3(32 * LT_NW), smem, stream, (const __nv_bfloat16*)ql, ql_tok, ql_head,
               (const __nv_bfloat16*)qr, ld_qr, head_qr, out, (__nv_bfloat16*)out_h, oh_tok, oh_head, part_o, part_ml, (const __nv_bfloat16*)cache, page_stride, positions, tok_seg, block_tables, H, C, R,

@@ -111,9 +111,8 @@ static int launch_rglru_gates(float* proj, long long ldp, int y_col, const float
     constexpr int BM = 4 * TM * WM, OUT = 8 * TN * WN / 2;
     constexpr size_t SMEM = gs_smem<float, float, BM, 2 * OUT>();
     const int Bs = R / B;
-    static const bool ready = SMEM <= 48 * 1024 || cudaFuncSetAttribute(k_rglru_gates<WM, WN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                                        (int)SMEM) == cudaSuccess;
-    if (!ready) return XR_ERR_LAUNCH;
+    static bool ready[XR_DEVICES];
+    if (SMEM > 48 * 1024 && !xr_once_per_device(ready, [] { return xr_allow_smem(k_rglru_gates<WM, WN, TM, TN>, SMEM); })) return XR_ERR_LAUNCH;
     const int vec = Bs % 4 == 0 && !(((uintptr_t)u | (uintptr_t)wa | (uintptr_t)wi) & 15);
     const dim3 grid((Bs + OUT - 1) / OUT, (n + BM - 1) / BM, B);
     if (grid.y > 65535) return XR_ERR_ARG;

@@ -1106,11 +1106,8 @@ static int launch_sample_block(const SampleArgs& a, int rows, float* scratch, in
     constexpr int DYN_MAX = SMP_DYN_MAX;
     const long long dyn = (long long)SMP_CAP * 16 + ((long long)(a.V + 31) / 32) * 4;
     if (shortcuts && dyn > DYN_MAX) return XR_ERR_ARG;              // (a vocabulary of more than 786,432; xr_sample checks before)
-    static bool configured = false;
-    if (!configured) {
-        if (cudaFuncSetAttribute(k_sample, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_MAX) != cudaSuccess) return XR_ERR_LAUNCH;
-        configured = true;
-    }
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_sample, DYN_MAX); })) return XR_ERR_LAUNCH;
     xr_launch(k_sample, dim3(rows), dim3(SMP_THREADS), shortcuts ? (size_t)dyn : 0, stream, a, scratch, shortcuts ? 1 : 0);
     return xr_launch_status();
 }
