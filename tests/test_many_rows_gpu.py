@@ -502,3 +502,43 @@ def test_route_few_against_its_parts(n, E, identity, top, mode, splits, align):
             assert tiles[r // align] == e and torch.equal(xs[r], h[p // top])
     used = sum(-(-ids.count(e) // align) for e in range(E))
     assert all(0 <= t < E for t in tiles[:used]) and all(t == -1 for t in tiles[used:])
+
+
+@pytest.mark.parametrize("kind,H,D,V", [("head", 2, 64, 64), ("key", 1, 128, 64), ("mlstm", 2, 64, 128)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_chunks_do_not_look_ahead(kind, H, D, V, bad):
+    """A value that is no number, in the middle of a chunk: the read-outs of the tokens before it, of other columns and of other
+    portions are bit for bit what they are without it, and those from it on are what the walk makes of them: no numbers."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(D + V)
+    f = lambda *s: torch.randn(*s, generator=g)
+    lens, token, column = [90, 70], 64 + 11, 5
+    n, S = sum(lens), 2
+    starts, slots = [0, 90], [1, 0]
+    state0 = f(2, H, D * V + D + 1 if kind == "mlstm" else D * V)
+    state0[..., -1] = 0.5
+    proj0, gates = f(n, 2 * H * D + 2 * H * V + 8) * 0.3, torch.cat([f(n, H), 3.0 + f(n, H)], dim=1)
+    dec, w_t, bias = torch.rand(H, generator=g) * 0.1 + 0.9, f(8, H * D), 2.0 + f(H * D)
+
+    def run(planted, chunked):
+        proj = proj0.clone()
+        if planted:
+            proj[token, 2 * H * D + column] = bad
+        proj, state, o = proj.to(DEV), state0.reshape(2, -1).to(DEV).clone(), torch.empty(n, H * V, device=DEV)
+        seg = (_i32(starts), _i32(lens), _i32(slots))
+        scratch = torch.full((kernels.chunked_floats(n, S, H, D, V, kind),), float("nan"), device=DEV) if chunked else None
+        if kind == "head":
+            kernels.decay_attention(proj, (0, H * D, 2 * H * D), dec.to(DEV), state, *seg, o, S, H, D, V, silu=False, scratch=scratch)
+        elif kind == "key":
+            kernels.key_decay_attention(proj, (0, H * D, 2 * H * D, 2 * H * D + 2 * H * V), 8, w_t.to(DEV), bias.to(DEV), 12.0,
+                                        torch.empty(n, H * D, device=DEV), state, *seg, o, S, H, D, V, scratch=scratch)
+        else:
+            kernels.mlstm(proj, (0, H * D, 2 * H * D, 2 * H * D + H * V), gates.to(DEV), state, torch.empty(n, 3 * H, device=DEV), o,
+                          torch.ones(H * V, device=DEV), torch.empty(n, H * V, device=DEV), *seg, S, H, D, V, 15.0, 1e-6, scratch=scratch)
+        return o.cpu()
+    clean, got, walk = run(False, True), run(True, True), run(True, False)
+    assert torch.isfinite(clean).all()
+    touched = torch.zeros(n, H * V, dtype=torch.bool)
+    touched[token:lens[0], column] = True
+    assert torch.equal(got[~touched], clean[~touched])
+    assert not torch.isfinite(got[touched]).any() and not torch.isfinite(walk[touched]).any() and torch.isfinite(walk[~touched]).all()

@@ -26,6 +26,8 @@
 
 #define CK_L 64                     // tokens a chunk
 #define CK_VT 64                    // value columns a block
+#define CK_KB 32                    // ck_out: terms a block of its sums
+#define CK_ST 3                     // ck_out: blocks in flight
 enum { CK_HEAD = 0, CK_TOKEN = 1, CK_KEY = 2 };
 
 struct ChunkArgs {
@@ -352,11 +354,25 @@ ck_scan(ChunkArgs a) {
     *st = S;
 }
 
+// Token i's read-out in columns v0 .. v0 + 3 once more, with the values up to its own only: the product above also takes the chunk's later
+// values, times zero, which is no zero where one of them is infinite or no number.  The same sums in the same order.
+template <int D>
+static __device__ __noinline__ float4 ck_out_causal(const float* row, const float* mem, const float* vals, long long ld_v, int V, int i) {
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k0 = 0; k0 <= D + i; k0 += CK_KB) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = k0; k < k0 + CK_KB && k <= D + i; k++) {
+            const float4 y = *reinterpret_cast<const float4*>(k < D ? mem + (size_t)k * V : vals + (size_t)(k - D) * ld_v);
+            acc = make_float4(fmaf(row[k], y.x, acc.x), fmaf(row[k], y.y, acc.y), fmaf(row[k], y.z, acc.z), fmaf(row[k], y.w, acc.w));
+        }
+        sum = make_float4(sum.x + acc.x, sum.y + acc.y, sum.z + acc.z, sum.w + acc.w);
+    }
+    return sum;
+}
+
 // ---- [q exp(c) | P] [S; v] ----------------------------------------------------------------------------------------------
 // 64 tokens x 64 columns a block of four warps; a thread 8 tokens (8 apart) x 4 columns; both operands in blocks of 32 through a ring
 // of three stages.  A block's 32 terms are summed on their own and then added: the sums' rounding grows with their length.
-#define CK_KB 32
-#define CK_ST 3
 template <int D, bool NORM>
 __global__ void __launch_bounds__(128)
 ck_out(ChunkArgs a) {
@@ -458,6 +474,8 @@ ck_out(ChunkArgs a) {
         const int i = tt + 8 * r;
         if (i >= p.count) continue;
         float4 y = make_float4(sum[r][0], sum[r][1], sum[r][2], sum[r][3]);
+        if (!(fabsf(y.x) < INFINITY && fabsf(y.y) < INFINITY && fabsf(y.z) < INFINITY && fabsf(y.w) < INFINITY))
+            y = ck_out_causal<D>(rows + (size_t)i * LR, mem + 4 * tc, vals + 4 * tc, a.ld_v, a.V, i);
         if (NORM) {
             const float f = den[i];
             y = make_float4(y.x / f, y.y / f, y.z / f, y.w / f);
