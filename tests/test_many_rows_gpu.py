@@ -542,3 +542,34 @@ def test_chunks_do_not_look_ahead(kind, H, D, V, bad):
     touched[token:lens[0], column] = True
     assert torch.equal(got[~touched], clean[~touched])
     assert not torch.isfinite(got[touched]).any() and not torch.isfinite(walk[touched]).any() and torch.isfinite(walk[~touched]).all()
+
+
+@pytest.mark.parametrize("token", [0, 70, 299])
+@pytest.mark.parametrize("which", ["forget", "input"])
+def test_gates_that_are_no_numbers_in_chunks(token, which):
+    """A gate of one head that is no number: the same read-outs, states and running maxima are numbers as in the walk, and what comes
+    before it, the other head and the other portion keep their bits."""
+    from xyntetik_runner_b200 import kernels
+    H, D, V = 2, 64, 64
+    g = torch.Generator().manual_seed(token)
+    f = lambda *s: torch.randn(*s, generator=g)
+    lens, starts, slots = [300, 40], [0, 300], [0, 1]
+    n, size = sum(lens), D * V + D + 1
+    proj, gates0, state0 = f(n, 2 * H * D + 2 * H * V), torch.cat([f(n, H), 3.0 + f(n, H)], dim=1), f(2, H, size)
+    state0[..., -1] = 0.5
+
+    def run(planted, chunked):
+        gates = gates0.clone()
+        if planted:
+            gates[token, (H if which == "forget" else 0) + 1] = float("nan")
+        state, o = state0.reshape(2, -1).to(DEV).clone(), torch.empty(n, H * V, device=DEV)
+        scratch = torch.empty(kernels.chunked_floats(n, 2, H, D, V, "mlstm"), device=DEV) if chunked else None
+        kernels.mlstm(proj.to(DEV), (0, H * D, 2 * H * D, 2 * H * D + H * V), gates.to(DEV), state, torch.empty(n, 3 * H, device=DEV), o,
+                      torch.ones(H * V, device=DEV), torch.empty(n, H * V, device=DEV), _i32(starts), _i32(lens), _i32(slots), 2, H, D, V, 15.0, 1e-6,
+                      scratch=scratch)
+        return o.cpu(), state.cpu()
+    (clean, clean_state), (got, state), (walk, walk_state) = run(False, True), run(True, True), run(True, False)
+    assert torch.equal(torch.isnan(got), torch.isnan(walk)) and torch.equal(torch.isnan(state), torch.isnan(walk_state))
+    assert torch.isnan(got[token:300, V:]).all() and torch.isfinite(clean).all()
+    for same in (got[:token] == clean[:token], got[:, :V] == clean[:, :V], got[300:] == clean[300:], state[1] == clean_state[1], state[0, :size] == clean_state[0, :size]):
+        assert same.all()

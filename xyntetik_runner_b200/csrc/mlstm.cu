@@ -24,6 +24,9 @@
 
 __device__ __forceinline__ float ml_logsigmoid(float x) { return fminf(x, 0.f) - log1pf(expf(-fabsf(x))); }
 
+// a decay's logarithm is at most zero; one that is no number stays so (fminf would make it zero, a decay of one)
+__device__ __forceinline__ float ml_log_decay(float x) { return x > 0.f ? 0.f : x; }
+
 // state layout per slot: [H][D * V + D + 1]
 __host__ __device__ __forceinline__ size_t ml_state_head(int D, int V) { return (size_t)D * V + D + 1; }
 
@@ -335,7 +338,7 @@ k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, floa
         const float m_new = fmaxf(lf + m, li);
         const size_t at = (size_t)(start + i) * H + h;
         if (i == i0) { first_m = m_new; first_lf = lf; }
-        else log_f[at] = fminf(lf + m - m_new, 0.f);
+        else log_f[at] = ml_log_decay(lf + m - m_new);
         in_scale[at] = expf(li - m_new); floor_n[at] = expf(-m_new);
         m = m_new;
     }
@@ -344,7 +347,7 @@ k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, floa
     __syncthreads();
     sa[tid] = m;
     __syncthreads();
-    if (i0 < i1) log_f[(size_t)(start + i0) * H + h] = fminf(first_lf + (tid == 0 ? m0 : sa[tid - 1]) - first_m, 0.f);
+    if (i0 < i1) log_f[(size_t)(start + i0) * H + h] = ml_log_decay(first_lf + (tid == 0 ? m0 : sa[tid - 1]) - first_m);
     if (len > 0 && i0 < len && i1 == len) *m_at = m;     // (every thread has read it, barriers ago)
 }
 
