@@ -573,3 +573,36 @@ def test_gates_that_are_no_numbers_in_chunks(token, which):
     assert torch.isnan(got[token:300, V:]).all() and torch.isfinite(clean).all()
     for same in (got[:token] == clean[:token], got[:, :V] == clean[:, :V], got[300:] == clean[300:], state[1] == clean_state[1], state[0, :size] == clean_state[0, :size]):
         assert same.all()
+
+
+@pytest.mark.parametrize("what", ["keys", "decays"])
+def test_scores_of_chunks_out_of_the_short_cuts_range(what):
+    """Decays per channel that reach exp(-59) over a chunk: with keys of 1e14 (and queries as small) exp(-c) k leaves float32's range where the
+    walk does not; and a decay that is no number leaves the tokens before it what they are, however far their decays have gone."""
+    from xyntetik_runner_b200 import kernels
+    H, D, V, n, token = 1, 64, 64, 150, 110
+    g = torch.Generator().manual_seed(9)
+    f = lambda *s: torch.randn(*s, generator=g)
+    scale = 1e14 if what == "keys" else 1.0
+    q, k, v = f(n, H * D) / scale, f(n, H * D) * D ** -0.5 * scale, f(n, H * V)
+    inner, w_t = torch.zeros(n, 8), torch.zeros(8, H * D)
+    w_t[0] = 1.0
+    if what == "decays":
+        inner[token:, 0] = float("nan")
+    z = -11.06 if what == "keys" else -20.0
+    proj = torch.cat([q, k, v, inner], 1).to(DEV)
+    state0 = f(1, H * D * V) * scale
+
+    def run(chunked):
+        state, o = state0.to(DEV).clone(), torch.empty(n, H * V, device=DEV)
+        kernels.key_decay_attention(proj, (0, H * D, 2 * H * D, 2 * H * D + H * V), 8, w_t.to(DEV), torch.full((H * D,), z).to(DEV), 12.0,
+                                    torch.empty(n, H * D, device=DEV), state, _i32([0]), _i32([n]), _i32([0]), o, 1, H, D, V,
+                                    scratch=torch.empty(kernels.chunked_floats(n, 1, H, D, V, "key"), device=DEV) if chunked else None)
+        return o.cpu()
+    walk, got = run(False), run(True)
+    upto = n if what == "keys" else token
+    decay = torch.exp(torch.nn.functional.logsigmoid(torch.tensor(z, dtype=torch.float64)) / 12.0).expand(upto, H, D)
+    want, _ = _walk(q[:upto].double().view(-1, H, D), k[:upto].double().view(-1, H, D), v[:upto].double().view(-1, H, V), decay,
+                    state0.double().view(H, V, D).transpose(1, 2))
+    _close(got[:upto], want.reshape(upto, -1), walk[:upto])
+    assert torch.equal(torch.isnan(got), torch.isnan(walk))

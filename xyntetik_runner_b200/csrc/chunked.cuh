@@ -97,10 +97,18 @@ ck_cumulate(const float* __restrict__ log_a, long long ld, double* __restrict__ 
 
 // ---- [q exp(c) | P] ----------------------------------------------------------------------------------------------------
 // 256 threads, 4 x 4 scores each.  CK_KEY: where no channel's decay over the chunk goes below exp(-CK_DEEP), P is the product of
-// q exp(c) and k exp(-c), which stay within float32's range.  Else, by sixteens of tokens with r the sum at the end of the sixteen
+// q exp(c) and k exp(-c), which stay within float32's range (a score whose keys are too large for that is summed pair by pair).  Else, by sixteens of tokens with r the sum at the end of the sixteen
 // before: a later sixteen's queries times exp(c_i - r) with the earlier keys times exp(r - c_j), both factors at most one, and inside a
 // sixteen every pair's exponentials channel by channel.
 #define CK_DEEP 60.0
+// CK_KEY: one score, every channel's exponential on its own.  q, k: the two tokens' rows of the head, ci, cj their sums c.
+template <int D>
+static __device__ __noinline__ float ck_pair(const float* q, const float* k, const double* ci, const double* cj) {
+    float sum = 0.f;
+    for (int d = 0; d < D; d++) sum = fmaf(q[d] * k[d], ck_exp(ci[d] - cj[d]), sum);
+    return sum;
+}
+
 template <int D, int KIND>
 __global__ void __launch_bounds__(256)
 ck_scores(ChunkArgs a) {
@@ -128,7 +136,8 @@ ck_scores(ChunkArgs a) {
         ends[tid] = f;
     }
     __syncthreads();
-    if (KIND == CK_KEY && tid < D && a.cum[((size_t)(p.t0 + p.count - 1) * a.H + h) * D + tid] < -CK_DEEP) deep = 1;
+    // (a sum that is no number says nothing about the tokens before it)
+    if (KIND == CK_KEY && tid < D && !(a.cum[((size_t)(p.t0 + p.count - 1) * a.H + h) * D + tid] >= -CK_DEEP)) deep = 1;
     if (KIND == CK_KEY) __syncthreads();
     float* out = a.rows + ((size_t)blockIdx.y * a.H + h) * CK_L * LR;
     float* keys = a.keys + ((size_t)blockIdx.y * a.H + h) * CK_L * D;
@@ -245,7 +254,12 @@ ck_scores(ChunkArgs a) {
             const int i = ti + 16 * r;
             float x = 0.f;
             if (j <= i && i < p.count) {
-                x = acc[r][s] * in;
+                x = acc[r][s];
+                if (KIND == CK_KEY && !(fabsf(x) < INFINITY)) {
+                    const size_t ti64 = (size_t)(p.t0 + i), tj64 = (size_t)(p.t0 + j);
+                    x = ck_pair<D>(a.q + ti64 * a.ld_q + h * D, a.k + tj64 * a.ld_k + h * D, a.cum + (ti64 * a.H + h) * D, a.cum + (tj64 * a.H + h) * D);
+                }
+                x *= in;
                 if (KIND != CK_KEY && i != j) x *= ck_exp(cs[i] - cs[j]);
             }
             out[i * LR + D + j] = x;
