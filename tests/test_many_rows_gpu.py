@@ -606,3 +606,29 @@ def test_scores_of_chunks_out_of_the_short_cuts_range(what):
                     state0.double().view(H, V, D).transpose(1, 2))
     _close(got[:upto], want.reshape(upto, -1), walk[:upto])
     assert torch.equal(torch.isnan(got), torch.isnan(walk))
+
+
+@pytest.mark.parametrize("each", [False, True])
+def test_gates_of_expanded_attention_keep_float32(each):
+    """Output gates far on either side: sigmoid(z) in float32 down to its smallest values; the results differ from float64 by their
+    rounding to bfloat16, the probabilities' and 2^-16 of a gate that float32 holds without its leading bit."""
+    from xyntetik_runner_b200 import kernels
+    H, D, R, V, n = 2, 64, 8, 64, 40
+    g = torch.Generator().manual_seed(1)
+    f = lambda *s: torch.randn(*s, generator=g).bfloat16()
+    q, kv, tail = f(n, H * (D + R)), f(n, H * (D + V)), f(n, R)
+    kv[:, H * D:] = (1000.0 + 100.0 * kv[:, H * D:].float()).bfloat16()
+    z = torch.tensor([-88.0, -87.5, -86.0, -60.0, -5.0, 0.0, 4.0, 60.0, 88.0, 100.0]).repeat(n, H * V // 10 + 1)[:, :H * V if each else H].bfloat16()
+    z = torch.stack([row.roll(t) for t, row in enumerate(z)]).contiguous() if each else z.flatten().roll(3).view(n, H).contiguous()
+    if not each:
+        z[:, 0] = torch.tensor([-88.0, -87.5, -60.0, 0.0, 88.0]).repeat(n // 5).bfloat16()
+    out = torch.empty(n, H * V, dtype=torch.bfloat16, device=DEV)
+    kernels.attention_tc_flat(q.to(DEV), kv.to(DEV), tail.to(DEV), out, _i32([0]), _i32([n]), _i32([0]), 1, H, D, R, V, 0, 0.05, 32, 1, gate=z.to(DEV),
+                              gate_each=each)
+    kernels.tc_check_status(torch.device(DEV))
+    see = torch.arange(n)[:, None] >= torch.arange(n)[None, :]
+    for h in range(H):
+        qh, kh, vh = (t.double() for t in (q[:, h * (D + R):(h + 1) * (D + R)], kv[:, h * D:(h + 1) * D], kv[:, H * D + h * V:H * D + (h + 1) * V]))
+        o = torch.softmax(((qh[:, :D] @ kh.T + qh[:, D:] @ tail.double().T) * 0.05).masked_fill(~see, float("-inf")), dim=-1) @ vh
+        o = o * torch.sigmoid(z.double()[:, h * V:(h + 1) * V] if each else z.double()[:, h:h + 1])
+        assert ((out[:, h * V:(h + 1) * V].double().cpu() - o).abs() <= (2.0 ** -8 + 2.0 ** -8) * o.abs()).all()

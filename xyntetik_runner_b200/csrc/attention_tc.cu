@@ -495,10 +495,11 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             // a sink has no key and no value: it only enters the sum, at the offset the sum carries
             if (live && a.sink != nullptr) l += ta_exp2(fmaf(a.sink[kvh * a.G + pr % a.G], 1.4426950408889634f, -m));
             float inv = live ? 1.0f / l : 0.f;
-            const __nv_bfloat16* gate = nullptr;                     // FLAT: this thread's gates
+            // FLAT: this thread's gates.  (expf and true divisions: __fdividef is zero where 1 + e^-z passes 2^126)
+            const __nv_bfloat16* gate = nullptr;
             if (FLAT && a.gate != nullptr && live) {
                 gate = a.gate + (long long)(tok_base + pr) * a.ld_gate + (a.gate_each ? kvh * HV + half * (HV / 2) : kvh);
-                if (!a.gate_each) inv = __fdividef(inv, 1.0f + __expf(-__bfloat162float(*gate)));
+                if (!a.gate_each) inv = inv / (1.0f + expf(-__bfloat162float(*gate)));
             }
             __nv_bfloat16* dst = a.out + ((long long)(tok_base + (live ? pr : 0) / a.G) * a.H + (kvh * a.G + (live ? pr : 0) % a.G)) * HV + half * (HV / 2);
             float v[32];
@@ -508,7 +509,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                 if (!live) continue;
                 if (FLAT && gate != nullptr && a.gate_each) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) v[i] = __fdividef(v[i], 1.0f + __expf(-__bfloat162float(gate[c * 32 + i])));
+                    for (int i = 0; i < 32; i++) v[i] *= 1.0f / (1.0f + expf(-__bfloat162float(gate[c * 32 + i])));
                 }
 #pragma unroll
                 for (int i = 0; i < 32; i += 8) {
