@@ -1,0 +1,41 @@
+"""Which steps expand the keys of a latent attention layer (LatentAttention._flat_plan): when it pays, what is left to the other order,
+how much memory it may take.  No GPU: the plan is arithmetic on a step's portions."""
+import types
+
+import numpy as np
+import pytest
+
+from xyntetik_runner_b200.parts.latent_attention import LatentAttention
+
+
+def plan(portions, H=16, D=128, R=64, V=128, C=512, window=0):
+    """portions: (position of the first token, tokens) each, in the order of the step."""
+    lens = np.array([m for _, m in portions], dtype=np.int32)
+    ctx = types.SimpleNamespace(host={"seg_len": lens, "seg_pos0": np.array([p for p, _ in portions], dtype=np.int32),
+                                      "seg_start": np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.int32)})
+    return LatentAttention._flat_plan(types.SimpleNamespace(H=H, D=D, R=R, V=V, C=C, window=window), ctx, int(lens.sum()))
+
+
+def test_what_is_expanded_and_what_is_left():
+    assert plan([(0, 2048)]) == (2048, 16, [])
+    # single tokens and short portions keep the other order, neighbours together
+    keys, tiles, rest = plan([(900, 1), (901, 1), (100, 500), (5, 31), (300, 1), (0, 700)])
+    assert (keys, tiles, rest) == (600 + 700, 4 + 6, [[0, 2], [502, 534]])
+    # only what a window's first token sees, down to a tile's border
+    assert plan([(5000, 512)], window=1024)[0] == 5512 - (5000 - 1023) // 128 * 128
+    # steps of single tokens, small layers, portions scattered between many others
+    assert plan([(3000, 1)] * 8) is None
+    assert plan([(0, 64)], H=2, D=64, R=32, V=64, C=64) is None
+    assert plan([(0, 512), (9, 1)] * 6) is None
+
+
+@pytest.mark.parametrize("H", [16, 32, 128])
+@pytest.mark.parametrize("at", [0, 7000, 30000, 65000, 200000])
+def test_memory_is_bounded(H, at):
+    """Whatever the reach, what is gathered and expanded takes at most half a gigabyte: the step could run without."""
+    got = plan([(at, 512)] * 3, H=H)
+    if got is not None:
+        room = 1 << (got[0] - 1).bit_length()                      # (buffers for a power of two of keys)
+        assert got[0] == 3 * (at + 512) and room * (H * 256 + 576) * 2 <= 1 << 29
+    else:
+        assert H * at > 16 * 7000

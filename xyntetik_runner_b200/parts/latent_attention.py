@@ -40,9 +40,15 @@ USE_MMA = True
 USE_FLAT = True
 counters = {"mma": 0, "simt": 0, "flat": 0}
 
-# Portions of at least so many tokens may have their keys expanded, over at most so many keys a step (16 KB a key and layer at
-# 32 heads of 128: what the expanded rows may take of the memory).
-FLAT_MIN, FLAT_KEYS = 32, 65536
+# Portions of at least so many tokens may have their keys expanded, as far as a step's gathered and expanded rows take no more than
+# so many bytes (9 KB a key at 16 heads of 128 + 128 over rows of 576: 32,768 keys).  They stay allocated beside the cached rows, and
+# the other order needs none of them.
+FLAT_MIN, FLAT_BYTES = 32, 1 << 29
+
+
+def _rows_for(keys: int) -> int:
+    """Rows of the buffers that hold `keys` expanded keys: a power of two (a buffer that grows invalidates the step graphs)."""
+    return 1 << (keys - 1).bit_length()
 
 
 class LatentAttention(Mixer):
@@ -152,7 +158,7 @@ class LatentAttention(Mixer):
         pairs = float((np.minimum(mean, window) if window else mean).dot(length[many]))
         keys = int((pos0 + length - kernels.flat_first_key(pos0, window))[many].sum())
         tokens = int(length[many].sum())
-        if keys > FLAT_KEYS:
+        if _rows_for(keys) * (H * (D + V) + C + R) * 2 > FLAT_BYTES:
             return None
         absorbed = pairs * H * 2 * (2 * C + R) / 70e6 + tokens * 2.0 * H * C * (D + V) / 300e6
         flat = 25.0 + keys * 2.0 * C * H * (D + V) / 900e6 + pairs * H * 2 * (D + R + V) / 300e6
@@ -236,8 +242,7 @@ class LatentAttention(Mixer):
             flat = ctx.once(("latent_flat", H, D, R, V, C, window), lambda: self._flat_plan(ctx, n)) if USE_FLAT and self.expand is not None else None
             if flat:
                 keys, tiles, rest = flat
-                # (rows for a power of two of keys: a buffer that grows invalidates the step graphs)
-                room = 1 << (keys - 1).bit_length()
+                room = _rows_for(keys)
                 rows = ctx.buf("latent_rows", (room, C + R), torch.bfloat16)[:keys]
                 kernels.flat_rows(cache_ptr, page_stride, rows, ctx.seg_len, ctx.seg_pos0, bt, ctx.n_seg, ctx.max_pages, ctx.page_size, window, FLAT_MIN)
                 kv = ctx.buf("latent_kv", (room, H * (D + V)), torch.bfloat16)[:keys]
