@@ -589,7 +589,7 @@ def test_scores_of_chunks_out_of_the_short_cuts_range(what):
     w_t[0] = 1.0
     if what == "decays":
         inner[token:, 0] = float("nan")
-    z = -11.06 if what == "keys" else -20.0
+    z = -11.06 if what == "keys" else -36.0
     proj = torch.cat([q, k, v, inner], 1).to(DEV)
     state0 = f(1, H * D * V) * scale
 
