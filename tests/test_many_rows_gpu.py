@@ -632,3 +632,31 @@ def test_gates_of_expanded_attention_keep_float32(each):
         o = torch.softmax(((qh[:, :D] @ kh.T + qh[:, D:] @ tail.double().T) * 0.05).masked_fill(~see, float("-inf")), dim=-1) @ vh
         o = o * torch.sigmoid(z.double()[:, h * V:(h + 1) * V] if each else z.double()[:, h:h + 1])
         assert ((out[:, h * V:(h + 1) * V].double().cpu() - o).abs() <= (2.0 ** -8 + 2.0 ** -8) * o.abs()).all()
+
+
+@pytest.mark.parametrize("n,n_out,k,wdt,skip,extra", [(9, 70, 34, torch.float32, 0, 2), (70, 600, 37, torch.float32, 1, 1), (300, 2001, 66, torch.bfloat16, 0, 0),
+                                                      (300, 2001, 68, torch.bfloat16, 0, 3), (70, 600, 64, torch.bfloat16, 2, 0), (65, 4800, 35, torch.float32, 0, 0),
+                                                      (300, 2001, 40, torch.bfloat16, 1, 0), (1, 33, 3, torch.bfloat16, 3, 5), (300, 2001, 16, torch.float32, 0, 0),
+                                                      (300, 2001, 4, torch.bfloat16, 0, 4)])
+def test_float32_product_off_the_copies_borders(n, n_out, k, wdt, skip, extra):
+    """Operands whose addresses, rows' distances or K do not allow 16-byte copies, and K of a few values, with few tiles and with many: the
+    same bits as the same numbers on 16-byte borders with zeros behind them, stored, added, as bfloat16 behind a factor and a bias."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + k + skip)
+    x, w = torch.randn(n, k, generator=g), torch.randn(n_out, k, generator=g).to(wdt)
+    xs = torch.full((n, k + extra), float("nan"), device=DEV)
+    xs[:, :k] = x.to(DEV)
+    flat = torch.full((n_out * k + 16,), float("nan"), dtype=wdt, device=DEV)
+    flat[skip:skip + n_out * k] = w.to(DEV).reshape(-1)
+    pad = -(-k // 8) * 8 + 8
+    off = (xs[:, :k], flat[skip:skip + n_out * k].view(n_out, k))
+    even = [torch.nn.functional.pad(t.to(DEV), (0, pad - k)).contiguous() for t in (x, w)]
+    base, bias = torch.randn(n, n_out, generator=g).to(DEV), torch.randn(n_out, generator=g).to(DEV)
+    for kind in ("store", "add", "bf16"):
+        got, want = ((base.clone() if kind == "add" else torch.empty(n, n_out, dtype=torch.bfloat16 if kind == "bf16" else torch.float32, device=DEV)) for _ in range(2))
+        for (a, b), out in ((off, got), (even, want)):
+            kernels.gemm_simt(a, b, out, bias if kind == "bf16" else None, kind == "add", 0.5 if kind == "bf16" else 1.0)
+        assert torch.equal(got, want), kind
+        if kind == "store":
+            bound = (x.double().abs() @ w.double().abs().T) * (k + 2) * 2.0 ** -24
+            assert ((got.cpu().double() - x.double() @ w.double().T).abs() <= bound).all()

@@ -42,9 +42,68 @@ k_gemm_simt(const TX* __restrict__ X, const TW* __restrict__ W, const float* __r
     }
 }
 
+// The same sums without the ring, for operands that 16-byte copies do not fit and for K of a few values: 64 x 64 outputs of 256 threads,
+// 16 values of k at a time through registers into shared memory, k-major.  Element by element the ring's copies are stores that every
+// later load waits for; here a thread has eight loads in flight and four blocks share an SM.  What bounds it: shared memory, 8 words
+// for 16 multiply-adds.
+#define GP_BM 64
+#define GP_BN 64
+#define GP_BK 16
+template <typename TX, typename TW, typename TO, bool ACCUM>
+__global__ void __launch_bounds__(256)
+k_gemm_simt_plain(const TX* __restrict__ X, const TW* __restrict__ W, const float* __restrict__ bias,
+                  TO* __restrict__ out, int n, int n_out, int K, long long ldx, long long ldo, float alpha) {
+    __shared__ float Xs[GP_BK][GP_BM + 4];
+    __shared__ float Ws[GP_BK][GP_BN + 4];
+    const int tid = threadIdx.x, t0 = blockIdx.y * GP_BM, r0 = blockIdx.x * GP_BN;
+    const int ty = tid / 16, tx = tid % 16, lrow = tid / 4, lk = (tid % 4) * 4;
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (int k0 = 0; k0 < K; k0 += GP_BK) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int k = k0 + lk + q, t = t0 + lrow, r = r0 + lrow;
+            Xs[lk + q][lrow] = t < n && k < K ? xr_to_f32<TX>(X[(size_t)t * ldx + k]) : 0.f;
+            Ws[lk + q][lrow] = r < n_out && k < K ? xr_to_f32<TW>(W[(size_t)r * K + k]) : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < GP_BK; kk++) {
+            float a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = Xs[kk][ty * 4 + i];
+#pragma unroll
+            for (int j = 0; j < 4; j++) b[j] = Ws[kk][tx * 4 + j];
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int t = t0 + ty * 4 + i;
+        if (t >= n) continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int r = r0 + tx * 4 + j;
+            if (r >= n_out) continue;
+            float v = alpha * acc[i][j];
+            if (bias) v += bias[r];
+            const size_t o = (size_t)t * ldo + r;
+            if (ACCUM) out[o] = xr_from_f32<TO>(xr_to_f32<TO>(out[o]) + v);
+            else out[o] = xr_from_f32<TO>(v);
+        }
+    }
+}
+
 template <typename TX, typename TW, typename TO, bool ACCUM, int WM, int WN, int TM, int TN>
 static int launch_simt_tile(const void* X, const void* W, const float* bias, void* out, int n, int n_out, int K, long long ldx, long long ldo,
-                            float alpha, cudaStream_t stream) {
+                            float alpha, int vec, cudaStream_t stream) {
     constexpr int BM = 4 * TM * WM, BN = 8 * TN * WN;
     constexpr size_t SMEM = gs_smem<TX, TW, BM, BN>();
     const dim3 grid((n_out + BN - 1) / BN, (n + BM - 1) / BM);
@@ -52,8 +111,6 @@ static int launch_simt_tile(const void* X, const void* W, const float* bias, voi
     static bool ready[XR_DEVICES];
     if (SMEM > 48 * 1024 && !xr_once_per_device(ready, [] { return xr_allow_smem(k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN>, SMEM); }))
         return XR_ERR_LAUNCH;
-    constexpr int PX = 16 / (int)sizeof(TX), PW = 16 / (int)sizeof(TW);
-    const int vec = !(((uintptr_t)X | (uintptr_t)W) & 15) && ldx % PX == 0 && K % PX == 0 && K % PW == 0;
     k_gemm_simt<TX, TW, TO, ACCUM, WM, WN, TM, TN><<<grid, 32 * WM * WN, SMEM, stream>>>((const TX*)X, (const TW*)W, bias, (TO*)out, n, n_out, K, ldx, ldo, alpha, vec);
     return xr_launch_status();
 }
@@ -62,12 +119,22 @@ static int launch_simt_tile(const void* X, const void* W, const float* bias, voi
 // wide ones read fewer words a multiply-add from shared memory, narrow ones spread a small product over more SMs.  Measured, us, tiles
 // 8x32 / 32x32 / 32x64 / 64x64 / 128x128: 44 x 1,024 x 1,024: 17 21 29 43 114; 256 x 1,024 x 1,024: 35 29 29 45 115; 256 x 5,632 x 1,024:
 // 163 103 91 98 117; 256 x 32,000 x 1,024: 881 535 464 433 451; 2,048 x 5,632 x 1,024: 1,235 745 642 613 577.
+// Operands off the 16-byte borders, and K of at most 16, take the kernel without the ring where its tiles fill a third of the SMs:
+// 760 x 1,525 x 5,123 625 / 477 (with the ring / without), 1,765 x 949 x 553 114 / 78, 1,097 x 152 x 3,633 238 / 215, 1,587 x 5,939 x 58 68 / 51, 1,487 x 3,097 x 4 17 / 12;
+// with fewer tiles the ring is ahead: 117 x 172 x 255 14 / 19, 756 x 258 x 179 37 / 51, 46 x 5 x 2,553 105 / 134.
 template <typename TX, typename TW, typename TO, bool ACCUM>
 static int launch_simt_out(const void* X, const void* W, const float* bias, void* out, int n, int n_out, int K, long long ldx, long long ldo,
                            float alpha, cudaStream_t stream) {
-#define GS(WM, WN, TM, TN) return launch_simt_tile<TX, TW, TO, ACCUM, WM, WN, TM, TN>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, stream)
+#define GS(WM, WN, TM, TN) return launch_simt_tile<TX, TW, TO, ACCUM, WM, WN, TM, TN>(X, W, bias, out, n, n_out, K, ldx, ldo, alpha, vec, stream)
     const long long sms = xr_sm_count();
+    constexpr int PX = 16 / (int)sizeof(TX), PW = 16 / (int)sizeof(TW);
+    const int vec = !(((uintptr_t)X | (uintptr_t)W) & 15) && ldx % PX == 0 && K % PX == 0 && K % PW == 0;
     auto tiles = [&](int bm, int bn) { return (long long)((n + bm - 1) / bm) * ((n_out + bn - 1) / bn); };
+    if ((!vec || K <= GP_BK) && n > 64 && 3 * tiles(GP_BM, GP_BN) > sms && (n + GP_BM - 1) / GP_BM <= 65535) {
+        k_gemm_simt_plain<TX, TW, TO, ACCUM><<<dim3((n_out + GP_BN - 1) / GP_BN, (n + GP_BM - 1) / GP_BM), 256, 0, stream>>>(
+            (const TX*)X, (const TW*)W, bias, (TO*)out, n, n_out, K, ldx, ldo, alpha);
+        return xr_launch_status();
+    }
     int pick;
     if (n <= 8 || tiles(32, 32) < sms) pick = 0;
     else if (tiles(128, 128) >= 4 * sms) pick = 4;
