@@ -122,14 +122,16 @@ static int launch_rglru_gates(float* proj, long long ldp, int y_col, const float
 
 // The convolution alone, a thread an element: u [n][R].  Ahead of k_rglru_gates_few, whose many small blocks would each compute
 // the whole tile again behind a chain of dependent loads.
+// I: a number of elements (32 bits as long as they do).
+template <typename I>
 __global__ void k_rglru_conv(const float* __restrict__ proj, long long ldp, int x_col, const float* __restrict__ conv_w,
                              const float* __restrict__ conv_b, const float* __restrict__ state, long long state_stride,
                              const int* __restrict__ tok_seg, const int* __restrict__ seg_start, const int* __restrict__ seg_slot,
                              float* __restrict__ u, int n, int R, int taps) {
     xr_pdl_launch();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n * R) return;
-    const int t = idx / R, ch = idx % R;
+    const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
+    if (idx >= (I)n * (I)R) return;
+    const int t = (int)(idx / R), ch = (int)(idx % R);
     const int seg = tok_seg[t], i = t - seg_start[seg];
     const float* tail = state + (size_t)seg_slot[seg] * state_stride + R;
     const float* w = conv_w + (size_t)ch * taps;
@@ -347,15 +349,19 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
         state_stride < (long long)R * taps)
         return XR_ERR_ARG;
     const int Bs = R / B;
-    if ((long long)n * R > 0x7fffffffLL - 255) return XR_ERR_ARG;
+    const long long elements = (long long)n * R;
+    if ((elements + 255) / 256 > 0x7fffffffLL) return XR_ERR_ARG;
     const bool rows = taps == 4 && n >= 64 && !((R | ldp | x_col | state_stride) & 3) &&
                       !(((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)state | (uintptr_t)u_s) & 15) && (n + RC_RUN - 1) / RC_RUN <= 65535;
     if (rows)
         xr_launch(k_rglru_conv_rows, dim3((R / 4 + 127) / 128, (n + RC_RUN - 1) / RC_RUN), dim3(128), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b,
                   (const float*)state, state_stride, tok_seg, seg_start, seg_slot, u_s, n, R);
+    else if (elements <= 0x7fffffffLL - 255)
+        xr_launch(k_rglru_conv<int>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b,
+                  (const float*)state, state_stride, tok_seg, seg_start, seg_slot, u_s, n, R, taps);
     else
-        xr_launch(k_rglru_conv, dim3((n * R + 255) / 256), dim3(256), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b, (const float*)state,
-                  state_stride, tok_seg, seg_start, seg_slot, u_s, n, R, taps);
+        xr_launch(k_rglru_conv<long long>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b,
+                  (const float*)state, state_stride, tok_seg, seg_start, seg_slot, u_s, n, R, taps);
     const size_t smem8 = (size_t)8 * Bs * sizeof(float);
     if (n <= 16 && smem8 <= 48 * 1024) {
         // (one token to a few: a warp an output, its lanes share the inputs)
