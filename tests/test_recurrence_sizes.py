@@ -17,4 +17,5 @@ def answer(n, R, B, taps=4):
 def test_sizes():
     assert answer(1901, 2560, 10) == NO_DEVICE and answer(1, 48, 2) == NO_DEVICE
     assert answer(900_000, 2560, 10) == NO_DEVICE               # more than 2^31 elements
+    assert answer(17, 6400, 1) == answer(1, 6400, 1) == NO_DEVICE and answer(17, 6408, 1) == answer(1, 6408, 1) == REFUSED
     assert answer(17, 48, 5) == REFUSED and answer(0, 48, 2) == REFUSED and answer(17, 48, 2, taps=17) == REFUSED

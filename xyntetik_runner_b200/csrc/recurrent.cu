@@ -226,6 +226,10 @@ k_rglru_gates_few(float* __restrict__ proj, long long ldp, int y_col, const floa
     }
 }
 
+// Channel blocks whose eight tokens fit this much shared memory take the kernel above, wider ones the tile product.  The whole part, one
+// token / sixteen, us, kernel above / tiles: blocks of 2,048 channels 20 66 / 46 84, of 3,072 38 133 / 67 137, of 4,096 109 389 / 90 115.
+#define RG_FEW_SMEM (100 * 1024)
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 k_rglru_scan(const float* __restrict__ proj, long long ldp, int y_col, int x_col, const float* __restrict__ a_in, const float* __restrict__ b_in,
@@ -350,7 +354,8 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
         return XR_ERR_ARG;
     const int Bs = R / B;
     const long long elements = (long long)n * R;
-    if ((elements + 255) / 256 > 0x7fffffffLL) return XR_ERR_ARG;
+    const size_t smem8 = (size_t)8 * Bs * sizeof(float);                // eight tokens of a channel block
+    if ((elements + 255) / 256 > 0x7fffffffLL || smem8 > 200 * 1024) return XR_ERR_ARG;
     const bool rows = taps == 4 && n >= 64 && !((R | ldp | x_col | state_stride) & 3) &&
                       !(((uintptr_t)proj | (uintptr_t)conv_w | (uintptr_t)state | (uintptr_t)u_s) & 15) && (n + RC_RUN - 1) / RC_RUN <= 65535;
     if (rows)
@@ -362,9 +367,10 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
     else
         xr_launch(k_rglru_conv<long long>, dim3((unsigned)((elements + 255) / 256)), dim3(256), 0, stream, (const float*)proj, ldp, x_col, conv_w, conv_b,
                   (const float*)state, state_stride, tok_seg, seg_start, seg_slot, u_s, n, R, taps);
-    const size_t smem8 = (size_t)8 * Bs * sizeof(float);
-    if (n <= 16 && smem8 <= 48 * 1024) {
+    if (n <= 16 && smem8 <= RG_FEW_SMEM) {
         // (one token to a few: a warp an output, its lanes share the inputs)
+        static bool ready[XR_DEVICES];
+        if (smem8 > 48 * 1024 && !xr_once_per_device(ready, [] { return xr_allow_smem(k_rglru_gates_few, RG_FEW_SMEM); })) return XR_ERR_LAUNCH;
         const int groups = (Bs + 7) / 8;
         xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, proj, ldp, y_col, wa, wi, ba, bi, lam, a_s, b_s,
                   n, R, Bs, c, groups, (const float*)u_s);
