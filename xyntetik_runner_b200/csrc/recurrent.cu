@@ -386,10 +386,19 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
     dim3 gs((R + 127) / 128, n_seg);
     // (a step with long portions is a few long-lived blocks: they start behind the gates kernel, not into its last wave)
     const bool behind = n > 4 * n_seg;
-    // (the true 32-bit path promises the same bits however portions are cut: a thread a channel there)
-    if (behind && dtype == XR_BF16)
+    // Segments where the chain of a portion's tokens is what counts: portions of 64 tokens on average, and of 3 / 5 of a token for every block of
+    // segments (two such blocks share an SM).  The whole part, us, segments / a thread a channel: 2,560 channels 1 x 64 tokens 30 / 30, 1 x 1,024
+    // 146 / 206, 2 x 64 45 / 41, 2 x 256 89 / 99, 8 x 128 155 / 145, 8 x 512 507 / 516, 48 x 16 195 / 97; 1,024 channels 1 x 128 17 / 22, 4 x 96
+    // 27 / 29, 16 x 64 52 / 37, 16 x 256 130 / 132.  (The true 32-bit path promises the same bits however portions are cut: a thread a
+    // channel there.)
+    const long long seg_blocks = (long long)((R + 31) / 32) * n_seg;
+    const bool segments = dtype == XR_BF16 && n >= 64LL * n_seg && 5LL * n >= 3 * seg_blocks * n_seg;
+    if (segments)
         xr_launch_behind((k_rglru_scan_segments<__nv_bfloat16>), dim3((R + 31) / 32, n_seg), dim3(32 * RS_WARPS), 0, stream, (const float*)proj, ldp, y_col,
                          x_col, (const float*)a_s, (const float*)b_s, state, state_stride, seg_start, seg_len, seg_slot, (__nv_bfloat16*)out, R, taps);
+    else if (behind && dtype == XR_BF16)
+        xr_launch_behind((k_rglru_scan<__nv_bfloat16>), gs, dim3(128), 0, stream, (const float*)proj, ldp, y_col, x_col, (const float*)a_s, (const float*)b_s, state,
+                         state_stride, seg_start, seg_len, seg_slot, (__nv_bfloat16*)out, R, taps);
     else if (behind && dtype == XR_F32)
         xr_launch_behind((k_rglru_scan<float>), gs, dim3(128), 0, stream, (const float*)proj, ldp, y_col, x_col, (const float*)a_s, (const float*)b_s, state,
                          state_stride, seg_start, seg_len, seg_slot, (float*)out, R, taps);
