@@ -39,3 +39,43 @@ def test_memory_is_bounded(H, at):
         assert got[0] == 3 * (at + 512) and room * (H * 256 + 576) * 2 <= 1 << 29
     else:
         assert H * at > 16 * 7000
+
+
+BIG, SMALL, WINDOW = (dict(H=16, D=128, R=64, V=128, C=512), dict(H=8, D=64, R=32, V=64, C=256), dict(H=16, D=128, R=64, V=128, C=512, window=1024))
+# keys held, tokens of the portion, single tokens at 600 keys beside it; microseconds a layer on one B200: over the latent rows, expanded
+MEASURED = [
+    (BIG, 0, 32, 0, 59, 44),
+    (BIG, 0, 512, 16, 216, 114),
+    (BIG, 0, 2048, 0, 1365, 137),
+    (BIG, 500, 64, 16, 105, 111),
+    (BIG, 2000, 32, 0, 92, 95),
+    (BIG, 2000, 48, 0, 135, 98),
+    (BIG, 2000, 48, 16, 124, 152),
+    (BIG, 2000, 96, 16, 249, 162),
+    (BIG, 8000, 32, 16, 221, 335),
+    (BIG, 8000, 48, 16, 286, 336),
+    (BIG, 8000, 200, 16, 1188, 346),
+    (BIG, 30000, 32, 16, 644, 902),
+    (BIG, 30000, 128, 0, 2754, 512),
+    (WINDOW, 0, 256, 0, 138, 84),
+    (WINDOW, 2000, 48, 16, 110, 142),
+    (WINDOW, 2000, 64, 16, 136, 152),
+    (WINDOW, 2000, 200, 16, 249, 154),
+    (WINDOW, 8000, 64, 16, 137, 143),
+    (SMALL, 0, 1024, 16, 301, 96),
+    (SMALL, 2000, 32, 16, 87, 120),
+    (SMALL, 8000, 32, 0, 155, 203),
+    (SMALL, 8000, 32, 16, 198, 278),
+    (SMALL, 8000, 48, 16, 260, 276),
+    (SMALL, 8000, 128, 0, 413, 131),
+]
+
+
+@pytest.mark.parametrize("sizes,held,tokens,singles,over_latents,expanded", MEASURED)
+def test_the_faster_order_is_taken(sizes, held, tokens, singles, over_latents, expanded):
+    """Never expanded where that takes a tenth longer, always where it takes two thirds at most."""
+    got = plan([(held, tokens)] + [(600, 1)] * singles, **sizes)
+    if expanded > 1.1 * over_latents:
+        assert got is None
+    if 1.5 * expanded < over_latents:
+        assert got is not None

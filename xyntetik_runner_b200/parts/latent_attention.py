@@ -144,37 +144,42 @@ class LatentAttention(Mixer):
                 + self.w_uv.numel() * self.w_uv.element_size() + (self.up_q.nbytes() if self.up_q is not None else 0))
 
     def _flat_plan(self, ctx, n: int):
-        """(keys to expand, 128-token tiles, token ranges left to the other order) where expanding keys pays, else None.  The times
-        (microseconds) behind it are rates measured on one B200: the kernel over the latent rows does 70 TFLOP/s on 2 C + R columns
-        a head and key, its per-head products 300; expanding costs a product at 900 TFLOP/s and attention at 300 on D + R + V columns,
-        and 25 us of launches.  2,048 tokens of one request, 16 heads of 128 + 64 over a latent of 512: 1,200 us a layer
-        over the latent rows, 85 so (51 of them attention); 512 of one request beside 16 single tokens, two layers: 540 us and 300."""
+        """(keys to expand, 128-token tiles, token ranges left to the other order) where expanding keys pays, else None.  Both sides' times
+        in microseconds, from one B200.  Over the latent rows: 50 TFLOP/s on 2 C + R columns a key and head (heads counted in sixteens), and
+        0.1 a token for what stands around it (at 16 heads over 512).  Expanded: a product at 900 TFLOP/s, then a CTA per 128 tokens and head walks its keys 128 at
+        a time, 1.33 each, 2.6 where some of its 128 tokens do not exist; the longest walk or all of them over 148 SMs, whichever is more.  Tokens that
+        are left to the other order cost its launches again for every run of neighbours, and splits over the step's longest reach.  Measured, a layer, latent rows / expanded,
+        16 heads of 128 + 64 over a latent of 512: 2,048 tokens 1,365 / 137; behind 2,000 keys 48 tokens 135 / 98, beside 16 single tokens 124 /
+        152, 96 and 16 249 / 162; behind 8,000 keys 32 and 16 221 / 335, 96 and 16 501 / 343; 8 heads of 64 + 32 over 256, behind 8,000
+        keys: 32 tokens 155 / 203, 64 262 / 207, 32 and 16 198 / 277."""
         H, D, R, V, C, window = self.H, self.D, self.R, self.V, self.C, self.window or 0
         length, pos0, start = (ctx.host[k].astype(np.int64) for k in ("seg_len", "seg_pos0", "seg_start"))
         many = length >= FLAT_MIN
         if not many.any():
             return None
-        mean = pos0[many] + (length[many] + 1) / 2.0
-        pairs = float((np.minimum(mean, window) if window else mean).dot(length[many]))
-        keys = int((pos0 + length - kernels.flat_first_key(pos0, window))[many].sum())
-        tokens = int(length[many].sum())
+        own, at = length[many], pos0[many]
+        mean = at + (own + 1) / 2.0
+        pairs = float((np.minimum(mean, window) if window else mean).dot(own))
+        reach = at + own - kernels.flat_first_key(at, window)
+        keys = int(reach.sum())
         if _rows_for(keys) * (H * (D + V) + C + R) * 2 > FLAT_BYTES:
             return None
-        absorbed = pairs * H * 2 * (2 * C + R) / 70e6 + tokens * 2.0 * H * C * (D + V) / 300e6
-        flat = 25.0 + keys * 2.0 * C * H * (D + V) / 900e6 + pairs * H * 2 * (D + R + V) / 300e6
-        if flat >= absorbed:
-            return None
-        # the tokens of the other portions, neighbours together
+        absorbed = pairs * -(-H // 16) * 16 * 2 * (2 * C + R) / 50e6 + 0.1 * float(own.sum()) * H * C / 8192
+        walk = reach / 128.0 * np.where(own % 128 > 0, 2.6, 1.33)
+        flat = 5.0 + keys * 2.0 * C * H * (D + V) / 900e6 + max(float(walk.max()), float(walk.dot(-(-own // 128))) * H / 148.0)
+        # the tokens of the other portions, neighbours together: a launch each
         rest = []
         for s in np.argsort(start[~many], kind="stable"):
-            at, end = int(start[~many][s]), int(start[~many][s] + length[~many][s])
-            if rest and rest[-1][1] == at:
+            first, end = int(start[~many][s]), int(start[~many][s] + length[~many][s])
+            if rest and rest[-1][1] == first:
                 rest[-1][1] = end
             else:
-                rest.append([at, end])
-        if len(rest) > 4:
-            return None                     # (scattered one by one between long portions: not worth a launch each)
-        return keys, int((-(-length[many] // 128)).sum()), rest
+                rest.append([first, end])
+        longest = int((pos0 + length).max())
+        flat += len(rest) * (45.0 + 0.005 * (min(longest, window) if window else longest))
+        if flat >= absorbed or len(rest) > 4:
+            return None
+        return keys, int((-(-own // 128)).sum()), rest
 
     def _absorbed(self, ctx, qt, positions, tok_seg, bt, cache_ptr, page_stride, o, gate, gate_col, window):
         """Attention over the latent rows of the tokens whose queries are qt's rows, into o's."""
