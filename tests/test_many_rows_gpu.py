@@ -660,3 +660,107 @@ def test_float32_product_off_the_copies_borders(n, n_out, k, wdt, skip, extra):
         if kind == "store":
             bound = (x.double().abs() @ w.double().abs().T) * (k + 2) * 2.0 ** -24
             assert ((got.cpu().double() - x.double() @ w.double().T).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("kind,H,D,V,lens", [("head", 2, 64, 64, [3, 900, 1, 64]), ("key", 1, 128, 64, [640, 1, 513]), ("key", 2, 64, 128, [1030]),
+                                             ("mlstm", 2, 64, 64, [1, 777, 65]), ("mlstm", 1, 128, 64, [1100])])
+def test_portions_of_many_chunks(kind, H, D, V, lens):
+    """Portions of nine to eighteen chunks, as steps bring them (the memories follow from one another eight chunks at a time), beside short
+    ones, in two launches, the second from the first's states: against float64 and beside the walk."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(sum(lens) + D)
+    f = lambda *s: torch.randn(*s, generator=g)
+    S, n = len(lens), sum(lens)
+    starts, slots = [sum(lens[:i]) for i in range(S)], list(range(S, 0, -1))
+    size = D * V + (D + 1 if kind == "mlstm" else 0)
+    state0 = f(S + 1, H, size)
+    if kind == "mlstm":
+        state0[..., -1] = 0.5
+    dec = torch.tensor([1.0 - 2.0 ** -(4 + 4 * h) for h in range(H)])
+    w_t, bias = f(8, H * D), 3.0 + f(H * D)
+    rows = []
+    for _ in range(2):
+        q, k, v = f(n, H * D), f(n, H * D) * (1.0 if kind == "mlstm" else D ** -0.5), f(n, H * V)
+        rows.append((torch.cat([q, k, v, f(n, H * V), f(n, 8)], 1), torch.cat([f(n, H), 4.0 + f(n, H)], 1)))
+
+    def run(chunked):
+        state, outs = state0.reshape(S + 1, -1).to(DEV).clone(), []
+        seg = (_i32(starts), _i32(lens), _i32(slots))
+        scratch = torch.full((kernels.chunked_floats(n, S, H, D, V, kind),), float("nan"), device=DEV) if chunked else None
+        for proj, gates in rows:
+            proj, o = proj.to(DEV), torch.empty(n, H * V, device=DEV)
+            if kind == "head":
+                kernels.decay_attention(proj, (0, H * D, 2 * H * D), dec.to(DEV), state, *seg, o, S, H, D, V, silu=False, scratch=scratch)
+            elif kind == "key":
+                kernels.key_decay_attention(proj, (0, H * D, 2 * H * D, 2 * H * D + 2 * H * V), 8, w_t.to(DEV), bias.to(DEV), 12.0,
+                                            torch.empty(n, H * D, device=DEV), state, *seg, o, S, H, D, V, scratch=scratch)
+            else:
+                kernels.mlstm(proj, (0, H * D, 2 * H * D, 2 * H * D + H * V), gates.to(DEV), state, torch.empty(n, 3 * H, device=DEV), o,
+                              torch.ones(H * V, device=DEV), torch.empty(n, H * V, device=DEV), *seg, S, H, D, V, 15.0, 1e-6, scratch=scratch)
+            outs.append(o.cpu())
+        return outs, state.cpu()
+    walk, walk_state = run(False)
+    got, state = run(True)
+    assert torch.equal(state[0], state0[0].reshape(-1))
+    for i, (m, slot) in enumerate(zip(lens, slots)):
+        at = slice(starts[i], starts[i] + m)
+        st = state0[slot].double()
+        if kind == "mlstm":
+            Sm, nm, mx = st[:, :D * V].reshape(H, D, V), st[:, D * V:D * V + D], st[:, -1]
+        else:
+            Sm = st.view(H, V, D).transpose(1, 2)
+        for part, (proj, gates) in enumerate(rows):
+            p = proj[at].double()
+            q, k, v = p[:, :H * D].view(m, H, D), p[:, H * D:2 * H * D].view(m, H, D), p[:, 2 * H * D:2 * H * D + H * V].view(m, H, V)
+            if kind == "mlstm":
+                q = q * D ** -0.5
+                li = 15.0 * torch.tanh(gates[at, :H].double() / 15.0)
+                lf = torch.nn.functional.logsigmoid(15.0 * torch.tanh(gates[at, H:].double() / 15.0))
+                want = []
+                for t in range(m):
+                    new = torch.maximum(lf[t] + mx, li[t])
+                    a, s = torch.exp(lf[t] + mx - new), torch.exp(li[t] - new)
+                    Sm = a[:, None, None] * Sm + s[:, None, None] * k[t][:, :, None] * v[t][:, None, :]
+                    nm, mx = a[:, None] * nm + s[:, None] * k[t], new
+                    want.append(torch.einsum("hdv,hd->hv", Sm, q[t]))            # the numerators: a denominator may cancel
+                    den = torch.maximum((nm * q[t]).sum(-1).abs(), torch.exp(-mx)) + 1e-6
+                    got[part][starts[i] + t] *= den.float().repeat_interleave(V)
+                    walk[part][starts[i] + t] *= den.float().repeat_interleave(V)
+                want = torch.stack(want)
+            else:
+                if kind == "head":
+                    decay = dec.double()[None, :, None].expand(m, H, D)
+                else:
+                    decay = torch.exp(torch.nn.functional.logsigmoid(p[:, -8:] @ w_t.double() + bias) / 12.0).view(m, H, D)
+                want, Sm = _walk(q, k, v, decay, Sm)
+            _close(got[part][at], want.reshape(m, -1), walk[part][at])
+        end = torch.cat([Sm.reshape(H, -1), nm, mx[:, None]], 1).reshape(-1) if kind == "mlstm" else Sm.transpose(1, 2).reshape(-1)
+        _close(state[slot], end, walk_state[slot])
+
+
+def test_gated_recurrence_in_segments_beside_short_portions():
+    """The route of long portions, taken for portions of a token, of fewer tokens than segments and of many in one launch: the same as each
+    portion alone, and the walk's results in float32."""
+    from xyntetik_runner_b200 import kernels
+    R, B, taps, lens = 48, 2, 4, [400, 1, 20, 33]
+    g = torch.Generator().manual_seed(2)
+    f = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    Bs, n, S = R // B, sum(lens), len(lens)
+    args = (f(R, taps), f(R), None, None, f(B, Bs, Bs) / Bs ** 0.5, f(B, Bs, Bs) / Bs ** 0.5, f(R), f(R), -4.0 + f(R))
+    proj0, state0 = f(n, 2 * R), f(S, kernels.rglru_state_floats(R, taps))
+    starts = [sum(lens[:i]) for i in range(S)]
+
+    def run(which, dtype):
+        rows = torch.cat([proj0[starts[s]:starts[s] + lens[s]] for s in which]).clone()
+        ln = [lens[s] for s in which]
+        m, state = len(rows), state0.clone()
+        a, b, u, out = torch.empty(m, R, device=DEV), torch.empty(m, R, device=DEV), torch.empty(m, R, device=DEV), torch.empty(m, R, dtype=dtype, device=DEV)
+        kernels.rglru(rows, *args, state, _i32([i for i, x in enumerate(ln) for _ in range(x)]), _i32([sum(ln[:i]) for i in range(len(ln))]), _i32(ln),
+                      _i32(which), a, b, u, out, len(ln), R, B, taps, 8.0)
+        return out, state
+    got, state = run([0, 1, 2, 3], torch.bfloat16)
+    want, want_state = run([0, 1, 2, 3], torch.float32)
+    # (a state is a sum of at most 400 terms in another order; a read-out is rounded to bfloat16 behind it)
+    assert torch.allclose(got.float(), want, rtol=2.0 ** -8, atol=1e-5) and torch.allclose(state, want_state, rtol=5e-5, atol=1e-5)
+    alone, alone_state = run([0], torch.bfloat16)
+    assert torch.allclose(got[:400].float(), alone.float(), rtol=2.0 ** -8, atol=1e-5) and torch.allclose(state[0], alone_state[0], rtol=5e-5, atol=1e-5)
