@@ -15,8 +15,9 @@
 // Why: the token-by-token walk (recurrent.cu, mlstm.cu) is a chain of as many steps as the portion has tokens and reads q, k and v
 // from shared memory for every few state elements; as products the same work is bound by the float32 FMA pipes and spread over all
 // chunks at once.  It costs about half as many operations again and the memories' way through L2, so it is for portions of many
-// tokens: the callers say from how many (a short portion beside a long one is a chunk of its own).  The sums come in another order
-// than the walk's, so a state depends in its last bits on where portions were cut; callers that promise the same bits take the walk.
+// tokens: parts/chunks.py compares the two by a step's portions (every one, a single token too, is a chunk of its own with a memory of its
+// own).  The sums come in another order than the walk's, so a state depends in its last bits on where portions were cut and on what stood
+// beside them; callers that promise the same bits take the walk.
 // 2,048 tokens of one request, 8 heads, us, walk / chunks: constant decay, 128 x 128 values: 166 / 75; decay per channel, 128 x 256:
 // 223 / 138; mLSTM, 128 x 256: 906 / 193.  Root mean square error of the read-outs against float64, 2,040 tokens, walk / chunks: 2.3e-7 /
 // 1.7e-7; 2.1e-6 / 1.8e-7; 6.9e-7 / 6.5e-7.

@@ -26,8 +26,9 @@
 //     S [H][V][N], then the last taps - 1 inputs of the convolution [taps-1][H V + 2 G N].
 //
 // Everything here is float32 in both precisions, and the walks go token by token: the state after a token does not depend
-// on how the tokens were cut into steps, bit for bit.  (Not so where a portion of many tokens of a bfloat16 model is cut into segments
-// or chunks: k_rglru_scan_segments, chunked.cuh; there the last bits depend on the cuts.)
+// on how the tokens were cut into steps, bit for bit.  (Not so in steps of a bfloat16 model whose portions are cut into segments or chunks:
+// k_rglru_scan_segments, chunked.cuh; there the last bits depend on the cuts and, since a step goes one way as a whole, on what else it
+// holds.)
 #include "simt_tile.cuh"
 #include "conv_tail.cuh"
 #include "chunked.cuh"
@@ -35,12 +36,6 @@
 
 #define RG_MAX_TAPS 16
 
-// a weight through the read-only path (blocks of the same SM read the same rows), pinned where it is written like xr_ld_now
-__device__ __forceinline__ float rc_ld_weight(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
-    return v;
-}
 __device__ __forceinline__ float rc_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float rc_softplus(float z) { return z > 30.0f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float rc_silu(float z) { return z < -80.0f ? 0.0f : z / (1.0f + expf(-z)); }

@@ -11,10 +11,9 @@
 #define GS_BK 32
 #define GS_STAGES 4
 
-template <int BYTES>
 __device__ __forceinline__ void gs_copy_async(void* dst, const void* src, bool live) {
     const unsigned at = (unsigned)__cvta_generic_to_shared(dst);
-    const int n = live ? BYTES : 0;                       // (bytes that are not copied are filled with zeros)
+    const int n = live ? 16 : 0;                          // (bytes that are not copied are filled with zeros)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(src), "r"(n) : "memory");
 }
 // four consecutive values of k
@@ -54,14 +53,14 @@ __device__ __forceinline__ void gs_tile(unsigned char* sm, int K, bool vec, XRow
                 const int row = e / (GS_BK / PX), k = e % (GS_BK / PX) * PX;
                 const TX* p = xrow(row);
                 const bool ok = p != nullptr && k0 + k < K;
-                gs_copy_async<16>(xd + row * SX + k, ok ? p + k0 + k : any_x, ok);
+                gs_copy_async(xd + row * SX + k, ok ? p + k0 + k : any_x, ok);
             }
 #pragma unroll
             for (int e = tid; e < BN * (GS_BK / PW); e += THREADS) {
                 const int row = e / (GS_BK / PW), k = e % (GS_BK / PW) * PW;
                 const TW* p = wrow(row);
                 const bool ok = p != nullptr && k0 + k < K;
-                gs_copy_async<16>(wd + row * SW + k, ok ? p + k0 + k : any_w, ok);
+                gs_copy_async(wd + row * SW + k, ok ? p + k0 + k : any_w, ok);
             }
         } else {
             for (int e = tid; e < BM * GS_BK; e += THREADS) {

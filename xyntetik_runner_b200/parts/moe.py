@@ -32,9 +32,10 @@ from .linear import Linear
 
 
 # A plan of more rows an expert than this (on average) goes to the product on CTA pairs, whose tiles hold what an expert has (up to
-# 256 rows).  Both products of an expert, microseconds, padded tiles of one CTA against pairs: 64 experts of 1,408 at width 2,048:
-# 19 rows 200 / 193, 38 rows 238 / 197, 73 rows 367 / 229, 192 rows 660 / 284; 16 of 1,408 at width 1,024: 25 rows 35 / 38,
-# 50 rows 41 / 39, 97 rows 66 / 48.
+# 256 rows).  Plan, gather and both products, rows drawn at random, microseconds, padded tiles of one CTA / pairs, at 16, 25, 36, 64 and
+# 192 rows: 64 experts of 1,408 at width 2,048: 193 215 252 318 753 / 189 193 199 220 281; 32 of 1,024 at 2,048: 82 92 109 117 261 / 84 85 88
+# 95 125; 16 of 2,816 at 2,048, ungated: 76 82 96 102 177 / 77 77 79 84 104; 16 of 1,408 at 1,024: 41 42 49 57 115 / 41 41 41 46 65.
+# (From 16 to 32 rows the pairs are ahead by up to a sixth; this line is on the safe side.)
 PAIRS_FROM = 32
 
 # The choice, the plan and the gather of a step of so few single tokens are one kernel: csrc/moe.cu, k_route_few.
