@@ -153,33 +153,35 @@ class LatentAttention(Mixer):
         152, 96 and 16 249 / 162; behind 8,000 keys 32 and 16 221 / 335, 96 and 16 501 / 343; 8 heads of 64 + 32 over 256, behind 8,000
         keys: 32 tokens 155 / 203, 64 262 / 207, 32 and 16 198 / 277."""
         H, D, R, V, C, window = self.H, self.D, self.R, self.V, self.C, self.window or 0
-        length, pos0, start = (ctx.host[k].astype(np.int64) for k in ("seg_len", "seg_pos0", "seg_start"))
-        many = length >= FLAT_MIN
-        if not many.any():
+        if int(ctx.host["seg_len"].max()) < FLAT_MIN:
             return None
-        own, at = length[many], pos0[many]
-        mean = at + (own + 1) / 2.0
-        pairs = float((np.minimum(mean, window) if window else mean).dot(own))
-        reach = at + own - kernels.flat_first_key(at, window)
-        keys = int(reach.sum())
+        # (plain numbers: a step's host time is not hidden, and an array operation a portion costs more than its portion)
+        keys = tokens = tiles = longest = 0
+        pairs = walk = walks = 0.0
+        others = []
+        for start, m, at in zip(ctx.host["seg_start"].tolist(), ctx.host["seg_len"].tolist(), ctx.host["seg_pos0"].tolist()):
+            longest = max(longest, at + m)
+            if m < FLAT_MIN:
+                others.append((start, start + m))
+                continue
+            reach, mean, own = at + m - int(kernels.flat_first_key(at, window)), at + (m + 1) / 2.0, -(-m // 128)
+            keys, tokens, tiles = keys + reach, tokens + m, tiles + own
+            pairs += (min(mean, window) if window else mean) * m
+            one = reach / 128.0 * (2.6 if m % 128 else 1.33)
+            walk, walks = max(walk, one), walks + one * own
         if _rows_for(keys) * (H * (D + V) + C + R) * 2 > FLAT_BYTES:
             return None
-        absorbed = pairs * -(-H // 16) * 16 * 2 * (2 * C + R) / 50e6 + 0.1 * float(own.sum()) * H * C / 8192
-        walk = reach / 128.0 * np.where(own % 128 > 0, 2.6, 1.33)
-        flat = 5.0 + keys * 2.0 * C * H * (D + V) / 900e6 + max(float(walk.max()), float(walk.dot(-(-own // 128))) * H / 148.0)
         # the tokens of the other portions, neighbours together: a launch each
         rest = []
-        for s in np.argsort(start[~many], kind="stable"):
-            first, end = int(start[~many][s]), int(start[~many][s] + length[~many][s])
+        for first, end in sorted(others):
             if rest and rest[-1][1] == first:
                 rest[-1][1] = end
             else:
                 rest.append([first, end])
-        longest = int((pos0 + length).max())
+        absorbed = pairs * -(-H // 16) * 16 * 2 * (2 * C + R) / 50e6 + 0.1 * tokens * H * C / 8192
+        flat = 5.0 + keys * 2.0 * C * H * (D + V) / 900e6 + max(walk, walks * H / 148.0)
         flat += len(rest) * (45.0 + 0.005 * (min(longest, window) if window else longest))
-        if flat >= absorbed or len(rest) > 4:
-            return None
-        return keys, int((-(-own // 128)).sum()), rest
+        return None if flat >= absorbed or len(rest) > 4 else (keys, tiles, rest)
 
     def _absorbed(self, ctx, qt, positions, tok_seg, bt, cache_ptr, page_stride, o, gate, gate_col, window):
         """Attention over the latent rows of the tokens whose queries are qt's rows, into o's."""
