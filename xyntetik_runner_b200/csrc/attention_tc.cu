@@ -170,6 +170,15 @@ __host__ __device__ constexpr uint32_t ta_idesc(bool b_mn, int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
+// 1 / (1 + e^-z) in float32's full precision over all of its range: with t = e^-|z| it is 1 / (1 + t) or t / (1 + t), whose divisor lies between 1
+// and 2, so that an approximate reciprocal and one step of Newton's iteration do, without the cases (and their branch, 64 times a thread:
+// 505 tokens beside 6, 16 heads, a gate an element: 51 us a launch with a true division of 1 by 1 + e^-z) that a division has to look for.
+__device__ __forceinline__ float ta_sigmoid(float z) {
+    const float t = expf(-fabsf(z)), y = 1.0f + t;
+    const float r0 = __fdividef(1.0f, y), r = fmaf(r0, fmaf(-y, r0, 1.0f), r0);
+    return z < 0.f ? t * r : r;
+}
+
 // The keys of a portion in the flat array: from this one on (the first its first token sees, at a tile's border) to its last.
 __host__ __device__ __forceinline__ int ta_flat_first(int pos0, int window) { return window > 0 && pos0 >= window ? (pos0 - window + 1) / TA_KEYS * TA_KEYS : 0; }
 
@@ -495,11 +504,10 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
             // a sink has no key and no value: it only enters the sum, at the offset the sum carries
             if (live && a.sink != nullptr) l += ta_exp2(fmaf(a.sink[kvh * a.G + pr % a.G], 1.4426950408889634f, -m));
             float inv = live ? 1.0f / l : 0.f;
-            // FLAT: this thread's gates.  (expf and true divisions: __fdividef is zero where 1 + e^-z passes 2^126)
-            const __nv_bfloat16* gate = nullptr;
+            const __nv_bfloat16* gate = nullptr;                     // FLAT: this thread's gates
             if (FLAT && a.gate != nullptr && live) {
                 gate = a.gate + (long long)(tok_base + pr) * a.ld_gate + (a.gate_each ? kvh * HV + half * (HV / 2) : kvh);
-                if (!a.gate_each) inv = inv / (1.0f + expf(-__bfloat162float(*gate)));
+                if (!a.gate_each) inv *= ta_sigmoid(__bfloat162float(*gate));
             }
             __nv_bfloat16* dst = a.out + ((long long)(tok_base + (live ? pr : 0) / a.G) * a.H + (kvh * a.G + (live ? pr : 0) % a.G)) * HV + half * (HV / 2);
             float v[32];
@@ -509,7 +517,7 @@ k_attention_tc(const __grid_constant__ CUtensorMap q_map, const __grid_constant_
                 if (!live) continue;
                 if (FLAT && gate != nullptr && a.gate_each) {
 #pragma unroll
-                    for (int i = 0; i < 32; i++) v[i] *= 1.0f / (1.0f + expf(-__bfloat162float(gate[c * 32 + i])));
+                    for (int i = 0; i < 32; i++) v[i] *= ta_sigmoid(__bfloat162float(gate[c * 32 + i]));
                 }
 #pragma unroll
                 for (int i = 0; i < 32; i += 8) {
