@@ -124,8 +124,8 @@ __global__ void k_rglru_conv(const float* __restrict__ proj, long long ldp, int 
                              const int* __restrict__ tok_seg, const int* __restrict__ seg_start, const int* __restrict__ seg_slot,
                              float* __restrict__ u, int n, int R, int taps) {
     xr_pdl_launch();
-    const I idx = (I)blockIdx.x * (I)blockDim.x + (I)threadIdx.x;
-    if (idx >= (I)n * (I)R) return;
+    const I idx = sizeof(I) == 4 ? (I)(blockIdx.x * blockDim.x + threadIdx.x) : (I)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (I)n * R) return;
     const int t = (int)(idx / R), ch = (int)(idx % R);
     const int seg = tok_seg[t], i = t - seg_start[seg];
     const float* tail = state + (size_t)seg_slot[seg] * state_stride + R;
