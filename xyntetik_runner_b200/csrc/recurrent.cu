@@ -876,12 +876,14 @@ static int launch_decay_scan(const float* proj, long long ldp, int q_col, int k_
 // proj [n][ldp] float32: q at q_col [H][D], k at k_col [H][D], v at v_col [H][V]; with `silu` their pre-activations (columns from the
 // first of q to the last of v, which a step of many tokens activates in place), else as they are; decay [H] float32; state
 // [slots][state_stride] float32, S [H][V][D];  o [n][H V] float32 receives the read-outs, times read_scale.
-// scratch (null: the walk): the recurrence in chunks (chunked.cuh), all decays then in (0, 1]; xr_chunked_floats says how much it takes.
+// scratch (null: the walk; on a 16-byte border): the recurrence in chunks (chunked.cuh), all decays then in (0, 1]; xr_chunked_floats says how
+// much it takes.
 XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_col, int v_col, const float* decay, float* state,
                                  long long state_stride, const int* seg_start, const int* seg_len, const int* seg_slot, float* o, int n, int n_seg,
                                  int H, int D, int V, int silu, float read_scale, float* scratch, long long scratch_floats, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || H < 1 || D < 1 || V < 1 || D > 256 || n_seg > 65535 || H > 65535 || state_stride < (long long)H * D * V)
         return XR_ERR_ARG;
+    if (scratch != nullptr && ck_takes(D, V) && (scratch_floats < ck_floats(n, n_seg, H, D, V, 0, false) || ((uintptr_t)scratch & 15))) return XR_ERR_ARG;
     // q, k, v lie side by side from q_col on (the caller's layout): one pass activates them all
     const bool many = silu && n > 16 && k_col == q_col + H * D && v_col == k_col + H * D;
     if (many) {
@@ -890,7 +892,6 @@ XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_co
         xr_launch(k_silu_cols, dim3(blocks), dim3(256), 0, stream, proj + q_col, ldp, 2 * H * D + H * V, total);
     }
     if (scratch != nullptr && ck_takes(D, V) && (many || !silu)) {
-        if (scratch_floats < ck_floats(n, n_seg, H, D, V, 0, false)) return XR_ERR_ARG;
         ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, decay, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
                     state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
         ck_lay_out(a, scratch, n, D, false);
@@ -955,7 +956,7 @@ XR_EXPORT int xr_key_decay_attention(const float* proj, long long ldp, int q_col
     ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
                 state_stride, (long long)D * V, 0, seg_start, seg_len, seg_slot, n_seg, o, read_scale, nullptr};
     const int chunked = scratch != nullptr && ck_takes(D, V) && ck_aligned(a) && ck_chunks(n, n_seg) <= 65535;
-    if (chunked && scratch_floats < ck_floats(n, n_seg, H, D, V, C, false)) return XR_ERR_ARG;
+    if (chunked && (scratch_floats < ck_floats(n, n_seg, H, D, V, C, false) || ((uintptr_t)scratch & 15))) return XR_ERR_ARG;
     const int early = chunked || n <= 4 * n_seg;
     if (n > 64) xr_launch((k_key_decay<16>), dim3((C + 127) / 128, (n + 15) / 16), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early, chunked);
     else xr_launch((k_key_decay<4>), dim3((C + 127) / 128, (n + 3) / 4), dim3(128), 0, stream, proj + a_col, ldp, w_t, bias, decays, n, R, C, 1.0f / tau, early, chunked);
