@@ -1,0 +1,73 @@
+"""Products of float32 rows with a bfloat16 matrix in three exact pieces on the tensor cores (csrc/split_product.cuh)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+# rows of W off and on the tiles' 128 (64 gated), tokens around every tile's 16, 32 and 64, K off its blocks of 64, of one slice and of eight
+SIZES = [(1, 8, 256), (15, 129, 264), (17, 128, 1024), (33, 127, 328), (64, 1000, 512), (65, 64, 4096), (129, 6000, 256), (300, 257, 2816), (300, 5001, 1024)]
+
+
+def _inputs(n, rows, k, seed=0):
+    g = torch.Generator().manual_seed(n * 7 + rows + k + seed)
+    x = torch.randn(n, k, generator=g) * torch.exp(2.0 * torch.randn(n, 1, generator=g))
+    return x, (torch.randn(rows, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("n,n_out,k", SIZES)
+def test_products_in_pieces(n, n_out, k):
+    """Stored behind a factor, a bias and an activation, added, gated, with strided rows; against float64.  A sum of k products rounded to
+    float32 at every step is off by at most (k + 2) 2^-24 times the sum of their sizes; as a whole it is no further off than the FMA
+    kernel's.  A token alone gives the same bits."""
+    from xyntetik_runner_b200 import kernels
+    x, w = _inputs(n, n_out, k)
+    xs = torch.full((n, k + 4), float("nan"), device=DEV)
+    xs[:, :k] = x.to(DEV)
+    xd, wd = xs[:, :k], w.to(DEV)
+    assert kernels.split_weight_ok(wd) and kernels.split_rows_ok(xd)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = size * (k + 2) * 2.0 ** -24
+    got, fma = (torch.empty(n, n_out, device=DEV) for _ in range(2))
+    kernels.gemm_split(xd, wd, got)
+    assert ((got.cpu().double() - want).abs() <= bound).all()
+    kernels.gemm_simt(xd, wd, fma)
+    off = lambda y: float(((y.cpu().double() - want) / size).square().mean().sqrt())
+    assert off(got) <= off(fma) * (1.0 if n * n_out > 2000 else 1.5), (off(got), off(fma))
+    for t in {0, n // 2, n - 1}:
+        one = torch.empty(1, n_out, device=DEV)
+        kernels.gemm_split(xd[t:t + 1], wd, one)
+        assert torch.equal(one[0], got[t]), t
+    bias, base = torch.randn(n_out, device=DEV), torch.randn(n, n_out + 3, device=DEV)
+    out = base.clone()[:, :n_out]
+    kernels.gemm_split(xd, wd, out, bias, True, -0.3)
+    assert torch.equal(out, base[:, :n_out] + (-0.3 * got + bias)) or (out - (base[:, :n_out] + (-0.3 * got + bias))).abs().max() <= 2e-6 * (got.abs().max() + 5)
+    kernels.gemm_split(xd, wd, out, bias, False, 0.5, kernels.ACT_SILU)
+    assert torch.allclose(out, torch.nn.functional.silu(0.5 * got + bias), rtol=2e-6, atol=2e-6)
+    F = n_out // 2
+    pair = torch.empty(n, F, device=DEV)
+    for act, limit in ((kernels.ACT_SILU, 0.0), (kernels.ACT_SWISH_CLAMP, 1.5)):
+        ref = torch.empty(n, F, device=DEV)
+        kernels.gemm_split(xd, wd[:2 * F], pair, act=act, gated=True, limit=limit)
+        kernels.act_mul(got[:, :2 * F].contiguous(), ref, act, True, limit)
+        assert torch.allclose(pair, ref, rtol=1e-6, atol=1e-7)
+
+
+def test_values_that_are_no_numbers_and_the_smallest():
+    """An infinite value makes its sums infinite, one that is no number makes them none, other rows stay; values near both ends of the range."""
+    from xyntetik_runner_b200 import kernels
+    x, w = _inputs(40, 200, 320)
+    x[3, 7], x[4, 8], x[5, 9], x[6] = float("inf"), float("-inf"), float("nan"), 3.0e38 * (torch.arange(320) == 11)
+    x[7] *= 1e-33
+    x[8, 1] = torch.tensor(0x7f800001, dtype=torch.int32).view(torch.float32)          # no number by its last bit alone
+    out, fma = (torch.empty(40, 200, device=DEV) for _ in range(2))
+    kernels.gemm_split(x.to(DEV), w.to(DEV), out)
+    kernels.gemm_simt(x.to(DEV), w.to(DEV), fma)
+    assert torch.equal(out.isnan(), fma.isnan()) and torch.equal(out.isinf(), fma.isinf())
+    # both are within (k + 2) 2^-24 of the products' sizes; pieces below 2^-126 may count as zero
+    x = torch.where(x.isfinite(), x, 0.0).double()
+    bound = x.abs() @ w.double().abs().T * (2 * 322 * 2.0 ** -24) + 320 * 2.0 ** -126
+    live = fma.isfinite().cpu()
+    assert ((out.cpu().double() - fma.cpu().double()).abs() <= bound)[live].all()
+    w[0, 0] = float("inf")
+    assert not kernels.split_weight_ok(w.to(DEV))

@@ -2,6 +2,7 @@
 // key/value store, SwiGLU.  The residual stream is float32 in both precisions;
 // "activation dtype" below is what matrix products read and write (bfloat16 in
 // the serving path, float32 in the true 32-bit path).
+#include "activation.cuh"
 #include "common.cuh"
 
 // ---------------------------------------------------------------------------
@@ -741,29 +742,9 @@ XR_EXPORT int xr_qk_norm_rope_store(const void* in, int dtype, long long ld_in, 
 }
 
 // ---------------------------------------------------------------------------
-// Activation of a feed-forward: gated, h = act(g) * u with g, u the two halves of each row of gu [n, 2F]
+// Activation of a feed-forward (activation.cuh): gated, h = act(g) * u with g, u the two halves of each row of gu [n, 2F]
 // (src/model.c:4425-4452, `gated_act`); ungated, h = act(x) of x [n, F] (src/model.c:6380-6396).
-// act 1: SiLU, g / (1 + exp(-g)), 0 for g < -80 (src/model.c:4451-4452; the reference's kernel is
-// src/kernels.cu:2868-2874); act 2: tanh-GELU, 0.5 g (1 + tanh(0.7978845608 (g + 0.044715 g^3)))
-// (src/model.c:4438-4441); act 4: the square of relu; act 0: none.  Full-precision expf and tanhf: this is the kernel of the true 32-bit path.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float xr_activation(int act, float g) {
-    if (act == 1) return g < -80.0f ? 0.0f : g / (1.0f + expf(-g));
-    if (act == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608f * (g + 0.044715f * g * g * g)));
-    if (act == 4) { const float r = fmaxf(g, 0.f); return r * r; }
-    return g;
-}
-
-// act 3 (gated only): with g' = min(g, limit) and u' = u clamped to [-limit, limit], h = g' sigmoid(1.702 g') (u' + 1).
-__device__ __forceinline__ float xr_gate(int act, float limit, float g, float u) {
-    if (act == 3) {
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-    }
-    return xr_activation(act, g) * u;
-}
-
 template <typename T>
 __global__ void k_act_mul(const T* gu, T* h, int n, int F, int act, int gated, float limit) {       // (h may be gu: no __restrict__)
     xr_pdl_launch();

@@ -31,15 +31,11 @@
 // The reference multiplies bf16 weights with scalar FMA kernels (`k_mv_bf16`, `k_mv_bf16_b`,
 // src/kernels.cu:534-549; `k_gemvb_bf16_x4/_x8`, src/kernels.cu:2814-2852) and adds the residual and
 // the activation in kernels of their own (`k_add` :2903, `k_silu_mul` :2868).
-#include "common.cuh"
-#include <cuda.h>
+#include "tc_product.cuh"
 
-#define TC_BM 128          // W rows per CTA (the M of the instruction)
-#define TC_BK 64           // K elements per stage: 128 bytes, one swizzle atom
 #define TC_THREADS 320       // producer warp, MMA warp, eight epilogue warps
 // a tile of 16 tokens is one chunk of accumulator columns: four epilogue warps are all it can use
 __host__ __device__ constexpr int tc_threads(int bn) { return bn <= 16 ? 192 : TC_THREADS; }
-#define XR_SPIN_LIMIT (1u << 24)
 
 #define TC_EPI_STORE 0     // out[t][r] = acc (+ bias), bfloat16 or float32
 #define TC_EPI_ADD 1       // out[t][r] += acc (+ bias), float32 residual stream
@@ -51,72 +47,6 @@ __host__ __device__ constexpr int tc_threads(int bn) { return bn <= 16 ? 192 : T
 #define TC_ACT_GELU_TANH 2
 #define TC_ACT_SWISH_CLAMP 3     // gated products only, see tc_gate
 #define TC_ACT_RELU2 4           // the square of relu
-
-// ---------------------------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded wait.  Returns false when it gave up (or another role already had).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-    for (uint32_t i = 0; i < XR_SPIN_LIMIT; i++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
-    }
-    *abort_flag = 1;
-    return false;
-}
-// One lane of a whole warp, the same one every time.  The copies', MMAs' and commits' operands live in registers that a warp shares:
-// behind this the compiler knows that one lane runs, behind `lane == 0` it does not and moves every operand over one by one.  Cycles a K
-// block of the pair kernel, `lane == 0` / elected: tiles of 64 and 128 tokens 620 / 323, of 256 tokens 620 / 512, which are the tensor
-// pipe's own; 2,048 x 4,096 x 4,096: 56 / 50 us.
-__device__ __forceinline__ bool tc_elect() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one != 0;
-}
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
-}
 
 // silu(g) = g / (1 + exp(-g)), 0 below -80 (src/model.c:4451-4452), with the hardware's approximate exp2 and
 // reciprocal: their error (about 2^-22) disappears in the bfloat16 rounding of the result, and an epilogue that
@@ -150,22 +80,6 @@ __device__ __forceinline__ float tc_gate(int act, float limit, float g, float u)
         return __fdividef(g, 1.0f + __expf(-1.702f * g)) * (u + 1.0f);
     }
     return tc_act(act, g) * u;
-}
-
-// K-major operand tile in shared memory, rows of 128 bytes, 128-byte swizzle, groups of 8 rows 1024 bytes
-// apart: start address and offsets in 16-byte units, descriptor version 1 (bit 46), layout type 2 (bits 61-63).
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;                 // leading byte offset (unused with a swizzled K-major tile)
-    d |= (uint64_t)(1024 >> 4) << 32;       // stride byte offset: 8 rows
-    d |= (uint64_t)1 << 46;                 // descriptor version
-    d |= (uint64_t)2 << 61;                 // SWIZZLE_128B
-    return d;
-}
-// kind::f16 instruction descriptor: D float32, A and B bfloat16, both K-major, M = 128, N = bn.
-__host__ __device__ constexpr uint32_t instr_desc(int bn) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
 
 struct TcParams {
@@ -442,16 +356,6 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
 // the end keeps a CTA from leaving while its partner may still signal it.  grid = 2 x clusters, cluster
 // (2, 1, 1); a tile is (token tile, pair of row tiles), CTA `rank` of the pair owns row tile 2 x pair + rank.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t tc_cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ void tc_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t tc_map_to_rank(uint32_t saddr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
 // copy into this CTA's shared memory, completion counted on a barrier that may be the partner's
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar_cluster_addr) {
     asm volatile(
@@ -697,38 +601,6 @@ __global__ void k_splitk_finish(FinishParams p) {
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                  const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void* ptr = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)ptr;
-    }
-    return fn;
-}
-
-// [rows, K] bfloat16, row stride `ld` elements; box = 64 (K) x box_rows; 128-byte swizzle; zero fill outside.
-static bool make_map(CUtensorMap* m, const void* base, long long rows, long long K, long long ld, int box_rows) {
-    EncodeTiledFn enc = get_encode();
-    if (!enc) return false;
-    const XrMapKey key{base, {(unsigned long long)K, (unsigned long long)rows, 0}, {(unsigned long long)ld * 2, 0}, {TC_BK, (unsigned)box_rows, 0}, 2, 0};
-    return xr_cached_map(m, key, [&](CUtensorMap* out) {
-        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-        cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-        cuuint32_t box[2] = {TC_BK, (cuuint32_t)box_rows};
-        cuuint32_t estr[2] = {1, 1};
-        return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    });
-}
-
 template <int BN, int STAGES, int MINB>
 static int launch_tc(const CUtensorMap& mw, const CUtensorMap& mx, const TcParams& p, dim3 grid, cudaStream_t stream) {
     constexpr int STAGE_BYTES = TC_BM * TC_BK * 2 + BN * TC_BK * 2;

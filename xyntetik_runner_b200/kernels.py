@@ -271,6 +271,41 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optiona
     _count()
 
 
+# The products in pieces round as a block of 64 values of k does in the tensor core, whatever K: 1.4 in units of 2^-24 of the result's size
+# at K 256, where the FMA kernel has 4.8.  Shorter sums, where the FMA kernel's error comes down to that and a product is a few
+# microseconds either way, stay with it.
+SPLIT_LEAST_K = 256
+
+
+def split_weight_ok(w: torch.Tensor) -> bool:
+    """Whether ``gemm_split`` multiplies by this matrix: bfloat16, every value finite, rows of at least SPLIT_LEAST_K values on 16-byte
+    borders."""
+    return (w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[1] >= SPLIT_LEAST_K
+            and w.data_ptr() % 16 == 0 and bool(torch.isfinite(w).all()))
+
+
+def split_rows_ok(x: torch.Tensor) -> bool:
+    return x.dtype == torch.float32 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, accumulate: bool = False,
+               alpha: float = 1.0, act: int = ACT_NONE, gated: bool = False, limit: float = 0.0) -> None:
+    """out[t][r] = act(alpha sum_k x[t][k] w[r][k] (+ bias[r])), or added to `out`, x and out float32, w as ``split_weight_ok`` takes it, in
+    float32's precision on the tensor cores: x as three exact bfloat16 pieces.  `gated`: w [2 F, K], out[t][f] = act(x.w[f]) * (x.w[F + f]).
+    A token's row is the same bits whatever other tokens are in the call.  Rows of x and out may be strided."""
+    for t in (x, w, out, bias):
+        if t is not None and not t.is_cuda:
+            raise KernelError("kernel arguments must be CUDA tensors")
+    n, k = x.shape
+    n_out = w.shape[0] // 2 if gated else w.shape[0]
+    assert w.shape == (n_out * (2 if gated else 1), k) and w.dtype == torch.bfloat16 and w.is_contiguous() and out.shape == (n, n_out)
+    assert x.dtype == torch.float32 and out.dtype == torch.float32 and x.stride(1) == 1 and out.stride(1) == 1
+    assert bias is None or (bias.dtype == torch.float32 and bias.numel() == n_out)
+    _check(_c.xr_gemm_split(x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), int(accumulate), int(gated), int(act), float(limit),
+                            float(alpha), n, n_out, k, x.stride(0), out.stride(0), workspace(out.device).status_ptr, _stream()), "gemm_split")
+    _count()
+
+
 def _check_bias(bias: Optional[torch.Tensor], H: int) -> None:
     _dev(bias)
     assert bias is None or (bias.dtype == torch.float32 and bias.dim() == 2 and bias.shape[0] == H and bias.shape[1] >= 1)

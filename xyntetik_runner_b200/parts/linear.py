@@ -2,9 +2,11 @@
 
 ``out[t][r] (+)= alpha sum_k x[t][k] W[r][k] (+ bias[r])``.  W keeps its stored dtype.  bfloat16 activations times
 a bfloat16 matrix go to the tensor-core kernel (tcgen05); for that the matrix is re-laid tile by tile when the
-part binds it (``prepare``), so that every tile the kernel streams is one contiguous read.  Everything else
--- the true 32-bit path above all -- goes to the float32 FMA kernel on the matrix as stored.  Which kernel
-ran is counted, so that a test can prove its subject ran.
+part binds it (``prepare``), so that every tile the kernel streams is one contiguous read.  The true 32-bit path's
+float32 activations times a bfloat16 matrix of some length go to the tensor cores too, in three exact pieces
+(``kernels.gemm_split``).  Everything else goes to the float32 FMA kernel on the matrix as stored.  Which kernel
+ran is counted, so that a test can prove its subject ran.  The choice hangs on the matrix and on how rows lie in memory,
+not on how many there are: in 32 bit a token's row is the same bits whatever stands beside it.
 """
 from __future__ import annotations
 
@@ -15,7 +17,7 @@ import torch
 from .. import kernels
 from . import linear_tc
 
-counters = {"tcgen05": 0, "simt": 0, "deferred": 0}
+counters = {"tcgen05": 0, "simt": 0, "deferred": 0, "split": 0}
 
 
 class Linear:
@@ -28,6 +30,7 @@ class Linear:
         self.n_out, self.k = self.weight.shape
         self.halves = halves
         self.packed: Optional[torch.Tensor] = None
+        self.split = False                     # multiplied by kernels.gemm_split
         self._nbytes = self.weight.numel() * self.weight.element_size()
 
     def prepare(self, rt, keep_plain: bool = False) -> "Linear":
@@ -37,6 +40,8 @@ class Linear:
             self.packed = kernels.pack_weight(self.weight, self.halves)
             if not keep_plain:
                 self.weight = None
+        elif linear_tc.ENABLED and rt.act_dtype == torch.float32:
+            self.split = kernels.split_weight_ok(self.weight)
         return self
 
     def nbytes(self) -> int:
@@ -55,6 +60,10 @@ class Linear:
             if pending is not None:
                 counters["deferred"] += 1
             return pending
+        if self.split and out.dtype == torch.float32 and kernels.split_rows_ok(x):
+            kernels.gemm_split(x, self.weight, out, self.bias, accumulate, alpha, act)
+            counters["split"] += 1
+            return None
         kernels.gemm_simt(x, self.weight, out, self.bias, accumulate, alpha)
         if act != kernels.ACT_NONE:
             kernels.act_mul(out, out, act, gated=False)
@@ -62,7 +71,7 @@ class Linear:
         return None
 
     def gated_fused(self) -> bool:
-        return self.halves == 2 and self.packed is not None
+        return self.halves == 2 and (self.packed is not None or self.split)
 
     def forward_gated(self, x: torch.Tensor, out: torch.Tensor, act: int = kernels.ACT_SILU,
                       scratch: Optional[torch.Tensor] = None, limit: float = 0.0) -> None:
@@ -73,6 +82,10 @@ class Linear:
         if self.packed is not None:
             kernels.gemm_tc(x, self.packed, out, None, kernels.EPI_GATED, packed_rows=self.n_out // 2, act=act, act_limit=limit)
             counters["tcgen05"] += 1
+            return
+        if self.split and (scratch is None or kernels.split_rows_ok(x)):
+            kernels.gemm_split(x, self.weight, out, act=act, gated=True, limit=limit)
+            counters["split"] += 1
             return
         assert scratch is not None and scratch.shape == (x.shape[0], self.n_out)
         kernels.gemm_simt(x, self.weight, scratch, None, False)
