@@ -71,3 +71,34 @@ def test_values_that_are_no_numbers_and_the_smallest():
     assert ((out.cpu().double() - fma.cpu().double()).abs() <= bound)[live].all()
     w[0, 0] = float("inf")
     assert not kernels.split_weight_ok(w.to(DEV))
+
+
+@pytest.mark.parametrize("n,R,B", [(63, 512, 2), (64, 768, 3), (65, 2560, 10), (200, 1320, 5), (777, 576, 2)])
+def test_recurrences_gates_in_pieces(n, R, B):
+    """The gates' products on the tensor cores beside the FMA kernel's: the recurrence's outputs and state from both, against float64."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + R)
+    Bs, taps = R // B, 4
+    dev = lambda t: t.to(DEV)
+    proj = dev(torch.randn(n, 2 * R, generator=g))
+    conv_w, conv_b = dev(torch.randn(R, taps, generator=g) * 0.5), dev(torch.randn(R, generator=g) * 0.1)
+    both = dev((torch.randn(2 * R, Bs, generator=g) * Bs ** -0.5).to(torch.bfloat16))
+    wa, wi = (both[i * R:(i + 1) * R].float().reshape(B, Bs, Bs).contiguous() for i in range(2))
+    ba, bi, lam = (dev(torch.randn(R, generator=g) * 0.5 - s) for s in (0.0, 0.0, 4.0))
+    ints = lambda *v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    seg = torch.zeros(n, dtype=torch.int32, device=DEV)
+    got = []
+    for gates in (None, both):
+        state = torch.zeros(1, kernels.rglru_state_floats(R, taps), device=DEV)
+        a, b, u, p = torch.empty(n, R, device=DEV), torch.empty(n, R, device=DEV), torch.empty(n, R, device=DEV), proj.clone()
+        out = torch.empty(n, R, device=DEV)
+        kernels.rglru(p, conv_w, conv_b, None, None, wa, wi, ba, bi, lam, state, seg, ints(0), ints(n), ints(0), a, b, u, out, 1, R, B, taps, 8.0, gates)
+        ud = u.double().view(n, B, Bs)
+        r, i = (torch.sigmoid(torch.einsum("tbi,boi->tbo", ud, w.double()).reshape(n, R) + c.double()) for w, c in ((wa, ba), (wi, bi)))
+        la = -8.0 * r * torch.nn.functional.softplus(lam.double())
+        want = torch.exp(la), torch.sqrt(-torch.expm1(2.0 * la)) * i * u.double()
+        got.append([float((x.double() - y).square().mean().sqrt()) for x, y in zip((a, b), want)] + [out, state, p])
+    for off, fma in zip(got[1][:2], got[0][:2]):
+        assert off <= 1.02 * fma + 1e-9
+    for x, y in zip(got[1][2:], got[0][2:]):
+        assert (x - y).abs().max() <= 2e-5 * y.abs().max()

@@ -32,6 +32,7 @@
 #include "simt_tile.cuh"
 #include "conv_tail.cuh"
 #include "chunked.cuh"
+#include "split_product.cuh"
 #include <math.h>
 
 #define RG_MAX_TAPS 16
@@ -114,6 +115,35 @@ static int launch_rglru_gates(float* proj, long long ldp, int y_col, const float
     xr_launch((k_rglru_gates<WM, WN, TM, TN>), grid, dim3(32 * WM * WN), SMEM, stream, proj, ldp, y_col, u, wa, wi, ba, bi, lam, a_s, b_s, n, R, Bs, c, vec);
     return XR_OK;
 }
+
+// The same on the tensor cores in float32's precision (split_product.cuh), where the matrices are bfloat16: rows of Wa and of Wi for the
+// same 64 outputs make a tile.  A block of 256 channels is four blocks of k: what a tile costs is its start and its end, not its product.
+// The whole part (convolution, gates, scan), us, FMA / tensor cores: 2,560 channels in ten blocks 32 tokens 20 / 21, 64 25 / 21, 128 33 / 27,
+// 512 72 / 43, 1,901 235 / 117; 1,280 in five 64 21 / 19, 512 48 / 31, 1,901 130 / 76.  Hence from 64 tokens on.
+__device__ __noinline__ float3 rg_finish_one(float ra, float ri, float u, float rate, float y) {       // (not inlined: see the end of k_split_product)
+    float3 v;
+    v.z = y;
+    rg_finish(ra, ri, u, rate, &v.x, &v.y, &v.z);
+    return v;
+}
+struct GateFinish {
+    float* proj; long long ldp;            // the gated branch's first column
+    const float* u; const float* ba; const float* bi; const float* lam;
+    float* a_out; float* b_out;
+    int R;
+    float c;
+    struct Row { float rate, a, i; };
+    using Pre = float2;                    // u, the gated branch
+    __device__ __forceinline__ Row row(int ch) const { return {-c * rc_softplus(lam[ch]), ba[ch], bi[ch]}; }
+    __device__ __forceinline__ Pre pre(int t, int ch) const { return make_float2(xr_ld_now(u + (size_t)t * R + ch), xr_ld_now(proj + (size_t)t * ldp + ch)); }
+    __device__ __forceinline__ void put(int t, int ch, float ra, float ri, Row w, Pre q) const {
+        const size_t at = (size_t)t * R + ch;
+        const float3 v = rg_finish_one(ra + w.a, ri + w.i, q.x, w.rate, q.y);
+        a_out[at] = v.x;
+        b_out[at] = v.y;
+        proj[(size_t)t * ldp + ch] = v.z;
+    }
+};
 
 // The convolution alone, a thread an element: u [n][R].  Ahead of k_rglru_gates_few, whose many small blocks would each compute
 // the whole tile again behind a chain of dependent loads.
@@ -339,11 +369,11 @@ k_rglru_scan_segments(const float* __restrict__ proj, long long ldp, int y_col, 
 
 // proj [n][ldp] float32: the gated branch's pre-activations at y_col, the convolution's inputs at x_col, R columns each.
 // conv_w [R][taps], conv_b [R]; wa, wi [B][R/B (out)][R/B (in)] as stored; ba, bi,
-// lam [R]; all float32.
+// lam [R]; all float32.  gates: null, or the same matrices as bfloat16, all of wa's and then all of wi's, where they are exactly that.
 // state [slots][state_stride] float32: S [R], tail [taps-1][R].  a_s, b_s, u_s [n][R] float32 scratch.  out [n][R] dtype `dtype`.
-XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
+XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const void* gates, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
                        const int* tok_seg, const int* seg_start, const int* seg_len, const int* seg_slot, float* a_s, float* b_s, float* u_s, void* out,
-                       int dtype, int n, int n_seg, int R, int B, int taps, float c, cudaStream_t stream) {
+                       int dtype, int n, int n_seg, int R, int B, int taps, float c, int* status, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || R < 1 || B < 1 || R % B || taps < 1 || taps > RG_MAX_TAPS || n_seg > 65535 || B > 65535 ||
         state_stride < (long long)R * taps)
         return XR_ERR_ARG;
@@ -369,6 +399,10 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
         const int groups = (Bs + 7) / 8;
         xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, proj, ldp, y_col, wa, wi, ba, bi, lam, a_s, b_s,
                   n, R, Bs, c, groups, (const float*)u_s);
+    } else if (gates != nullptr && n >= 64 && split_takes(u_s, n, R, gates, Bs)) {
+        SplitParams p{u_s, R, n, Bs, Bs, R, 0, status};
+        const int rc = run_split<true>(gates, 2LL * R, p, GateFinish{proj + y_col, ldp, u_s, ba, bi, lam, a_s, b_s, R, c}, B, stream);
+        if (rc != XR_OK) return rc;
     } else {
         int rc;
         // enough tiles of 64 tokens x 32 outputs to fill the machine twice, else of 16 x 16.  The whole part (convolution, gates, scan) at 2,560

@@ -1293,11 +1293,13 @@ def rglru_state_floats(R: int, taps: int) -> int:
 
 
 def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, state: torch.Tensor, tok_seg, seg_start, seg_len, seg_slot,
-          a_s: torch.Tensor, b_s: torch.Tensor, u_s: torch.Tensor, out: torch.Tensor, n_seg: int, R: int, B: int, taps: int, c: float) -> None:
+          a_s: torch.Tensor, b_s: torch.Tensor, u_s: torch.Tensor, out: torch.Tensor, n_seg: int, R: int, B: int, taps: int, c: float,
+          gates: Optional[torch.Tensor] = None) -> None:
     """The real-gated linear recurrent unit over the step's tokens, request by request, from and into `state`.  proj [n, >= 2R]
     float32 (rows may be strided): the gated branch's pre-activations in columns [0, R), the convolution's inputs in [R, 2R).
     out [n, R] = S * gelu_tanh(gated branch).  wa, wi: the gates' matrices [B, out, in]; wa_t, wi_t: the same transposed to
-    [B, in, out], or None (no kernel reads them).  See csrc/recurrent.cu for the other arguments."""
+    [B, in, out], or None (no kernel reads them).  `gates`: both matrices once more as bfloat16 [2 R, in], wa's rows first, where they are
+    exactly that (``split_weight_ok``).  See csrc/recurrent.cu for the other arguments."""
     _dev(conv_w, conv_b, wa, wi, ba, bi, lam, state, tok_seg, seg_start, seg_len, seg_slot, a_s, b_s, u_s, out)
     n = proj.shape[0]
     Bs = R // B
@@ -1306,10 +1308,11 @@ def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, s
     assert all(t.dtype == torch.float32 for t in (conv_w, conv_b, wa, wi, ba, bi, lam, state, a_s, b_s))
     assert conv_w.shape == (R, taps) and all(t.shape == (B, Bs, Bs) for t in (wa, wi)) and a_s.numel() >= n * R and b_s.numel() >= n * R
     assert state.dim() == 2 and state.shape[1] >= rglru_state_floats(R, taps)
+    assert gates is None or (gates.is_cuda and gates.is_contiguous() and gates.dtype == torch.bfloat16 and gates.shape == (2 * R, Bs))
     _check(_c.xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(),
-                          wa.data_ptr(), wi.data_ptr(), ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
+                          wa.data_ptr(), wi.data_ptr(), _ptr(gates), ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
                           seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), u_s.data_ptr(), out.data_ptr(),
-                          dtype_code(out.dtype), n, n_seg, R, B, taps, float(c), _stream()), "rglru")
+                          dtype_code(out.dtype), n, n_seg, R, B, taps, float(c), workspace(out.device).status_ptr, _stream()), "rglru")
     _count(3)
 
 

@@ -59,6 +59,8 @@ class GatedLinearRecurrence(Mixer):
         del ws
         self.out = Linear(tensors[n["o"]]).prepare(rt)
         self.conv_w, self.conv_b = f32(n["conv"]), f32(n["conv"] + b)
+        both = torch.cat([tensors[n["ra"]], tensors[n["ri"]]]).reshape(2 * self.R, -1)
+        self.gates = both if kernels.split_weight_ok(both) else None
         self.wa, self.wi = f32(n["ra"]), f32(n["ri"])
         self.ba, self.bi, self.lam = f32(n["ra"] + b).reshape(-1), f32(n["ri"] + b).reshape(-1), f32(n["lam"])
         self._small = (self.wa.numel() + self.wi.numel() + self.conv_w.numel() + 4 * self.R) * 4
@@ -76,7 +78,7 @@ class GatedLinearRecurrence(Mixer):
         u_s = ctx.buf("rglru_u", (n, R), torch.float32)
         y = ctx.buf("rglru_out", (n, R), ctx.act_dtype)
         kernels.rglru(proj, self.conv_w, self.conv_b, None, None, self.wa, self.wi, self.ba, self.bi, self.lam, lay.state, ctx.tok_seg,
-                      ctx.seg_start, ctx.seg_len, ctx.seg_slot, a_s, b_s, u_s, y, ctx.n_seg, R, self.B, self.taps, self.rate)
+                      ctx.seg_start, ctx.seg_len, ctx.seg_slot, a_s, b_s, u_s, y, ctx.n_seg, R, self.B, self.taps, self.rate, self.gates)
         ctx.set_pending(x, self.out.forward(y, x, accumulate=True, defer=True))
 
 
