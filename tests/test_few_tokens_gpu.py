@@ -1,0 +1,82 @@
+"""Products of one token or two on CUDA cores (csrc/gemv.cuh): the entry points' other road for so few."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _close(got, want, size, k, dtype):
+    """A sum of k exact products rounded to float32 at every step, then once to `dtype`."""
+    bound = size * (k + 4) * 2.0 ** -24 + (want.abs() * 2.0 ** -8 if dtype == torch.bfloat16 else 0.0) + 1e-6
+    assert ((got.double().cpu() - want).abs() <= bound).all()
+
+
+# rows off a unit's 8 (4 features) and a tile's 128, K off its blocks of 64, one block, fewer than warps, more than are held ahead, more units than
+# are walked at once
+@pytest.mark.parametrize("n", [1, 2, 3])
+@pytest.mark.parametrize("n_out,k", [(1, 8), (7, 72), (130, 64), (129, 1000), (2048, 1024), (500, 4096), (96, 2504), (300, 4104), (28411, 64), (20003, 320)])
+def test_products_of_a_few_tokens(n, n_out, k):
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n * 31 + n_out + k)
+    x = torch.randn(n, k, generator=g).to(torch.bfloat16)
+    wide = torch.full((n, k + 8), float("nan"), dtype=torch.bfloat16, device=DEV)      # (rows apart, what lies between is nobody's)
+    wide[:, :k] = x.to(DEV)
+    xd = wide[:, :k]
+    w = (torch.randn(n_out, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+    bias = torch.randn(n_out, generator=g)
+    packed = kernels.pack_weight(w.to(DEV))
+    torch.cuda.synchronize()                    # (weights are at rest when a product is launched)
+    want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.empty(n, n_out, dtype=dtype, device=DEV)
+        kernels.gemm_tc(xd, packed, out, bias.to(DEV), packed_rows=n_out, alpha=-0.5)
+        _close(out, -0.5 * want + bias.double(), size + bias.double().abs(), k, dtype)
+        kernels.gemm_tc(xd, packed, out, None, packed_rows=n_out, act=kernels.ACT_RELU2)
+        _close(out, want.clamp(min=0) ** 2, 2 * size * size + size, k, dtype)
+    base = torch.randn(n, n_out + 3, generator=g)
+    acc = base.to(DEV)[:, :n_out]
+    kernels.gemm_tc(xd, packed, acc, bias.to(DEV), kernels.EPI_ADD, packed_rows=n_out)
+    _close(acc, base[:, :n_out].double() + want + bias.double(), size + base[:, :n_out].double().abs() + bias.double().abs(), k, torch.float32)
+    # left to the next kernel
+    x0 = torch.randn(n, n_out, generator=g)
+    rows = x0.to(DEV)
+    sums = kernels.gemm_tc_deferred(xd, packed, rows, bias.to(DEV), kernels.EPI_ADD, packed_rows=n_out)
+    if sums is not None:                         # (None: the product was not left to anyone)
+        assert torch.equal(rows.cpu(), x0)
+        kernels.finish_plain(sums.partial, sums.splits, bias.to(DEV), rows, True)
+        sums.release()
+    _close(rows, x0.double() + want + bias.double(), size + x0.double().abs() + bias.double().abs(), k, torch.float32)
+    assert kernels.workspace(torch.device(DEV)).live == 0
+    # gated: gate rows, then up rows
+    F = (n_out + 1) // 2
+    pair = (torch.randn(2 * F, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+    gate, up = (x.double() @ pair[i * F:(i + 1) * F].double().T for i in range(2))
+    out = torch.empty(n, F, dtype=torch.bfloat16, device=DEV)
+    both = kernels.pack_weight(pair.to(DEV), 2)
+    torch.cuda.synchronize()
+    kernels.gemm_tc(xd, both, out, None, kernels.EPI_GATED, packed_rows=F)
+    ref = torch.nn.functional.silu(gate) * up
+    assert ((out.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5 * (gate.abs() + 1) * (up.abs() + 1)).all()
+
+
+@pytest.mark.parametrize("n,E,top,width,inner", [(1, 16, 2, 1024, 1408), (2, 64, 6, 264, 72), (2, 5, 3, 136, 200), (1, 12, 1, 64, 128)])
+def test_experts_products_of_a_few_tokens(n, E, top, width, inner):
+    """The rows of the first tiles alone, every one by its tile's matrix, against plain products; other rows stay as they are."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + E)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)])
+    used = sorted(set(ids.reshape(-1).tolist()))
+    tiles, bn = len(used) + 2, 16
+    group = torch.tensor(used + [-1, -1], dtype=torch.int32, device=DEV)
+    x = torch.randn(tiles * bn, width, generator=g).to(torch.bfloat16)
+    up = (torch.randn(E, inner, width, generator=g) * width ** -0.5).to(torch.bfloat16)
+    out = torch.full((tiles * bn, inner), 7.0, device=DEV)
+    packed = kernels.pack_weight_groups(up.to(DEV))
+    torch.cuda.synchronize()
+    kernels.gemm_tc_grouped(x.to(DEV), packed, out, group, bn, inner, kernels.EPI_STORE, kernels.ACT_RELU2, live_rows=n, live_tiles=n * top)
+    got = out.cpu().double().view(tiles, bn, inner)
+    for t, e in enumerate(used):
+        want = (x.view(tiles, bn, width)[t, :n].double() @ up[e].double().T).clamp(min=0) ** 2
+        assert ((got[t, :n] - want).abs() <= 1e-4 * (want + 1)).all()
+    assert (got[:, n:] == 7).all() and (got[len(used):] == 7).all()

@@ -108,6 +108,8 @@ struct TcParams {
     const int* tiles = nullptr;
 };
 
+#include "gemv.cuh"
+
 // ---------------------------------------------------------------------------------------------
 // Epilogue of one tile (`bn` tokens from tok0 on, those from n_end on do not exist), run by warps 2..9 once the accumulator is complete.  A warp may only read the 32
 // tensor-memory lanes of its index mod 4, so two warps share each quarter and take alternate 16-column
@@ -800,6 +802,15 @@ XR_EXPORT int xr_gemm_tc(const void* X, const void* W, const float* bias, void* 
     const bool gated = epilogue == TC_EPI_GATED;
     if (act != TC_ACT_NONE && act != TC_ACT_SILU && act != TC_ACT_GELU_TANH && act != TC_ACT_RELU2 && !(act == TC_ACT_SWISH_CLAMP && gated)) return XR_ERR_ARG;
     if (gated && (!w_packed || bias != nullptr || alpha != 1.0f)) return XR_ERR_ARG;
+    if (w_packed && force_splits == 0 && gemv_takes(n, K, 2LL * K * n_out * (gated ? 2 : 1), false)) {
+        // (float32 that is stored is what the sum would be: nothing is left for the caller's next kernel)
+        const bool defer = defer_finish && !gated && (epilogue == TC_EPI_ADD || out_dtype == XR_BF16) && scratch != nullptr && scratch_floats >= (long long)n * n_out;
+        if (splits_used) *splits_used = defer ? GV_DEFERRED : 1;
+        TcParams p{out, bias, scratch, status, ldo, n, n_out, K, 1, defer ? TC_EPI_PARTIAL : epilogue, out_dtype, act, act_limit, gated ? 1 : 0, 0, 1,
+                   (K + TC_BK - 1) / TC_BK, 1, 0};
+        p.alpha = alpha;
+        return launch_gemv(X, W, ldx, p, 1, stream);
+    }
     const TcPlan pl = plan_product(n, n_out, K, gated, force_splits, defer_finish != 0, scratch ? scratch_floats : 0);
     CUtensorMap mw, mx;
     const int rows_padded = gated ? (int)pl.rows : (n_out + TC_BM - 1) / TC_BM * TC_BM;
@@ -845,10 +856,11 @@ XR_EXPORT int xr_gemm_tc(const void* X, const void* W, const float* bias, void* 
 // and rows of X sorted by the matrix they meet, every group's rows starting at a multiple of `bn` (16, 32, 64 or 128):
 // token tile t of X multiplies by matrix tile_group[t] (an int per tile, on the device; below zero: no rows).  n is the
 // number of rows of X and out that the plan may use (a multiple of bn).  Store and gated epilogues; never cut along K.
+// live_rows, live_tiles (0: not known): only the first tiles can have a matrix, and of theirs only the first rows are looked at.
 // ---------------------------------------------------------------------------------------------
 XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit,
                                  int n, int n_out, int K, long long ldx, long long ldo, int bn, const int* tile_group, int groups,
-                                 int* status, cudaStream_t stream) {
+                                 int live_rows, int live_tiles, int* status, cudaStream_t stream) {
     if (n < 1 || n_out < 1 || K < 8 || (K % 8) != 0 || (ldx % 8) != 0 || ldx < K || ldo < n_out || groups < 1) return XR_ERR_ARG;
     if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || tile_group == nullptr) return XR_ERR_ARG;
     if (bn != 16 && bn != 32 && bn != 64 && bn != 128) return XR_ERR_ARG;
@@ -860,7 +872,12 @@ XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int ou
     const int row_tiles = gated ? (n_out + 63) / 64 : (n_out + TC_BM - 1) / TC_BM;
     const int total_kb = (K + TC_BK - 1) / TC_BK;
     const int tok_tiles = n / bn;
-    if (row_tiles > 65535) return XR_ERR_ARG;
+    if (row_tiles > 65535 || live_rows < 0 || live_rows > bn || live_tiles < 0) return XR_ERR_ARG;
+    if (live_rows > 0 && live_tiles > 0 && gemv_takes(live_rows, K, 2LL * K * n_out * (gated ? 2 : 1) * (live_tiles < tok_tiles ? live_tiles : tok_tiles), true)) {
+        TcParams p{out, nullptr, nullptr, status, ldo, live_rows, n_out, K, 1, epilogue, out_dtype, act, act_limit, gated ? 1 : 0, bn, 1, total_kb, 1, 0,
+                   tile_group, row_tiles};
+        return launch_gemv(X, W, ldx, p, live_tiles < tok_tiles ? live_tiles : tok_tiles, stream);
+    }
     CUtensorMap mw, mx;
     if (!make_map(&mw, W, (long long)groups * row_tiles * TC_BM * total_kb, TC_BK, TC_BK, TC_BM)) return -3;
     if (!make_map(&mx, X, n, K, ldx, bn)) return -3;

@@ -531,6 +531,9 @@ class PartialSums:
 
 
 
+ONE_DEFERRED = 1 << 16          # xr_gemm_tc's answer where it left one slice of sums, not cut, to the caller's next kernel
+
+
 def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, act_limit=0.0, alpha=1.0):
     # (called once or several times a layer: shapes and strides are asked for once)
     n, k = x.shape
@@ -558,6 +561,8 @@ def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, a
     if splits < 0:
         _check(splits, "gemm_tc")
     _count(1 if (splits == 1 or defer) else 2)
+    if splits == ONE_DEFERRED:
+        return PartialSums(ws, ws.take(n * n_out), 1)
     if defer and splits > 1:
         rows = tiles * TILE_ROWS if (gated and packed_rows is not None) else n_out
         return PartialSums(ws, ws.take(splits * n * rows), splits)
@@ -578,7 +583,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[
 def gemm_tc_deferred(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
                      epilogue: int = EPI_STORE, force_splits: int = 0, packed_rows: Optional[int] = None,
                      alpha: float = 1.0) -> Optional[PartialSums]:
-    """The same product, its sum left to the caller when it was cut along K: returns ``PartialSums`` ([splits][n][n_out]
+    """The same product, its sum left to the caller when it was cut along K (or, for a few tokens, all the same): returns ``PartialSums`` ([splits][n][n_out]
     float32 in a slab of the workspace, `alpha` applied; `out` is NOT written, and the bias not added) for the caller's next kernel
     (``finish_*``) to sum, then ``release()``.  Returns None when the product was not cut: `out` is complete."""
     r = _gemm_tc(x, w, out, bias, epilogue, ACT_NONE, force_splits, True, packed_rows, 0.0, alpha)
@@ -1164,9 +1169,10 @@ def pack_weight_groups(w: torch.Tensor, halves: int = 1) -> torch.Tensor:
 
 
 def gemm_tc_grouped(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, tile_group: torch.Tensor, bn: int, n_out: int,
-                    epilogue: int = EPI_STORE, act: int = ACT_NONE, act_limit: float = 0.0) -> None:
-    """bfloat16 product on tcgen05 of rows sorted by group: tile t of `bn` rows of x multiplies by matrix
-    tile_group[t] of w_packed (from ``pack_weight_groups``); tiles with tile_group below zero are skipped.
+                    epilogue: int = EPI_STORE, act: int = ACT_NONE, act_limit: float = 0.0, live_rows: int = 0, live_tiles: int = 0) -> None:
+    """bfloat16 product of rows sorted by group: tile t of `bn` rows of x multiplies by matrix
+    tile_group[t] of w_packed (from ``pack_weight_groups``); tiles with tile_group below zero are skipped.  With `live_rows` and
+    `live_tiles` only the first tiles may have a group and only their first rows are anybody's: other rows of `out` may stay as they are.
     EPI_STORE: out[r] = x[r] . w^T; EPI_GATED (halves = 2 packing): out[r][f] = gate_act(x . w_gate[f], x . w_up[f])."""
     _dev(x, w_packed, out, tile_group)
     n, k = x.shape
@@ -1177,7 +1183,7 @@ def gemm_tc_grouped(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, 
     ws = workspace(x.device)
     _check(_c.xr_gemm_tc_grouped(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
                                     float(act_limit), n, n_out, k, x.stride(0), out.stride(0), bn, tile_group.data_ptr(),
-                                    w_packed.shape[0], ws.status_ptr, _stream()), "gemm_tc_grouped")
+                                    w_packed.shape[0], int(live_rows), int(live_tiles), ws.status_ptr, _stream()), "gemm_tc_grouped")
     _count()
 
 

@@ -209,9 +209,10 @@ class RoutedExperts(FeedForward):
                                           self.act, self.limit)
             kernels.gemm_tc_grouped_pairs(y, self.w_down, zz, tiles, max_tiles, self.width)
         elif self.tensor_cores:
+            live = dict(live_rows=n, live_tiles=pairs) if n <= align else {}          # (an expert meets a token once; used tiles come first)
             kernels.gemm_tc_grouped(xs, self.w_gate_up, y, tile_group, align, self.inner, kernels.EPI_GATED if self.gated else kernels.EPI_STORE,
-                                    self.act, self.limit)
-            kernels.gemm_tc_grouped(y, self.w_down, zz, tile_group, align, self.width)
+                                    self.act, self.limit, **live)
+            kernels.gemm_tc_grouped(y, self.w_down, zz, tile_group, align, self.width, **live)
         else:
             kernels.moe_gemm(h, self.w_gate_up, y, row_src, tile_group, top, self.gated, self.act, self.limit, gather=True)
             kernels.moe_gemm(y, self.w_down, zz, row_src, tile_group, top, False)
