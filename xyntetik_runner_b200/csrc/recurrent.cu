@@ -371,7 +371,7 @@ k_rglru_scan_segments(const float* __restrict__ proj, long long ldp, int y_col, 
 // conv_w [R][taps], conv_b [R]; wa, wi [B][R/B (out)][R/B (in)] as stored; ba, bi,
 // lam [R]; all float32.  gates: null, or the same matrices as bfloat16, all of wa's and then all of wi's, where they are exactly that.
 // state [slots][state_stride] float32: S [R], tail [taps-1][R].  a_s, b_s, u_s [n][R] float32 scratch.  out [n][R] dtype `dtype`.
-XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const void* gates, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
+static int run_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const void* gates, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
                        const int* tok_seg, const int* seg_start, const int* seg_len, const int* seg_slot, float* a_s, float* b_s, float* u_s, void* out,
                        int dtype, int n, int n_seg, int R, int B, int taps, float c, int* status, cudaStream_t stream) {
     if (n < 1 || n_seg < 1 || R < 1 || B < 1 || R % B || taps < 1 || taps > RG_MAX_TAPS || n_seg > 65535 || B > 65535 ||
@@ -439,6 +439,20 @@ XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const f
                   state_stride, seg_start, seg_len, seg_slot, (__nv_bfloat16*)out, R, taps);
     else return XR_ERR_ARG;
     return xr_launch_status();
+}
+XR_EXPORT int xr_rglru(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
+                       const int* tok_seg, const int* seg_start, const int* seg_len, const int* seg_slot, float* a_s, float* b_s, float* u_s, void* out,
+                       int dtype, int n, int n_seg, int R, int B, int taps, float c, cudaStream_t stream) {
+    return run_rglru(proj, ldp, y_col, x_col, conv_w, conv_b, wa, wi, nullptr, ba, bi, lam, state, state_stride, tok_seg, seg_start, seg_len, seg_slot, a_s, b_s, u_s,
+                     out, dtype, n, n_seg, R, B, taps, c, nullptr, stream);
+}
+// The same with the matrices as bfloat16 too, and the word that a wait which gave up is written to.
+XR_EXPORT int xr_rglru_gates(float* proj, long long ldp, int y_col, int x_col, const float* conv_w, const float* conv_b, const float* wa, const float* wi, const void* gates, const float* ba, const float* bi, const float* lam, float* state, long long state_stride,
+                             const int* tok_seg, const int* seg_start, const int* seg_len, const int* seg_slot, float* a_s, float* b_s, float* u_s, void* out,
+                             int dtype, int n, int n_seg, int R, int B, int taps, float c, int* status, cudaStream_t stream) {
+    if (gates == nullptr || status == nullptr) return XR_ERR_ARG;
+    return run_rglru(proj, ldp, y_col, x_col, conv_w, conv_b, wa, wi, gates, ba, bi, lam, state, state_stride, tok_seg, seg_start, seg_len, seg_slot, a_s, b_s, u_s,
+                     out, dtype, n, n_seg, R, B, taps, c, status, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

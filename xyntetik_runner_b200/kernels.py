@@ -1315,10 +1315,14 @@ def rglru(proj: torch.Tensor, conv_w, conv_b, wa_t, wi_t, wa, wi, ba, bi, lam, s
     assert conv_w.shape == (R, taps) and all(t.shape == (B, Bs, Bs) for t in (wa, wi)) and a_s.numel() >= n * R and b_s.numel() >= n * R
     assert state.dim() == 2 and state.shape[1] >= rglru_state_floats(R, taps)
     assert gates is None or (gates.is_cuda and gates.is_contiguous() and gates.dtype == torch.bfloat16 and gates.shape == (2 * R, Bs))
-    _check(_c.xr_rglru(proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(),
-                          wa.data_ptr(), wi.data_ptr(), _ptr(gates), ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
-                          seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), u_s.data_ptr(), out.data_ptr(),
-                          dtype_code(out.dtype), n, n_seg, R, B, taps, float(c), workspace(out.device).status_ptr, _stream()), "rglru")
+    head = (proj.data_ptr(), proj.stride(0), 0, R, conv_w.data_ptr(), conv_b.data_ptr(), wa.data_ptr(), wi.data_ptr())
+    tail = (ba.data_ptr(), bi.data_ptr(), lam.data_ptr(), state.data_ptr(), state.stride(0), tok_seg.data_ptr(),
+            seg_start.data_ptr(), seg_len.data_ptr(), seg_slot.data_ptr(), a_s.data_ptr(), b_s.data_ptr(), u_s.data_ptr(), out.data_ptr(),
+            dtype_code(out.dtype), n, n_seg, R, B, taps, float(c))
+    if gates is None:
+        _check(_c.xr_rglru(*head, *tail, _stream()), "rglru")
+    else:
+        _check(_c.xr_rglru_gates(*head, gates.data_ptr(), *tail, workspace(out.device).status_ptr, _stream()), "rglru")
     _count(3)
 
 
