@@ -80,3 +80,30 @@ def test_experts_products_of_a_few_tokens(n, E, top, width, inner):
         want = (x.view(tiles, bn, width)[t, :n].double() @ up[e].double().T).clamp(min=0) ** 2
         assert ((got[t, :n] - want).abs() <= 1e-4 * (want + 1)).all()
     assert (got[:, n:] == 7).all() and (got[len(used):] == 7).all()
+
+
+@pytest.mark.parametrize("n,ctx,chunk,page,skew", [(1, 33, 128, 8, 0), (3, 700, 128, 8, 0), (2, 1030, 512, 16, 2), (40, 300, 128, 64, 0), (9, 2000, 128, 64, 0), (1, 2100, 2112, 8, 0)])
+def test_latent_attention_by_stages_and_pages(n, ctx, chunk, page, skew):
+    """Both depths of the ring (every CTA an SM to itself or not), more pages a split than are kept in shared memory, queries off 16-byte borders, tiles
+    that end early; against float64 of the same bfloat16 numbers.  Probabilities are rounded to bfloat16: 2^-8 of the values' size."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + ctx)
+    H, C, R = 16, 128, 32
+    W, mp = C + R, -(-ctx // page)
+    cache = torch.randn(n * mp + 1, page, W, generator=g).to(torch.bfloat16)
+    bt = torch.arange(n * mp).reshape(n, mp).flip(1).contiguous()
+    pos = torch.tensor([max(0, ctx - 1 - 17 * (i % 5)) for i in range(n)])
+    wide = torch.randn(n, H * R + 8, generator=g).to(torch.bfloat16)
+    ql = torch.randn(n, H * C, generator=g).to(torch.bfloat16)
+    splits = -(-ctx // chunk)
+    dev = lambda t, d=torch.int32: t.to(d).to(DEV)
+    out = torch.full((n, H * C), float("nan"), device=DEV)
+    po, pm = torch.empty(n * splits * 16 * C, device=DEV), torch.empty(n * splits * 32, device=DEV)
+    cd = cache.to(DEV)
+    kernels.latent_attention_mma(ql.to(DEV), wide.to(DEV), skew, R, out, po, pm, cd.data_ptr(), page * W, dev(pos), dev(torch.arange(n)), dev(bt), H, C, R, mp, page,
+                                 0.1, chunk, splits)
+    for t in range(n):
+        rows = torch.cat([cache[b] for b in bt[t]])[:int(pos[t]) + 1].double()
+        q = torch.cat([ql[t].view(H, C), wide[t, skew:skew + H * R].view(H, R)], 1).double()
+        want = torch.softmax(0.1 * q @ rows.T, -1) @ rows[:, :C]
+        assert (out[t].cpu().double().view(H, C) - want).abs().max() <= 2.0 ** -7 * rows[:, :C].abs().max()

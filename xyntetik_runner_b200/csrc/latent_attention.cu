@@ -294,7 +294,11 @@ XR_EXPORT int xr_latent_attention(const float* ql, const void* qr, int dtype, lo
 // are multiples of 64 up to 512 and rotated parts that are multiples of 8.
 //
 // A CTA of four warps takes one token and up to sixteen of its heads (the rows of the M = 16 tile: all heads read the
-// same cached rows) over a range of keys, in tiles of 32 keys that cp.async brings to shared memory two deep.
+// same cached rows) over a range of keys, in tiles of 32 keys that cp.async brings to shared memory, LT_DEEP stages of them where every
+// CTA has an SM to itself (a split's 128 keys are then all on their way at once), else two.
+// What bounds it: a split is a chain of trips to L2.  So all that needs no result of this step, the zeros and the split's pages, comes
+// before the wait, and queries and keys are copied side by side.  8 tokens, 16 heads, 512 + 64 columns, context 2,000, a launch inside a
+// step: 32.1 -> 18.4 us, the same bits.
 //   scores   S [16 x 32] = Q [16 x Wp] K^T: warp w takes keys 8w .. 8w + 7 of the tile (Wp = C + R rounded up to 16,
 //            the padding zero on both sides); the scores go to shared memory, times `scale`, keys beyond the range -inf;
 //   softmax  every warp reads S in the layout of the A operand (rows g and g + 8, g = lane / 4), keeps the running
@@ -307,6 +311,8 @@ XR_EXPORT int xr_latent_attention(const float* ql, const void* qr, int dtype, lo
 // ---------------------------------------------------------------------------------------------
 #define LT_KT 32
 #define LT_NW 4
+#define LT_DEEP 4
+#define LT_PAGES 64          // a split's pages that are kept in shared memory
 #define LT_MAX_NT 16         // n8 tiles of O per warp: C / 4 / 8 <= 16, so C <= 512
 
 __device__ __forceinline__ uint32_t lt_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -334,6 +340,7 @@ __device__ __forceinline__ uint32_t lt_pack(float a, float b) {
 // reads lie in different banks
 static __host__ __device__ inline int lt_row_bytes(int Wp) { int u = Wp / 8; return ((u & 1) ? u : u + 1) * 16; }
 
+template <int S>
 __global__ void __launch_bounds__(32 * LT_NW)
 k_latent_attention_mma(const __nv_bfloat16* __restrict__ ql, long long ql_tok, long long ql_head,
                        const __nv_bfloat16* __restrict__ qr, long long ld_qr, int head_qr,
@@ -341,13 +348,14 @@ k_latent_attention_mma(const __nv_bfloat16* __restrict__ ql, long long ql_tok, l
                        float* __restrict__ part_o, float* __restrict__ part_ml,
                        const __nv_bfloat16* __restrict__ cache, long long page_stride, const int* __restrict__ positions,
                        const int* __restrict__ tok_seg, const int* __restrict__ block_tables, int H, int C, int R, int max_pages,
-                       int page_size, float scale, int chunk, int splits, int window) {
+                       int page_size, float scale, int chunk, int splits, int window, int vec) {
     xr_pdl_launch();
     extern __shared__ __align__(16) uint8_t lt_sm[];
+    __shared__ int kept_pages[LT_PAGES];
     const int W = C + R, Wp = (W + 15) / 16 * 16, rb = lt_row_bytes(Wp);
     uint8_t* Qs = lt_sm;                                   // [16][rb]
-    uint8_t* Ks = Qs + 16 * rb;                            // [2][32][rb]
-    float* Ss = reinterpret_cast<float*>(Ks + 2 * LT_KT * rb);   // [16][33]
+    uint8_t* Ks = Qs + 16 * rb;                            // [S][32][rb]
+    float* Ss = reinterpret_cast<float*>(Ks + S * LT_KT * rb);   // [16][33]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int t = blockIdx.x, h0 = blockIdx.y * 16, split = blockIdx.z;
     const int pos = positions[t];
@@ -357,38 +365,53 @@ k_latent_attention_mma(const __nv_bfloat16* __restrict__ ql, long long ql_tok, l
     const int mt = gridDim.y;
     float* my_ml = part_ml + (((size_t)t * mt + blockIdx.y) * splits + split) * 32;
     float* my_o = part_o + (((size_t)t * mt + blockIdx.y) * splits + split) * 16 * (size_t)C;
-    xr_pdl_wait();
     if (kend <= kbeg) {                                    // nothing for this split (only with splits > 1)
+        xr_pdl_wait();
         if (threadIdx.x < 16) { my_ml[threadIdx.x * 2] = -INFINITY; my_ml[threadIdx.x * 2 + 1] = 0.f; }
         return;
     }
+    const int page0 = kbeg / page_size, n_pages = (kend - 1) / page_size - page0 + 1;
+    const bool kept = n_pages <= LT_PAGES;
+    if (kept) for (int i = threadIdx.x; i < n_pages; i += blockDim.x) kept_pages[i] = bt[page0 + i];
     // zeros everywhere first: the padding columns stay zero, and rows that a last, partial tile leaves alone hold
     // finite values (a weight of zero times them must be zero)
-    for (int i = threadIdx.x; i < (16 + 2 * LT_KT) * rb / 16; i += blockDim.x) reinterpret_cast<uint4*>(lt_sm)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = threadIdx.x; i < (16 + S * LT_KT) * rb / 16; i += blockDim.x) reinterpret_cast<uint4*>(lt_sm)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
+    xr_pdl_wait();
     const int n_tiles = (kend - kbeg + LT_KT - 1) / LT_KT;
     const int chunks16 = W / 8;                            // 16-byte pieces of a cached row
     auto fetch = [&](int tile, int buf) {
         // a warp per key (its page and row worked out once), the lanes over the row's 16-byte pieces
         const int k0 = kbeg + tile * LT_KT, cnt = min(LT_KT, kend - k0);
         for (int j = warp; j < cnt; j += LT_NW) {
-            const int kp = k0 + j;
-            const __nv_bfloat16* src = cache + (size_t)bt[kp / page_size] * page_stride + (size_t)(kp % page_size) * W;
+            const int kp = k0 + j, pg = kp / page_size;
+            const __nv_bfloat16* src = cache + (size_t)(kept ? kept_pages[pg - page0] : bt[pg]) * page_stride + (size_t)(kp - pg * page_size) * W;
             const uint32_t dst = lt_smem(Ks + ((size_t)buf * LT_KT + j) * rb);
             for (int piece = lane; piece < chunks16; piece += 32) lt_cp16(dst + piece * 16, src + piece * 8);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0, 0);
-    // the queries: [latent part | rotated part] of heads h0 .. h0 + 15 (rows of heads that do not exist stay zero)
-    for (int i = threadIdx.x; i < 16 * (W / 2); i += blockDim.x) {
-        const int r = i / (W / 2), e = (i % (W / 2)) * 2, h = h0 + r;
-        if (h >= H) continue;
-        uint32_t v;
-        if (e < C) v = *reinterpret_cast<const uint32_t*>(ql + (size_t)t * ql_tok + (size_t)h * ql_head + e);
-        else v = *reinterpret_cast<const uint32_t*>(qr + (size_t)t * ld_qr + (size_t)h * head_qr + (e - C));
-        *reinterpret_cast<uint32_t*>(Qs + (size_t)r * rb + e * 2) = v;
+    // the queries: [latent part | rotated part] of heads h0 .. h0 + 15 (rows of heads that do not exist stay zero); with the first tile
+    if (vec) {
+        for (int i = threadIdx.x; i < 16 * chunks16; i += blockDim.x) {
+            const int r = i / chunks16, e = (i % chunks16) * 8, h = h0 + r;
+            if (h < H) lt_cp16(lt_smem(Qs + (size_t)r * rb + e * 2), e < C ? ql + (size_t)t * ql_tok + (size_t)h * ql_head + e : qr + (size_t)t * ld_qr + (size_t)h * head_qr + (e - C));
+        }
     }
+#pragma unroll
+    for (int i = 0; i < S - 1; i++) {
+        if (i < n_tiles) fetch(i, i);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (!vec)
+        for (int i = threadIdx.x; i < 16 * (W / 2); i += blockDim.x) {
+            const int r = i / (W / 2), e = (i % (W / 2)) * 2, h = h0 + r;
+            if (h >= H) continue;
+            uint32_t v;
+            if (e < C) v = *reinterpret_cast<const uint32_t*>(ql + (size_t)t * ql_tok + (size_t)h * ql_head + e);
+            else v = *reinterpret_cast<const uint32_t*>(qr + (size_t)t * ld_qr + (size_t)h * head_qr + (e - C));
+            *reinterpret_cast<uint32_t*>(Qs + (size_t)r * rb + e * 2) = v;
+        }
     const int DW = C / LT_NW, NT = DW / 8;                 // this warp's columns of O and their n8 tiles
     float acc[LT_MAX_NT][4];
 #pragma unroll
@@ -396,13 +419,10 @@ k_latent_attention_mma(const __nv_bfloat16* __restrict__ ql, long long ql_tok, l
     float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;       // rows g and g + 8
     const uint32_t q_addr = lt_smem(Qs) + (lane & 15) * rb + (lane >> 4) * 16;
     for (int tile = 0; tile < n_tiles; tile++) {
-        const int buf = tile & 1;
-        if (tile + 1 < n_tiles) {
-            fetch(tile + 1, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
+        const int buf = tile % S;
+        if (tile + S - 1 < n_tiles) fetch(tile + S - 1, (tile + S - 1) % S);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(S - 1) : "memory");
         __syncthreads();
         const uint32_t k_base = lt_smem(Ks + (size_t)buf * LT_KT * rb);
         // ---- scores of keys 8 warp .. 8 warp + 7
@@ -489,7 +509,7 @@ k_latent_attention_mma(const __nv_bfloat16* __restrict__ ql, long long ql_tok, l
                 }
             }
         }
-        __syncthreads();                                   // S and this buffer are free for the tile after next
+        __syncthreads();                                   // the scores and this buffer are free
     }
     // ---- results
     if (splits == 1) {
@@ -606,13 +626,20 @@ XR_EXPORT int xr_latent_attention_mma(const void* ql, long long ql_tok, long lon
     if ((ql_tok | ql_head | oh_tok | oh_head) & 1) return XR_ERR_ARG;            // pairs of bfloat16 are read and written
     if (splits > 65535 || (H + 15) / 16 > 65535) return XR_ERR_ARG;
     const int Wp = (C + R + 15) / 16 * 16;
-    const size_t smem = (size_t)(16 + 2 * LT_KT) * lt_row_bytes(Wp) + 16 * 33 * sizeof(float);
-    static bool ready[XR_DEVICES];
-    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_latent_attention_mma, 200 * 1024); })) return XR_ERR_LAUNCH;
     const int mt = (H + 15) / 16;
-    xr_launch(k_latent_attention_mma, dim3(n, mt, splits), dim3(32 * LT_NW), smem, stream, (const __nv_bfloat16*)ql, ql_tok, ql_head,
-              (const __nv_bfloat16*)qr, ld_qr, head_qr, out, (__nv_bfloat16*)out_h, oh_tok, oh_head, part_o, part_ml, (const __nv_bfloat16*)cache, page_stride, positions, tok_seg, block_tables, H, C, R,
-              max_pages, page_size, scale, chunk, splits, window);
+    auto smem_of = [&](int stages) { return (size_t)(16 + stages * LT_KT) * lt_row_bytes(Wp) + 16 * 33 * sizeof(float); };
+    static bool ready[XR_DEVICES];
+    if (!xr_once_per_device(ready, [] { return xr_allow_smem(k_latent_attention_mma<2>, 200 * 1024) && xr_allow_smem(k_latent_attention_mma<LT_DEEP>, 200 * 1024); }))
+        return XR_ERR_LAUNCH;
+    // (queries by 16-byte copies: addresses and distances of eight values)
+    const int vec = !(((uintptr_t)ql | (uintptr_t)qr) & 15) && !((ql_tok | ql_head | ld_qr | head_qr) & 7);
+    const bool deep = (long long)n * mt * splits <= xr_sm_count() && smem_of(LT_DEEP) <= 200 * 1024;
+#define LT(S) xr_launch((k_latent_attention_mma<S>), dim3(n, mt, splits), dim3(32 * LT_NW), smem_of(S), stream, (const __nv_bfloat16*)ql, ql_tok, ql_head,             \
+              (const __nv_bfloat16*)qr, ld_qr, head_qr, out, (__nv_bfloat16*)out_h, oh_tok, oh_head, part_o, part_ml, (const __nv_bfloat16*)cache, page_stride, positions, tok_seg, \
+              block_tables, H, C, R, max_pages, page_size, scale, chunk, splits, window, vec)
+    if (deep) LT(LT_DEEP);
+    else LT(2);
+#undef LT
     if (splits > 1) {
         xr_launch(k_latent_merge, dim3((unsigned)n * (unsigned)H), dim3(128), 0, stream, (const float*)part_o, (const float*)part_ml, out, (__nv_bfloat16*)out_h, oh_tok, oh_head, n, H, C, mt, splits);
     }
