@@ -107,3 +107,31 @@ def test_latent_attention_by_stages_and_pages(n, ctx, chunk, page, skew):
         q = torch.cat([ql[t].view(H, C), wide[t, skew:skew + H * R].view(H, R)], 1).double()
         want = torch.softmax(0.1 * q @ rows.T, -1) @ rows[:, :C]
         assert (out[t].cpu().double().view(H, C) - want).abs().max() <= 2.0 ** -7 * rows[:, :C].abs().max()
+
+
+@pytest.mark.parametrize("n,top,E", [(1, 1, 3), (300, 6, 64), (4096, 4, 7), (4097, 4, 16), (6000, 6, 64)])
+def test_plan_of_many_pairs(n, top, E):
+    """Pairs around and beyond what a thread keeps (16,384 in all), rows of identity experts among them: every pair has a row of its own among its
+    expert's, the tiles cover every expert's rows, and the gather brings every row its token, rows of four blocks and a remainder."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + E)
+    ids = torch.stack([torch.randperm(E + 2, generator=g)[:top] for _ in range(n)]).int()
+    pairs = n * top
+    max_tiles, rows = kernels.moe_tiles_room(pairs, E)
+    row_src, pair_row, tiles = (torch.full((m,), -7, dtype=torch.int32, device=DEV) for m in (rows, pairs, 1 + 3 * max_tiles))
+    kernels.moe_plan_tiles(ids.to(DEV), row_src, pair_row, tiles, E)
+    src, at, table = row_src.cpu(), pair_row.cpu().long(), tiles.cpu()
+    flat = ids.reshape(-1).long()
+    real = flat < E
+    assert (at[~real] == -1).all() and at[real].unique().numel() == int(real.sum())
+    assert torch.equal(src[at[real]].long(), torch.arange(pairs)[real]) and int((src >= 0).sum()) == int(real.sum())
+    owner = torch.full((rows,), -1, dtype=torch.long)
+    for e, first, count in table[1:1 + 3 * int(table[0])].view(-1, 3).tolist():
+        assert (owner[first:first + count] == -1).all()
+        owner[first:first + count] = e
+    assert torch.equal(owner[at[real]], flat[real]) and int((owner >= 0).sum()) == int(real.sum())
+    h = torch.randn(n, 40, generator=g).to(torch.bfloat16)
+    xs = torch.full((rows, 40), 7.0, dtype=torch.bfloat16, device=DEV)
+    kernels.moe_gather(h.to(DEV), xs, row_src, None, top)
+    want = torch.where((src >= 0)[:, None], h[src.clamp(min=0).long() // top], torch.tensor(7.0, dtype=torch.bfloat16))
+    assert torch.equal(xs.cpu(), want)
