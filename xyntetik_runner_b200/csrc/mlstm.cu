@@ -292,6 +292,70 @@ k_mlstm_out(const float* __restrict__ o, const TG* __restrict__ proj, long long 
         dst[i] = xr_from_f32<T>(src[i] * inv * (w != nullptr ? w[(size_t)h * w_head + i] : 1.0f) * gate);
     }
 }
+// The same with a head's values, gates and weights in a warp's registers, four columns an access (PER accesses a lane), all on their way at once:
+// heads of up to 512 values, a multiple of four, on borders of an access.  2,048 tokens, 8 heads of 256, inside a step: 17.4 -> 9.8 us (gates in bfloat16), 20.3
+// -> 10.5 (in float32).
+__device__ __forceinline__ float4 ml_read4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 ml_read4(const __nv_bfloat16* p) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
+__device__ __forceinline__ void ml_write4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void ml_write4(__nv_bfloat16* p, float4 v) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+}
+template <typename T, typename TG, int PER>
+__global__ void __launch_bounds__(128)
+k_mlstm_out_vec(const float* __restrict__ o, const TG* __restrict__ proj, long long ldp, int g_col, const float* __restrict__ w,
+                T* __restrict__ y, int n, int H, int V, float eps, int w_head, int gate_silu) {
+    xr_pdl_launch();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long idx = (long long)blockIdx.x * 4 + warp;
+    xr_pdl_wait();
+    if (idx >= (long long)n * H) return;
+    const int t = (int)(idx / H), h = (int)(idx % H);
+    const float* src = o + ((size_t)t * H + h) * V;
+    const TG* g = proj + (size_t)t * ldp + g_col + (size_t)h * V;
+    T* dst = y + (size_t)t * H * V + (size_t)h * V;
+    float4 x[PER], z[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int i = 4 * (lane + 32 * k);
+        x[k] = z[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (i < V) { x[k] = ml_read4(src + i); z[k] = ml_read4(g + i); }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < PER; k++) { ss = fmaf(x[k].x, x[k].x, ss); ss = fmaf(x[k].y, x[k].y, ss); ss = fmaf(x[k].z, x[k].z, ss); ss = fmaf(x[k].w, x[k].w, ss); }
+    ss = xr_warp_sum(ss);
+    const float inv = 1.0f / sqrtf(ss / (float)V + eps);
+    auto one = [&](float v, float z, float wt) {
+        float gate = 1.0f / (1.0f + expf(-z));
+        if (gate_silu) gate *= z;
+        return v * inv * wt * gate;
+    };
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int i = 4 * (lane + 32 * k);
+        if (i >= V) continue;
+        const float4 wt = w != nullptr ? ml_read4(w + (size_t)h * w_head + i) : make_float4(1.f, 1.f, 1.f, 1.f);
+        ml_write4(dst + i, make_float4(one(x[k].x, z[k].x, wt.x), one(x[k].y, z[k].y, wt.y), one(x[k].z, z[k].z, wt.z), one(x[k].w, z[k].w, wt.w)));
+    }
+}
+template <typename T, typename TG>
+static void launch_mlstm_out(const float* o, const TG* proj, long long ldp, int g_col, const float* w, T* y, int n, int H, int V, float eps, int w_head, int gate_silu,
+                             cudaStream_t stream) {
+    const dim3 grid((unsigned)(((long long)n * H + 3) / 4)), block(128);
+    const bool vec = V <= 512 && !((V | g_col | w_head) & 3) && ldp % 4 == 0 && !(((uintptr_t)o | (uintptr_t)w) & 15) && !((uintptr_t)proj & (4 * sizeof(TG) - 1)) &&
+                     !((uintptr_t)y & (4 * sizeof(T) - 1));
+#define MO(PER) xr_launch((k_mlstm_out_vec<T, TG, PER>), grid, block, 0, stream, o, proj, ldp, g_col, w, y, n, H, V, eps, w_head, gate_silu)
+    if (vec && V <= 128) MO(1);
+    else if (vec && V <= 256) MO(2);
+    else if (vec) MO(4);
+    else xr_launch((k_mlstm_out<T, TG>), grid, block, 0, stream, o, proj, ldp, g_col, w, y, n, H, V, eps, w_head, gate_silu);
+#undef MO
+}
 
 // ---------------------------------------------------------------------------------------------
 // Portions of many tokens go through the recurrence in chunks (chunked.cuh), with  a_t = f  and  s_t = i  in logarithms:
@@ -299,6 +363,7 @@ k_mlstm_out(const float* __restrict__ o, const TG* __restrict__ proj, long long 
 // m is a running maximum of sums, m_t = max(m_(t-1) + lf_t, li_t): a block per (head, portion), a thread a run of tokens; a run is
 // the map m -> max(m + A, B), the runs' maps are joined over the block, then every thread walks its run from its own start.
 // ---------------------------------------------------------------------------------------------
+#define ML_RUN 8
 __global__ void __launch_bounds__(256)
 k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, float* __restrict__ log_f, float* __restrict__ in_scale,
                 float* __restrict__ floor_n, const int* __restrict__ seg_start, const int* __restrict__ seg_len, const int* __restrict__ seg_slot,
@@ -310,17 +375,41 @@ k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, floa
     const int per = (len + 255) / 256, i0 = min(len, tid * per), i1 = min(len, i0 + per);
     float* m_at = state + ((size_t)seg_slot[seg] * H + h) * ml_state_head(D, V) + (size_t)D * V + D;
     xr_pdl_wait();
+    if (len <= 0) return;
     const float m0 = *m_at;
     auto logs = [&](int i, float& li, float& lf) {
         const float* row = gates + (size_t)(start + i) * 2 * H + h;
         li = cap * tanhf(row[0] / cap);
         lf = ml_logsigmoid(cap * tanhf(row[H] / cap));
     };
+    // a run of up to ML_RUN tokens (portions of up to 2,048): both logarithms of all of them in registers, their loads on their way at once and the
+    // functions taken once.  8 heads, 2,048 tokens inside a step, 18 to 24 -> 11.8 us.
+    float lis[ML_RUN], lfs[ML_RUN];
+    const bool held = per <= ML_RUN;
+    if (held) {
+#pragma unroll
+        for (int k = 0; k < ML_RUN; k++) {
+            const float* row = gates + (size_t)(start + min(i0 + k, len - 1)) * 2 * H + h;
+            lis[k] = xr_ld_now(row); lfs[k] = xr_ld_now(row + H);
+        }
+#pragma unroll
+        for (int k = 0; k < ML_RUN; k++) { xr_ld_fence(lis[k]); xr_ld_fence(lfs[k]); }
+#pragma unroll
+        for (int k = 0; k < ML_RUN; k++)
+            if (i0 + k < i1) { lis[k] = cap * tanhf(lis[k] / cap); lfs[k] = ml_logsigmoid(cap * tanhf(lfs[k] / cap)); }
+    }
     float A = 0.f, B = -INFINITY;
-    for (int i = i0; i < i1; i++) {
-        float li, lf;
-        logs(i, li, lf);
-        B = fmaxf(B + lf, li); A += lf;
+    auto join = [&](float li, float lf) { B = fmaxf(B + lf, li); A += lf; };
+    if (held) {
+#pragma unroll
+        for (int k = 0; k < ML_RUN; k++)
+            if (i0 + k < i1) join(lis[k], lfs[k]);
+    } else {
+        for (int i = i0; i < i1; i++) {
+            float li, lf;
+            logs(i, li, lf);
+            join(li, lf);
+        }
     }
     sa[tid] = A; sb[tid] = B;
     __syncthreads();
@@ -332,15 +421,24 @@ k_mlstm_scalars(const float* __restrict__ gates, float* __restrict__ state, floa
         __syncthreads();
     }
     float m = tid == 0 ? m0 : fmaxf(m0 + sa[tid - 1], sb[tid - 1]), first_m = 0.f, first_lf = 0.f;
-    for (int i = i0; i < i1; i++) {
-        float li, lf;
-        logs(i, li, lf);
+    auto token = [&](int i, float li, float lf) {
         const float m_new = fmaxf(lf + m, li);
         const size_t at = (size_t)(start + i) * H + h;
         if (i == i0) { first_m = m_new; first_lf = lf; }
         else log_f[at] = ml_log_decay(lf + m - m_new);
         in_scale[at] = expf(li - m_new); floor_n[at] = expf(-m_new);
         m = m_new;
+    };
+    if (held) {
+#pragma unroll
+        for (int k = 0; k < ML_RUN; k++)
+            if (i0 + k < i1) token(i0 + k, lis[k], lfs[k]);
+    } else {
+        for (int i = i0; i < i1; i++) {
+            float li, lf;
+            logs(i, li, lf);
+            token(i, li, lf);
+        }
     }
     // a run's first decay leads over from the very m that the run before ended with (joined in another order, the sums differ in
     // their last bits, and S is kept relative to m)
@@ -365,6 +463,26 @@ k_mlstm_rows(const T* __restrict__ proj, long long ldp, int q_col, int k_col, in
         out[e] = c < HD ? xr_to_f32<T>(row[q_col + c]) * qs : (c < 2 * HD ? xr_to_f32<T>(row[k_col + c - HD]) : xr_to_f32<T>(row[v_col + c - 2 * HD]));
     }
 }
+// Eight columns a thread (grid: columns, tokens) of bfloat16 rows on 16-byte borders: without a division an element.  2,048 tokens of 4,096
+// columns inside a step, 23.9 -> 10.2 us.
+static __global__ void __launch_bounds__(256)
+k_mlstm_rows_vec(const __nv_bfloat16* __restrict__ proj, long long ldp, int q_col, int k_col, int v_col, float* __restrict__ out, int n, int HD, int HV, float qs) {
+    xr_pdl_launch();
+    const int cols = 2 * HD + HV, c = (blockIdx.x * 256 + threadIdx.x) * 8;
+    xr_pdl_wait();
+    if (c >= cols) return;
+    const int from = c < HD ? q_col + c : (c < 2 * HD ? k_col + c - HD : v_col + c - 2 * HD);
+    const float f = c < HD ? qs : 1.0f;
+    for (int t = blockIdx.y; t < n; t += gridDim.y) {
+        const uint4 u = *reinterpret_cast<const uint4*>(proj + (size_t)t * ldp + from);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        float4* dst = reinterpret_cast<float4*>(out + (size_t)t * cols + c);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            dst[i] = make_float4(__uint_as_float(w[2 * i] << 16) * f, __uint_as_float(w[2 * i] & 0xffff0000u) * f, __uint_as_float(w[2 * i + 1] << 16) * f,
+                                 __uint_as_float(w[2 * i + 1] & 0xffff0000u) * f);
+    }
+}
 
 template <typename T>
 static int mlstm_chunked(const T* proj, long long ldp, int q_col, int k_col, int v_col, const float* gates, float* state, float* o, const int* seg_start,
@@ -385,7 +503,10 @@ static int mlstm_chunked(const T* proj, long long ldp, int q_col, int k_col, int
     a.cum = cum;
     const size_t total = (size_t)n * cols;
     const int most = xr_sm_count() * 8, blocks = (int)((total + 255) / 256 < (size_t)most ? (total + 255) / 256 : most);
-    xr_launch((k_mlstm_rows<T>), dim3(blocks), dim3(256), 0, stream, proj, ldp, q_col, k_col, v_col, rows, n, HD, HV, 1.0f / sqrtf((float)D));
+    if (sizeof(T) == 2 && !((ldp | q_col | k_col | v_col | HD | HV) & 7) && !(((uintptr_t)proj | (uintptr_t)rows) & 15))
+        xr_launch(k_mlstm_rows_vec, dim3(((2 * HD + HV) / 8 + 255) / 256, n < 65535 ? n : 65535), dim3(256), 0, stream, (const __nv_bfloat16*)proj, ldp, q_col, k_col,
+                  v_col, rows, n, HD, HV, 1.0f / sqrtf((float)D));
+    else xr_launch((k_mlstm_rows<T>), dim3(blocks), dim3(256), 0, stream, proj, ldp, q_col, k_col, v_col, rows, n, HD, HV, 1.0f / sqrtf((float)D));
     xr_launch(k_mlstm_scalars, dim3(H, n_seg), dim3(256), 0, stream, gates, state, log_f, in_scale, floor_n, seg_start, seg_len, seg_slot, H, D, V, cap);
     xr_launch(ck_cumulate, dim3((H + 127) / 128, (unsigned)ck_chunks(n, n_seg)), dim3(128), 0, stream, (const float*)log_f, (long long)H, cum, H, a);
     return ck_run<CK_TOKEN, true>(a, n, D, stream);
@@ -408,8 +529,6 @@ XR_EXPORT int xr_mlstm(const void* proj, int dtype, long long ldp, int q_col, in
     const size_t smem_s = ((size_t)D * ML_VS + 2 * (size_t)ML_CHUNK * D + ML_CHUNK * ML_VS + ML_CHUNK * ML_RG * ML_VS + ML_CHUNK * 3) * sizeof(float);
     if (smem_g > 48 * 1024 || smem_s > 220 * 1024) return XR_ERR_ARG;
     dim3 gg(H, n_seg), gs((V + ML_VS - 1) / ML_VS, H, n_seg);
-    const long long warps = (long long)n * H;
-    const unsigned gb = (unsigned)((warps + 3) / 4);
 #define SCAN_ARGS(T) gs, dim3(ML_VS * ML_RG), 0, stream, (const T*)proj, ldp, q_col, k_col, v_col, (const float*)coef, state, o, seg_start, seg_len, seg_slot, H, D, V
 #define SCAN(T)                                                                                                                       \
     do {                                                                                                                              \
@@ -434,8 +553,7 @@ XR_EXPORT int xr_mlstm(const void* proj, int dtype, long long ldp, int q_col, in
                   seg_len, seg_slot, H, D, V, cap, stage);                                                                            \
         SCAN(T);                                                                                                                      \
         }                                                                                                                             \
-        xr_launch((k_mlstm_out<T>), dim3(gb), dim3(128), 0, stream, (const float*)o, (const T*)proj, ldp, g_col, norm_w, (T*)y, n, H, \
-                  V, eps, V, 0);                                                                                                         \
+        launch_mlstm_out<T, T>((const float*)o, (const T*)proj, ldp, g_col, norm_w, (T*)y, n, H, V, eps, V, 0, stream);               \
     } while (0)
     if (dtype == XR_F32) ML(float);
     else if (dtype == XR_BF16) ML(__nv_bfloat16);
@@ -452,15 +570,13 @@ XR_EXPORT int xr_mlstm(const void* proj, int dtype, long long ldp, int q_col, in
 XR_EXPORT int xr_head_norm_gate(const float* o, const void* gate, int gate_dtype, long long ld_gate, const float* w, int w_head, int gate_silu,
                                 void* y, int dtype, int n, int H, int V, float eps, cudaStream_t stream) {
     if (n < 1 || H < 1 || V < 1 || w_head < 0) return XR_ERR_ARG;
-    const long long warps = (long long)n * H;
-    const unsigned gb = (unsigned)((warps + 3) / 4);
     typedef __nv_bfloat16 bf;
     if (dtype == XR_F32 && gate_dtype == XR_F32)
-        xr_launch((k_mlstm_out<float, float>), dim3(gb), dim3(128), 0, stream, o, (const float*)gate, ld_gate, 0, w, (float*)y, n, H, V, eps, w_head, gate_silu);
+        launch_mlstm_out(o, (const float*)gate, ld_gate, 0, w, (float*)y, n, H, V, eps, w_head, gate_silu, stream);
     else if (dtype == XR_BF16 && gate_dtype == XR_BF16)
-        xr_launch((k_mlstm_out<bf, bf>), dim3(gb), dim3(128), 0, stream, o, (const bf*)gate, ld_gate, 0, w, (bf*)y, n, H, V, eps, w_head, gate_silu);
+        launch_mlstm_out(o, (const bf*)gate, ld_gate, 0, w, (bf*)y, n, H, V, eps, w_head, gate_silu, stream);
     else if (dtype == XR_BF16 && gate_dtype == XR_F32)
-        xr_launch((k_mlstm_out<bf, float>), dim3(gb), dim3(128), 0, stream, o, (const float*)gate, ld_gate, 0, w, (bf*)y, n, H, V, eps, w_head, gate_silu);
+        launch_mlstm_out(o, (const float*)gate, ld_gate, 0, w, (bf*)y, n, H, V, eps, w_head, gate_silu, stream);
     else return XR_ERR_ARG;
     return xr_launch_status();
 }

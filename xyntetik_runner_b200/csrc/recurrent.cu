@@ -485,6 +485,20 @@ struct KeyDecayArgs {
     float read_scale;            // factor on the read-outs (DS_HEAD too)
 };
 
+// A thread four columns of a row (grid: columns, rows), where rows lie on 16-byte borders: without a division an element, which bound the
+// kernel behind it: 1,901 tokens of 3,072 columns inside a step, 16.6 -> 7.9 us.
+__global__ void __launch_bounds__(256)
+k_silu_cols_vec(float* __restrict__ rows, long long ld, int quads, int n) {
+    xr_pdl_launch();
+    const int c = blockIdx.x * 256 + threadIdx.x;
+    xr_pdl_wait();
+    if (c >= quads) return;
+    for (int t = blockIdx.y; t < n; t += gridDim.y) {
+        float4* p = reinterpret_cast<float4*>(rows + (size_t)t * ld) + c;
+        const float4 v = *p;
+        *p = make_float4(rc_silu(v.x), rc_silu(v.y), rc_silu(v.z), rc_silu(v.w));
+    }
+}
 __global__ void k_silu_cols(float* __restrict__ rows, long long ld, int cols, size_t total) {
     xr_pdl_launch();
     xr_pdl_wait();
@@ -936,8 +950,10 @@ XR_EXPORT int xr_decay_attention(float* proj, long long ldp, int q_col, int k_co
     const bool many = silu && n > 16 && k_col == q_col + H * D && v_col == k_col + H * D;
     if (many) {
         const size_t total = (size_t)n * (2 * H * D + H * V);
-        const int blocks = (int)((total + 255) / 256 < (size_t)xr_sm_count() * 16 ? (total + 255) / 256 : xr_sm_count() * 16);
-        xr_launch(k_silu_cols, dim3(blocks), dim3(256), 0, stream, proj + q_col, ldp, 2 * H * D + H * V, total);
+        const int blocks = (int)((total + 255) / 256 < (size_t)xr_sm_count() * 16 ? (total + 255) / 256 : xr_sm_count() * 16), cols = 2 * H * D + H * V;
+        if (!((cols | ldp) & 3) && !((uintptr_t)(proj + q_col) & 15))
+            xr_launch(k_silu_cols_vec, dim3((cols / 4 + 255) / 256, n < 65535 ? n : 65535), dim3(256), 0, stream, proj + q_col, ldp, cols / 4, n);
+        else xr_launch(k_silu_cols, dim3(blocks), dim3(256), 0, stream, proj + q_col, ldp, 2 * H * D + H * V, total);
     }
     if (scratch != nullptr && ck_takes(D, V) && (many || !silu)) {
         ChunkArgs a{proj + q_col, proj + k_col, proj + v_col, ldp, ldp, ldp, H, V, decay, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, state,
