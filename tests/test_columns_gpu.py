@@ -30,3 +30,17 @@ def test_head_norm_gate(n, H, V, skip, dtype, gate_dtype, silu):
     want = (od / torch.sqrt((od * od).mean(-1, keepdim=True) + 1e-5)).view(n, -1) * w.double() * torch.sigmoid(z) * (z if silu else 1.0)
     # float32 sums of V squares and a few functions: 1e-5 of the value; stored once
     assert ((y.double().cpu() - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 1e-5) + 1e-6).all()
+
+
+@pytest.mark.parametrize("n,width,groups,skip", [(1, 4, 1, 0), (3, 512, 1, 0), (3, 516, 1, 0), (2, 2048, 1, 4), (777, 2048, 1, 0), (4, 2048, 4, 0), (2, 2048, 1, 1), (2, 8192, 1, 0), (2, 8196, 1, 0), (3, 30, 3, 0)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_silu_gate_norm(n, width, groups, skip, dtype):
+    """Groups of one and of four accesses a thread, wider ones, gates off the borders."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n + width)
+    o, gate, w = torch.randn(n, width, generator=g), torch.randn(n, width + 8, generator=g), 1 + 0.1 * torch.randn(width, generator=g)
+    y = torch.empty(n, width, dtype=dtype, device=DEV)
+    kernels.silu_gate_norm(o.to(DEV), gate.to(DEV), skip, w.to(DEV), y, groups, 1e-5)
+    z = (o.double() * torch.nn.functional.silu(gate[:, skip:skip + width].double())).view(n, groups, -1)
+    want = (z / torch.sqrt((z * z).mean(-1, keepdim=True) + 1e-5)).view(n, -1) * w.double()
+    assert ((y.double().cpu() - want).abs() <= want.abs() * (2.0 ** -8 if dtype == torch.bfloat16 else 1e-5) + 1e-6).all()
