@@ -135,3 +135,36 @@ def test_plan_of_many_pairs(n, top, E):
     kernels.moe_gather(h.to(DEV), xs, row_src, None, top)
     want = torch.where((src >= 0)[:, None], h[src.clamp(min=0).long() // top], torch.tensor(7.0, dtype=torch.bfloat16))
     assert torch.equal(xs.cpu(), want)
+
+
+def test_a_token_meets_an_expert_once():
+    """Scores that leave nothing to choose by (one token's are no numbers, or fewer outputs than are chosen have a finite correction): the choices
+    of a token still differ, so an expert has as many rows as there are tokens at most, and the other token's rows are all computed."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(4)
+    n, E, top, width, inner, align = 2, 12, 3, 64, 136, 16
+    z = torch.randn(n, E, generator=g)
+    z[0, 5], z[1, 0] = float("nan"), 6.0                        # (expert 0 is the other token's)
+    few = torch.full((E,), float("-inf"))
+    few[7] = 0.0
+    for correction in (None, few):
+        cd = None if correction is None else correction.to(DEV)
+        ids, w = torch.empty(n, top, dtype=torch.int32, device=DEV), torch.empty(n, top, device=DEV)
+        kernels.route_groups(z.to(DEV), ids, w, top, cd, 4, 2, 1.0)
+        assert all(len(set(r)) == top and 0 <= min(r) and max(r) < E for r in ids.tolist()), ids
+    h = torch.randn(n, width, generator=g).to(torch.bfloat16)
+    up = (torch.randn(E, inner, width, generator=g) * width ** -0.5).to(torch.bfloat16)
+    tiles = kernels.moe_max_tiles(n * top, E, align)
+    pair_row, group = (torch.full((m,), -7, dtype=torch.int32, device=DEV) for m in (n * top, tiles))
+    wts, xs = torch.empty(n, top, device=DEV), torch.zeros(tiles * align, width, dtype=torch.bfloat16, device=DEV)
+    zs = z.to(DEV)
+    kernels.route_few(zs, 1, zs, E, E, top, wts, pair_row, group, align, h.to(DEV), xs, 2, None, 4, 2, 1.0)
+    out = torch.full((tiles * align, inner), 7.0, device=DEV)
+    packed = kernels.pack_weight_groups(up.to(DEV))
+    torch.cuda.synchronize()
+    kernels.gemm_tc_grouped(xs, packed, out, group, align, inner, live_rows=n, live_tiles=n * top)
+    rows, of = pair_row.cpu().view(n, top)[1].tolist(), group.cpu()
+    assert int(of[rows[0] // align]) == 0
+    for r in rows:
+        want = h[1].double() @ up[int(of[r // align])].double().T
+        assert (out[r].cpu().double() - want).abs().max() <= 1e-4

@@ -126,8 +126,14 @@ __device__ __forceinline__ void route_groups_row(const float* row, float* c, int
         for (int e = lane; e < E; e += 32)
             if (c[e] > bv) { bv = c[e]; be = e; }
         route_argmax(bv, be);
-        if (be >= E) be = 0;                                       // (nothing left to choose: scores that are no numbers)
         if (lane == 0) {
+            // nothing left to choose by (scores that are no numbers, corrections of -inf): the lowest output that is not chosen yet, because an
+            // expert meets a token once at most (a grouped product of few tokens computes no more rows of a tile than there are tokens)
+            if (be >= E) {
+                be = 0;
+                for (int k = 0; k < j; k++)
+                    if (ids[k] == be) { be++; k = -1; }
+            }
             ids[j] = be;
             wts[j] = expf(row[be] - m) / sum * scale;
             c[be] = -INFINITY;
