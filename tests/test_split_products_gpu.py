@@ -102,3 +102,45 @@ def test_recurrences_gates_in_pieces(n, R, B):
         assert off <= 1.02 * fma + 1e-9
     for x, y in zip(got[1][2:], got[0][2:]):
         assert (x - y).abs().max() <= 2e-5 * y.abs().max()
+
+
+@pytest.mark.parametrize("R,B", [(512, 2), (1320, 5)])
+def test_a_recurrence_in_32_bits_cut_anywhere(R, B):
+    """The true 32-bit path with bfloat16 gate matrices, portions of more than sixteen tokens: outputs and state are the same bits whatever
+    portions a text is cut into (around every width of the products' token tiles, and the 64 tokens that serving steps go by) and whatever stands
+    beside one."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(R)
+    n, Bs, taps = 200, R // B, 4
+    dev = lambda t: t.to(DEV)
+    proj = dev(torch.randn(n, 2 * R, generator=g))
+    conv_w, conv_b = dev(torch.randn(R, taps, generator=g) * 0.5), dev(torch.randn(R, generator=g) * 0.1)
+    gates = dev((torch.randn(2 * R, Bs, generator=g) * Bs ** -0.5).to(torch.bfloat16))
+    assert kernels.split_weight_ok(gates)
+    wa, wi = (gates[i * R:(i + 1) * R].float().reshape(B, Bs, Bs).contiguous() for i in range(2))
+    ba, bi, lam = (dev(torch.randn(R, generator=g) * 0.5 - s) for s in (0.0, 0.0, 4.0))
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+
+    def step(rows, lengths, state):
+        m = rows.shape[0]
+        a, b, u, out = (torch.empty(m, R, device=DEV) for _ in range(4))
+        seg = ints([i for i, k in enumerate(lengths) for _ in range(k)])
+        starts = [sum(lengths[:i]) for i in range(len(lengths))]
+        kernels.rglru(rows.clone(), conv_w, conv_b, None, None, wa, wi, ba, bi, lam, state, seg, ints(starts), ints(lengths), ints(list(range(len(lengths)))), a, b, u, out,
+                      len(lengths), R, B, taps, 8.0, gates)
+        return out
+
+    def text(cuts):
+        state = torch.zeros(1, kernels.rglru_state_floats(R, taps), device=DEV)
+        outs, at = [], 0
+        for k in cuts:
+            outs.append(step(proj[at:at + k], [k], state))
+            at += k
+        return torch.cat(outs), state
+    whole, state = text([200])
+    for cuts in ([100, 100], [17, 63, 64, 56], [40, 33, 65, 62], [136, 32, 32]):
+        got, st = text(cuts)
+        assert torch.equal(got, whole) and torch.equal(st, state), cuts
+    two = torch.zeros(2, kernels.rglru_state_floats(R, taps), device=DEV)
+    beside = step(torch.cat([proj[:40], proj]), [40, 200], two)
+    assert torch.equal(beside[:40], whole[:40]) and torch.equal(beside[40:], whole) and torch.equal(two[1:], state)

@@ -119,7 +119,9 @@ static int launch_rglru_gates(float* proj, long long ldp, int y_col, const float
 // The same on the tensor cores in float32's precision (split_product.cuh), where the matrices are bfloat16: rows of Wa and of Wi for the
 // same 64 outputs make a tile.  A block of 256 channels is four blocks of k: what a tile costs is its start and its end, not its product.
 // The whole part (convolution, gates, scan), us, FMA / tensor cores: 2,560 channels in ten blocks 32 tokens 20 / 21, 64 25 / 21, 128 33 / 27,
-// 512 72 / 43, 1,901 235 / 117; 1,280 in five 64 21 / 19, 512 48 / 31, 1,901 130 / 76.  Hence from 64 tokens on.
+// 512 72 / 43, 1,901 235 / 117; 1,280 in five 64 21 / 19, 512 48 / 31, 1,901 130 / 76.  Hence from 64 tokens on, and in the true 32-bit path
+// from 17 on: which of the two a step takes would else hang on how a text is cut, and their last bits differ.  That costs nothing there, us, launches
+// back to back: 2,560 channels 17 tokens 21.1 / 11.7, 32 22.2 / 14.3, 63 24.5 / 17.1; 1,280 17 15.3 / 11.3, 63 23.0 / 15.2.
 __device__ __noinline__ float3 rg_finish_one(float ra, float ri, float u, float rate, float y) {       // (not inlined: see the end of k_split_product)
     float3 v;
     v.z = y;
@@ -399,7 +401,7 @@ static int run_rglru(float* proj, long long ldp, int y_col, int x_col, const flo
         const int groups = (Bs + 7) / 8;
         xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, proj, ldp, y_col, wa, wi, ba, bi, lam, a_s, b_s,
                   n, R, Bs, c, groups, (const float*)u_s);
-    } else if (gates != nullptr && n >= 64 && split_takes(u_s, n, R, gates, Bs)) {
+    } else if (gates != nullptr && (n >= 64 || dtype == XR_F32) && split_takes(u_s, n, R, gates, Bs)) {
         SplitParams p{u_s, R, n, Bs, Bs, R, 0, status};
         const int rc = run_split<true>(gates, 2LL * R, p, GateFinish{proj + y_col, ldp, u_s, ba, bi, lam, a_s, b_s, R, c}, B, stream);
         if (rc != XR_OK) return rc;
@@ -418,8 +420,8 @@ static int run_rglru(float* proj, long long ldp, int y_col, int x_col, const flo
     // Segments where the chain of a portion's tokens is what counts: portions of 64 tokens on average, and of 3 / 5 of a token for every block of
     // segments (two such blocks share an SM).  The whole part, us, segments / a thread a channel: 2,560 channels 1 x 64 tokens 30 / 30, 1 x 1,024
     // 146 / 206, 2 x 64 45 / 41, 2 x 256 89 / 99, 8 x 128 155 / 145, 8 x 512 507 / 516, 48 x 16 195 / 97; 1,024 channels 1 x 128 17 / 22, 4 x 96
-    // 27 / 29, 16 x 64 52 / 37, 16 x 256 130 / 132.  (The true 32-bit path promises the same bits however portions are cut: a thread a
-    // channel there.)
+    // 27 / 29, 16 x 64 52 / 37, 16 x 256 130 / 132.  (The true 32-bit path promises the same bits however portions of more than sixteen
+    // tokens are cut: a thread a channel there.)
     const long long seg_blocks = (long long)((R + 31) / 32) * n_seg;
     const bool segments = dtype == XR_BF16 && n >= 64LL * n_seg && 5LL * n >= 3 * seg_blocks * n_seg;
     if (segments)
