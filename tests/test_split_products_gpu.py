@@ -144,3 +144,24 @@ def test_a_recurrence_in_32_bits_cut_anywhere(R, B):
     two = torch.zeros(2, kernels.rglru_state_floats(R, taps), device=DEV)
     beside = step(torch.cat([proj[:40], proj]), [40, 200], two)
     assert torch.equal(beside[:40], whole[:40]) and torch.equal(beside[40:], whole) and torch.equal(two[1:], state)
+
+
+@pytest.mark.parametrize("n,n_out,k", [(1, 129, 1024), (3, 33, 2048), (20, 161, 4096), (40, 255, 2816), (70, 97, 512), (300, 1, 1024)])
+def test_rows_that_part_a_warp(n, n_out, k):
+    """Outputs that end inside a warp's 32, K in slices and whole, activations with branches that lanes take apart: what every warp does as one behind
+    them (the cluster's barrier, tensor memory's release) still comes to its end, twice over, with the same bits."""
+    from xyntetik_runner_b200 import kernels
+    x, w = _inputs(n, n_out, k)
+    x *= 60.0                                          # (SiLU below and above -80)
+    xd, wd = x.to(DEV), w.to(DEV)
+    want = x.double() @ w.double().T
+    bound = x.double().abs() @ w.double().abs().T * (k + 2) * 2.0 ** -24
+    for act, ref in ((kernels.ACT_SILU, torch.nn.functional.silu(want)), (kernels.ACT_RELU2, want.clamp(min=0) ** 2)):
+        out, again = (torch.empty(n, n_out, device=DEV) for _ in range(2))
+        kernels.gemm_split(xd, wd, out, act=act)
+        kernels.gemm_split(xd, wd, again, act=act)
+        # an error e of the sum: 1.1 e of SiLU (its largest slope), 2 |sum| e + e^2 of the square; functions and the last rounding 2^-20 of the value
+        slope = 1.1 * bound if act == kernels.ACT_SILU else 2 * want.abs() * bound + bound * bound
+        assert ((out.cpu().double() - ref).abs() <= slope + ref.abs() * 2.0 ** -20 + 1e-30).all()
+        assert torch.equal(out, again)
+    assert int(kernels.workspace(torch.device(DEV)).status.sum()) == 0

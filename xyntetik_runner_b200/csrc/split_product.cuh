@@ -181,7 +181,8 @@ k_split_product(const __grid_constant__ CUtensorMap map_w, SplitParams p, Epi ep
 #pragma unroll
         for (int c = 0; c < COLS; c++) acc[c] = 0.f;
         auto add = [&](int i) {            // block i's accumulator
-            if (!mbar_wait(&acc_full[i & 1], (i >> 1) & 1, abort_flag)) return false;
+            // (a lane may see the barrier's end ahead of others, and tcgen05.ld is for a warp that has come together)
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[i & 1], (i >> 1) & 1, abort_flag))) return false;
             tc_fence_after();
             float v[COLS];
             sp_ld<COLS>(taddr + (i & 1) * BN, v);
@@ -211,8 +212,8 @@ k_split_product(const __grid_constant__ CUtensorMap map_w, SplitParams p, Epi ep
         uint32_t s = 0, phase = 0;
         const uint32_t at = (uint32_t)(r0 * 128 + (((k4 >> 1) ^ (r0 & 7)) << 4) + (k4 & 1) * 8);       // (rows 8 apart: the same place in the swizzle)
         auto turn = [&](int i, float4 (&v)[XI]) {
-            // (W's copy was made when the stage was free)
-            if (!mbar_wait(&full_w[s], phase, abort_flag)) return false;
+            // (W's copy was made when the stage was free; a wait that gave up has set the flag, and all waits behind it are short)
+            mbar_wait(&full_w[s], phase, abort_flag);
             uint8_t* dst = smem + s * Sh::STAGE + Sh::W_BYTES + at;
             float2 none = make_float2(0.f, 0.f);
 #pragma unroll
@@ -317,6 +318,7 @@ k_split_product(const __grid_constant__ CUtensorMap map_w, SplitParams p, Epi ep
             }
         }
     }
+    __syncwarp();                                 // (outputs that are not there, and the functions' branches, part a warp's lanes)
     if (slices > 1) tc_cluster_sync();            // (no CTA leaves while another reads its sums)
     if (warp == 1) {
         tc_fence_after();
