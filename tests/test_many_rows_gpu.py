@@ -764,3 +764,29 @@ def test_gated_recurrence_in_segments_beside_short_portions():
     assert torch.allclose(got.float(), want, rtol=2.0 ** -8, atol=1e-5) and torch.allclose(state, want_state, rtol=5e-5, atol=1e-5)
     alone, alone_state = run([0], torch.bfloat16)
     assert torch.allclose(got[:400].float(), alone.float(), rtol=2.0 ** -8, atol=1e-5) and torch.allclose(state[0], alone_state[0], rtol=5e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("n,n_out", [(33, 33), (33, 1000), (100, 129), (64, 257), (300, 97), (300, 257), (700, 1)])
+def test_products_whose_rows_part_a_warp(n, n_out):
+    """Rows of W that end inside a warp's 32 while tokens go on for more chunks of sixteen than one: lanes without a row leave a chunk early, and the
+    next read of tensor memory is for the whole warp again.  Stored, added, gated."""
+    from xyntetik_runner_b200 import kernels
+    k = 328
+    g = torch.Generator().manual_seed(n + n_out)
+    x = torch.randn(n, k, generator=g).to(torch.bfloat16)
+    w = (torch.randn(2 * n_out, k, generator=g) * k ** -0.5).to(torch.bfloat16)
+    gate, up = (x.double() @ w[i * n_out:(i + 1) * n_out].double().T for i in range(2))
+    # float32 sums of k exact products: (k + 2) 2^-24 of the products' sizes
+    bound = x.double().abs() @ w[:n_out].double().abs().T * (k + 2) * 2.0 ** -24
+    xd, one, both = x.to(DEV), kernels.pack_weight(w[:n_out].to(DEV)), kernels.pack_weight(w.to(DEV), 2)
+    torch.cuda.synchronize()
+    out = torch.empty(n, n_out, device=DEV)
+    kernels.gemm_tc(xd, one, out, packed_rows=n_out)
+    assert ((out.cpu().double() - gate).abs() <= bound).all()
+    kernels.gemm_tc(xd, one, out, None, kernels.EPI_ADD, packed_rows=n_out)
+    assert ((out.cpu().double() - 2 * gate).abs() <= 2 * bound + gate.abs() * 2.0 ** -22).all()
+    pair = torch.empty(n, n_out, dtype=torch.bfloat16, device=DEV)
+    kernels.gemm_tc(xd, both, pair, None, kernels.EPI_GATED, packed_rows=n_out)
+    ref = torch.nn.functional.silu(gate) * up
+    assert ((pair.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5 * (gate.abs() + 1) * (up.abs() + 1)).all()
+    assert int(kernels.workspace(torch.device(DEV)).status.item()) == 0

@@ -138,6 +138,7 @@ __device__ __forceinline__ void tc_epilogue(const TcParams& p, uint32_t tmem_bas
 #pragma unroll 1
     for (int c0 = chunk_first * 16; c0 < bn; c0 += 16 * warps_per_quarter) {
         if (tok0 + c0 >= n_end) break;             // warp-uniform
+        __syncwarp();                              // (lanes whose row does not exist come here ahead of the others)
         float g[16];
         tc_ld16(taddr + c0, g);
         if (gated_out) {
@@ -331,10 +332,11 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
         }
     } else {
         // ---------------- epilogue: warps 2..9 ----------------
-        bool ok = mbar_wait(acc_ready, 0, abort_flag);
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(acc_ready, 0, abort_flag));
         tc_fence_after();
         if (ok) tc_epilogue<(BN > 64)>(p, tmem_base, row0, tok0, warp, lane, 2, (int)blockIdx.z, p.bn, p.n);
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -529,7 +531,7 @@ k_gemm_tc_pair(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
         for (int item = cluster_id; item < pair_tiles * p.splits; item += n_clusters, j++) {
             const int tile = item % pair_tiles, split = item / pair_tiles;
             const int b = j % ACC_BUFS;
-            if (!mbar_wait(&acc_full[b], (j / ACC_BUFS) & 1, abort_flag)) break;
+            if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[b], (j / ACC_BUFS) & 1, abort_flag))) break;
             tc_fence_after();
             const TcTile at = tc_pair_tile<GROUPED>(p, tile, tok_tiles);
             const int row0 = (2 * at.pair + (int)rank) * TC_BM;
