@@ -858,11 +858,9 @@ XR_EXPORT int xr_gemm_tc(const void* X, const void* W, const float* bias, void* 
 // and rows of X sorted by the matrix they meet, every group's rows starting at a multiple of `bn` (16, 32, 64 or 128):
 // token tile t of X multiplies by matrix tile_group[t] (an int per tile, on the device; below zero: no rows).  n is the
 // number of rows of X and out that the plan may use (a multiple of bn).  Store and gated epilogues; never cut along K.
-// live_rows, live_tiles (0: not known): only the first tiles can have a matrix, and of theirs only the first rows are looked at.
 // ---------------------------------------------------------------------------------------------
-XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit,
-                                 int n, int n_out, int K, long long ldx, long long ldo, int bn, const int* tile_group, int groups,
-                                 int live_rows, int live_tiles, int* status, cudaStream_t stream) {
+static int run_grouped(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit, int n, int n_out, int K, long long ldx,
+                       long long ldo, int bn, const int* tile_group, int groups, int live_rows, int live_tiles, int* status, cudaStream_t stream) {
     if (n < 1 || n_out < 1 || K < 8 || (K % 8) != 0 || (ldx % 8) != 0 || ldx < K || ldo < n_out || groups < 1) return XR_ERR_ARG;
     if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || tile_group == nullptr) return XR_ERR_ARG;
     if (bn != 16 && bn != 32 && bn != 64 && bn != 128) return XR_ERR_ARG;
@@ -892,6 +890,19 @@ XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int ou
         case 64: return launch_tc<64, 4, 2>(mw, mx, p, grid, stream);
         default: return launch_tc<128, 5, 1>(mw, mx, p, grid, stream);
     }
+}
+
+XR_EXPORT int xr_gemm_tc_grouped(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit,
+                                 int n, int n_out, int K, long long ldx, long long ldo, int bn, const int* tile_group, int groups,
+                                 int* status, cudaStream_t stream) {
+    return run_grouped(X, W, out, out_dtype, epilogue, act, act_limit, n, n_out, K, ldx, ldo, bn, tile_group, groups, 0, 0, status, stream);
+}
+// The same where only the first live_tiles tiles can have a matrix, and only the first live_rows rows of theirs are anybody's (0: not known): other
+// rows of `out` may stay as they are.
+XR_EXPORT int xr_gemm_tc_grouped_live(const void* X, const void* W, void* out, int out_dtype, int epilogue, int act, float act_limit,
+                                      int n, int n_out, int K, long long ldx, long long ldo, int bn, const int* tile_group, int groups,
+                                      int live_rows, int live_tiles, int* status, cudaStream_t stream) {
+    return run_grouped(X, W, out, out_dtype, epilogue, act, act_limit, n, n_out, K, ldx, ldo, bn, tile_group, groups, live_rows, live_tiles, status, stream);
 }
 
 // The same on CTA pairs, for groups that meet many rows: `tiles` (int [1 + 3 max_tiles], on the device) holds the number of token

@@ -1181,9 +1181,12 @@ def gemm_tc_grouped(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, 
     assert w_packed.shape[1] == tiles and w_packed.shape[2] == -(-k // TILE_K) and out.shape == (n, n_out)
     assert tile_group.dtype == torch.int32 and tile_group.numel() >= n // bn
     ws = workspace(x.device)
-    _check(_c.xr_gemm_tc_grouped(x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act),
-                                    float(act_limit), n, n_out, k, x.stride(0), out.stride(0), bn, tile_group.data_ptr(),
-                                    w_packed.shape[0], int(live_rows), int(live_tiles), ws.status_ptr, _stream()), "gemm_tc_grouped")
+    args = (x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), n, n_out, k, x.stride(0),
+            out.stride(0), bn, tile_group.data_ptr(), w_packed.shape[0])
+    if live_rows and live_tiles:
+        _check(_c.xr_gemm_tc_grouped_live(*args, int(live_rows), int(live_tiles), ws.status_ptr, _stream()), "gemm_tc_grouped")
+    else:
+        _check(_c.xr_gemm_tc_grouped(*args, ws.status_ptr, _stream()), "gemm_tc_grouped")
     _count()
 
 
