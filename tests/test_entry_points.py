@@ -20,3 +20,21 @@ def test_grouped_products():
     live = kernels._c.xr_gemm_tc_grouped_live
     assert live(*head(), 1, 4, P, 0) in NOT_LAUNCHED and live(*head(), 0, 0, P, 0) in NOT_LAUNCHED
     assert live(*head(), 17, 4, P, 0) == REFUSED and live(*head(), -1, 4, P, 0) == REFUSED
+
+
+@without_device
+@pytest.mark.parametrize("n,n_out,k", [(1, 1024, 1024), (2, 4096, 1024), (1, 2048, 4096), (8, 1024, 4096)])
+def test_slices_that_a_product_leaves(n, n_out, k):
+    """What xr_gemm_tc says of a product whose sum is left to the caller: how many slices lie in the scratch, within the room it was given.  That one
+    slice of a product that is not cut may lie there is said to callers of xr_gemm_tc_uncut alone."""
+    lib, room = kernels.lib(), 16 * n * n_out
+    said = []
+    for entry in (lib.xr_gemm_tc, lib.xr_gemm_tc_uncut):
+        slices = ctypes.c_int(-7)
+        rc = entry(P, P, None, P, kernels.F32, kernels.EPI_ADD, 0, 0.0, 1.0, n, n_out, k, k, n_out, P, room, P, 0, 1, ctypes.byref(slices), 1, None)
+        assert rc in NOT_LAUNCHED
+        said.append(slices.value)
+    if n <= 2:                                    # (on CUDA cores: nothing is cut)
+        assert said == [1, kernels.ONE_DEFERRED]
+    else:                                         # (no tensor map, no answer)
+        assert set(said) <= {-7} | set(range(1, 17))

@@ -531,7 +531,7 @@ class PartialSums:
 
 
 
-ONE_DEFERRED = 1 << 16          # xr_gemm_tc's answer where it left one slice of sums, not cut, to the caller's next kernel
+ONE_DEFERRED = 1 << 16          # xr_gemm_tc_uncut's answer where it left one slice of sums, not cut, to the caller's next kernel
 
 
 def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, act_limit=0.0, alpha=1.0):
@@ -555,9 +555,9 @@ def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, a
     assert not defer or not gated
     ws = workspace(x.device)
     at, room = ws.room()
-    splits = _c.xr_gemm_tc(x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), float(alpha),
-                           n, n_out, k, ldx, out.stride(0), at, room,
-                           ws.status_ptr, force_splits, int(defer), int(packed_rows is not None), _stream())
+    splits = _c.xr_gemm_tc_uncut(x.data_ptr(), w.data_ptr(), _ptr(bias), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), float(alpha),
+                                 n, n_out, k, ldx, out.stride(0), at, room,
+                                 ws.status_ptr, force_splits, int(defer), int(packed_rows is not None), _stream())
     if splits < 0:
         _check(splits, "gemm_tc")
     _count(1 if (splits == 1 or defer) else 2)
