@@ -168,3 +168,69 @@ def test_a_token_meets_an_expert_once():
     for r in rows:
         want = h[1].double() @ up[int(of[r // align])].double().T
         assert (out[r].cpu().double() - want).abs().max() <= 1e-4
+
+
+@pytest.mark.parametrize("n,n_out,k,few", [(1, 1024, 4096, True), (1, 1024, 4104, False), (1, 2504, 64, True), (2, 2048, 1536, True), (2, 2048, 1544, False),
+                                           (2, 16, 8, True), (3, 1024, 1024, False)])
+def test_which_road_a_product_takes(n, n_out, k, few):
+    """The road of one token or two says so and is counted apart, stored, added, left to the next kernel and gated; K 8 further on and one token more
+    are counted as products on tcgen05."""
+    from types import SimpleNamespace
+    from xyntetik_runner_b200 import kernels
+    from xyntetik_runner_b200.parts import linear
+    rt = SimpleNamespace(act_dtype=torch.bfloat16)
+    w = torch.randn(n_out, k, device=DEV).to(torch.bfloat16)
+    one, both = linear.Linear(w).prepare(rt), linear.Linear(w, halves=2).prepare(rt)
+    x, stored, added = torch.randn(n, k, device=DEV).to(torch.bfloat16), torch.empty(n, n_out, device=DEV), torch.zeros(n, n_out, device=DEV)
+    pair = torch.empty(n, n_out // 2, device=DEV, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    before, kept = dict(linear.counters), kernels.few_products
+    one.forward(x, stored)
+    one.forward(x, added, accumulate=True)
+    both.forward_gated(x, pair)
+    pending = one.forward(x, added, accumulate=True, defer=True)
+    if few:
+        assert pending is not None and pending.splits == 1
+    if pending is not None:
+        pending.finish()
+    gone = {name: linear.counters[name] - before[name] for name in before}
+    assert (gone["few"], gone["tcgen05"]) == ((4, 0) if few else (0, 4)) and kernels.few_products - kept == gone["few"]
+    assert (added - 2 * stored).abs().max() <= 1e-4 * stored.abs().max()
+    assert kernels.gemm_tc(x, one.packed, stored, packed_rows=n_out) == 1 or not few
+
+
+def test_an_engines_single_tokens_take_it(tmp_path):
+    import tiny
+    from xyntetik_runner_b200.engine.runner import Runner
+    from xyntetik_runner_b200.parts import linear
+    tiny.make_folder(str(tmp_path), "B", "bfloat16")
+    before = dict(linear.counters)
+    Runner(str(tmp_path), dtype="bfloat16", ctx=64, parallel=2, page_size=8).generate(list(range(3, 12)), n=4, temp=0.0, ignore_eos=True)
+    assert linear.counters["few"] > before["few"] + 4 and linear.counters["tcgen05"] > before["tcgen05"] + 4
+
+
+@pytest.mark.parametrize("n,E,top,width,inner,act,limit", [(1, 16, 2, 1024, 1408, 1, 0.0), (2, 64, 6, 264, 72, 3, 7.0), (2, 12, 2, 1024, 1400, 2, 0.0)])
+def test_gated_experts_of_a_few_tokens(n, E, top, width, inner, act, limit):
+    """Gated experts' first product in bfloat16 as their layer asks for it: the rows that live against plain products, all others untouched."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(n * 3 + E)
+    used = sorted(set(torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).reshape(-1).tolist()))
+    tiles, bn = len(used) + 2, 16
+    group = torch.tensor(used + [-1, -1], dtype=torch.int32, device=DEV)
+    x = torch.randn(tiles * bn, width, generator=g).to(torch.bfloat16)
+    w = (torch.randn(E, 2 * inner, width, generator=g) * width ** -0.5).to(torch.bfloat16)
+    out = torch.full((tiles * bn, inner), 7.0, device=DEV, dtype=torch.bfloat16)
+    packed = kernels.pack_weight_groups(w.to(DEV), 2)
+    torch.cuda.synchronize()
+    kernels.gemm_tc_grouped(x.to(DEV), packed, out, group, bn, inner, kernels.EPI_GATED, act, limit, live_rows=n, live_tiles=n * top)
+    got = out.cpu().double().view(tiles, bn, inner)
+    for t, e in enumerate(used):
+        gate, up = (x.view(tiles, bn, width)[t, :n].double() @ w[e, i * inner:(i + 1) * inner].double().T for i in range(2))
+        if act == 3:
+            gate, up = gate.clamp(max=limit), up.clamp(-limit, limit)
+            want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+        else:
+            want = (torch.nn.functional.silu(gate) if act == 1 else torch.nn.functional.gelu(gate, approximate="tanh")) * up
+        # one rounding to bfloat16; float32 sums and the hardware's approximate functions 2e-5 of both factors' size
+        assert ((got[t, :n] - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * (gate.abs() + 1) * (up.abs() + 2)).all()
+    assert (got[:, n:] == 7).all() and (got[len(used):] == 7).all()

@@ -793,7 +793,8 @@ XR_EXPORT long long xr_gemm_tc_scratch_floats(int n, int n_out, int gated) {
 // device int, set non-zero if a wait gave up.
 // alpha: factor on every sum, ahead of bias and activation (1 for gated products); partial sums carry it.
 // defer_finish: partial sums are left in `scratch` for the caller's next kernel.  *splits_used: how many slices of them; 1: `out` is complete.
-// defer_uncut (with defer_finish): a product of a few tokens may leave the one slice of its sums too, *splits_used is then GV_DEFERRED.
+// defer_uncut: the caller is told of a product on CUDA cores (gemv.cuh), *splits_used GV_COMPLETE; with defer_finish that may leave the one slice
+// of its sums too, *splits_used GV_DEFERRED.
 static int run_gemm_tc(const void* X, const void* W, const float* bias, void* out, int out_dtype, int epilogue, int act, float act_limit, float alpha,
                        int n, int n_out, int K, long long ldx, long long ldo, float* scratch, long long scratch_floats, int* status, int force_splits,
                        int defer_finish, bool defer_uncut, int* splits_used, int w_packed, cudaStream_t stream) {
@@ -808,7 +809,7 @@ static int run_gemm_tc(const void* X, const void* W, const float* bias, void* ou
     if (w_packed && force_splits == 0 && gemv_takes(n, K, 2LL * K * n_out * (gated ? 2 : 1), false)) {
         // (float32 that is stored is what the sum would be: nothing is left for the caller's next kernel)
         const bool defer = defer_finish && defer_uncut && !gated && (epilogue == TC_EPI_ADD || out_dtype == XR_BF16) && scratch != nullptr && scratch_floats >= (long long)n * n_out;
-        if (splits_used) *splits_used = defer ? GV_DEFERRED : 1;
+        if (splits_used) *splits_used = defer ? GV_DEFERRED : (defer_uncut ? GV_COMPLETE : 1);
         TcParams p{out, bias, scratch, status, ldo, n, n_out, K, 1, defer ? TC_EPI_PARTIAL : epilogue, out_dtype, act, act_limit, gated ? 1 : 0, 0, 1,
                    (K + TC_BK - 1) / TC_BK, 1, 0};
         p.alpha = alpha;
@@ -861,7 +862,7 @@ XR_EXPORT int xr_gemm_tc(const void* X, const void* W, const float* bias, void* 
     return run_gemm_tc(X, W, bias, out, out_dtype, epilogue, act, act_limit, alpha, n, n_out, K, ldx, ldo, scratch, scratch_floats, status, force_splits,
                        defer_finish, false, splits_used, w_packed, stream);
 }
-// The same for callers that know GV_DEFERRED.
+// The same for callers that know GV_DEFERRED and GV_COMPLETE.
 XR_EXPORT int xr_gemm_tc_uncut(const void* X, const void* W, const float* bias, void* out, int out_dtype, int epilogue, int act, float act_limit, float alpha,
                                int n, int n_out, int K, long long ldx, long long ldo, float* scratch,
                                long long scratch_floats, int* status, int force_splits, int defer_finish, int* splits_used,

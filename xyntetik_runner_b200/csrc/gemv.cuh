@@ -15,7 +15,9 @@
 #pragma once
 
 #define GV_AHEAD 4                  // K blocks of weights that a lane holds
-#define GV_DEFERRED (1 << 16)       // "splits used" of a product whose one slice of sums is left to the caller's next kernel
+// "splits used" of a product that ran here: its one slice of sums is left to the caller's next kernel, or it is complete
+#define GV_DEFERRED (1 << 16)
+#define GV_COMPLETE (1 << 17)
 
 __device__ __forceinline__ uint4 gv_load(const __nv_bfloat16* p) {
     uint4 v;

@@ -531,7 +531,9 @@ class PartialSums:
 
 
 
-ONE_DEFERRED = 1 << 16          # xr_gemm_tc_uncut's answer where it left one slice of sums, not cut, to the caller's next kernel
+# xr_gemm_tc_uncut's answers for a product of a few tokens that ran on CUDA cores: one slice of sums is left to the caller's next kernel; it is complete
+ONE_DEFERRED, ONE_COMPLETE = 1 << 16, 1 << 17
+few_products = 0                # how many of them ran
 
 
 def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, act_limit=0.0, alpha=1.0):
@@ -560,9 +562,12 @@ def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, a
                                  ws.status_ptr, force_splits, int(defer), int(packed_rows is not None), _stream())
     if splits < 0:
         _check(splits, "gemm_tc")
+    if splits >= ONE_DEFERRED:
+        global few_products
+        few_products += 1
+        _count()
+        return PartialSums(ws, ws.take(n * n_out), 1) if splits == ONE_DEFERRED else 1
     _count(1 if (splits == 1 or defer) else 2)
-    if splits == ONE_DEFERRED:
-        return PartialSums(ws, ws.take(n * n_out), 1)
     if defer and splits > 1:
         rows = tiles * TILE_ROWS if (gated and packed_rows is not None) else n_out
         return PartialSums(ws, ws.take(splits * n * rows), splits)
@@ -572,7 +577,8 @@ def _gemm_tc(x, w, out, bias, epilogue, act, force_splits, defer, packed_rows, a
 def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None,
             epilogue: int = EPI_STORE, force_splits: int = 0, packed_rows: Optional[int] = None, act: Optional[int] = None,
             act_limit: float = 0.0, alpha: float = 1.0) -> int:
-    """bfloat16 product on tcgen05.  EPI_STORE: out[t][r] = act(alpha x.w + bias); EPI_ADD: float32 out += alpha x.w + bias;
+    """bfloat16 product on tcgen05, or for a few tokens on CUDA cores (``few_products``).  EPI_STORE: out[t][r] = act(alpha x.w + bias);
+    EPI_ADD: float32 out += alpha x.w + bias;
     EPI_GATED: w from ``pack_weight(w, halves=2)``, out[t][f] = act(x.w_gate[f]) * (x.w_up[f]) (act defaults to SiLU).
     Returns the number of K splits used."""
     if act is None:

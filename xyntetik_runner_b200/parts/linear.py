@@ -1,12 +1,13 @@
 """A weight matrix and the choice of kernel that multiplies by it.
 
 ``out[t][r] (+)= alpha sum_k x[t][k] W[r][k] (+ bias[r])``.  W keeps its stored dtype.  bfloat16 activations times
-a bfloat16 matrix go to the tensor-core kernel (tcgen05); for that the matrix is re-laid tile by tile when the
-part binds it (``prepare``), so that every tile the kernel streams is one contiguous read.  The true 32-bit path's
+a bfloat16 matrix go to the tensor-core kernel (tcgen05), or where one token or two are all there is to CUDA cores (by K and bytes:
+``gemv_takes`` in csrc/gemv.cuh); for both the matrix is re-laid tile by tile when the
+part binds it (``prepare``), so that every tile a kernel streams is one contiguous read.  The true 32-bit path's
 float32 activations times a bfloat16 matrix of some length go to the tensor cores too, in three exact pieces
 (``kernels.gemm_split``).  Everything else goes to the float32 FMA kernel on the matrix as stored.  Which kernel
-ran is counted, so that a test can prove its subject ran.  The choice hangs on the matrix and on how rows lie in memory,
-not on how many there are: in 32 bit a token's row is the same bits whatever stands beside it.
+ran is counted, so that a test can prove its subject ran.  In 32 bit the choice hangs on the matrix and on how rows lie in memory,
+not on how many there are: a token's row is the same bits whatever stands beside it.
 """
 from __future__ import annotations
 
@@ -17,7 +18,7 @@ import torch
 from .. import kernels
 from . import linear_tc
 
-counters = {"tcgen05": 0, "simt": 0, "deferred": 0, "split": 0}
+counters = {"tcgen05": 0, "few": 0, "simt": 0, "deferred": 0, "split": 0}
 
 
 class Linear:
@@ -55,8 +56,9 @@ class Linear:
         assert self.halves == 1, "a matrix of two halves is multiplied by forward_gated"
         assert act == kernels.ACT_NONE or not (accumulate or defer)
         if self.packed is not None or linear_tc.usable(self, x, out, accumulate):
-            counters["tcgen05"] += 1
+            before = kernels.few_products
             pending = linear_tc.run(self, x, out, accumulate, defer, act, alpha)
+            counters["tcgen05" if kernels.few_products == before else "few"] += 1
             if pending is not None:
                 counters["deferred"] += 1
             return pending
@@ -80,8 +82,9 @@ class Linear:
         activation kernel."""
         assert self.halves == 2
         if self.packed is not None:
+            before = kernels.few_products
             kernels.gemm_tc(x, self.packed, out, None, kernels.EPI_GATED, packed_rows=self.n_out // 2, act=act, act_limit=limit)
-            counters["tcgen05"] += 1
+            counters["tcgen05" if kernels.few_products == before else "few"] += 1
             return
         if self.split and (scratch is None or kernels.split_rows_ok(x)):
             kernels.gemm_split(x, self.weight, out, act=act, gated=True, limit=limit)
