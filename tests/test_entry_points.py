@@ -38,3 +38,24 @@ def test_slices_that_a_product_leaves(n, n_out, k):
         assert said == [1, kernels.ONE_DEFERRED]
     else:                                         # (no tensor map, no answer)
         assert set(said) <= {-7} | set(range(1, 17))
+
+
+def test_what_a_products_grid_does_not_hold_goes_by_another():
+    """Sizes beyond the grid, or beyond the addresses, of the products in pieces stay with the float32 FMA kernel, which takes them (storage on no device:
+    only sizes are looked at)."""
+    rows = lambda n, ld, k=256, dtype=torch.float32: torch.empty_strided((n, k), (ld, 1), dtype=dtype, device="meta")
+    assert kernels.split_rows_ok(rows(300, 256)) and kernels.split_rows_ok(rows(65535 * 64, 256)) and kernels.split_rows_ok(rows(7, (1 << 31) + 4))
+    assert not kernels.split_rows_ok(rows(65535 * 64 + 1, 256)) and not kernels.split_rows_ok(rows(9, 1 << 31)) and not kernels.split_rows_ok(rows(3, 258))
+    matrix = lambda r, k: torch.empty(r, k, dtype=torch.bfloat16, device="meta")
+    assert kernels.split_shape_ok(matrix(65535 * 128, 256)) and not kernels.split_shape_ok(matrix(65535 * 128 + 1, 256))
+    assert not kernels.split_shape_ok(matrix(100, 248)) and not kernels.split_shape_ok(matrix(100, 260))
+
+
+@without_device
+def test_a_recurrence_of_more_blocks_than_the_products_grid_holds():
+    """20,000 blocks of 256 channels: four tiles each are more than the grid of the products in pieces holds, and the FMA kernel takes them."""
+    R, B = 256 * 20000, 20000
+    p = P
+    for n in (17, 64):
+        args = (p, 2 * R, 0, R, p, p, p, p, p, p, p, p, p, R * 4, p, p, p, p, p, p, p, p, kernels.F32, n, 1, R, B, 4, 8.0, p, 0)
+        assert kernels._c.xr_rglru_gates(*args) == -2            # (the products in pieces would ask for a tensor map first)

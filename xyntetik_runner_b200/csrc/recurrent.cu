@@ -401,7 +401,7 @@ static int run_rglru(float* proj, long long ldp, int y_col, int x_col, const flo
         const int groups = (Bs + 7) / 8;
         xr_launch(k_rglru_gates_few, dim3((n + 7) / 8, B * groups), dim3(256), smem8, stream, proj, ldp, y_col, wa, wi, ba, bi, lam, a_s, b_s,
                   n, R, Bs, c, groups, (const float*)u_s);
-    } else if (gates != nullptr && (n >= 64 || dtype == XR_F32) && split_takes(u_s, n, R, gates, Bs)) {
+    } else if (gates != nullptr && (n >= 64 || dtype == XR_F32) && split_takes(u_s, n, R, gates, Bs) && split_fits<true>(n, Bs, B)) {
         SplitParams p{u_s, R, n, Bs, Bs, R, 0, status};
         const int rc = run_split<true>(gates, 2LL * R, p, GateFinish{proj + y_col, ldp, u_s, ba, bi, lam, a_s, b_s, R, c}, B, stream);
         if (rc != XR_OK) return rc;

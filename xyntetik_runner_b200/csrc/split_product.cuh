@@ -359,6 +359,11 @@ static int launch_split(const CUtensorMap& mw, const SplitParams& p, const Epi& 
 static inline bool split_takes(const float* x, int n, long long ldx, const void* W, int K) {
     return K % 8 == 0 && ldx % 4 == 0 && (long long)n * ldx < (1LL << 34) && !(((uintptr_t)x | (uintptr_t)W) & 15);
 }
+// What the grid holds: `rows` rows of W (TWO: features) a block.
+template <bool TWO> static inline bool split_fits(int n, int rows, int blocks) {
+    constexpr int per = TWO ? TC_BM / 2 : TC_BM;
+    return (long long)((rows + per - 1) / per) * blocks <= 65535 && n <= 65535 * 64;
+}
 // `blocks` blocks of X's columns.  64 tokens a tile, or 32 while these still fit the SMs at once; 16 for a few.
 template <bool TWO, class Epi>
 static int run_split(const void* W, long long w_rows, SplitParams p, const Epi& epi, int blocks, cudaStream_t stream) {

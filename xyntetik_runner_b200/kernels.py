@@ -278,14 +278,21 @@ SPLIT_LEAST_K = 256
 
 
 def split_weight_ok(w: torch.Tensor) -> bool:
-    """Whether ``gemm_split`` multiplies by this matrix: bfloat16, every value finite, rows of at least SPLIT_LEAST_K values on 16-byte
-    borders."""
-    return (w.is_cuda and w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[1] >= SPLIT_LEAST_K
-            and w.data_ptr() % 16 == 0 and bool(torch.isfinite(w).all()))
+    """Whether ``gemm_split`` multiplies by this matrix: bfloat16, every value finite (read once, where the matrix is bound), rows of at least
+    SPLIT_LEAST_K values on 16-byte borders, and no more of them than its grid holds."""
+    return w.is_cuda and split_shape_ok(w) and w.data_ptr() % 16 == 0 and bool(torch.isfinite(w).all())
+
+
+def split_shape_ok(w: torch.Tensor) -> bool:
+    return (w.dtype == torch.bfloat16 and w.is_contiguous() and w.shape[1] % 8 == 0 and w.shape[1] >= SPLIT_LEAST_K
+            and w.shape[0] <= 65535 * TILE_ROWS)
 
 
 def split_rows_ok(x: torch.Tensor) -> bool:
-    return x.dtype == torch.float32 and x.stride(1) == 1 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
+    """Whether ``gemm_split`` reads these rows: float32 on 16-byte borders, within 2^34 values of memory and 65,535 tiles of 64 tokens."""
+    n, ld = x.shape[0], x.stride(0)
+    return (x.dtype == torch.float32 and x.stride(1) == 1 and ld % 4 == 0 and x.data_ptr() % 16 == 0 and n * ld < 1 << 34
+            and n <= 65535 * 64)
 
 
 def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor] = None, accumulate: bool = False,

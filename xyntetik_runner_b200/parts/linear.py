@@ -86,10 +86,12 @@ class Linear:
             kernels.gemm_tc(x, self.packed, out, None, kernels.EPI_GATED, packed_rows=self.n_out // 2, act=act, act_limit=limit)
             counters["tcgen05" if kernels.few_products == before else "few"] += 1
             return
-        if self.split and (scratch is None or kernels.split_rows_ok(x)):
+        if self.split and kernels.split_rows_ok(x):
             kernels.gemm_split(x, self.weight, out, act=act, gated=True, limit=limit)
             counters["split"] += 1
             return
+        if self.split and scratch is None:               # (rows that gemm_split does not read: the caller was told of no scratch)
+            scratch = torch.empty((x.shape[0], self.n_out), dtype=out.dtype, device=out.device)
         assert scratch is not None and scratch.shape == (x.shape[0], self.n_out)
         kernels.gemm_simt(x, self.weight, scratch, None, False)
         counters["simt"] += 1
