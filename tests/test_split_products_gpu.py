@@ -165,3 +165,15 @@ def test_rows_that_part_a_warp(n, n_out, k):
         assert ((out.cpu().double() - ref).abs() <= slope + ref.abs() * 2.0 ** -20 + 1e-30).all()
         assert torch.equal(out, again)
     assert int(kernels.workspace(torch.device(DEV)).status.sum()) == 0
+
+
+def test_the_switch_reaches_a_recurrences_gates(monkeypatch):
+    """With the tensor cores switched off to bisect a difference, the gates go to the FMA kernel too."""
+    from types import SimpleNamespace
+    from xyntetik_runner_b200.parts import linear_tc
+    from xyntetik_runner_b200.parts.rglru import GatedLinearRecurrence
+    for on in (True, False):
+        monkeypatch.setattr(linear_tc, "ENABLED", on)
+        part = GatedLinearRecurrence(64, 512, 2, 4, "")
+        part.bind({name: torch.randn(spec.shape, device=DEV).to(torch.bfloat16) for name, spec in part.tensors().items()}, SimpleNamespace(act_dtype=torch.bfloat16))
+        assert (part.gates is not None) == on and (part.out.packed is not None) == on

@@ -15,6 +15,7 @@ import torch
 
 from .. import kernels
 from ..weights.loader import TensorSpec
+from . import linear_tc
 from .base import Mixer, StateNeed, register_mixer
 from .linear import Linear
 
@@ -60,12 +61,13 @@ class GatedLinearRecurrence(Mixer):
         self.out = Linear(tensors[n["o"]]).prepare(rt)
         self.conv_w, self.conv_b = f32(n["conv"]), f32(n["conv"] + b)
         both = torch.cat([tensors[n["ra"]], tensors[n["ri"]]]).reshape(2 * self.R, -1)
-        self.gates = both if kernels.split_weight_ok(both) else None
+        self.gates = both if linear_tc.ENABLED and kernels.split_weight_ok(both) else None
         self.wa, self.wi = f32(n["ra"]), f32(n["ri"])
         self.ba, self.bi, self.lam = f32(n["ra"] + b).reshape(-1), f32(n["ri"] + b).reshape(-1), f32(n["lam"])
         self._small = (self.wa.numel() + self.wi.numel() + self.conv_w.numel() + 4 * self.R) * 4
 
     def weight_bytes(self):
+        # a step reads the gates' matrices in one of their two forms: in float32 a step of single tokens, which is what is counted
         return self.proj.nbytes() + self.out.nbytes() + self._small
 
     def forward(self, ctx, h, x, lay):
