@@ -790,3 +790,27 @@ def test_products_whose_rows_part_a_warp(n, n_out):
     ref = torch.nn.functional.silu(gate) * up
     assert ((pair.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 2e-5 * (gate.abs() + 1) * (up.abs() + 1)).all()
     assert int(kernels.workspace(torch.device(DEV)).status.item()) == 0
+
+
+@pytest.mark.parametrize("lens", [[2048], [2049, 3], [1700, 2500]])
+def test_portions_whose_gates_a_thread_holds_and_does_not(lens):
+    """mLSTM's running maxima: a thread's run of eight tokens, the most that it keeps both logarithms of, and of nine and ten; against float64."""
+    test_portions_of_many_chunks("mlstm", 1, 64, 64, lens)
+
+
+@pytest.mark.parametrize("tiles,align", [(127, 16), (128, 16), (517, 16), (33, 64), (2053, 1)])
+@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 40), (torch.bfloat16, 33), (torch.float32, 300)])
+def test_gather_of_planned_tiles(tiles, align, dtype, width):
+    """Rows below and above the 2,048 from which four go to a block, in tiles that the plan uses, uses in part and leaves alone: a row's token, zeros in
+    padding, unused tiles as they were."""
+    from xyntetik_runner_b200 import kernels
+    g = torch.Generator().manual_seed(tiles + width)
+    rows, top, n = tiles * align, 3, 97
+    group = torch.where(torch.rand(tiles, generator=g) < 0.7, torch.randint(0, 9, (tiles,), generator=g), torch.tensor(-1)).int()
+    src = torch.where(torch.rand(rows, generator=g) < 0.8, torch.randint(0, n * top, (rows,), generator=g), torch.tensor(-1)).int()
+    h = torch.randn(n, width, generator=g).to(dtype)
+    out = torch.full((rows, width), 7.0, dtype=dtype, device=DEV)
+    kernels.moe_gather(h.to(DEV), out, src.to(DEV), group.to(DEV), top, align)
+    want = torch.where((src >= 0)[:, None], h[src.clamp(min=0).long() // top], torch.tensor(0.0, dtype=dtype))
+    want[(group < 0).repeat_interleave(align)] = 7.0
+    assert torch.equal(out.cpu(), want)
