@@ -6,9 +6,10 @@
 // Other scores, a correction of the choice, groups of experts and a factor on the weights: see k_route_topk and k_route_groups.
 // The router may have more outputs than there are experts: the outputs from E on are identity experts, whose output is h[t]
 // itself.  They take part in the choice, have no rows in the plan (pair_row -1), and the weighted sum adds weight * h[t] for them.
-// An expert is a feed-forward: y = gate_act(W_gate h, W_up h), or act(W_up h) without a gate, then W_down y (see xr_gate below for the
+// An expert is a feed-forward: y = gate_act(W_gate h, W_up h), or act(W_up h) without a gate, then W_down y (see activation.cuh for the
 // activations).  No step reads anything back to the host: the plan of who computes what is made on the device, and
 // the grids are sized for the worst case (every tile index beyond the plan's count returns at once).
+#include "activation.cuh"
 #include "common.cuh"
 #include <math.h>
 
@@ -521,18 +522,6 @@ XR_EXPORT int xr_route_few(const float* z, int splits, float* zs, int ldz, int n
 #define MOE_TM 64
 XR_EXPORT int xr_moe_tile_rows() { return MOE_TM; }
 
-__device__ __forceinline__ float moe_gate(int act, float limit, float g, float u) {
-    if (act == 3) {                  // g' sigmoid(1.702 g') (u' + 1), g' = min(g, limit), u' = clamp(u, -limit, limit)
-        g = fminf(g, limit);
-        u = fminf(fmaxf(u, -limit), limit);
-        return g / (1.0f + expf(-1.702f * g)) * (u + 1.0f);
-    }
-    if (act == 1) return (g < -80.0f ? 0.0f : g / (1.0f + expf(-g))) * u;
-    if (act == 2) return 0.5f * g * (1.0f + tanhf(0.7978845608f * (g + 0.044715f * g * g * g))) * u;
-    if (act == 4) { const float r = fmaxf(g, 0.f); return r * r * u; }
-    return g * u;
-}
-
 template <typename TA, typename TW, typename TO>
 __global__ void __launch_bounds__(256)
 k_moe_gemm(const TA* __restrict__ A, long long lda, const TW* __restrict__ W, TO* __restrict__ out, long long ldo,
@@ -589,13 +578,13 @@ k_moe_gemm(const TA* __restrict__ A, long long lda, const TW* __restrict__ W, TO
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const int f = c0 + tx + 16 * j;
-                if (f < N) orow[f] = xr_from_f32<TO>(moe_gate(act, limit, acc[i][j], acc[i][j + 2]));
+                if (f < N) orow[f] = xr_from_f32<TO>(xr_gate(act, limit, acc[i][j], acc[i][j + 2]));
             }
         } else {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 const int c = c0 + tx + 16 * j;
-                if (c < N) orow[c] = xr_from_f32<TO>(moe_gate(act, limit, acc[i][j], 1.0f));
+                if (c < N) orow[c] = xr_from_f32<TO>(xr_gate(act, limit, acc[i][j], 1.0f));
             }
         }
     }
