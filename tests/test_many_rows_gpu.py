@@ -798,10 +798,10 @@ def test_portions_whose_gates_a_thread_holds_and_does_not(lens):
     test_portions_of_many_chunks("mlstm", 1, 64, 64, lens)
 
 
-@pytest.mark.parametrize("tiles,align", [(127, 16), (128, 16), (517, 16), (33, 64), (2053, 1)])
-@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 40), (torch.bfloat16, 33), (torch.float32, 300)])
+@pytest.mark.parametrize("tiles,align", [(127, 16), (192, 16), (517, 16), (47, 64), (3073, 1), (12291, 1)])
+@pytest.mark.parametrize("dtype,width", [(torch.bfloat16, 40), (torch.bfloat16, 33), (torch.float32, 300), (torch.bfloat16, 2056)])
 def test_gather_of_planned_tiles(tiles, align, dtype, width):
-    """Rows below and above the 2,048 from which four go to a block, in tiles that the plan uses, uses in part and leaves alone: a row's token, zeros in
+    """Rows below and above the 3,072 (wide ones 12,288) from which four go to a block, in tiles that the plan uses, uses in part and leaves alone: a row's token, zeros in
     padding, unused tiles as they were."""
     from xyntetik_runner_b200 import kernels
     g = torch.Generator().manual_seed(tiles + width)

@@ -316,7 +316,9 @@ XR_EXPORT int xr_moe_plan(const int* ids, int* row_src, int* pair_row, int* tile
 // padding are left as they are, nobody reads what they come to.
 // ---------------------------------------------------------------------------------------------
 // ROWS rows a block, side by side: a row is two trips to memory, one behind the other.  12,288 rows of 2,048 bfloat16
-// inside a step: a row a block 15.7 us, so 11.0.
+// inside a step: a row a block 15.7 us, so 11.0.  Where it pays, us, launches back to back, a row a block / so: rows of 1,024 bfloat16
+// 1,024 1.8 / 2.2, 2,048 2.5 / 3.2, 3,072 3.6 / 3.3, 12,288 13.1 / 5.7; of 2,048 2,048 3.3 / 3.7, 3,072 4.3 / 4.0, 4,096 5.1 / 4.5; of 4,096, which
+// are two accesses a thread already, 3,072 5.5 / 6.1, 4,096 6.7 / 7.4, 12,288 28.8 / 26.6.
 template <typename T, int ROWS>
 __global__ void __launch_bounds__(256)
 k_moe_gather_rows(const T* __restrict__ h, long long ldh, T* __restrict__ out, const int* __restrict__ row_src,
@@ -369,7 +371,7 @@ XR_EXPORT int xr_moe_gather(const void* h, int dtype, long long ldh, void* out, 
 #define GATHER(T, DIV)                                                                                                                       \
     do {                                                                                                                                     \
         const int units = width / (DIV), threads = units >= 256 ? 256 : (units + 31) / 32 * 32;                                              \
-        if (max_rows >= 2048)                                                                                                                \
+        if (max_rows >= (units <= 256 ? 3072 : 12288))                                                                                       \
             xr_launch((k_moe_gather_rows<T, 4>), dim3((max_rows + 3) / 4), dim3(threads), 0, stream, (const T*)h, ldh / (DIV), (T*)out, row_src,         \
                       tile_group, top, units, align, max_rows);                                                                              \
         else                                                                                                                                 \
