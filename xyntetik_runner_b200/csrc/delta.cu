@@ -57,7 +57,7 @@ k_delta_prep(const T* __restrict__ proj, long long ldp, const float* __restrict_
                 const float* w = conv_w + (size_t)c * taps;
                 float acc = 0.f;
                 if (taps == 4 && i >= 3) {
-                    // (every input is a row of this step: the four side by side; one behind the other, 505 tokens of 8 heads took 17.5 us
+                    // (four taps, which is what models have, and every input a row of this step: the four side by side; one behind the other, 505 tokens of 8 heads took 17.5 us
                     // inside a step, so 14.5)
                     float x[4], u[4];
 #pragma unroll

@@ -293,9 +293,11 @@ k_silu_gate_norm(const float* __restrict__ o, const float* __restrict__ g, long 
 }
 
 // Four columns an access, KEEP accesses a thread, all on their way at once: groups of up to 4 KEEP columns a thread on 16-byte borders.  777 tokens of
-// 2,048 columns inside a step: 11.9 -> 6.2 us.
+// 2,048 columns inside a step: 11.9 -> 6.2 us.  Few rows take it too: four accesses side by side hide more than a row's own 1,024 threads do.  us, launches
+// back to back, a column an access / so: 512 columns 1 row 2.6 / 1.6, 64 rows 3.1 / 1.8; 2,048 columns 1 3.6 / 3.1, 64 3.8 / 3.3, 777 8.6 / 5.6; 8,192 columns
+// 1 5.3 / 3.7, 777 31.8 / 12.3; behind it in 128 rows of 4,096 alone, 4.4 / 4.6.
 template <typename T, int KEEP>
-__global__ void __launch_bounds__(KEEP == 1 ? 1024 : 512)
+__global__ void __launch_bounds__(KEEP == 1 ? 128 : 512)
 k_silu_gate_norm_vec(const float* __restrict__ o, const float* __restrict__ g, long long ld_g, const float* __restrict__ w, T* __restrict__ y,
                      int width, int per, float eps) {
     xr_pdl_launch();
@@ -336,12 +338,10 @@ XR_EXPORT int xr_silu_gate_norm(const float* o, const float* g, long long ld_g, 
                                 float eps, cudaStream_t stream) {
     if (n < 1 || width < 1 || groups < 1 || width % groups || groups > 65535) return XR_ERR_ARG;
     const int per = width / groups;
-    // (few rows: nothing but a row's own threads hides its loads' latency)
-    const int most = (long long)n * groups <= xr_sm_count() ? 1024 : 256, threads = per >= most ? most : (per + 31) / 32 * 32;
     const dim3 grid(n, groups);
-    // (the block's size, and with it the order of the sum, is a function of the group's width alone)
     if (dtype != XR_F32 && dtype != XR_BF16) return XR_ERR_ARG;
     if (!((per | width) & 3) && per <= 8192 && ld_g % 4 == 0 && !(((uintptr_t)o | (uintptr_t)g | (uintptr_t)w | (uintptr_t)y) & 15)) {
+        // (the block's size, and with it the order of the sum, is a function of the group's width alone)
         const int quads = per / 4, wide = (quads + 31) / 32 * 32, each = ((quads + 3) / 4 + 31) / 32 * 32;
 #define SGN(T)                                                                                                                       \
     do {                                                                                                                             \
@@ -353,6 +353,8 @@ XR_EXPORT int xr_silu_gate_norm(const float* o, const float* g, long long ld_g, 
 #undef SGN
         return xr_launch_status();
     }
+    // (few rows, a column an access: nothing but a row's own threads hides its loads' latency)
+    const int most = (long long)n * groups <= xr_sm_count() ? 1024 : 256, threads = per >= most ? most : (per + 31) / 32 * 32;
     if (dtype == XR_F32) xr_launch((k_silu_gate_norm<float>), grid, dim3(threads), 0, stream, o, g, ld_g, w, (float*)y, width, per, eps);
     else if (dtype == XR_BF16) xr_launch((k_silu_gate_norm<__nv_bfloat16>), grid, dim3(threads), 0, stream, o, g, ld_g, w, (__nv_bfloat16*)y, width, per, eps);
     else return XR_ERR_ARG;
