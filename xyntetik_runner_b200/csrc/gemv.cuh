@@ -145,12 +145,17 @@ k_gemv(const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* X, long long ld
 }
 
 // Whether a product of n tokens goes here, by K and the bytes of all matrices that it may read.  Where the lines lie is what whole decode
-// steps took (us, tensor cores / here); the product alone says less, because behind it others wait with their weights fetched, and a
+// steps took (us; runs of one rule differ by 0.2 %); the product alone says less, because behind it others wait with their weights fetched, and a
 // product here keeps registers where one on tensor cores keeps shared memory.
-//   one token, up to 64 MB (experts' 128 MB): Lilalorn w1024 440 / 285, Turudra w2048 776 / 634, Besolix w1024 320 / 242, Pitolix w2048 312 / 279,
-//   Llama-3-8B 3,039 / 2,981; with the 67 MB of Llama-3.2-1B's gate and up too 723 / 729.  K 8,192 there 719 / 781, 5,632 in Pitolix 300 / 305.
-//   two tokens, K up to 1,536, up to 24 MB: Lilalorn w1024 446 / 334, Turudra w1024 529 / 429, Pitolix w1024 234 / 211; K 2,048 in Llama-3.2-1B
-//   750 / 785.  Three and more need as many multiply-adds again for bytes that are the same: four tokens 243 / 260 at Pitolix w1024.
+//   one token, tensor cores alone / this rule: Lilalorn w1024 428 / 271, w2048 552 / 387, Turudra w2048 734 / 587, Besolix w2048 376 / 350, Llama-3.2-1B 739 /
+//   731, Llama-3-8B 3,015 / 2,974.  K: up to 3,072 alone 8B 3,024; 5,632 too Besolix w2048 341, Pitolix w2048 281 (280), 8,192 too Llama-3.2-1B 793, Semesun w2048
+//   333 (343): up to 4,096 no model is slower than without.  Bytes: up to 32 MB alone Turudra w2048 691, Pitolix w2048 301 (280); 100 MB, which
+//   takes in gate and up of Llama-3.2-1B (67 MB) and heads of 66, 738 there, Lilalorn w2048 394, Semesun w1024 213 (217).  Experts' up to 64 MB alone
+//   Turudra w2048 (69 MB) 657; nothing measured lies above.
+//   two tokens: Lilalorn w1024 434 / 319, Turudra w1024 508 / 404, Semesun w1024 309 / 271; models 2,048 wide, of which few products are so short, stay within
+//   1 % (Lilalorn 566 / 571, Turudra 775 / 774).  K up to 1,024 alone Lilalorn w1024 369; 2,048 too Llama-3.2-1B 759 -> 786, Turudra w2048 788, Lilalorn w2048
+//   540.  Up to 8 MB alone Lilalorn w1024 374, up to 16 Buzarax w1024 336 (328), up to 40 the same as 24.  Three tokens and more need as many multiply-adds
+//   again for bytes that are the same: four tokens 243 / 260 at Pitolix w1024.
 static inline bool gemv_takes(int n, int K, long long bytes, bool grouped) {
     if (n == 1) return K <= 4096 && bytes <= (grouped ? 128000000 : 64000000);
     return n == 2 && K <= 1536 && bytes <= 24000000;
