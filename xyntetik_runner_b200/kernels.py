@@ -271,8 +271,8 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optiona
     _count()
 
 
-# The products in pieces round as a block of 64 values of k does in the tensor core, whatever K: 1.4 in units of 2^-24 of the result's size
-# at K 256, where the FMA kernel has 4.8.  Shorter sums, where the FMA kernel's error comes down to that and a product is a few
+# The upper piece's sums, which are the result's size, round as a block of 64 values of k does in the tensor core, whatever K (the lower pieces'
+# run over all of a slice of K, 2^-8 of that): 1.4 in units of 2^-24 of the result's size at K 256, where the FMA kernel has 4.8.  Shorter sums, where the FMA kernel's error comes down to that and a product is a few
 # microseconds either way, stay with it.
 SPLIT_LEAST_K = 256
 
