@@ -272,8 +272,8 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optiona
 
 
 # The upper piece's sums, which are the result's size, round as a block of 64 values of k does in the tensor core, whatever K (the lower pieces'
-# run over all of a slice of K, 2^-8 of that): 1.4 in units of 2^-24 of the result's size at K 256, where the FMA kernel has 4.8.  Shorter sums, where the FMA kernel's error comes down to that and a product is a few
-# microseconds either way, stay with it.
+# run over all of a slice of K, 2^-8 of that): 1.4 in units of 2^-24 of the result's size at K 256, where the FMA kernel has 4.8.  Shorter sums,
+# where the FMA kernel's error comes down to that and a product is a few microseconds either way, stay with it.
 SPLIT_LEAST_K = 256
 
 
@@ -1196,7 +1196,7 @@ def gemm_tc_grouped(x: torch.Tensor, w_packed: torch.Tensor, out: torch.Tensor, 
     ws = workspace(x.device)
     args = (x.data_ptr(), w_packed.data_ptr(), out.data_ptr(), dtype_code(out.dtype), epilogue, int(act), float(act_limit), n, n_out, k, x.stride(0),
             out.stride(0), bn, tile_group.data_ptr(), w_packed.shape[0])
-    if live_rows and live_tiles:
+    if live_rows or live_tiles:
         _check(_c.xr_gemm_tc_grouped_live(*args, int(live_rows), int(live_tiles), ws.status_ptr, _stream()), "gemm_tc_grouped")
     else:
         _check(_c.xr_gemm_tc_grouped(*args, ws.status_ptr, _stream()), "gemm_tc_grouped")
